@@ -465,6 +465,63 @@ void bind_ops(py::module_& m) {
                  "embed_bwd");
   }, py::arg("ids"), py::arg("dy"), py::arg("dtok"), py::arg("dpos") = py::none(), py::arg("seq") = 1, py::arg("scale") = 1.0,
         "Adds scale * dy[t] into dtok[ids[t]] and dpos[t % seq] (either table may be None).");
+  m.def("rope_qk_fwd", [](const at::Tensor& qkv, const at::Tensor& cos_t, const at::Tensor& sin_t) {
+    need(qkv, at::kBFloat16, "rope(qkv)");
+    need(cos_t, at::kFloat, "rope(cos)");
+    need(sin_t, at::kFloat, "rope(sin)");
+    MCCL_CHECK_TENSOR(qkv.dim() == 5 && qkv.size(2) == 3, "rope: qkv [batch, seq, 3, heads, head_dim] expected");
+    const int64_t B = qkv.size(0), S = qkv.size(1), H = qkv.size(3), D = qkv.size(4);
+    MCCL_CHECK_TENSOR(cos_t.sizes() == sin_t.sizes() && cos_t.dim() == 2 && cos_t.size(0) >= S && cos_t.size(1) * 2 == D,
+                      "rope: tables [>= seq, head_dim / 2] expected");
+    c10::cuda::CUDAGuard guard(qkv.device());
+    at::Tensor qk = at::empty({B, S, 2, H, D}, qkv.options());
+    check_launch(ops::rope_qk_fwd(bf(qkv), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), bf(qk), B * S, static_cast<int>(S),
+                                  static_cast<int>(H), static_cast<int>(D), stream_of(qkv)),
+                 "rope_qk_fwd");
+    return qk;
+  });
+  m.def("rope_qkv_bwd", [](const at::Tensor& dq, const at::Tensor& dk, const at::Tensor& dv, const at::Tensor& cos_t, const at::Tensor& sin_t) {
+    ops::StridedGrad g[3];
+    const at::Tensor* in[3] = {&dq, &dk, &dv};
+    for (int i = 0; i < 3; ++i) {
+      need_cuda(*in[i], "rope_bwd(gradient)");
+      MCCL_CHECK_TENSOR(in[i]->scalar_type() == at::kBFloat16 && in[i]->dim() == 4 && in[i]->sizes() == dq.sizes() && in[i]->stride(3) == 1,
+                        "rope_bwd: bf16 gradients [batch, heads, seq, head_dim] with contiguous head_dim expected");
+      g[i] = {bf(*in[i]), in[i]->stride(0), in[i]->stride(1), in[i]->stride(2)};
+    }
+    need(cos_t, at::kFloat, "rope_bwd(cos)");
+    need(sin_t, at::kFloat, "rope_bwd(sin)");
+    const int64_t B = dq.size(0), H = dq.size(1), S = dq.size(2), D = dq.size(3);
+    MCCL_CHECK_TENSOR(cos_t.sizes() == sin_t.sizes() && cos_t.dim() == 2 && cos_t.size(0) >= S && cos_t.size(1) * 2 == D,
+                      "rope_bwd: tables [>= seq, head_dim / 2] expected");
+    c10::cuda::CUDAGuard guard(dq.device());
+    at::Tensor dqkv = at::empty({B, S, 3, H, D}, dq.options());
+    check_launch(ops::rope_qkv_bwd(g, cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), bf(dqkv), B * S, static_cast<int>(S),
+                                   static_cast<int>(H), static_cast<int>(D), stream_of(dq)),
+                 "rope_qkv_bwd");
+    return dqkv;
+  });
+  m.def("swiglu_fwd", [](const at::Tensor& gu) {
+    need(gu, at::kBFloat16, "swiglu(gate_up)");
+    MCCL_CHECK_TENSOR(gu.dim() >= 1 && gu.size(-1) % 16 == 0, "swiglu: last dimension must be a multiple of 16");
+    c10::cuda::CUDAGuard guard(gu.device());
+    const int64_t f = gu.size(-1) / 2;
+    auto shape = gu.sizes().vec();
+    shape.back() = f;
+    at::Tensor h = at::empty(shape, gu.options());
+    check_launch(ops::swiglu_fwd(bf(gu), bf(h), h.numel() / f, static_cast<int>(f), stream_of(gu)), "swiglu_fwd");
+    return h;
+  });
+  m.def("swiglu_bwd", [](const at::Tensor& dh, const at::Tensor& gu) {
+    need(dh, at::kBFloat16, "swiglu_bwd(dh)");
+    need(gu, at::kBFloat16, "swiglu_bwd(gate_up)");
+    MCCL_CHECK_TENSOR(gu.numel() == 2 * dh.numel() && gu.size(-1) == 2 * dh.size(-1) && dh.size(-1) % 8 == 0, "swiglu_bwd: bad shapes");
+    c10::cuda::CUDAGuard guard(gu.device());
+    const int64_t f = dh.size(-1);
+    at::Tensor dgu = at::empty_like(gu);
+    check_launch(ops::swiglu_bwd(bf(dh), bf(gu), bf(dgu), dh.numel() / f, static_cast<int>(f), stream_of(gu)), "swiglu_bwd");
+    return dgu;
+  });
 }
 
 }  // namespace mccl

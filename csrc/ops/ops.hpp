@@ -74,6 +74,22 @@ cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse
 cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, const __nv_bfloat16* d_o, const float* lse,
                           __nv_bfloat16* dqkv, int B, int S, int H, float softmax_scale, cudaStream_t stream);
 
+// ---- rotary embedding of the fused QKV projection's output (pairs of even and odd elements; cos / sin: fp32
+// [>= seq, head_dim / 2]; token t has position t % seq).  qkv [tokens, 3, H, hd] -> qk [tokens, 2, H, hd].
+cudaError_t rope_qk_fwd(const __nv_bfloat16* qkv, const float* cos_t, const float* sin_t, __nv_bfloat16* qk, long long tokens, int seq,
+                        int heads, int head_dim, cudaStream_t stream);
+// A gradient [batch, head, position, head_dim] with contiguous head_dim and these strides (elements, multiples of 8).
+struct StridedGrad {
+  const __nv_bfloat16* p;
+  long long sb, sh, ss;
+};
+// d: gradients of the rotated q, the rotated k, and v -> dqkv [tokens, 3, H, hd], every element written.
+cudaError_t rope_qkv_bwd(const StridedGrad (&d)[3], const float* cos_t, const float* sin_t, __nv_bfloat16* dqkv, long long tokens, int seq,
+                         int heads, int head_dim, cudaStream_t stream);
+// ---- SwiGLU on the fused projection [rows, 2 f] = [gate | up]: h = silu(gate) * up, and the gradient of [gate | up].
+cudaError_t swiglu_fwd(const __nv_bfloat16* gu, __nv_bfloat16* h, long long rows, int f, cudaStream_t stream);
+cudaError_t swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gu, __nv_bfloat16* dgu, long long rows, int f, cudaStream_t stream);
+
 // ---- tcgen05 GEMM: D[M,N] = A[M,K] · B[N,K]^T (+ bias[N]) (GELU) ; A, B bf16 with K contiguous.
 enum GemmEpilogue : int {
   EPI_NONE = 0,       // D = acc

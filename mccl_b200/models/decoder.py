@@ -68,11 +68,28 @@ PRESETS = {
 _FUSE_RESIDUAL_GRAD = os.environ.get("MCCL_FUSE_RESIDUAL_GRAD", "1") != "0"
 
 
+_rope_cache: dict = {}
+
+
 def _rope_tables(seq: int, dim: int, device, base: float = 10000.0):
+    """cos / sin of position x frequency, fp32 [seq, dim / 2].  The last few tables are kept: they depend on nothing but the
+    arguments, and making them takes ten small kernels.  (Not during a graph capture: what is made there is only valid
+    once the graph has run.)"""
+    key = (seq, dim, str(device), base)
+    tables = _rope_cache.get(key)
+    if tables is not None:
+        return tables
     inv = 1.0 / (base ** (torch.arange(0, dim, 2, device=device, dtype=torch.float32) / dim))
     t = torch.arange(seq, device=device, dtype=torch.float32)
     f = torch.outer(t, inv)
-    return f.cos(), f.sin()
+    tables = f.cos(), f.sin()
+    if not (torch.is_inference_mode_enabled() or (f.is_cuda and torch.cuda.is_current_stream_capturing())):
+        if f.is_cuda:
+            torch.cuda.current_stream(f.device).synchronize()   # any stream may use them from now on
+        while len(_rope_cache) >= 16:
+            _rope_cache.pop(next(iter(_rope_cache)))
+        _rope_cache[key] = tables
+    return tables
 
 
 def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
@@ -151,6 +168,9 @@ class Block(nn.Module):
         if native and rope is None:
             from .. import ops
             a = ops.causal_attention(qkv, cfg.n_heads)   # own kernels for head dimension 64, S in {128, 256}
+        elif native:
+            from .. import ops
+            a = ops.rope_attention(qkv, cfg.n_heads, *rope)
         else:
             qkv = qkv.view(B, S, 3, cfg.n_heads, cfg.head_dim)
             # unbind, not three selects: its backward is one stack instead of three zero-filled tensors and two adds
@@ -161,8 +181,13 @@ class Block(nn.Module):
         x = self.proj(a, native, residual=x)
         h, x = self.ln2.with_residual(x, native)
         if cfg.act == "swiglu":
-            g, u = self.gate_up(h, native).chunk(2, dim=-1)
-            h = F.silu(g) * u
+            gu = self.gate_up(h, native)
+            if native:
+                from .. import ops
+                h = ops.swiglu(gu)
+            else:
+                g, u = gu.chunk(2, dim=-1)
+                h = F.silu(g) * u
         elif native:
             from .. import ops
             return ops.mlp_gelu(h, self.up.weight, self.up.bias, self.down.weight, self.down.bias, residual=x)

@@ -10,7 +10,7 @@ import torch.nn.functional as F
 from .. import _C
 
 _HAS = {name: hasattr(_C, name) for name in ("gemm_bf16", "norm_fwd", "norm_bwd", "adamw_flat", "ce_fwd_bwd", "embed_fwd",
-                                             "attn_fwd")}
+                                             "attn_fwd", "rope_qk_fwd", "swiglu_fwd")}
 _launches = 0
 
 
@@ -71,6 +71,32 @@ def causal_attention(qkv: torch.Tensor, n_heads: int) -> torch.Tensor:
     q, k, v = (t.transpose(1, 2) for t in q5.unbind(2))
     a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
     return a.transpose(1, 2).reshape(B, S, n_heads * hd)
+
+
+def rope_attention(qkv: torch.Tensor, n_heads: int, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
+    """Causal self-attention with rotary positions.  qkv: [B, S, 3 * n_heads * head_dim], cos / sin: fp32 [>= S, head_dim / 2];
+    returns [B, S, n_heads * head_dim].  On CUDA the rotation is one kernel each way around the attention."""
+    from ..models.decoder import apply_rope
+    B, S = qkv.shape[0], qkv.shape[1]
+    hd = qkv.numel() // (B * S * 3 * n_heads)
+    q5 = qkv.view(B, S, 3, n_heads, hd)
+    if qkv.is_cuda and qkv.dtype == torch.bfloat16 and hd % 8 == 0 and _HAS["rope_qk_fwd"]:
+        from .native import RopeQkvFn
+        q, k, v = RopeQkvFn.apply(q5, cos, sin)
+    else:
+        q, k, v = (t.transpose(1, 2) for t in q5.unbind(2))
+        q, k = apply_rope(q, cos, sin), apply_rope(k, cos, sin)
+    a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
+    return a.transpose(1, 2).reshape(B, S, n_heads * hd)
+
+
+def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
+    """silu(gate) * up of the fused projection [..., 2 F] = [gate | up], in one kernel each way on CUDA."""
+    if gate_up.is_cuda and gate_up.dtype == torch.bfloat16 and gate_up.shape[-1] % 16 == 0 and _HAS["swiglu_fwd"]:
+        from .native import SwigluFn
+        return SwigluFn.apply(gate_up)
+    g, u = gate_up.chunk(2, dim=-1)
+    return F.silu(g) * u
 
 
 def mlp_gelu(x: torch.Tensor, w1: torch.Tensor, b1, w2: torch.Tensor, b2, residual=None) -> torch.Tensor:

@@ -266,6 +266,39 @@ class CausalAttentionFn(torch.autograd.Function):
         return _C.attn_bwd(q5, o, d, lse, ctx.scale), None
 
 
+class RopeQkvFn(torch.autograd.Function):
+    """Fused QKV projection output [B, S, 3, H, hd] -> rotated q, rotated k, v, each [B, H, S, hd] (views).  One kernel
+    each way: the backward turns dq and dk back and gathers all three into the gradient of the whole projection."""
+
+    @staticmethod
+    def forward(ctx, qkv, cos, sin):
+        q5 = qkv if qkv.is_contiguous() else qkv.contiguous()
+        qk = _C.rope_qk_fwd(q5, cos, sin)
+        ctx.tables = (cos, sin)
+        return qk[:, :, 0].transpose(1, 2), qk[:, :, 1].transpose(1, 2), q5[:, :, 2].transpose(1, 2)
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv):
+        def usable(g):
+            return g if g.stride(3) == 1 and all(s % 8 == 0 for s in g.stride()[:3]) and g.data_ptr() % 16 == 0 else g.contiguous()
+        return _C.rope_qkv_bwd(usable(dq), usable(dk), usable(dv), *ctx.tables), None, None
+
+
+class SwigluFn(torch.autograd.Function):
+    """silu(gate) * up for [..., 2 F] = [gate | up], one kernel each way."""
+
+    @staticmethod
+    def forward(ctx, gu):
+        g2 = gu if gu.is_contiguous() else gu.contiguous()
+        ctx.save_for_backward(g2)
+        return _C.swiglu_fwd(g2)
+
+    @staticmethod
+    def backward(ctx, dh):
+        (gu,) = ctx.saved_tensors
+        return _C.swiglu_bwd(dh if dh.is_contiguous() else dh.contiguous(), gu)
+
+
 class NormFn(torch.autograd.Function):
     """LayerNorm (bias given) or RMSNorm (bias None) over the last dimension; fp32 weight / bias."""
 

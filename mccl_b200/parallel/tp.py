@@ -211,7 +211,11 @@ class ParallelAttention(nn.Module):
     def forward(self, x: torch.Tensor, rope) -> torch.Tensor:
         from ..models.decoder import apply_rope
         B, S, H, D = self.batch, self.seq, self.heads_local, self.head_dim
-        qkv = self.qkv(x).view(B, S, 3, H, D)
+        qkv = self.qkv(x)
+        if self.ctx.native and rope is not None:
+            from .. import ops
+            return self.proj(ops.rope_attention(qkv.view(B, S, 3 * H * D), H, *rope).view(B * S, H * D))
+        qkv = qkv.view(B, S, 3, H, D)
         q, k, v = (t.transpose(1, 2) for t in qkv.unbind(2))
         if rope is not None:
             q, k = apply_rope(q, *rope), apply_rope(k, *rope)
@@ -229,7 +233,11 @@ class ParallelMLP(nn.Module):
         self.down = RowParallelLinear(d_ff, d_model, ctx, std=0.02 / (2 * n_layers) ** 0.5)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        gate, up = self.gate_up(x).chunk(2, dim=-1)
+        gate_up = self.gate_up(x)
+        if self.ctx.native:
+            from .. import ops
+            return self.down(ops.swiglu(gate_up))
+        gate, up = gate_up.chunk(2, dim=-1)
         return self.down(F.silu(gate) * up)
 
 
