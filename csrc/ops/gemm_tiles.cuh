@@ -1,0 +1,640 @@
+// The bf16 GEMM of the model operators: D[M, N] = A[M, K] * B[N, K]^T on tcgen05, one persistent kernel template.
+//
+// Two shapes of tile:
+//   one CTA    128 x BN (BN 64 or 128): cta_group::1; every SM works alone, no cluster launch, no cluster barriers
+//   CTA pair   256 x 256: cta_group::2; each CTA loads its 128 rows of A and half of the B tile and the even CTA issues
+//              the MMAs for both, so a 128 x 256 block costs 32 KB of operands per 64 of K instead of 48
+//
+// What bounds it, from probes that ran loads and MMAs apart and together (148 SMs, operands in L2):
+//   * L2 to shared memory is not the limit: 90 B / clk / SM for every SM at once (over 20 TB/s).
+//   * Issue is.  Under `lane == 0` a k-block (two loads, four MMAs, a commit, two waits) took 608 clocks whatever the
+//     tile; under elect.sync 430-515, of which the barrier round trips are half.  Hence elect_one() around the two role
+//     loops, stage and phase counters instead of divisions, and 128 of K per stage where shared memory has room for it:
+//     half the waits per MMA, and one 3-D TMA load fetches both 64-wide swizzle atoms of an operand.
+//   * A tile's epilogue was 1.8 us for 64 columns per warp, 3.6 us with a residual: instruction fetch and exposed
+//     global loads.  Extra inputs with the layout of the output (residual, multiplier) are therefore fetched by TMA into
+//     the staging buffer the result will leave from, before the accumulator is awaited; bias comes as broadcast 16-byte
+//     loads; and a trip of the epilogue loop is 32 columns.
+//
+//   warp 0        producer: one elected thread issues the TMA loads
+//   warp 1        MMA issuer (even CTA of a pair), tensor-memory allocation
+//   warps 2..     epilogue, two per tensor-memory lane quarter (one where BN is 64); the accumulator is double buffered
+//
+// No load uses cluster multicast.  Every wait is bounded (two seconds); a wait that runs out sets the error word the
+// host checks, the roles leave their loops, and the CTAs of a pair still meet before tensor memory is freed.
+#pragma once
+
+#include "gemm_common.cuh"
+
+#include "../core/launch.hpp"
+
+#include <atomic>
+
+namespace mccl {
+namespace ops {
+namespace tiles {
+
+enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2 };
+
+template <int BN, bool kPair>
+struct Shape {
+  static constexpr int kBK = kPair ? 64 : 128;
+  static constexpr int kStages = kPair ? 5 : (BN == 64 ? 4 : 3);
+  static constexpr int kRowsB = kPair ? BN / 2 : BN;   // rows of the B tile this CTA loads
+  static constexpr int kABytes = BM * kBK * 2;
+  static constexpr int kBBytes = kRowsB * kBK * 2;
+  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kEpiWarps = BN == 64 ? 4 : 8;
+  static constexpr int kThreads = 64 + 32 * kEpiWarps;
+  static constexpr int kCols = BN / (kEpiWarps / 4);   // accumulator columns per epilogue warp
+  static constexpr int kBufs = kCols / 64;             // 4 KB staging buffers per epilogue warp
+  static constexpr int kTiles = kStages * kStageBytes;
+  static constexpr int kStagingOff = kTiles;
+  static constexpr int kBarOff = kStagingOff + kEpiWarps * kBufs * 4096;
+  static constexpr int kBarriers = 2 * kStages + 4 + kEpiWarps * kBufs;
+  static constexpr int kTotal = kBarOff + kBarriers * 8 + 16 + 1024;
+  static_assert(kTotal <= 227 * 1024, "shared memory of one CTA");
+};
+
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+static __device__ __noinline__ bool wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  const unsigned long long t0 = now_ns();
+  for (uint32_t i = 0;; ++i) {
+    if (tc::mbar_try_wait(bar, parity)) return true;
+    if ((i & 255u) == 255u) {
+      if (*abort_flag) return false;
+      if (now_ns() - t0 > 2000000000ull) return false;
+    }
+  }
+}
+__device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (tc::mbar_try_wait(bar, parity)) return true;
+  return wait_slow(bar, parity, abort_flag);
+}
+
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Address, in the cluster's shared window, of the even CTA's copy of a shared-memory object of this CTA.
+__device__ __forceinline__ uint32_t leader_addr(const void* p) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(tc::smem_u32(p)), "r"(0));
+  return a;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The bytes land in this CTA's shared memory and complete on a barrier of the cluster window (the even CTA's).
+__device__ __forceinline__ void load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void mma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
+  uint32_t acc = accumulate ? 1u : 0u;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(acc)
+      : "memory");
+}
+// Arrives on the barrier at this offset in BOTH CTAs once every MMA issued so far has finished (an mbarrier arrive, not a load).
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  const uint16_t mask = 3;
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(tc::smem_u32(bar)), "h"(mask)
+               : "memory");
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t bar_cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
+}
+__device__ __forceinline__ void store_2d(const CUtensorMap* map, const void* src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(src)), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void reduce_add_2d(const CUtensorMap* map, const void* src, int x, int y) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(src)), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// All but the last N groups committed by this thread have read their shared-memory source.
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  uint4 pk;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+  return pk;
+}
+__device__ __forceinline__ void unpack8(const uint4& pk, float (&v)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&pk);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(h[i]);
+    v[2 * i] = t.x;
+    v[2 * i + 1] = t.y;
+  }
+}
+
+// tma_x: the second output of the GELU instantiation, or the extra input (multiplier / residual) of the bf16 one.
+template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut>
+__global__ void __launch_bounds__(Shape<BN, kPair>::kThreads, 1)
+gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+                 const __grid_constant__ CUtensorMap tma_d, const __grid_constant__ CUtensorMap tma_x, GemmDev g, int splits) {
+  using S = Shape<BN, kPair>;
+  constexpr int kBK = S::kBK, kStages = S::kStages, kTileM = kPair ? 2 * BM : BM;
+  extern __shared__ uint8_t smem_raw[];
+  // the same offset in both CTAs of a pair: the MMA addresses the peer's operands by this CTA's offsets
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::kBarOff);
+  uint64_t* empty = full + kStages;
+  uint64_t* acc_full = empty + kStages;   // [2]
+  uint64_t* acc_empty = acc_full + 2;     // [2]
+  uint64_t* extra_full = acc_empty + 2;   // [epilogue warp][buffer]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(extra_full + S::kEpiWarps * S::kBufs);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  pdl_trigger();
+  const unsigned long long tl_t0 = tl_begin(g.tl);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = kPair ? cluster_ctarank() : 0u;
+  const int worker = static_cast<int>(kPair ? blockIdx.x >> 1 : blockIdx.x), workers = static_cast<int>(kPair ? gridDim.x >> 1 : gridDim.x);
+  const int m_tiles = (g.m + kTileM - 1) / kTileM, n_tiles = (g.n + BN - 1) / BN;
+  const int total = m_tiles * n_tiles * splits;
+  const int all_kb = (g.k + kBK - 1) / kBK;
+
+  if (warp == 0 && tc::elect_one()) {
+    for (int s = 0; s < kStages; ++s) {
+      tc::mbar_init(&full[s], 1);     // the (even CTA's) producer arrives once and expects the bytes of every load
+      tc::mbar_init(&empty[s], 1);    // one commit per use
+    }
+    for (int b = 0; b < 2; ++b) {
+      tc::mbar_init(&acc_full[b], 1);
+      tc::mbar_init(&acc_empty[b], (kPair ? 2 : 1) * S::kEpiWarps);
+    }
+    for (int b = 0; b < S::kEpiWarps * S::kBufs; ++b) tc::mbar_init(&extra_full[b], 1);
+    *abort_flag = 0;
+    tc::mbar_init_fence();
+    tc::tma_prefetch_desc(&tma_a);
+    tc::tma_prefetch_desc(&tma_b);
+    tc::tma_prefetch_desc(&tma_d);
+    tc::tma_prefetch_desc(&tma_x);
+  }
+  if (warp == 1) {
+    if constexpr (kPair) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(2 * BN) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      tc::tmem_alloc(tmem_slot, 2 * BN);
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  // the peer's barriers exist and its tensor memory is allocated before anything is sent its way
+  if constexpr (kPair) cluster_sync_all();
+  tc::fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();   // set-up done: from here on operands are read and outputs written
+  if (tl_t0 != 0ull && tl_detail(g.tl)) tl_mark(g.tl, tl_t0, tl_now(), TL_GEMM_PHASE, 0u);
+
+  auto tile_coords = [&](int w, int& m_blk, int& n_blk, int& kb0, int& kb1) {
+    const int t = splits > 1 ? w / splits : w;
+    const int s = w - t * splits;
+    kb0 = splits > 1 ? all_kb * s / splits : 0;
+    kb1 = splits > 1 ? all_kb * (s + 1) / splits : all_kb;
+    m_blk = t / n_tiles;
+    n_blk = t - m_blk * n_tiles;
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------ TMA producer --
+    if (tc::elect_one()) {
+      bool ok = true;
+      int s = 0;
+      uint32_t parity = 1;   // a fresh barrier counts as the phase before the first: the first round does not wait
+      for (int w = worker; w < total && ok; w += workers) {
+        int m_blk, n_blk, kb0, kb1;
+        tile_coords(w, m_blk, n_blk, kb0, kb1);
+        const int a_row = m_blk * kTileM + static_cast<int>(rank) * BM;
+        const int b_row = n_blk * BN + static_cast<int>(rank) * S::kRowsB;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          ok = wait(&empty[s], parity, abort_flag);
+          if (!ok) break;
+          uint8_t* a_dst = smem + s * S::kStageBytes;
+          uint8_t* b_dst = a_dst + S::kABytes;
+          const int k0 = kb * kBK;
+          if constexpr (kPair) {
+            if (rank == 0) tc::mbar_expect_tx(&full[s], 2 * S::kStageBytes);
+            const uint32_t bar = leader_addr(&full[s]);
+            if (kAMn) {
+#pragma unroll
+              for (int q = 0; q < BM / 64; ++q) load_2d_pair(a_dst + q * (kBK * 128), &tma_a, bar, a_row + q * 64, k0);
+            } else {
+              load_2d_pair(a_dst, &tma_a, bar, k0, a_row);
+            }
+            if (kBMn) {
+#pragma unroll
+              for (int q = 0; q < S::kRowsB / 64; ++q) load_2d_pair(b_dst + q * (kBK * 128), &tma_b, bar, b_row + q * 64, k0);
+            } else {
+              load_2d_pair(b_dst, &tma_b, bar, k0, b_row);
+            }
+          } else {
+            tc::mbar_expect_tx(&full[s], S::kStageBytes);
+            if (kAMn) {
+#pragma unroll
+              for (int q = 0; q < BM / 64; ++q) tc::tma_load_2d(a_dst + q * (kBK * 128), &tma_a, &full[s], a_row + q * 64, k0);
+            } else {
+              load_3d(a_dst, &tma_a, &full[s], 0, a_row, kb * (kBK / 64));
+            }
+            if (kBMn) {
+#pragma unroll
+              for (int q = 0; q < S::kRowsB / 64; ++q) tc::tma_load_2d(b_dst + q * (kBK * 128), &tma_b, &full[s], b_row + q * 64, k0);
+            } else {
+              load_3d(b_dst, &tma_b, &full[s], 0, b_row, kb * (kBK / 64));
+            }
+          }
+          if (++s == kStages) {
+            s = 0;
+            parity ^= 1u;
+          }
+        }
+      }
+      if (!ok) {
+        *abort_flag = 1;
+        atomicExch(g.err, 11);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // -------------------------------------------------------- MMA issuer --
+    if (rank == 0 && tc::elect_one()) {
+      constexpr uint32_t idesc = tc::idesc_bf16(kTileM, BN, kAMn, kBMn);
+      // 16 of K further: 32 bytes within a swizzled row, or 16 rows of 128 bytes; 64 of K further: the next atom, or 64 rows
+      constexpr uint64_t a_step = kAMn ? 128 : 2, b_step = kBMn ? 128 : 2;
+      constexpr uint64_t a_half = kAMn ? 512 : (BM * 128) >> 4, b_half = kBMn ? 512 : (S::kRowsB * 128) >> 4;
+      bool ok = true;
+      int s = 0, i = 0;
+      uint32_t parity = 0;
+      for (int w = worker; w < total; w += workers, ++i) {
+        int m_blk, n_blk, kb0, kb1;
+        tile_coords(w, m_blk, n_blk, kb0, kb1);
+        const int buf = i & 1;
+        if (i >= 2) {
+          ok = wait(&acc_empty[buf], ((i >> 1) - 1) & 1, abort_flag);
+          if (!ok) break;
+          tc::fence_after_sync();
+        }
+        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * BN);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          ok = wait(&full[s], parity, abort_flag);
+          if (!ok) break;
+          tc::fence_after_sync();
+          const uint8_t* a_tile = smem + s * S::kStageBytes;
+          const uint64_t da = kAMn ? tc::smem_desc_mn_sw128(a_tile, kBK * 128) : tc::smem_desc_k_sw128(a_tile);
+          const uint64_t db = kBMn ? tc::smem_desc_mn_sw128(a_tile + S::kABytes, kBK * 128) : tc::smem_desc_k_sw128(a_tile + S::kABytes);
+#pragma unroll
+          for (int h = 0; h < kBK / 64; ++h) {
+            if (h > 0 && kb * kBK + h * 64 >= g.k) break;   // the rest of the last block is zero fill
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint64_t xa = da + a_half * h + a_step * q, xb = db + b_half * h + b_step * q;
+              if constexpr (kPair) mma_pair(tmem_d, xa, xb, idesc, h > 0 || q > 0 || kb != kb0);
+              else tc::mma_bf16(tmem_d, xa, xb, idesc, h > 0 || q > 0 || kb != kb0);
+            }
+          }
+          if constexpr (kPair) commit_pair(&empty[s]);
+          else tc::mma_commit(&empty[s]);
+          if (++s == kStages) {
+            s = 0;
+            parity ^= 1u;
+          }
+        }
+        if (!ok) break;
+        if constexpr (kPair) commit_pair(&acc_full[buf]);
+        else tc::mma_commit(&acc_full[buf]);
+      }
+      if (!ok) {
+        *abort_flag = 1;
+        atomicExch(g.err, 12);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ----------------------------------------------------------- epilogue --
+    const int e = warp - 2, quarter = warp & 3, part = e >> 2;
+    uint8_t* stage = smem + S::kStagingOff + e * S::kBufs * 4096;
+    uint64_t* xfull = extra_full + e * S::kBufs;
+    const bool has_bias = kOut != OUT_F32 && (g.epilogue == EPI_BIAS || g.epilogue == EPI_BIAS_GELU || g.epilogue == EPI_BIAS_GELU_D);
+    const bool has_extra = kOut == OUT_BF16 && (g.mul != nullptr || g.residual != nullptr);
+    const bool multiply = g.mul != nullptr;
+    const bool gelu_d = g.epilogue == EPI_BIAS_GELU_D || g.epilogue == EPI_GELU_D;
+    bool ok = true;
+    int i = 0;
+    uint32_t xparity = 0;   // one bit per staging buffer
+    for (int w = worker; w < total; w += workers, ++i) {
+      int m_blk, n_blk, kb0, kb1;
+      tile_coords(w, m_blk, n_blk, kb0, kb1);
+      const int buf = i & 1;
+      const bool stamp = warp == 2 && lane == 0 && tl_detail(g.tl);
+      const unsigned long long ts0 = stamp ? tl_now() : 0ull;
+      const int col0 = n_blk * BN + part * S::kCols;
+      const int row0 = m_blk * kTileM + static_cast<int>(rank) * BM + quarter * 32;
+      const bool inside = row0 < g.m && col0 < g.n;   // uniform over the warp
+      // the staging buffers are free again; fetch what the epilogue will need while the MMAs of the tile still run
+      if (tc::elect_one()) {
+        bulk_wait_read<0>();
+        if (has_extra && inside) {
+#pragma unroll
+          for (int b = 0; b < S::kBufs; ++b) {
+            if (col0 + b * 64 < g.n) {
+              tc::mbar_expect_tx(&xfull[b], 4096);
+              tc::tma_load_2d(stage + b * 4096, &tma_x, &xfull[b], col0 + b * 64, row0);
+            }
+          }
+        }
+      }
+      if (has_bias && lane * 32 < S::kCols && col0 + lane * 32 < g.n) prefetch_l1(g.bias + col0 + lane * 32);
+      __syncwarp();
+      ok = wait(&acc_full[buf], (i >> 1) & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc::fence_after_sync();
+      const unsigned long long ts1 = stamp ? tl_now() : 0ull;
+      const uint32_t taddr = tmem_base + static_cast<uint32_t>(buf * BN + part * S::kCols) + (static_cast<uint32_t>(quarter * 32) << 16);
+      auto last_read = [&]() {
+        // every column of this warp's part is in registers: hand the buffer back to the MMA thread
+        tc::fence_before_sync();
+        if (lane == 0) {
+          if constexpr (kPair) arrive_cluster(leader_addr(&acc_empty[buf]));
+          else tc::mbar_arrive(&acc_empty[buf]);
+        }
+      };
+      if constexpr (kOut == OUT_F32) {
+        const bool add = g.atomic_add || g.accumulate;
+#pragma unroll 1
+        for (int c = 0; c < S::kCols; c += 32) {
+          uint32_t r[32];
+          tc::tmem_ld_32x32(taddr + static_cast<uint32_t>(c), r);
+          tc::tmem_ld_wait();
+          if (c + 32 >= S::kCols) last_read();
+          if (row0 >= g.m || col0 + c >= g.n) continue;
+          uint8_t* dst = stage + (S::kBufs > 1 ? ((c >> 5) & 1) * 4096 : 0);
+          if (tc::elect_one()) bulk_wait_read<S::kBufs - 1>();
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) *stage_unit(dst, lane, j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          fence_async_smem();
+          __syncwarp();
+          if (tc::elect_one()) {
+            if (add) reduce_add_2d(&tma_d, dst, col0 + c, row0);
+            else store_2d(&tma_d, dst, col0 + c, row0);
+            bulk_commit();
+          }
+          __syncwarp();
+        }
+      } else {
+        uint4 second[kOut == OUT_GELU ? 8 : 1];   // the second output waits here until the first has left the staging buffer
+#pragma unroll 1
+        for (int c = 0; c < S::kCols; c += 64) {
+          const int cg = col0 + c;
+          const bool active = row0 < g.m && cg < g.n;   // uniform over the warp
+          uint8_t* buf_c = stage + (c >> 6) * 4096;
+          if (has_extra && active) {
+            ok = wait(&xfull[c >> 6], (xparity >> (c >> 6)) & 1u, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            xparity ^= 1u << (c >> 6);
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t r[32];
+            tc::tmem_ld_32x32(taddr + static_cast<uint32_t>(c + 32 * h), r);
+            tc::tmem_ld_wait();
+            if (h == 1 && c + 64 >= S::kCols) last_read();
+            if (!active) continue;
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj) {
+              const int j = 4 * h + jj;
+              float v[8];
+#pragma unroll
+              for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(r[jj * 8 + q]);
+              if (has_bias && cg + j * 8 < g.n) {   // N is a multiple of 8
+                const float4 b0 = __ldg(reinterpret_cast<const float4*>(g.bias + cg + j * 8));
+                const float4 b1 = __ldg(reinterpret_cast<const float4*>(g.bias + cg + j * 8 + 4));
+                v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
+                v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
+              }
+              if constexpr (kOut == OUT_GELU) {
+                if (gelu_d) {
+                  // value and derivative share one exponential; the derivative is what backward needs, so it is saved instead of z
+                  float dv[8];
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) gelu_value_grad(v[q], v[q], dv[q]);
+                  second[j] = pack8(dv);
+                } else {
+                  second[j] = pack8(v);
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) v[q] = gelu_erf(v[q]);
+                }
+              } else if (has_extra) {
+                float x[8];
+                unpack8(*stage_unit(buf_c, lane, j), x);
+                if (multiply) {
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) v[q] *= x[q];
+                } else {
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) v[q] += x[q];
+                }
+              }
+              *stage_unit(buf_c, lane, j) = pack8(v);
+            }
+          }
+          if (!active) continue;
+          fence_async_smem();
+          __syncwarp();
+          if (tc::elect_one()) {
+            store_2d(&tma_d, buf_c, cg, row0);
+            bulk_commit();
+            if constexpr (kOut == OUT_GELU) bulk_wait_read<0>();
+          }
+          __syncwarp();
+          if constexpr (kOut == OUT_GELU) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) *stage_unit(buf_c, lane, j) = second[j];
+            fence_async_smem();
+            __syncwarp();
+            if (tc::elect_one()) {
+              store_2d(&tma_x, buf_c, cg, row0);
+              bulk_commit();
+            }
+            __syncwarp();
+          }
+        }
+        if (!ok) break;
+      }
+      if (stamp) {
+        const unsigned long long ts2 = tl_now();   // before the records below: their atomics take a microsecond
+        tl_mark(g.tl, ts0, ts1, TL_GEMM_PHASE, (1u << 24) | static_cast<uint32_t>(i));
+        tl_mark(g.tl, ts1, ts2, TL_GEMM_PHASE, (2u << 24) | static_cast<uint32_t>(i));
+      }
+    }
+    if (tc::elect_one()) bulk_wait_read<0>();   // the stores have read this warp's staging; kernel completion publishes them
+    if (!ok && lane == 0) {
+      *abort_flag = 1;
+      atomicExch(g.err, 13);
+    }
+    __syncwarp();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (*abort_flag) {
+    // a wait ran out somewhere: loads still in flight get time to land before shared memory is given up
+    const unsigned long long t0 = now_ns();
+    while (now_ns() - t0 < 50000ull) __nanosleep(1000);
+  }
+  // nothing of the peer is touched after this: its shared memory (operands the MMAs read) and barriers (remote arrives)
+  if constexpr (kPair) cluster_sync_all();
+  if (warp == 1) {
+    tc::fence_after_sync();
+    if constexpr (kPair) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * BN) : "memory");
+    else tc::tmem_dealloc(tmem_base, 2 * BN);
+  }
+  tl_end(g.tl, tl_t0, TL_GEMM, (static_cast<uint32_t>(m_tiles * (kPair ? 2 : 1)) << 16) | static_cast<uint32_t>(n_tiles * splits));
+}
+
+// K-major operand [rows, K] as [K / 64][rows][64]: a box of two atoms is 128 of K in one load (zero fill past K).
+inline bool encode_k_atoms(CUtensorMap* map, const void* base, int rows, int k, int ld_elems, int box_rows, int atoms) {
+  const CuDriver& cu = CuDriver::get();
+  if (!cu.loaded || !cu.TensorMapEncodeTiled) return false;
+  int device = 0;
+  cudaGetDevice(&device);
+  cu.ensure_context(device);
+  cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(k / 64)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld_elems) * 2, 128};
+  cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(atoms)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return cu.TensorMapEncodeTiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Launches `workers` CTAs (pairs) over the tiles of `a`, K cut into `splits` (fp32 sums added into D).
+template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut>
+cudaError_t launch_tiles(const GemmArgs& a, int workers, int splits, cudaStream_t stream) {
+  using S = Shape<BN, kPair>;
+  auto kernel = gemm_tile_kernel<BN, kPair, kAMn, kBMn, kOut>;
+  static std::atomic<bool> configured{false};
+  if (!configured.load(std::memory_order_acquire)) {
+    cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
+    if (rc != cudaSuccess) return rc;
+    configured.store(true, std::memory_order_release);
+  }
+  CUtensorMap ma, mb, md, mx;
+  // MN-major: boxes of 64 columns x one k-block of rows
+  const bool oka = kAMn ? encode_map(&ma, a.a, a.k, a.m, a.lda, S::kBK)
+                        : (kPair ? encode_map(&ma, a.a, a.m, a.k, a.lda, BM) : encode_k_atoms(&ma, a.a, a.m, a.k, a.lda, BM, S::kBK / 64));
+  const bool okb = kBMn ? encode_map(&mb, a.b, a.k, a.n, a.ldb, S::kBK)
+                        : (kPair ? encode_map(&mb, a.b, a.n, a.k, a.ldb, S::kRowsB) : encode_k_atoms(&mb, a.b, a.n, a.k, a.ldb, S::kRowsB, S::kBK / 64));
+  if (!oka || !okb || !encode_out_map(&md, a.d, a.m, a.n, a.ldd, kOut == OUT_F32)) return cudaErrorNotSupported;
+  const void* x = kOut == OUT_GELU ? a.aux : (kOut == OUT_BF16 ? (a.mul ? a.mul : a.residual) : nullptr);
+  if (x == nullptr) mx = md;   // never used
+  else if (!encode_out_map(&mx, x, a.m, a.n, a.ldd, false)) return cudaErrorNotSupported;
+  GemmDev g;
+  g.d = a.d;
+  g.aux = a.aux;
+  g.bias = a.bias;
+  g.residual = a.residual;
+  g.mul = a.mul;
+  g.m = a.m;
+  g.n = a.n;
+  g.k = a.k;
+  g.ldd = a.ldd;
+  g.d_fp32 = kOut == OUT_F32 ? 1 : 0;
+  g.accumulate = a.accumulate ? 1 : 0;
+  g.epilogue = a.epilogue;
+  g.atomic_add = splits > 1 ? 1 : 0;
+  g.err = gemm_error_device_ptr();
+  if (!g.err) return cudaErrorNotSupported;
+  g.tl = timeline_device_ptr();
+  // partial sums are added into the output: start from zero unless the caller accumulates anyway
+  if (splits > 1 && !a.accumulate) {
+    cudaError_t rc = cudaMemsetAsync(a.d, 0, static_cast<size_t>(a.m) * a.n * sizeof(float), stream);
+    if (rc != cudaSuccess) return rc;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(kPair ? 2 * workers : workers));
+  cfg.blockDim = dim3(S::kThreads);
+  cfg.dynamicSmemBytes = S::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  if (kPair) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = 2;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (pdl_enabled()) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  cudaLaunchKernelEx(&cfg, kernel, ma, mb, md, mx, g, splits);
+  ::mccl::launch_record("gemm_tile_kernel", __FILE__, __LINE__, cfg.gridDim, cfg.blockDim, S::kTotal, stream);
+  count_launch();
+  return ::mccl::launch_status();
+}
+
+// Pairs of this instantiation that can be resident at once (GPCs with an odd number of free SMs leave one SM out).
+template <int BN, bool kAMn, bool kBMn, int kOut>
+int max_pairs() {
+  using S = Shape<BN, true>;
+  static std::atomic<int> cached{0};
+  int n = cached.load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  auto kernel = gemm_tile_kernel<BN, true, kAMn, kBMn, kOut>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * 74);
+  cfg.blockDim = dim3(S::kThreads);
+  cfg.dynamicSmemBytes = S::kTotal;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+    (void)cudaGetLastError();
+    n = gemm_sm_count() / 2 - 2;
+  }
+  cached.store(n, std::memory_order_relaxed);
+  return n;
+}
+
+}  // namespace tiles
+}  // namespace ops
+}  // namespace mccl

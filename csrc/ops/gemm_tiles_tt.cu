@@ -1,0 +1,19 @@
+// Instantiations of the GEMM kernel: both operands MN-major (weight gradients).
+#include "gemm_tiles.cuh"
+
+namespace mccl {
+namespace ops {
+namespace tiles {
+
+template cudaError_t launch_tiles<64, false, true, true, OUT_BF16>(const GemmArgs&, int, int, cudaStream_t);
+template cudaError_t launch_tiles<128, false, true, true, OUT_BF16>(const GemmArgs&, int, int, cudaStream_t);
+template cudaError_t launch_tiles<256, true, true, true, OUT_BF16>(const GemmArgs&, int, int, cudaStream_t);
+template int max_pairs<256, true, true, OUT_BF16>();
+template cudaError_t launch_tiles<64, false, true, true, OUT_F32>(const GemmArgs&, int, int, cudaStream_t);
+template cudaError_t launch_tiles<128, false, true, true, OUT_F32>(const GemmArgs&, int, int, cudaStream_t);
+template cudaError_t launch_tiles<256, true, true, true, OUT_F32>(const GemmArgs&, int, int, cudaStream_t);
+template int max_pairs<256, true, true, OUT_F32>();
+
+}  // namespace tiles
+}  // namespace ops
+}  // namespace mccl

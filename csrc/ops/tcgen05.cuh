@@ -18,6 +18,16 @@ namespace tc {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
+// One lane of a full warp, known to the compiler to be the only active one.  TMA and tcgen05 instructions take their
+// operands from uniform registers: under `lane == 0` every operand is first made uniform by a loop over the (one)
+// active lane, which costs more than the instruction (measured: a k-block of two loads, four MMAs and a commit takes
+// 608 clocks of issue under `lane == 0` and 430 under elect.sync, whatever the tile).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+
 // ------------------------------------------------------------- mbarrier ----
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

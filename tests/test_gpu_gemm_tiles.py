@@ -1,0 +1,69 @@
+"""Every tile of the GEMM kernel at the edges of its tiles and of its k-blocks, against fp32 matmul."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).abs().max() / b.double().abs().max().clamp_min(1e-6)).item()
+
+
+@pytest.fixture(params=["tile64", "tile128", "pair256", ""])
+def C(request):
+    from mccl_b200 import _C
+    _C.set_gemm_kernel(request.param)
+    yield _C
+    _C.set_gemm_kernel("")
+    torch.cuda.synchronize()
+    assert _C.gemm_error_flag() == 0
+
+
+# one row, an edge in every dimension, several rounds of tiles per CTA, an odd number of 64-wide k-blocks
+SHAPES = [(1, 8, 64), (37, 1536, 512), (129, 72, 192), (256, 256, 128), (257, 264, 320), (1000, 2056, 64), (8000, 2048, 576)]
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True), (True, False), (True, True)])
+def test_product(C, M, N, K, a_t, b_t):
+    if a_t:
+        M = (M + 7) // 8 * 8
+    torch.manual_seed(M + N + K)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    ref = a.float() @ b.float().t()
+    aa, bb = (a.t().contiguous() if a_t else a), (b.t().contiguous() if b_t else b)
+    d, _ = C.gemm_bf16(aa, bb, None, "none", False, None, False, a_t, b_t)
+    assert _rel(d, ref) < 1e-2
+    d, _ = C.gemm_bf16(aa, bb, None, "none", True, None, False, a_t, b_t)
+    assert _rel(d, ref) < 1e-5 * max(1, K // 64)
+    acc = torch.randn(M, N, device="cuda")
+    want = acc + ref
+    C.gemm_bf16(aa, bb, None, "none", True, acc, True, a_t, b_t)
+    assert _rel(acc, want) < 1e-5 * max(1, K // 64)
+    mul = torch.randn(M, N, device="cuda").bfloat16()
+    d, _ = C.gemm_bf16(aa, bb, None, "none", False, None, False, a_t, b_t, None, mul)
+    assert _rel(d, ref * mul.float()) < 1e-2
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+def test_epilogues(C, M, N, K):
+    torch.manual_seed(M * 3 + N + K)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16() * 0.1
+    bias, res = torch.randn(N, device="cuda"), torch.randn(M, N, device="cuda").bfloat16()
+    z = a.float() @ b.float().t() + bias
+    assert _rel(C.gemm_bf16(a, b, bias)[0], z) < 1e-2
+    assert _rel(C.gemm_bf16(a, b, bias, "none", False, None, False, False, False, res)[0], z + res.float()) < 1e-2
+    d, saved = C.gemm_bf16(a, b, bias, "gelu")
+    assert _rel(d, F.gelu(z)) < 1e-2 and _rel(saved, z) < 1e-2
+    d, saved = C.gemm_bf16(a, b, bias, "gelu_d")
+    zz = z.clone().requires_grad_(True)
+    F.gelu(zz).sum().backward()
+    assert _rel(d, F.gelu(z)) < 1e-2 and _rel(saved, zz.grad) < 1e-2
+
+
+def test_long_contraction_is_split(C):
+    torch.manual_seed(0)
+    a, b = torch.randn(16384, 512, device="cuda").bfloat16(), torch.randn(16384, 256, device="cuda").bfloat16()
+    d, _ = C.gemm_bf16(a, b, None, "none", True, None, False, True, True)
+    assert _rel(d, a.float().t() @ b.float()) < 3e-5
