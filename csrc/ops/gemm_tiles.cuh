@@ -13,8 +13,9 @@
 //     half the waits per MMA, and one 3-D TMA load fetches both 64-wide swizzle atoms of an operand.
 //   * A tile's epilogue was 1.8 us for 64 columns per warp, 3.6 us with a residual: instruction fetch and exposed
 //     global loads.  Extra inputs with the layout of the output (residual, multiplier) are therefore fetched by TMA into
-//     the staging buffer the result will leave from, before the accumulator is awaited; bias comes as broadcast 16-byte
-//     loads; and a trip of the epilogue loop is 32 columns.
+//     the staging buffer the result will leave from, before the accumulator is awaited; bias is fetched then too, four
+//     values per lane, and spread by shuffles (read where it is used, even from L1, it cost 0.9 us); and a trip of the
+//     epilogue loop is 32 columns.
 //
 //   warp 0        producer: one elected thread issues the TMA loads
 //   warp 1        MMA issuer (even CTA of a pair), tensor-memory allocation
@@ -140,8 +141,6 @@ __device__ __forceinline__ void bulk_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
-
 __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
   uint4 pk;
   __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
@@ -376,7 +375,9 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           }
         }
       }
-      if (has_bias && lane * 32 < S::kCols && col0 + lane * 32 < g.n) prefetch_l1(g.bias + col0 + lane * 32);
+      // lane l keeps the bias of columns [col0 + 4 l, col0 + 4 l + 4); the loop below spreads it by shuffles
+      float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (has_bias && 4 * lane < S::kCols && col0 + 4 * lane < g.n) bias4 = __ldg(reinterpret_cast<const float4*>(g.bias + col0 + 4 * lane));
       __syncwarp();
       ok = wait(&acc_full[buf], (i >> 1) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
@@ -440,11 +441,16 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               float v[8];
 #pragma unroll
               for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(r[jj * 8 + q]);
-              if (has_bias && cg + j * 8 < g.n) {   // N is a multiple of 8
-                const float4 b0 = __ldg(reinterpret_cast<const float4*>(g.bias + cg + j * 8));
-                const float4 b1 = __ldg(reinterpret_cast<const float4*>(g.bias + cg + j * 8 + 4));
-                v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
-                v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
+              if (has_bias) {
+                const int src = (c >> 2) + 2 * j;
+                v[0] += __shfl_sync(0xffffffffu, bias4.x, src);
+                v[1] += __shfl_sync(0xffffffffu, bias4.y, src);
+                v[2] += __shfl_sync(0xffffffffu, bias4.z, src);
+                v[3] += __shfl_sync(0xffffffffu, bias4.w, src);
+                v[4] += __shfl_sync(0xffffffffu, bias4.x, src + 1);
+                v[5] += __shfl_sync(0xffffffffu, bias4.y, src + 1);
+                v[6] += __shfl_sync(0xffffffffu, bias4.z, src + 1);
+                v[7] += __shfl_sync(0xffffffffu, bias4.w, src + 1);
               }
               if constexpr (kOut == OUT_GELU) {
                 if (gelu_d) {
