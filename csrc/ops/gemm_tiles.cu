@@ -59,9 +59,9 @@ Plan choose(const GemmArgs& a, int forced, int sms, int pairs, bool gelu, bool s
     if (bn == 256 && (gelu || pairs < 1)) continue;
     const int workers = bn == 256 ? pairs : sms;
     const int tiles = ceil_div(a.m, bn == 256 ? 256 : 128) * ceil_div(a.n, bn);
-    const int num_kb = ceil_div(a.k, bn == 256 ? 64 : 128);
+    const int num_kb = ceil_div(a.k, 64);
     for (int s = 1; s <= 16; s = s < 4 ? s + 1 : s + 2) {
-      if (s > 1 && (!splittable || num_kb / s < 2 || tiles * (s - 1) >= 2 * workers)) break;
+      if (s > 1 && (!splittable || num_kb / s < 4 || tiles * (s - 1) >= 2 * workers)) break;
       const double c = cost(bn, a.m, a.n, a.k, workers, s, gelu);
       if (best.bn == 0 || c < best_cost) {
         best_cost = c;

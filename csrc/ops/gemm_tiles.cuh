@@ -8,9 +8,11 @@
 // What bounds it, from probes that ran loads and MMAs apart and together (148 SMs, operands in L2):
 //   * L2 to shared memory is not the limit: 90 B / clk / SM for every SM at once (over 20 TB/s).
 //   * Issue is.  Under `lane == 0` a k-block (two loads, four MMAs, a commit, two waits) took 608 clocks whatever the
-//     tile; under elect.sync 430-515, of which the barrier round trips are half.  Hence elect_one() around the two role
-//     loops, stage and phase counters instead of divisions, and 128 of K per stage where shared memory has room for it:
-//     half the waits per MMA, and one 3-D TMA load fetches both 64-wide swizzle atoms of an operand.
+//     tile; under elect.sync 430-515.  Hence elect_one() around the two role loops, and stage and phase counters
+//     instead of divisions.
+//   * Then the TMA unit: about 105 B / clk / SM and 50 clocks per load, so the 32 KB of a 128 x 128 k-block take 342
+//     clocks (measured, at its bound) where its MMAs need 256.  Six stages of 64 of K do better than three of 128
+//     (4096 x 512 x 2048: 11.8 -> 11.2 us): a stage is refilled sooner.
 //   * A tile's epilogue was 1.8 us for 64 columns per warp, 3.6 us with a residual: instruction fetch and exposed
 //     global loads.  Extra inputs with the layout of the output (residual, multiplier) are therefore fetched by TMA into
 //     the staging buffer the result will leave from, before the accumulator is awaited; bias is fetched then too, four
@@ -39,11 +41,10 @@ enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2 };
 
 template <int BN, bool kPair>
 struct Shape {
-  static constexpr int kBK = kPair ? 64 : 128;
-  static constexpr int kStages = kPair ? 5 : (BN == 64 ? 4 : 3);
+  static constexpr int kStages = kPair ? 5 : (BN == 64 ? 8 : 6);
   static constexpr int kRowsB = kPair ? BN / 2 : BN;   // rows of the B tile this CTA loads
-  static constexpr int kABytes = BM * kBK * 2;
-  static constexpr int kBBytes = kRowsB * kBK * 2;
+  static constexpr int kABytes = BM * BK * 2;
+  static constexpr int kBBytes = kRowsB * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kEpiWarps = BN == 64 ? 4 : 8;
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
@@ -97,12 +98,6 @@ __device__ __forceinline__ void load_2d_pair(void* dst, const CUtensorMap* map, 
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y)
-      : "memory");
-}
-__device__ __forceinline__ void load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
 __device__ __forceinline__ void mma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
@@ -164,7 +159,7 @@ __global__ void __launch_bounds__(Shape<BN, kPair>::kThreads, 1)
 gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ CUtensorMap tma_d, const __grid_constant__ CUtensorMap tma_x, GemmDev g, int splits) {
   using S = Shape<BN, kPair>;
-  constexpr int kBK = S::kBK, kStages = S::kStages, kTileM = kPair ? 2 * BM : BM;
+  constexpr int kStages = S::kStages, kTileM = kPair ? 2 * BM : BM;
   extern __shared__ uint8_t smem_raw[];
   // the same offset in both CTAs of a pair: the MMA addresses the peer's operands by this CTA's offsets
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -183,7 +178,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int worker = static_cast<int>(kPair ? blockIdx.x >> 1 : blockIdx.x), workers = static_cast<int>(kPair ? gridDim.x >> 1 : gridDim.x);
   const int m_tiles = (g.m + kTileM - 1) / kTileM, n_tiles = (g.n + BN - 1) / BN;
   const int total = m_tiles * n_tiles * splits;
-  const int all_kb = (g.k + kBK - 1) / kBK;
+  const int all_kb = (g.k + BK - 1) / BK;
 
   if (warp == 0 && tc::elect_one()) {
     for (int s = 0; s < kStages; ++s) {
@@ -244,19 +239,19 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           if (!ok) break;
           uint8_t* a_dst = smem + s * S::kStageBytes;
           uint8_t* b_dst = a_dst + S::kABytes;
-          const int k0 = kb * kBK;
+          const int k0 = kb * BK;
           if constexpr (kPair) {
             if (rank == 0) tc::mbar_expect_tx(&full[s], 2 * S::kStageBytes);
             const uint32_t bar = leader_addr(&full[s]);
             if (kAMn) {
 #pragma unroll
-              for (int q = 0; q < BM / 64; ++q) load_2d_pair(a_dst + q * (kBK * 128), &tma_a, bar, a_row + q * 64, k0);
+              for (int q = 0; q < BM / 64; ++q) load_2d_pair(a_dst + q * (BK * 128), &tma_a, bar, a_row + q * 64, k0);
             } else {
               load_2d_pair(a_dst, &tma_a, bar, k0, a_row);
             }
             if (kBMn) {
 #pragma unroll
-              for (int q = 0; q < S::kRowsB / 64; ++q) load_2d_pair(b_dst + q * (kBK * 128), &tma_b, bar, b_row + q * 64, k0);
+              for (int q = 0; q < S::kRowsB / 64; ++q) load_2d_pair(b_dst + q * (BK * 128), &tma_b, bar, b_row + q * 64, k0);
             } else {
               load_2d_pair(b_dst, &tma_b, bar, k0, b_row);
             }
@@ -264,15 +259,15 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             tc::mbar_expect_tx(&full[s], S::kStageBytes);
             if (kAMn) {
 #pragma unroll
-              for (int q = 0; q < BM / 64; ++q) tc::tma_load_2d(a_dst + q * (kBK * 128), &tma_a, &full[s], a_row + q * 64, k0);
+              for (int q = 0; q < BM / 64; ++q) tc::tma_load_2d(a_dst + q * (BK * 128), &tma_a, &full[s], a_row + q * 64, k0);
             } else {
-              load_3d(a_dst, &tma_a, &full[s], 0, a_row, kb * (kBK / 64));
+              tc::tma_load_2d(a_dst, &tma_a, &full[s], k0, a_row);
             }
             if (kBMn) {
 #pragma unroll
-              for (int q = 0; q < S::kRowsB / 64; ++q) tc::tma_load_2d(b_dst + q * (kBK * 128), &tma_b, &full[s], b_row + q * 64, k0);
+              for (int q = 0; q < S::kRowsB / 64; ++q) tc::tma_load_2d(b_dst + q * (BK * 128), &tma_b, &full[s], b_row + q * 64, k0);
             } else {
-              load_3d(b_dst, &tma_b, &full[s], 0, b_row, kb * (kBK / 64));
+              tc::tma_load_2d(b_dst, &tma_b, &full[s], k0, b_row);
             }
           }
           if (++s == kStages) {
@@ -291,9 +286,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     // -------------------------------------------------------- MMA issuer --
     if (rank == 0 && tc::elect_one()) {
       constexpr uint32_t idesc = tc::idesc_bf16(kTileM, BN, kAMn, kBMn);
-      // 16 of K further: 32 bytes within a swizzled row, or 16 rows of 128 bytes; 64 of K further: the next atom, or 64 rows
+      // 16 of K further: 32 bytes within a swizzled row, or 16 rows of 128 bytes
       constexpr uint64_t a_step = kAMn ? 128 : 2, b_step = kBMn ? 128 : 2;
-      constexpr uint64_t a_half = kAMn ? 512 : (BM * 128) >> 4, b_half = kBMn ? 512 : (S::kRowsB * 128) >> 4;
       bool ok = true;
       int s = 0, i = 0;
       uint32_t parity = 0;
@@ -312,17 +306,12 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           if (!ok) break;
           tc::fence_after_sync();
           const uint8_t* a_tile = smem + s * S::kStageBytes;
-          const uint64_t da = kAMn ? tc::smem_desc_mn_sw128(a_tile, kBK * 128) : tc::smem_desc_k_sw128(a_tile);
-          const uint64_t db = kBMn ? tc::smem_desc_mn_sw128(a_tile + S::kABytes, kBK * 128) : tc::smem_desc_k_sw128(a_tile + S::kABytes);
+          const uint64_t da = kAMn ? tc::smem_desc_mn_sw128(a_tile, BK * 128) : tc::smem_desc_k_sw128(a_tile);
+          const uint64_t db = kBMn ? tc::smem_desc_mn_sw128(a_tile + S::kABytes, BK * 128) : tc::smem_desc_k_sw128(a_tile + S::kABytes);
 #pragma unroll
-          for (int h = 0; h < kBK / 64; ++h) {
-            if (h > 0 && kb * kBK + h * 64 >= g.k) break;   // the rest of the last block is zero fill
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const uint64_t xa = da + a_half * h + a_step * q, xb = db + b_half * h + b_step * q;
-              if constexpr (kPair) mma_pair(tmem_d, xa, xb, idesc, h > 0 || q > 0 || kb != kb0);
-              else tc::mma_bf16(tmem_d, xa, xb, idesc, h > 0 || q > 0 || kb != kb0);
-            }
+          for (int q = 0; q < BK / UMMA_K; ++q) {
+            if constexpr (kPair) mma_pair(tmem_d, da + a_step * q, db + b_step * q, idesc, q > 0 || kb != kb0);
+            else tc::mma_bf16(tmem_d, da + a_step * q, db + b_step * q, idesc, q > 0 || kb != kb0);
           }
           if constexpr (kPair) commit_pair(&empty[s]);
           else tc::mma_commit(&empty[s]);
@@ -531,22 +520,6 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   tl_end(g.tl, tl_t0, TL_GEMM, (static_cast<uint32_t>(m_tiles * (kPair ? 2 : 1)) << 16) | static_cast<uint32_t>(n_tiles * splits));
 }
 
-// K-major operand [rows, K] as [K / 64][rows][64]: a box of two atoms is 128 of K in one load (zero fill past K).
-inline bool encode_k_atoms(CUtensorMap* map, const void* base, int rows, int k, int ld_elems, int box_rows, int atoms) {
-  const CuDriver& cu = CuDriver::get();
-  if (!cu.loaded || !cu.TensorMapEncodeTiled) return false;
-  int device = 0;
-  cudaGetDevice(&device);
-  cu.ensure_context(device);
-  cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(k / 64)};
-  cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld_elems) * 2, 128};
-  cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(atoms)};
-  cuuint32_t estr[3] = {1, 1, 1};
-  return cu.TensorMapEncodeTiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // Launches `workers` CTAs (pairs) over the tiles of `a`, K cut into `splits` (fp32 sums added into D).
 template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut>
 cudaError_t launch_tiles(const GemmArgs& a, int workers, int splits, cudaStream_t stream) {
@@ -559,11 +532,9 @@ cudaError_t launch_tiles(const GemmArgs& a, int workers, int splits, cudaStream_
     configured.store(true, std::memory_order_release);
   }
   CUtensorMap ma, mb, md, mx;
-  // MN-major: boxes of 64 columns x one k-block of rows
-  const bool oka = kAMn ? encode_map(&ma, a.a, a.k, a.m, a.lda, S::kBK)
-                        : (kPair ? encode_map(&ma, a.a, a.m, a.k, a.lda, BM) : encode_k_atoms(&ma, a.a, a.m, a.k, a.lda, BM, S::kBK / 64));
-  const bool okb = kBMn ? encode_map(&mb, a.b, a.k, a.n, a.ldb, S::kBK)
-                        : (kPair ? encode_map(&mb, a.b, a.n, a.k, a.ldb, S::kRowsB) : encode_k_atoms(&mb, a.b, a.n, a.k, a.ldb, S::kRowsB, S::kBK / 64));
+  // K-major: boxes of 64 of K x the tile's rows; MN-major: boxes of 64 columns x 64 of K (zero fill past K)
+  const bool oka = kAMn ? encode_map(&ma, a.a, a.k, a.m, a.lda, BK) : encode_map(&ma, a.a, a.m, a.k, a.lda, BM);
+  const bool okb = kBMn ? encode_map(&mb, a.b, a.k, a.n, a.ldb, BK) : encode_map(&mb, a.b, a.n, a.k, a.ldb, S::kRowsB);
   if (!oka || !okb || !encode_out_map(&md, a.d, a.m, a.n, a.ldd, kOut == OUT_F32)) return cudaErrorNotSupported;
   const void* x = kOut == OUT_GELU ? a.aux : (kOut == OUT_BF16 ? (a.mul ? a.mul : a.residual) : nullptr);
   if (x == nullptr) mx = md;   // never used
