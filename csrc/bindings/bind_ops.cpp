@@ -95,7 +95,7 @@ void bind_ops(py::module_& m) {
       "gemm_bf16",
       [](const at::Tensor& a, const at::Tensor& b, const c10::optional<at::Tensor>& bias, const std::string& epilogue,
          bool out_fp32, const c10::optional<at::Tensor>& out, bool accumulate, bool a_t, bool b_t,
-         const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& mul) {
+         const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& mul, const c10::optional<at::Tensor>& colsum) {
         need_cuda(a, "gemm(a)");
         need_cuda(b, "gemm(b)");
         MCCL_CHECK_TENSOR(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16, "gemm: operands must be bf16");
@@ -154,6 +154,12 @@ void bind_ops(py::module_& m) {
                             "gemm: mul must be a contiguous [M, N] bf16 tensor and the output bf16");
           g.mul = bf(*mul);
         }
+        if (colsum.has_value() && colsum->defined()) {
+          need(*colsum, at::kFloat, "gemm(colsum)");
+          MCCL_CHECK_TENSOR(colsum->numel() == N && !a_t && b_t && !out_fp32 && !g.bias && !g.residual && g.epilogue == ops::EPI_NONE,
+                            "gemm: colsum must have N elements and goes with a bf16 output, an MN-major B and no bias, activation or residual");
+          g.colsum = colsum->data_ptr<float>();
+        }
         cudaError_t rc = ops::gemm_bf16_tn(g, stream_of(a));
         MCCL_CHECK_T(rc == cudaSuccess, CudaError,
                      "gemm_bf16 [" << M << "x" << N << "x" << K << ", lda " << g.lda << ", ldb " << g.ldb << ", ldd " << g.ldd
@@ -162,7 +168,44 @@ void bind_ops(py::module_& m) {
       },
       py::arg("a"), py::arg("b"), py::arg("bias") = py::none(), py::arg("epilogue") = "none", py::arg("out_fp32") = false,
       py::arg("out") = py::none(), py::arg("accumulate") = false, py::arg("a_t") = false, py::arg("b_t") = false,
-      py::arg("residual") = py::none(), py::arg("mul") = py::none());
+      py::arg("residual") = py::none(), py::arg("mul") = py::none(), py::arg("colsum") = py::none());
+
+  // dW_i[N_i, K_i] = dY_i[tokens, N_i]^T · X_i[tokens, K_i], four products per launch.  items: (dY, X, dW or None); with
+  // accumulate every dW is given and added into.  Returns the dW.
+  m.def(
+      "gemm_group",
+      [](const std::vector<std::tuple<at::Tensor, at::Tensor, c10::optional<at::Tensor>>>& items, bool accumulate) {
+        std::vector<at::Tensor> out;
+        std::vector<ops::GemmArgs> args;
+        MCCL_CHECK_TENSOR(!items.empty(), "gemm_group: no products");
+        c10::cuda::CUDAGuard guard(std::get<0>(items[0]).device());
+        for (const auto& it : items) {
+          const at::Tensor &a = std::get<0>(it), &b = std::get<1>(it);
+          need(a, at::kBFloat16, "gemm_group(dY)");
+          need(b, at::kBFloat16, "gemm_group(X)");
+          MCCL_CHECK_TENSOR(a.dim() == 2 && b.dim() == 2 && a.size(0) == b.size(0), "gemm_group: dY [tokens, N] and X [tokens, K] expected");
+          MCCL_CHECK_TENSOR(std::get<2>(it).has_value() || !accumulate, "gemm_group: accumulate needs outputs to add into");
+          at::Tensor d = std::get<2>(it).has_value() ? *std::get<2>(it) : at::empty({a.size(1), b.size(1)}, a.options().dtype(at::kFloat));
+          need(d, at::kFloat, "gemm_group(dW)");
+          MCCL_CHECK_TENSOR(d.numel() == a.size(1) * b.size(1), "gemm_group: bad output shape");
+          ops::GemmArgs g;
+          g.a = bf(a);
+          g.b = bf(b);
+          g.d = d.data_ptr();
+          g.a_mn_major = g.b_mn_major = g.d_fp32 = true;
+          g.accumulate = accumulate;
+          g.m = static_cast<int>(a.size(1));
+          g.n = static_cast<int>(b.size(1));
+          g.k = static_cast<int>(a.size(0));
+          g.lda = g.m;
+          g.ldb = g.ldd = g.n;
+          args.push_back(g);
+          out.push_back(d);
+        }
+        check_launch(ops::gemm_group(args.data(), static_cast<int>(args.size()), stream_of(std::get<0>(items[0]))), "gemm_group");
+        return out;
+      },
+      py::arg("items"), py::arg("accumulate") = false);
 
   m.def(
       "norm_fwd",

@@ -47,7 +47,9 @@ const char* gemm_last_reason() { return t_reason; }
 cudaError_t gemm_bf16_tn(const GemmArgs& a, cudaStream_t stream) {
   t_reason = "";
   if (a.m <= 0 || a.n <= 0 || a.k <= 0) return cudaErrorInvalidValue;
-  if (a.k % BK != 0 || a.n % 8 != 0) return unsupported("K must be a multiple of 64 and N a multiple of 8");
+  // (a contraction over rows of both operands may end anywhere: the tile kernel loads zeros past the last row)
+  if ((a.k % BK != 0 && !(a.a_mn_major && a.b_mn_major)) || a.n % 8 != 0)
+    return unsupported("K must be a multiple of 64 and N a multiple of 8");
   if (a.lda % 8 != 0 || a.ldb % 8 != 0 || a.ldd % (a.d_fp32 ? 4 : 8) != 0)
     return unsupported("row strides must keep rows 16-byte aligned");
   if ((reinterpret_cast<uintptr_t>(a.a) | reinterpret_cast<uintptr_t>(a.b) | reinterpret_cast<uintptr_t>(a.d)) & 15u)
@@ -67,7 +69,8 @@ cudaError_t gemm_bf16_tn(const GemmArgs& a, cudaStream_t stream) {
   }();
   const int forced = g_gemm_kernel_override.load(std::memory_order_relaxed);
   const int choice = forced != -2 ? forced : env_choice;
-  cudaError_t rc = choice == kPersistent ? launch_gemm_persistent(a, FusedDev{}, 0, stream) : launch_gemm_tiles(a, choice, stream);
+  const bool tile_only = a.k % BK != 0 || a.colsum;   // what only the tile kernel does
+  cudaError_t rc = choice == kPersistent && !tile_only ? launch_gemm_persistent(a, FusedDev{}, 0, stream) : launch_gemm_tiles(a, choice, stream);
   if (rc == cudaErrorNotSupported) return unsupported("cuTensorMapEncodeTiled rejected an operand");
   return rc;
 }

@@ -37,7 +37,21 @@ namespace mccl {
 namespace ops {
 namespace tiles {
 
-enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2 };
+// OUT_BF16_SUM: the bf16 output and, added into GemmDev::colsum, its column sums (a bias gradient).
+enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3 };
+
+// One product, or several with the same K whose tiles one launch works through (the weight gradients of a layer: alone,
+// a 512 x 2048 gradient is 64 tiles and leaves half the SMs without one; together they fill two rounds).
+constexpr int kMaxGroup = 4;
+template <int kMax>
+struct Problems {
+  CUtensorMap a[kMax], b[kMax], d[kMax];
+  CUtensorMap x;              // the second output of the GELU instantiation, or the extra input of the bf16 ones
+  int m[kMax], n[kMax];
+  int first[kMax + 1];        // first tile of each product
+  int n_tiles[kMax];
+  int count;
+};
 
 template <int BN, bool kPair>
 struct Shape {
@@ -153,11 +167,10 @@ __device__ __forceinline__ void unpack8(const uint4& pk, float (&v)[8]) {
   }
 }
 
-// tma_x: the second output of the GELU instantiation, or the extra input (multiplier / residual) of the bf16 one.
-template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut>
+template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut, int kMax>
 __global__ void __launch_bounds__(Shape<BN, kPair>::kThreads, 1)
-gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                 const __grid_constant__ CUtensorMap tma_d, const __grid_constant__ CUtensorMap tma_x, GemmDev g, int splits) {
+gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits) {
+  constexpr bool kBf16 = kOut == OUT_BF16 || kOut == OUT_BF16_SUM;
   using S = Shape<BN, kPair>;
   constexpr int kStages = S::kStages, kTileM = kPair ? 2 * BM : BM;
   extern __shared__ uint8_t smem_raw[];
@@ -176,8 +189,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = kPair ? cluster_ctarank() : 0u;
   const int worker = static_cast<int>(kPair ? blockIdx.x >> 1 : blockIdx.x), workers = static_cast<int>(kPair ? gridDim.x >> 1 : gridDim.x);
-  const int m_tiles = (g.m + kTileM - 1) / kTileM, n_tiles = (g.n + BN - 1) / BN;
-  const int total = m_tiles * n_tiles * splits;
+  const int total = P.first[P.count] * splits;
   const int all_kb = (g.k + BK - 1) / BK;
 
   if (warp == 0 && tc::elect_one()) {
@@ -192,10 +204,12 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     for (int b = 0; b < S::kEpiWarps * S::kBufs; ++b) tc::mbar_init(&extra_full[b], 1);
     *abort_flag = 0;
     tc::mbar_init_fence();
-    tc::tma_prefetch_desc(&tma_a);
-    tc::tma_prefetch_desc(&tma_b);
-    tc::tma_prefetch_desc(&tma_d);
-    tc::tma_prefetch_desc(&tma_x);
+    for (int p = 0; p < P.count; ++p) {
+      tc::tma_prefetch_desc(&P.a[p]);
+      tc::tma_prefetch_desc(&P.b[p]);
+      tc::tma_prefetch_desc(&P.d[p]);
+    }
+    if (kMax == 1) tc::tma_prefetch_desc(&P.x);
   }
   if (warp == 1) {
     if constexpr (kPair) {
@@ -214,13 +228,24 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   pdl_wait();   // set-up done: from here on operands are read and outputs written
   if (tl_t0 != 0ull && tl_detail(g.tl)) tl_mark(g.tl, tl_t0, tl_now(), TL_GEMM_PHASE, 0u);
 
-  auto tile_coords = [&](int w, int& m_blk, int& n_blk, int& kb0, int& kb1) {
-    const int t = splits > 1 ? w / splits : w;
+  // product, tile row, tile column and range of k-blocks of work item w
+  struct Item {
+    int p, m_blk, n_blk, kb0, kb1;
+  };
+  auto item = [&](int w) {
+    Item it;
+    int t = splits > 1 ? w / splits : w;
     const int s = w - t * splits;
-    kb0 = splits > 1 ? all_kb * s / splits : 0;
-    kb1 = splits > 1 ? all_kb * (s + 1) / splits : all_kb;
-    m_blk = t / n_tiles;
-    n_blk = t - m_blk * n_tiles;
+    it.kb0 = splits > 1 ? all_kb * s / splits : 0;
+    it.kb1 = splits > 1 ? all_kb * (s + 1) / splits : all_kb;
+    it.p = 0;
+    if constexpr (kMax > 1) {
+      while (it.p + 1 < P.count && t >= P.first[it.p + 1]) ++it.p;
+      t -= P.first[it.p];
+    }
+    it.m_blk = t / P.n_tiles[it.p];
+    it.n_blk = t - it.m_blk * P.n_tiles[it.p];
+    return it;
   };
 
   if (warp == 0) {
@@ -230,11 +255,12 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int s = 0;
       uint32_t parity = 1;   // a fresh barrier counts as the phase before the first: the first round does not wait
       for (int w = worker; w < total && ok; w += workers) {
-        int m_blk, n_blk, kb0, kb1;
-        tile_coords(w, m_blk, n_blk, kb0, kb1);
-        const int a_row = m_blk * kTileM + static_cast<int>(rank) * BM;
-        const int b_row = n_blk * BN + static_cast<int>(rank) * S::kRowsB;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        const Item it = item(w);
+        const CUtensorMap* map_a = &P.a[it.p];
+        const CUtensorMap* map_b = &P.b[it.p];
+        const int a_row = it.m_blk * kTileM + static_cast<int>(rank) * BM;
+        const int b_row = it.n_blk * BN + static_cast<int>(rank) * S::kRowsB;
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
           ok = wait(&empty[s], parity, abort_flag);
           if (!ok) break;
           uint8_t* a_dst = smem + s * S::kStageBytes;
@@ -245,29 +271,29 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             const uint32_t bar = leader_addr(&full[s]);
             if (kAMn) {
 #pragma unroll
-              for (int q = 0; q < BM / 64; ++q) load_2d_pair(a_dst + q * (BK * 128), &tma_a, bar, a_row + q * 64, k0);
+              for (int q = 0; q < BM / 64; ++q) load_2d_pair(a_dst + q * (BK * 128), map_a, bar, a_row + q * 64, k0);
             } else {
-              load_2d_pair(a_dst, &tma_a, bar, k0, a_row);
+              load_2d_pair(a_dst, map_a, bar, k0, a_row);
             }
             if (kBMn) {
 #pragma unroll
-              for (int q = 0; q < S::kRowsB / 64; ++q) load_2d_pair(b_dst + q * (BK * 128), &tma_b, bar, b_row + q * 64, k0);
+              for (int q = 0; q < S::kRowsB / 64; ++q) load_2d_pair(b_dst + q * (BK * 128), map_b, bar, b_row + q * 64, k0);
             } else {
-              load_2d_pair(b_dst, &tma_b, bar, k0, b_row);
+              load_2d_pair(b_dst, map_b, bar, k0, b_row);
             }
           } else {
             tc::mbar_expect_tx(&full[s], S::kStageBytes);
             if (kAMn) {
 #pragma unroll
-              for (int q = 0; q < BM / 64; ++q) tc::tma_load_2d(a_dst + q * (BK * 128), &tma_a, &full[s], a_row + q * 64, k0);
+              for (int q = 0; q < BM / 64; ++q) tc::tma_load_2d(a_dst + q * (BK * 128), map_a, &full[s], a_row + q * 64, k0);
             } else {
-              tc::tma_load_2d(a_dst, &tma_a, &full[s], k0, a_row);
+              tc::tma_load_2d(a_dst, map_a, &full[s], k0, a_row);
             }
             if (kBMn) {
 #pragma unroll
-              for (int q = 0; q < S::kRowsB / 64; ++q) tc::tma_load_2d(b_dst + q * (BK * 128), &tma_b, &full[s], b_row + q * 64, k0);
+              for (int q = 0; q < S::kRowsB / 64; ++q) tc::tma_load_2d(b_dst + q * (BK * 128), map_b, &full[s], b_row + q * 64, k0);
             } else {
-              tc::tma_load_2d(b_dst, &tma_b, &full[s], k0, b_row);
+              tc::tma_load_2d(b_dst, map_b, &full[s], k0, b_row);
             }
           }
           if (++s == kStages) {
@@ -292,9 +318,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int s = 0, i = 0;
       uint32_t parity = 0;
       for (int w = worker; w < total; w += workers, ++i) {
-        int m_blk, n_blk, kb0, kb1;
-        tile_coords(w, m_blk, n_blk, kb0, kb1);
-        const int buf = i & 1;
+        const Item it = item(w);
+        const int kb0 = it.kb0, kb1 = it.kb1, buf = i & 1;
         if (i >= 2) {
           ok = wait(&acc_empty[buf], ((i >> 1) - 1) & 1, abort_flag);
           if (!ok) break;
@@ -336,37 +361,38 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     uint8_t* stage = smem + S::kStagingOff + e * S::kBufs * 4096;
     uint64_t* xfull = extra_full + e * S::kBufs;
     const bool has_bias = kOut != OUT_F32 && (g.epilogue == EPI_BIAS || g.epilogue == EPI_BIAS_GELU || g.epilogue == EPI_BIAS_GELU_D);
-    const bool has_extra = kOut == OUT_BF16 && (g.mul != nullptr || g.residual != nullptr);
+    const bool has_extra = kBf16 && (g.mul != nullptr || g.residual != nullptr);
     const bool multiply = g.mul != nullptr;
     const bool gelu_d = g.epilogue == EPI_BIAS_GELU_D || g.epilogue == EPI_GELU_D;
     bool ok = true;
     int i = 0;
     uint32_t xparity = 0;   // one bit per staging buffer
     for (int w = worker; w < total; w += workers, ++i) {
-      int m_blk, n_blk, kb0, kb1;
-      tile_coords(w, m_blk, n_blk, kb0, kb1);
+      const Item it = item(w);
+      const CUtensorMap* map_d = &P.d[it.p];
+      const int m = P.m[it.p], n = P.n[it.p];
       const int buf = i & 1;
       const bool stamp = warp == 2 && lane == 0 && tl_detail(g.tl);
       const unsigned long long ts0 = stamp ? tl_now() : 0ull;
-      const int col0 = n_blk * BN + part * S::kCols;
-      const int row0 = m_blk * kTileM + static_cast<int>(rank) * BM + quarter * 32;
-      const bool inside = row0 < g.m && col0 < g.n;   // uniform over the warp
+      const int col0 = it.n_blk * BN + part * S::kCols;
+      const int row0 = it.m_blk * kTileM + static_cast<int>(rank) * BM + quarter * 32;
+      const bool inside = row0 < m && col0 < n;   // uniform over the warp
       // the staging buffers are free again; fetch what the epilogue will need while the MMAs of the tile still run
       if (tc::elect_one()) {
         bulk_wait_read<0>();
         if (has_extra && inside) {
 #pragma unroll
           for (int b = 0; b < S::kBufs; ++b) {
-            if (col0 + b * 64 < g.n) {
+            if (col0 + b * 64 < n) {
               tc::mbar_expect_tx(&xfull[b], 4096);
-              tc::tma_load_2d(stage + b * 4096, &tma_x, &xfull[b], col0 + b * 64, row0);
+              tc::tma_load_2d(stage + b * 4096, &P.x, &xfull[b], col0 + b * 64, row0);
             }
           }
         }
       }
       // lane l keeps the bias of columns [col0 + 4 l, col0 + 4 l + 4); the loop below spreads it by shuffles
       float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (has_bias && 4 * lane < S::kCols && col0 + 4 * lane < g.n) bias4 = __ldg(reinterpret_cast<const float4*>(g.bias + col0 + 4 * lane));
+      if (has_bias && 4 * lane < S::kCols && col0 + 4 * lane < n) bias4 = __ldg(reinterpret_cast<const float4*>(g.bias + col0 + 4 * lane));
       __syncwarp();
       ok = wait(&acc_full[buf], (i >> 1) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
@@ -390,7 +416,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           tc::tmem_ld_32x32(taddr + static_cast<uint32_t>(c), r);
           tc::tmem_ld_wait();
           if (c + 32 >= S::kCols) last_read();
-          if (row0 >= g.m || col0 + c >= g.n) continue;
+          if (row0 >= m || col0 + c >= n) continue;
           uint8_t* dst = stage + (S::kBufs > 1 ? ((c >> 5) & 1) * 4096 : 0);
           if (tc::elect_one()) bulk_wait_read<S::kBufs - 1>();
           __syncwarp();
@@ -399,8 +425,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           fence_async_smem();
           __syncwarp();
           if (tc::elect_one()) {
-            if (add) reduce_add_2d(&tma_d, dst, col0 + c, row0);
-            else store_2d(&tma_d, dst, col0 + c, row0);
+            if (add) reduce_add_2d(map_d, dst, col0 + c, row0);
+            else store_2d(map_d, dst, col0 + c, row0);
             bulk_commit();
           }
           __syncwarp();
@@ -410,7 +436,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll 1
         for (int c = 0; c < S::kCols; c += 64) {
           const int cg = col0 + c;
-          const bool active = row0 < g.m && cg < g.n;   // uniform over the warp
+          const bool active = row0 < m && cg < n;   // uniform over the warp
           uint8_t* buf_c = stage + (c >> 6) * 4096;
           if (has_extra && active) {
             ok = wait(&xfull[c >> 6], (xparity >> (c >> 6)) & 1u, abort_flag);
@@ -465,13 +491,30 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 }
               }
               *stage_unit(buf_c, lane, j) = pack8(v);
+              if constexpr (kOut == OUT_BF16_SUM) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) r[jj * 8 + q] = __float_as_uint(v[q]);
+              }
+            }
+            if constexpr (kOut == OUT_BF16_SUM) {
+              // sums of 32 columns over the warp's 32 rows by halving: 31 shuffles, lane l ends up with column l
+#pragma unroll
+              for (int o = 16; o >= 1; o >>= 1) {
+#pragma unroll
+                for (int q = 0; q < o; ++q) {
+                  const float lo = __uint_as_float(r[q]), hi = __uint_as_float(r[q + o]);
+                  const float other = __shfl_xor_sync(0xffffffffu, (lane & o) ? lo : hi, o);
+                  r[q] = __float_as_uint(((lane & o) ? hi : lo) + other);
+                }
+              }
+              if (cg + 32 * h + lane < n) atomicAdd(g.colsum + cg + 32 * h + lane, __uint_as_float(r[0]));
             }
           }
           if (!active) continue;
           fence_async_smem();
           __syncwarp();
           if (tc::elect_one()) {
-            store_2d(&tma_d, buf_c, cg, row0);
+            store_2d(map_d, buf_c, cg, row0);
             bulk_commit();
             if constexpr (kOut == OUT_GELU) bulk_wait_read<0>();
           }
@@ -482,7 +525,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             fence_async_smem();
             __syncwarp();
             if (tc::elect_one()) {
-              store_2d(&tma_x, buf_c, cg, row0);
+              store_2d(&P.x, buf_c, cg, row0);
               bulk_commit();
             }
             __syncwarp();
@@ -517,34 +560,51 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     if constexpr (kPair) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * BN) : "memory");
     else tc::tmem_dealloc(tmem_base, 2 * BN);
   }
-  tl_end(g.tl, tl_t0, TL_GEMM, (static_cast<uint32_t>(m_tiles * (kPair ? 2 : 1)) << 16) | static_cast<uint32_t>(n_tiles * splits));
+  tl_end(g.tl, tl_t0, TL_GEMM, (static_cast<uint32_t>(total / (P.n_tiles[0] * splits) * (kPair ? 2 : 1)) << 16) | static_cast<uint32_t>(P.n_tiles[0] * splits));
 }
 
-// Launches `workers` CTAs (pairs) over the tiles of `a`, K cut into `splits` (fp32 sums added into D).
-template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut>
-cudaError_t launch_tiles(const GemmArgs& a, int workers, int splits, cudaStream_t stream) {
+// Launches `workers` CTAs (pairs) over the tiles of `count` products with the same K, which is cut into `splits` (fp32
+// sums added into D).
+template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut, int kMax>
+cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int splits, cudaStream_t stream) {
   using S = Shape<BN, kPair>;
-  auto kernel = gemm_tile_kernel<BN, kPair, kAMn, kBMn, kOut>;
+  auto kernel = gemm_tile_kernel<BN, kPair, kAMn, kBMn, kOut, kMax>;
   static std::atomic<bool> configured{false};
   if (!configured.load(std::memory_order_acquire)) {
     cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
     if (rc != cudaSuccess) return rc;
     configured.store(true, std::memory_order_release);
   }
-  CUtensorMap ma, mb, md, mx;
-  // K-major: boxes of 64 of K x the tile's rows; MN-major: boxes of 64 columns x 64 of K (zero fill past K)
-  const bool oka = kAMn ? encode_map(&ma, a.a, a.k, a.m, a.lda, BK) : encode_map(&ma, a.a, a.m, a.k, a.lda, BM);
-  const bool okb = kBMn ? encode_map(&mb, a.b, a.k, a.n, a.ldb, BK) : encode_map(&mb, a.b, a.n, a.k, a.ldb, S::kRowsB);
-  if (!oka || !okb || !encode_out_map(&md, a.d, a.m, a.n, a.ldd, kOut == OUT_F32)) return cudaErrorNotSupported;
-  const void* x = kOut == OUT_GELU ? a.aux : (kOut == OUT_BF16 ? (a.mul ? a.mul : a.residual) : nullptr);
-  if (x == nullptr) mx = md;   // never used
-  else if (!encode_out_map(&mx, x, a.m, a.n, a.ldd, false)) return cudaErrorNotSupported;
+  Problems<kMax> P;
+  P.count = count;
+  P.first[0] = 0;
+  for (int p = 0; p < count; ++p) {
+    const GemmArgs& a = args[p];
+    // K-major: boxes of 64 of K x the tile's rows; MN-major: boxes of 64 columns x 64 of K (zero fill past K)
+    const bool oka = kAMn ? encode_map(&P.a[p], a.a, a.k, a.m, a.lda, BK) : encode_map(&P.a[p], a.a, a.m, a.k, a.lda, BM);
+    const bool okb = kBMn ? encode_map(&P.b[p], a.b, a.k, a.n, a.ldb, BK) : encode_map(&P.b[p], a.b, a.n, a.k, a.ldb, S::kRowsB);
+    if (!oka || !okb || !encode_out_map(&P.d[p], a.d, a.m, a.n, a.ldd, kOut == OUT_F32)) return cudaErrorNotSupported;
+    P.m[p] = a.m;
+    P.n[p] = a.n;
+    P.n_tiles[p] = (a.n + BN - 1) / BN;
+    P.first[p + 1] = P.first[p] + P.n_tiles[p] * ((a.m + (kPair ? 2 * BM : BM) - 1) / (kPair ? 2 * BM : BM));
+    // partial sums are added into the output: start from zero unless the caller accumulates anyway
+    if (splits > 1 && !a.accumulate) {
+      cudaError_t rc = cudaMemsetAsync(a.d, 0, static_cast<size_t>(a.m) * a.n * sizeof(float), stream);
+      if (rc != cudaSuccess) return rc;
+    }
+  }
+  const GemmArgs& a = args[0];
+  const void* x = kOut == OUT_GELU ? a.aux : (kOut == OUT_F32 ? nullptr : (a.mul ? a.mul : a.residual));
+  if (x == nullptr) P.x = P.d[0];   // never used
+  else if (!encode_out_map(&P.x, x, a.m, a.n, a.ldd, false)) return cudaErrorNotSupported;
   GemmDev g;
   g.d = a.d;
   g.aux = a.aux;
   g.bias = a.bias;
   g.residual = a.residual;
   g.mul = a.mul;
+  g.colsum = a.colsum;
   g.m = a.m;
   g.n = a.n;
   g.k = a.k;
@@ -556,11 +616,6 @@ cudaError_t launch_tiles(const GemmArgs& a, int workers, int splits, cudaStream_
   g.err = gemm_error_device_ptr();
   if (!g.err) return cudaErrorNotSupported;
   g.tl = timeline_device_ptr();
-  // partial sums are added into the output: start from zero unless the caller accumulates anyway
-  if (splits > 1 && !a.accumulate) {
-    cudaError_t rc = cudaMemsetAsync(a.d, 0, static_cast<size_t>(a.m) * a.n * sizeof(float), stream);
-    if (rc != cudaSuccess) return rc;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(kPair ? 2 * workers : workers));
   cfg.blockDim = dim3(S::kThreads);
@@ -579,20 +634,20 @@ cudaError_t launch_tiles(const GemmArgs& a, int workers, int splits, cudaStream_
     attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++cfg.numAttrs;
   }
-  cudaLaunchKernelEx(&cfg, kernel, ma, mb, md, mx, g, splits);
+  cudaLaunchKernelEx(&cfg, kernel, P, g, splits);
   ::mccl::launch_record("gemm_tile_kernel", __FILE__, __LINE__, cfg.gridDim, cfg.blockDim, S::kTotal, stream);
   count_launch();
   return ::mccl::launch_status();
 }
 
 // Pairs of this instantiation that can be resident at once (GPCs with an odd number of free SMs leave one SM out).
-template <int BN, bool kAMn, bool kBMn, int kOut>
+template <int BN, bool kAMn, bool kBMn, int kOut, int kMax>
 int max_pairs() {
   using S = Shape<BN, true>;
   static std::atomic<int> cached{0};
   int n = cached.load(std::memory_order_relaxed);
   if (n > 0) return n;
-  auto kernel = gemm_tile_kernel<BN, true, kAMn, kBMn, kOut>;
+  auto kernel = gemm_tile_kernel<BN, true, kAMn, kBMn, kOut, kMax>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * 74);
   cfg.blockDim = dim3(S::kThreads);

@@ -109,6 +109,7 @@ struct GemmArgs {
   const float* bias = nullptr;       // [N]
   const __nv_bfloat16* residual = nullptr;  // [M, N] added after bias / activation, row stride ldd
   const __nv_bfloat16* mul = nullptr;       // [M, N]: D = acc * mul (e.g. the saved gelu'(z): the input gradient through a GELU), row stride ldd
+  float* colsum = nullptr;                  // [N] fp32: column sums of D are added here (bf16 output without bias or residual, B MN-major)
   int m = 0, n = 0, k = 0;
   int lda = 0, ldb = 0, ldd = 0;
   bool d_fp32 = false;
@@ -118,6 +119,10 @@ struct GemmArgs {
 // Returns cudaErrorNotSupported for shapes the kernel does not cover
 // (K % 64 != 0, N % 8 != 0, unaligned pointers); the caller falls back.
 cudaError_t gemm_bf16_tn(const GemmArgs& args, cudaStream_t stream);
+// Up to any number of weight gradients dW[N, K] = dY[tokens, N]^T · X[tokens, K] over the same tokens, worked through together
+// (four products per launch).  A product is a GemmArgs with both operands MN-major, fp32 output, no epilogue; all of them
+// accumulate, or none.
+cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream);
 // Caps the number of CTAs (= SMs) plain GEMM launches occupy from now on; 0 restores one CTA per SM.  A
 // data-parallel trainer lowers it during backward so that a few SMs stay free for the gradient collectives
 // that run beside the GEMMs.  The value is read at launch time, so it is baked into a captured CUDA graph.

@@ -67,3 +67,40 @@ def test_long_contraction_is_split(C):
     a, b = torch.randn(16384, 512, device="cuda").bfloat16(), torch.randn(16384, 256, device="cuda").bfloat16()
     d, _ = C.gemm_bf16(a, b, None, "none", True, None, False, True, True)
     assert _rel(d, a.float().t() @ b.float()) < 3e-5
+
+
+@pytest.mark.parametrize("K", [8, 72, 1000])
+def test_ragged_contraction_of_row_major_operands(C, K):
+    """Weight gradients over any number of tokens: past the last row the loads are zeros."""
+    torch.manual_seed(K)
+    a, b = torch.randn(K, 264, device="cuda").bfloat16(), torch.randn(K, 136, device="cuda").bfloat16()
+    assert _rel(C.gemm_bf16(a, b, None, "none", True, None, False, True, True)[0], a.float().t() @ b.float()) < 1e-5
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 64), (300, 200, 128), (4096, 2048, 512)])
+def test_column_sums_of_the_output(C, M, N, K):
+    torch.manual_seed(M)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
+    mul, acc = torch.randn(M, N, device="cuda").bfloat16(), torch.randn(N, device="cuda")
+    want, ref = acc.clone(), (a.float() @ b.float()) * mul.float()
+    d, _ = C.gemm_bf16(a, b, None, "none", False, None, False, False, True, None, mul, acc)
+    assert _rel(d, ref) < 1e-2 and _rel(acc, want + ref.sum(0)) < 1e-4
+
+
+@pytest.mark.parametrize("tokens,shapes", [(64, [(8, 8)]), (200, [(128, 64), (264, 128), (64, 512)]),
+                                           (4096, [(512, 2048), (2048, 512), (512, 512), (1536, 512), (104, 72), (512, 128)])])
+def test_group(tokens, shapes):
+    from mccl_b200 import _C
+    torch.manual_seed(tokens)
+    pairs = [(torch.randn(tokens, n, device="cuda").bfloat16(), torch.randn(tokens, k, device="cuda").bfloat16()) for n, k in shapes]
+    refs = [a.float().t() @ b.float() for a, b in pairs]
+    tol = 1e-5 * max(1, tokens // 64)
+    for d, r in zip(_C.gemm_group([(a, b, None) for a, b in pairs]), refs):
+        assert _rel(d, r) < tol
+    accs = [torch.randn_like(r) for r in refs]
+    wants = [a + r for a, r in zip(accs, refs)]
+    _C.gemm_group([(a, b, d) for (a, b), d in zip(pairs, accs)], True)
+    for d, w in zip(accs, wants):
+        assert _rel(d, w) < tol
+    torch.cuda.synchronize()
+    assert _C.gemm_error_flag() == 0
