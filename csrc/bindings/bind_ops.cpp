@@ -323,39 +323,50 @@ void bind_ops(py::module_& m) {
       "attn_fwd",
       [](const at::Tensor& qkv, double scale) {
         need(qkv, at::kBFloat16, "attention(qkv)");
-        MCCL_CHECK_TENSOR(qkv.dim() == 5 && qkv.size(2) == 3 && qkv.size(4) == 64, "attention: qkv must be [B, S, 3, H, 64]");
-        const int64_t B = qkv.size(0), S = qkv.size(1), H = qkv.size(3);
+        MCCL_CHECK_TENSOR(qkv.dim() == 5 && qkv.size(2) == 3, "attention: qkv must be [B, S, 3, H, head_dim]");
+        const int64_t B = qkv.size(0), S = qkv.size(1), H = qkv.size(3), D = qkv.size(4);
         c10::cuda::CUDAGuard guard(qkv.device());
-        at::Tensor o = at::empty({B, S, H * 64}, qkv.options());
+        at::Tensor o = at::empty({B, S, H * D}, qkv.options());
         at::Tensor lse = at::empty({B, H, S}, qkv.options().dtype(at::kFloat));
         cudaError_t rc = ops::attention_fwd(bf(qkv), bf(o), lse.data_ptr<float>(), static_cast<int>(B), static_cast<int>(S),
-                                            static_cast<int>(H), static_cast<float>(scale), stream_of(qkv));
-        MCCL_CHECK_T(rc == cudaSuccess, CudaError, "attention forward [B " << B << ", S " << S << ", H " << H << "] failed: "
+                                            static_cast<int>(H), static_cast<int>(D), static_cast<float>(scale), stream_of(qkv));
+        MCCL_CHECK_T(rc == cudaSuccess, CudaError, "attention forward [B " << B << ", S " << S << ", H " << H << ", head_dim " << D << "] failed: "
                                                                            << cudaGetErrorString(rc));
         return std::make_pair(o, lse);
       },
-      py::arg("qkv"), py::arg("scale"), "Causal attention; returns (o [B, S, H*64] bf16, lse [B, H, S] fp32, log2 domain).  S % 128 == 0.");
+      py::arg("qkv"), py::arg("scale"), "Causal attention; returns (o [B, S, H*hd] bf16, lse [B, H, S] fp32, log2 domain).  S <= 256 and head_dim <= 64 (a "
+      "multiple of 8), or head_dim 64 with S a multiple of 128.");
+  m.def("attention_supported", [](int64_t seq, int64_t head_dim) {
+    return seq < (1 << 30) && head_dim < (1 << 30) && ops::attention_supported(static_cast<int>(seq), static_cast<int>(head_dim));
+  });
   m.def(
       "attn_bwd",
-      [](const at::Tensor& qkv, const at::Tensor& o, const at::Tensor& d_o, const at::Tensor& lse, double scale) {
+      [](const at::Tensor& qkv, const at::Tensor& o, const at::Tensor& d_o, const at::Tensor& lse, double scale,
+         const c10::optional<at::Tensor>& colsum) {
         need(qkv, at::kBFloat16, "attention_bwd(qkv)");
         need(o, at::kBFloat16, "attention_bwd(o)");
         need(d_o, at::kBFloat16, "attention_bwd(d_o)");
         need(lse, at::kFloat, "attention_bwd(lse)");
-        MCCL_CHECK_TENSOR(qkv.dim() == 5 && qkv.size(2) == 3 && qkv.size(4) == 64, "attention_bwd: qkv must be [B, S, 3, H, 64]");
-        const int64_t B = qkv.size(0), S = qkv.size(1), H = qkv.size(3);
-        MCCL_CHECK_TENSOR(o.numel() == B * S * H * 64 && d_o.numel() == o.numel() && lse.numel() == B * H * S,
+        MCCL_CHECK_TENSOR(qkv.dim() == 5 && qkv.size(2) == 3, "attention_bwd: qkv must be [B, S, 3, H, head_dim]");
+        const int64_t B = qkv.size(0), S = qkv.size(1), H = qkv.size(3), D = qkv.size(4);
+        float* cs = nullptr;
+        if (colsum.has_value() && colsum->defined()) {
+          need(*colsum, at::kFloat, "attention_bwd(colsum)");
+          MCCL_CHECK_TENSOR(colsum->numel() == 3 * H * D, "attention_bwd: colsum must have 3 * heads * head_dim elements");
+          cs = colsum->data_ptr<float>();
+        }
+        MCCL_CHECK_TENSOR(o.numel() == B * S * H * D && d_o.numel() == o.numel() && lse.numel() == B * H * S,
                           "attention_bwd: operand sizes do not match qkv");
         c10::cuda::CUDAGuard guard(qkv.device());
         at::Tensor dqkv = at::empty_like(qkv);
-        cudaError_t rc = ops::attention_bwd(bf(qkv), bf(o), bf(d_o), lse.data_ptr<float>(), bf(dqkv), static_cast<int>(B),
-                                            static_cast<int>(S), static_cast<int>(H), static_cast<float>(scale), stream_of(qkv));
+        cudaError_t rc = ops::attention_bwd(bf(qkv), bf(o), bf(d_o), lse.data_ptr<float>(), bf(dqkv), cs, static_cast<int>(B),
+                                            static_cast<int>(S), static_cast<int>(H), static_cast<int>(D), static_cast<float>(scale), stream_of(qkv));
         MCCL_CHECK_T(rc == cudaSuccess, CudaError, "attention backward [B " << B << ", S " << S << ", H " << H << "] failed: "
                                                                             << cudaGetErrorString(rc));
         return dqkv;
       },
-      py::arg("qkv"), py::arg("o"), py::arg("d_o"), py::arg("lse"), py::arg("scale"),
-      "Gradient of the whole qkv tensor.  S must be 128 or 256.");
+      py::arg("qkv"), py::arg("o"), py::arg("d_o"), py::arg("lse"), py::arg("scale"), py::arg("colsum") = py::none(),
+      "Gradient of the whole qkv tensor (see attention_supported); its column sums are added into colsum.");
 
   // ---- tensor-parallel GEMMs fused with their collective ----
   py::class_<ops::TpGemm>(m, "TpGemm")

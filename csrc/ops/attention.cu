@@ -1,26 +1,35 @@
-// Causal self-attention for sm_100a, head dimension 64, forward and backward, on the 5th-generation tensor cores.
+// Causal self-attention for sm_100a, forward and backward, on the 5th-generation tensor cores.
 //
-// Operands come straight from the fused QKV projection: qkv is [B, S, 3, H, 64] bf16 (the projection's output
-// viewed, not copied), so q, k and v tiles of a (batch, head) are boxes of one 2-D tensor map over the
-// [B*S, 3*H*64] matrix, fetched by TMA into 128-byte-swizzled shared memory.  The output is written as
-// [B, S, H, 64], which is the layout the output projection reads, and backward produces the gradient of the whole
+// Operands come straight from the fused QKV projection: qkv is [B, S, 3, H, hd] bf16 (the projection's output
+// viewed, not copied), so q, k and v tiles of a (batch, head) are boxes of one tensor map,
+// fetched by TMA into 128-byte-swizzled shared memory.  The output is written as [B, S, H, hd], which is the layout the output projection reads, and backward produces the gradient of the whole
 // qkv tensor in one piece.  Nothing is transposed, sliced or concatenated around the kernels.
 //
-// Forward, one CTA per (batch, head, block of 128 queries), looping over the key blocks up to the diagonal:
-//   S = Q K^T           tcgen05.mma, fp32 accumulator in tensor memory (128 lanes x 128 columns)
-//   P = exp2(S*c - m)   tcgen05.ld, one query row per thread, running max / sum (online softmax), P written as bf16
-//                       into shared memory in the layout the next MMA reads as its A operand
-//   O += P V            tcgen05.mma into a second tensor-memory region, folded into registers with the rescale
-// Backward, one CTA per (batch, head) for S = 256 (two blocks; dQ, dK, dV accumulate in tensor memory):
-//   per block pair (i, j <= i):  S = Q_i K_j^T,  P = exp2(S*c - L_i),  dP = dO_i V_j^T,  dS = P (dP - delta_i) c,
-//                                dV_j += P^T dO_i,  dK_j += dS^T Q_i,  dQ_i += dS K_j
-// The transposed products read P / dS from the same shared-memory tile through an MN-major operand descriptor.
+// Sequences of up to 256 and head dimensions of up to 64 (multiples of 8), which is what the models train with:
+//   Forward, one CTA of two warpgroups per (batch, head, block of 128 queries).  A row of scores is at most 256 wide, so
+//   all of them fit tensor memory: one S = Q K^T for every key, one softmax without running rescale (the warpgroups take
+//   half of the columns each and exchange maximum and sum), one O = P V.  P overwrites Q and K in shared memory and O the
+//   scores in tensor memory, so two CTAs share an SM.
+//   Backward, one CTA of two warpgroups per (batch, head); per block pair (i, j <= i):
+//     S = Q_i K_j^T and dP = dO_i V_j^T together,  P = exp2(S*c - L_i),  dS = P (dP - delta_i) c,
+//     dV_j += P^T dO_i,  dK_j += dS^T Q_i,  dQ_i += dS K_j
+//   The next pair's S and dP are issued ahead of this pair's gradient products, so the tensor cores work on them while
+//   the gradients finish.  The transposed products read P / dS from the same tile through an MN-major descriptor.  Column
+//   sums of the qkv gradient (the projection's bias gradient) are taken on the way out.
+//   Both are bound by the latency of one CTA's chain (load, MMA, exponentials, MMA, store), not by any rate: at batch 16,
+//   8 heads, 256 x 64 the tensor cores would need 1 us forward and 3 backward.  Hence two threads per row, MMAs issued
+//   under elect.sync, no online rescale, and one wait where the products allow it.
+//   A tile row past the sequence or a column past the head dimension is zero fill of the TMA load, so ragged sizes take
+//   the same path.
+// Longer sequences (forward, head dimension 64): one warpgroup per 128 queries, looping over key blocks with the online softmax.
 //
 // The reference has no attention kernel (its models call PyTorch's); this one exists because attention and the
 // copies around it are a tenth of the headline training step.  Every wait is bounded: on a timeout the kernel sets
 // the GEMM error word, frees its tensor memory and returns.
 #include "../core/launch.hpp"
 #include "gemm_common.cuh"
+
+#include <atomic>
 
 namespace mccl {
 namespace ops {
@@ -55,8 +64,8 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// ------------------------------------------------------------------ forward --
-__global__ void __launch_bounds__(128) attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, AttnDev a) {
+// -------------------------------------------------- forward, long sequences --
+__global__ void __launch_bounds__(128) attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tm_qkv, AttnDev a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;                       // 16 KiB
@@ -252,304 +261,533 @@ __global__ void __launch_bounds__(128) attn_fwd_kernel(const __grid_constant__ C
   }
 }
 
-constexpr int kFwdSmem = 6 * kTile + 64 + 1024;   // 97 KiB: two CTAs per SM
+constexpr int kLongSmem = 6 * kTile + 64 + 1024;   // 97 KiB: two CTAs per SM
 
-// ----------------------------------------------------------------- backward --
-struct AttnBwdDev {
-  const __nv_bfloat16* o;    // [B, S, H, 64]
-  const __nv_bfloat16* d_o;  // [B, S, H, 64]
-  const float* lse;          // [B, H, S], log2 domain
-  __nv_bfloat16* dqkv;       // [B, S, 3, H, 64]
-  int S, H;
+// ------------------------------------------------- forward, up to 256 keys --
+struct AttnArgs {
+  const __nv_bfloat16* o;     // [B, S, H, hd]: backward reads it, forward writes through o_out
+  const __nv_bfloat16* d_o;   // [B, S, H, hd]
+  __nv_bfloat16* o_out;
+  float* lse;                 // [B, H, S], log2 domain: m + log2(l)
+  __nv_bfloat16* dqkv;        // [B, S, 3, H, hd]
+  float* colsum;              // optional: column sums of dqkv are added here, fp32 [3 * H * hd]
+  int S, H, hd;
   float scale, scale_log2;
   int* err;
 };
 
-// One CTA per (batch, head); the sequence is one or two blocks of 128 (S = 128 or 256).  Tensor memory, 512 columns:
-//   [0,128) dQ_0, dQ_1   [128,256) dK_0, dK_1   [256,384) dV_0, dV_1   [384,512) scratch: S, then dP
-__global__ void __launch_bounds__(128) attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv,
-                                                       const __grid_constant__ CUtensorMap tm_do, AttnBwdDev a) {
+// Box [128 rows of the sequence x 64 columns] of part `slot` (head, or part * H + head): zero fill past S and past hd.
+__device__ __forceinline__ void load_tile(void* dst, const CUtensorMap* map, uint64_t* bar, int slot, int row, int b) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(bar)), "r"(0), "r"(slot), "r"(row), "r"(b)
+      : "memory");
+}
+
+__global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, AttnArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* sQ = smem;                 // [2] x 16 KiB
-  uint8_t* sK = sQ + 2 * kTile;       // [2]
-  uint8_t* sV = sK + 2 * kTile;       // [2]
-  uint8_t* sDO = sV + 2 * kTile;      // [2]
-  uint8_t* sP = sDO + 2 * kTile;      // 32 KiB
-  uint8_t* sDS = sP + 2 * kTile;      // 32 KiB
-  uint64_t* in_full = reinterpret_cast<uint64_t*>(sDS + 2 * kTile);
-  uint64_t* mma_bar = in_full + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_bar + 1);
+  uint8_t* sK = smem;                // 2 tiles
+  uint8_t* sQ = smem + 2 * kTile;    // then one tile of room: P, up to four [128 x 64] sub-tiles, overwrites K, Q and this
+  uint8_t* sP = smem;
+  uint8_t* sV = smem + 4 * kTile;    // 2 tiles
+  float* s_max = reinterpret_cast<float*>(smem + 6 * kTile);   // [2][128]
+  float* s_sum = s_max + 256;                                  // [2][128]
+  uint64_t* qk_full = reinterpret_cast<uint64_t*>(s_sum + 256);
+  uint64_t* v_full = qk_full + 1;
+  uint64_t* s_done = v_full + 1;
+  uint64_t* o_done = s_done + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
   volatile int* bad = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   pdl_trigger();
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int nblk = a.S / kBlk;   // 1 or 2
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int qi = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);   // long rows first
+  const int h = blockIdx.y, b = blockIdx.z, nblk = qi + 1, nk = nblk * kBlk;
+  if (warp == 0 && tc::elect_one()) {
+    tc::mbar_init(qk_full, 1);
+    tc::mbar_init(v_full, 1);
+    tc::mbar_init(s_done, 1);
+    tc::mbar_init(o_done, 1);
+    *bad = 0;
+    tc::mbar_init_fence();
+    tc::tma_prefetch_desc(&tm_qkv);
+    pdl_wait();
+    tc::mbar_expect_tx(qk_full, static_cast<uint32_t>((1 + nblk) * kTile));
+    load_tile(sQ, &tm_qkv, qk_full, h, qi * kBlk, b);
+    for (int j = 0; j < nblk; ++j) load_tile(sK + j * kTile, &tm_qkv, qk_full, a.H + h, j * kBlk, b);
+    tc::mbar_expect_tx(v_full, static_cast<uint32_t>(nblk * kTile));
+    for (int j = 0; j < nblk; ++j) load_tile(sV + j * kTile, &tm_qkv, v_full, 2 * a.H + h, j * kBlk, b);
+  }
+  __syncwarp();
+  if (warp == 1) tc::tmem_alloc(tmem_slot, 256);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();
+
+  if (warp == 0) {
+    bool w = tc::mbar_wait(qk_full, 0);
+    w = __all_sync(0xffffffffu, w);
+    tc::fence_after_sync();
+    if (tc::elect_one()) {
+      if (w) {
+        const uint64_t da = tc::smem_desc_k_sw128(sQ), db = tc::smem_desc_k_sw128(sK);
+        const uint32_t idesc = nblk == 2 ? tc::idesc_bf16(kBlk, 256) : tc::idesc_bf16(kBlk, 128);
+#pragma unroll
+        for (int k4 = 0; k4 < kHd / UMMA_K; ++k4) tc::mma_bf16(tmem, da + 2 * k4, db + 2 * k4, idesc, k4 != 0);
+      } else {
+        *bad = 1;
+      }
+      tc::mma_commit(s_done);   // also on the failure path: releases the waiters below
+    }
+    __syncwarp();
+  }
+  bool ok = tc::mbar_wait(s_done, 0);
+  ok = __all_sync(0xffffffffu, ok);
+  tc::fence_after_sync();
+
+  const int wg = warp >> 2, row = (warp & 3) * 32 + lane;      // two threads per query row, half of the keys each
+  const int cols = nk >> 1, c_begin = wg * cols, limit = qi * kBlk + row;   // keys after `limit` are masked
+  const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  float mx = -INFINITY;
+#pragma unroll 1
+  for (int c0 = c_begin; c0 < c_begin + cols; c0 += 32) {
+    float s[32];
+    tmem_ld32(lane_base + static_cast<uint32_t>(c0), s);
+    if (c0 + 31 <= limit) {
+#pragma unroll
+      for (int e = 0; e < 32; ++e) mx = fmaxf(mx, s[e]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 32; ++e) mx = c0 + e <= limit ? fmaxf(mx, s[e]) : mx;
+    }
+  }
+  s_max[wg * 128 + row] = mx;
+  __syncthreads();
+  const float m = fmaxf(s_max[row], s_max[128 + row]) * a.scale_log2;   // key 0 is never masked: finite
+  float sum = 0.f;
+#pragma unroll 1
+  for (int c0 = c_begin; c0 < c_begin + cols; c0 += 32) {
+    float s[32];
+    tmem_ld32(lane_base + static_cast<uint32_t>(c0), s);
+    uint8_t* sub = sP + (c0 >> 6) * kTile;
+#pragma unroll
+    for (int c8 = 0; c8 < 4; ++c8) {
+      uint4 pk;
+      __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
+#pragma unroll
+      for (int e2 = 0; e2 < 4; ++e2) {
+        const int e = c8 * 8 + e2 * 2;
+        const float p0 = c0 + e <= limit ? exp2f(s[e] * a.scale_log2 - m) : 0.f;
+        const float p1 = c0 + e + 1 <= limit ? exp2f(s[e + 1] * a.scale_log2 - m) : 0.f;
+        hp[e2] = __floats2bfloat162_rn(p0, p1);
+        // the sum uses the rounded values: they are what multiplies V
+        const float2 back = __bfloat1622float2(hp[e2]);
+        sum += back.x + back.y;
+      }
+      *reinterpret_cast<uint4*>(sub + sw128_offset(row, ((c0 & 63) >> 3) + c8)) = pk;
+    }
+  }
+  s_sum[wg * 128 + row] = sum;
+  fence_async_smem();          // the MMA reads P through the async proxy
+  tc::fence_before_sync();
+  __syncthreads();             // P is complete and everybody has read S: O may overwrite it
+  if (warp == 0) {
+    bool w = tc::mbar_wait(v_full, 0);
+    w = __all_sync(0xffffffffu, w);
+    tc::fence_after_sync();
+    if (tc::elect_one()) {
+      if (w) {
+        constexpr uint32_t idesc = tc::idesc_bf16(kBlk, kHd, false, true);
+        const uint64_t dv = tc::smem_desc_mn_sw128(sV, kTile), dp = tc::smem_desc_k_sw128(sP);
+        for (int t = 0; t < 2 * nblk; ++t) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            tc::mma_bf16(tmem, dp + (kTile >> 4) * t + 2 * q, dv + 512 * t + 128 * q, idesc, t + q != 0);
+        }
+      } else {
+        *bad = 1;
+      }
+      tc::mma_commit(o_done);
+    }
+    __syncwarp();
+  }
+  ok = tc::mbar_wait(o_done, 0) && ok;
+  ok = __all_sync(0xffffffffu, ok);
+  tc::fence_after_sync();
+  {
+    float o[32];
+    tmem_ld32(lane_base + static_cast<uint32_t>(wg * 32), o);
+    const int q_row = qi * kBlk + row;
+    const float l = s_sum[row] + s_sum[128 + row], inv = 1.f / l;
+    if (q_row < a.S && ok && *bad == 0) {
+      __nv_bfloat16* orow = a.o_out + ((static_cast<size_t>(b) * a.S + q_row) * a.H + h) * a.hd + wg * 32;
+#pragma unroll
+      for (int c8 = 0; c8 < 4; ++c8) {
+        if (wg * 32 + c8 * 8 < a.hd) {
+          uint4 pk;
+          __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
+#pragma unroll
+          for (int e2 = 0; e2 < 4; ++e2) hp[e2] = __floats2bfloat162_rn(o[c8 * 8 + 2 * e2] * inv, o[c8 * 8 + 2 * e2 + 1] * inv);
+          reinterpret_cast<uint4*>(orow)[c8] = pk;
+        }
+      }
+      if (wg == 0) a.lse[(static_cast<size_t>(b) * a.H + h) * a.S + q_row] = m + log2f(l);
+    }
+  }
+  if ((!ok || *bad) && tid == 0) {
+    atomicExch(a.err, 11);
+    tc::mbar_wait(qk_full, 0, 1u << 20);   // loads that were issued must land before the CTA retires
+    tc::mbar_wait(v_full, 0, 1u << 20);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, 256);
+  }
+}
+
+constexpr int kFwdSmem = 6 * kTile + 2048 + 64 + 1024;   // 99 KiB: two CTAs per SM
+
+// ------------------------------------------------ backward, up to 256 keys --
+// Sum of each of 32 per-lane values over the warp's lanes, by halving: lane l returns column l.
+__device__ __forceinline__ float column_sum32(float (&v)[32], int lane) {
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+#pragma unroll
+    for (int q = 0; q < o; ++q) {
+      const float lo = v[q], hi = v[q + o];
+      const float other = __shfl_xor_sync(0xffffffffu, (lane & o) ? lo : hi, o);
+      v[q] = ((lane & o) ? hi : lo) + other;
+    }
+  }
+  return v[0];
+}
+
+// Tensor memory, 512 columns: [0,128) S  [128,256) dP  [256,384) dQ_0, dQ_1  [384,448) dK_j  [448,512) dV_j
+__global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv,
+                                                          const __grid_constant__ CUtensorMap tm_do, AttnArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* sQ = smem;                 // [2] tiles each
+  uint8_t* sK = sQ + 2 * kTile;
+  uint8_t* sV = sK + 2 * kTile;
+  uint8_t* sDO = sV + 2 * kTile;
+  uint8_t* sP = sDO + 2 * kTile;      // two [128 x 64] sub-tiles each
+  uint8_t* sDS = sP + 2 * kTile;
+  float* s_delta = reinterpret_cast<float*>(sDS + 2 * kTile);   // [256]
+  float* s_lse = s_delta + 256;                                 // [256]
+  uint64_t* in_full = reinterpret_cast<uint64_t*>(s_lse + 256);   // [2]: one per block
+  uint64_t* s_done = in_full + 2;
+  uint64_t* g_done = s_done + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(g_done + 1);
+  volatile int* bad = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  pdl_trigger();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nblk = (a.S + kBlk - 1) / kBlk;   // 1 or 2
   const int h = blockIdx.x, b = blockIdx.y;
-  const int HD = a.H * kHd;
-  if (tid == 0) {
-    tc::mbar_init(in_full, 1);
-    tc::mbar_init(mma_bar, 1);
+  if (warp == 0 && tc::elect_one()) {
+    tc::mbar_init(&in_full[0], 1);
+    tc::mbar_init(&in_full[1], 1);
+    tc::mbar_init(s_done, 1);
+    tc::mbar_init(g_done, 1);
     *bad = 0;
     tc::mbar_init_fence();
     tc::tma_prefetch_desc(&tm_qkv);
     tc::tma_prefetch_desc(&tm_do);
+    pdl_wait();
+    for (int i = nblk - 1; i >= 0; --i) {   // the last block first: its pair is the first one computed
+      tc::mbar_expect_tx(&in_full[i], 4 * kTile);
+      load_tile(sQ + i * kTile, &tm_qkv, &in_full[i], h, i * kBlk, b);
+      load_tile(sK + i * kTile, &tm_qkv, &in_full[i], a.H + h, i * kBlk, b);
+      load_tile(sDO + i * kTile, &tm_do, &in_full[i], h, i * kBlk, b);
+      load_tile(sV + i * kTile, &tm_qkv, &in_full[i], 2 * a.H + h, i * kBlk, b);
+    }
   }
-  if (warp == 0) tc::tmem_alloc(tmem_slot, 512);
+  __syncwarp();
+  if (warp == 1) tc::tmem_alloc(tmem_slot, 512);
+  pdl_wait();
+  {
+    // delta[row] = sum_d dO[row, d] * O[row, d] and the row's log-sum-exp.  Rows past the sequence get an infinite one: P = 0.
+    float acc = 0.f, l = INFINITY;
+    if (tid < a.S) {
+      const size_t r = (static_cast<size_t>(b) * a.S + tid) * a.H + h;
+      const uint4* po = reinterpret_cast<const uint4*>(a.o + r * a.hd);
+      const uint4* pd = reinterpret_cast<const uint4*>(a.d_o + r * a.hd);
+#pragma unroll
+      for (int c = 0; c < kHd / 8; ++c) {
+        if (c * 8 < a.hd) {
+          const uint4 vo = __ldg(po + c), vd = __ldg(pd + c);
+          const __nv_bfloat162* ho = reinterpret_cast<const __nv_bfloat162*>(&vo);
+          const __nv_bfloat162* hd = reinterpret_cast<const __nv_bfloat162*>(&vd);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 x = __bfloat1622float2(ho[e]), y = __bfloat1622float2(hd[e]);
+            acc += x.x * y.x + x.y * y.y;
+          }
+        }
+      }
+      l = a.lse[(static_cast<size_t>(b) * a.H + h) * a.S + tid];
+    }
+    s_delta[tid] = acc;
+    s_lse[tid] = l;
+  }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem0 = *tmem_slot;
-  const uint32_t tm_dq = tmem0, tm_dk = tmem0 + 128, tm_dv = tmem0 + 256, tm_sc = tmem0 + 384;
-  const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-  pdl_wait();
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tm_dq = tmem + 256, tm_dk = tmem + 384, tm_dv = tmem + 448;
+  const int wg = warp >> 2, row = (warp & 3) * 32 + lane;
+  const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
 
-  const int row0 = b * a.S;
-  if (tid == 0) {
-    tc::mbar_expect_tx(in_full, static_cast<uint32_t>(4 * nblk * kTile));
-    for (int i = 0; i < nblk; ++i) {
-      tc::tma_load_2d(sQ + i * kTile, &tm_qkv, in_full, h * kHd, row0 + i * kBlk);
-      tc::tma_load_2d(sK + i * kTile, &tm_qkv, in_full, HD + h * kHd, row0 + i * kBlk);
-      tc::tma_load_2d(sV + i * kTile, &tm_qkv, in_full, 2 * HD + h * kHd, row0 + i * kBlk);
-      tc::tma_load_2d(sDO + i * kTile, &tm_do, in_full, h * kHd, row0 + i * kBlk);
-    }
-  }
-  // delta_i[row] = sum_d dO[row, d] * O[row, d] and the row's log-sum-exp, one row per thread and block
-  float delta[2] = {0.f, 0.f}, lse[2] = {0.f, 0.f};
-  for (int i = 0; i < nblk; ++i) {
-    const size_t r = static_cast<size_t>(row0 + i * kBlk + tid);
-    const uint4* po = reinterpret_cast<const uint4*>(a.o + (r * a.H + h) * kHd);
-    const uint4* pd = reinterpret_cast<const uint4*>(a.d_o + (r * a.H + h) * kHd);
-    float acc = 0.f;
-#pragma unroll
-    for (int c = 0; c < kHd / 8; ++c) {
-      const uint4 vo = po[c], vd = pd[c];
-      const __nv_bfloat162* ho = reinterpret_cast<const __nv_bfloat162*>(&vo);
-      const __nv_bfloat162* hd = reinterpret_cast<const __nv_bfloat162*>(&vd);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 x = __bfloat1622float2(ho[e]), y = __bfloat1622float2(hd[e]);
-        acc += x.x * y.x + x.y * y.y;
-      }
-    }
-    delta[i] = acc;
-    lse[i] = a.lse[(static_cast<size_t>(b) * a.H + h) * a.S + i * kBlk + tid];
-  }
-
-  uint32_t mma_phase = 0;
-  bool ok = true;
-  auto wait_mma = [&]() -> bool {
-    bool w = tc::mbar_wait(mma_bar, mma_phase) && *bad == 0;
-    mma_phase ^= 1u;
-    tc::fence_after_sync();
-    return __syncthreads_and(w ? 1 : 0) != 0;
-  };
   constexpr uint32_t idesc_qk = tc::idesc_bf16(kBlk, kBlk, false, false);    // S, dP: both operands K-major
   constexpr uint32_t idesc_tt = tc::idesc_bf16(kBlk, kHd, true, true);       // dV, dK: A transposed (MN-major), B MN-major
   constexpr uint32_t idesc_nt = tc::idesc_bf16(kBlk, kHd, false, true);      // dQ: A K-major, B MN-major
-
-  bool first = true;
-  for (int i = 0; i < nblk && ok; ++i) {
-    for (int j = 0; j <= i && ok; ++j) {
-      const bool diag = i == j;
-      // ---- S = Q_i K_j^T
-      if (tid == 0) {
-        bool w = true;
-        if (first) w = tc::mbar_wait(in_full, 0);
-        if (!w) *bad = 1;
-        tc::fence_after_sync();
-        if (w) {
-          const uint64_t da = tc::smem_desc_k_sw128(sQ + i * kTile), db = tc::smem_desc_k_sw128(sK + j * kTile);
+  // pairs in order: (1,1), (1,0), (0,0) for two blocks, (0,0) for one
+  const int pairs = nblk == 2 ? 3 : 1;
+  auto pair_i = [&](int p) { return nblk == 2 && p < 2 ? 1 : 0; };
+  auto pair_j = [&](int p) { return nblk == 2 && p < 1 ? 1 : 0; };
+  auto issue_scores = [&](int i, int j) {   // elected thread of warp 0
+    const uint64_t dq = tc::smem_desc_k_sw128(sQ + i * kTile), dk = tc::smem_desc_k_sw128(sK + j * kTile);
 #pragma unroll
-          for (int k4 = 0; k4 < kHd / UMMA_K; ++k4) tc::mma_bf16(tm_sc, da + 2 * k4, db + 2 * k4, idesc_qk, k4 != 0);
-        }
-        tc::mma_commit(mma_bar);   // completes after every earlier product too: P and dS may be overwritten below
-      }
-      first = false;
-      if (!wait_mma()) {
-        ok = false;
-        break;
-      }
-      // ---- P = exp2(S c - L_i), written as bf16 for the products that follow
-#pragma unroll 1
-      for (int c0 = 0; c0 < kBlk; c0 += 32) {
-        float s[32];
-        tmem_ld32(tm_sc + lane_base + static_cast<uint32_t>(c0), s);
-        uint8_t* sub = sP + (c0 >> 6) * kTile;
+    for (int k4 = 0; k4 < kHd / UMMA_K; ++k4) tc::mma_bf16(tmem, dq + 2 * k4, dk + 2 * k4, idesc_qk, k4 != 0);
+    const uint64_t dd = tc::smem_desc_k_sw128(sDO + i * kTile), dv = tc::smem_desc_k_sw128(sV + j * kTile);
 #pragma unroll
-        for (int c8 = 0; c8 < 4; ++c8) {
+    for (int k4 = 0; k4 < kHd / UMMA_K; ++k4) tc::mma_bf16(tmem + 128, dd + 2 * k4, dv + 2 * k4, idesc_qk, k4 != 0);
+    tc::mma_commit(s_done);
+  };
+  // one row of 32 gradient columns [c0, c0 + 32) of part t (0: dQ, 1: dK, 2: dV), block blk, out of tensor memory
+  auto write_out = [&](uint32_t taddr, int t, int blk, int c0) {
+    float v[32];
+    tmem_ld32(taddr + lane_base + static_cast<uint32_t>(c0), v);
+    const int r = blk * kBlk + row;
+    if (r < a.S) {
+      uint4* grow = reinterpret_cast<uint4*>(a.dqkv + (((static_cast<size_t>(b) * a.S + r) * 3 + t) * a.H + h) * a.hd + c0);
+#pragma unroll
+      for (int c8 = 0; c8 < 4; ++c8) {
+        if (c0 + c8 * 8 < a.hd) {
           uint4 pk;
           __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
-          for (int e2 = 0; e2 < 4; ++e2) {
-            float p[2];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const int e = c8 * 8 + e2 * 2 + q;
-              const bool masked = diag && (c0 + e > tid);
-              p[q] = masked ? 0.f : exp2f(s[e] * a.scale_log2 - lse[i]);
-            }
-            hp[e2] = __floats2bfloat162_rn(p[0], p[1]);
-          }
-          *reinterpret_cast<uint4*>(sub + sw128_offset(tid, ((c0 & 63) >> 3) + c8)) = pk;
+          for (int e2 = 0; e2 < 4; ++e2) hp[e2] = __floats2bfloat162_rn(v[c8 * 8 + 2 * e2], v[c8 * 8 + 2 * e2 + 1]);
+          grow[c8] = pk;
         }
-      }
-      fence_async_smem();
-      tc::fence_before_sync();
-      __syncthreads();   // P is complete, and nobody reads the scratch columns any more
-      // ---- dP = dO_i V_j^T into the scratch columns; dV_j += P^T dO_i
-      if (tid == 0) {
-        tc::fence_after_sync();
-        const uint64_t da = tc::smem_desc_k_sw128(sDO + i * kTile), db = tc::smem_desc_k_sw128(sV + j * kTile);
-#pragma unroll
-        for (int k4 = 0; k4 < kHd / UMMA_K; ++k4) tc::mma_bf16(tm_sc, da + 2 * k4, db + 2 * k4, idesc_qk, k4 != 0);
-        const uint64_t dpt = tc::smem_desc_mn_sw128(sP, kTile), ddo = tc::smem_desc_mn_sw128(sDO + i * kTile, kTile);
-#pragma unroll
-        for (int kk = 0; kk < kBlk / UMMA_K; ++kk)
-          tc::mma_bf16(tm_dv + static_cast<uint32_t>(j * kHd), dpt + 128 * kk, ddo + 128 * kk, idesc_tt, (kk != 0) || !diag);
-        tc::mma_commit(mma_bar);
-      }
-      if (!wait_mma()) {
-        ok = false;
-        break;
-      }
-      // ---- dS = P (dP - delta_i) c
-#pragma unroll 1
-      for (int c0 = 0; c0 < kBlk; c0 += 32) {
-        float dp[32];
-        tmem_ld32(tm_sc + lane_base + static_cast<uint32_t>(c0), dp);
-        const uint8_t* psub = sP + (c0 >> 6) * kTile;
-        uint8_t* dsub = sDS + (c0 >> 6) * kTile;
-#pragma unroll
-        for (int c8 = 0; c8 < 4; ++c8) {
-          const uint32_t off = sw128_offset(tid, ((c0 & 63) >> 3) + c8);
-          const uint4 pv = *reinterpret_cast<const uint4*>(psub + off);
-          const __nv_bfloat162* hp = reinterpret_cast<const __nv_bfloat162*>(&pv);
-          uint4 pk;
-          __nv_bfloat162* hs = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-          for (int e2 = 0; e2 < 4; ++e2) {
-            const float2 p = __bfloat1622float2(hp[e2]);
-            const int e = c8 * 8 + e2 * 2;
-            hs[e2] = __floats2bfloat162_rn(p.x * (dp[e] - delta[i]) * a.scale, p.y * (dp[e + 1] - delta[i]) * a.scale);
-          }
-          *reinterpret_cast<uint4*>(dsub + off) = pk;
-        }
-      }
-      fence_async_smem();
-      tc::fence_before_sync();
-      __syncthreads();
-      // ---- dK_j += dS^T Q_i ; dQ_i += dS K_j
-      if (tid == 0) {
-        tc::fence_after_sync();
-        const uint64_t dst = tc::smem_desc_mn_sw128(sDS, kTile), dq = tc::smem_desc_mn_sw128(sQ + i * kTile, kTile);
-#pragma unroll
-        for (int kk = 0; kk < kBlk / UMMA_K; ++kk)
-          tc::mma_bf16(tm_dk + static_cast<uint32_t>(j * kHd), dst + 128 * kk, dq + 128 * kk, idesc_tt, (kk != 0) || !diag);
-        const uint64_t dk = tc::smem_desc_mn_sw128(sK + j * kTile, kTile);
-#pragma unroll
-        for (int kk = 0; kk < kBlk / UMMA_K; ++kk) {
-          const uint64_t dsn = tc::smem_desc_k_sw128(sDS + (kk >> 2) * kTile) + 2 * (kk & 3);
-          tc::mma_bf16(tm_dq + static_cast<uint32_t>(i * kHd), dsn, dk + 128 * kk, idesc_nt, (kk != 0) || (j != 0));
-        }
-        // no commit here: the next block pair's first commit (or the final one) covers these products
       }
     }
-  }
-  if (tid == 0) tc::mma_commit(mma_bar);
-  ok = wait_mma() && ok;
+    if (a.colsum != nullptr && c0 < a.hd) {   // rows past the sequence are zero
+      const float sum = column_sum32(v, lane);
+      if (c0 + lane < a.hd) atomicAdd(a.colsum + (t * a.H + h) * a.hd + c0 + lane, sum);
+    }
+  };
 
-  if (ok) {
-    // gradients out of tensor memory, one row per thread, straight into the [B, S, 3, H, 64] gradient of qkv
-    for (int t = 0; t < 3; ++t) {          // 0: dQ, 1: dK, 2: dV
-      const uint32_t base = t == 0 ? tm_dq : (t == 1 ? tm_dk : tm_dv);
-      for (int i = 0; i < nblk; ++i) {
-        __nv_bfloat16* grow = a.dqkv + ((static_cast<size_t>(row0 + i * kBlk + tid) * 3 + t) * a.H + h) * kHd;
+  if (warp == 0) {
+    bool w = tc::mbar_wait(&in_full[nblk - 1], 0);
+    w = __all_sync(0xffffffffu, w);
+    tc::fence_after_sync();
+    if (tc::elect_one()) {
+      if (!w) *bad = 1;
+      issue_scores(nblk - 1, nblk - 1);
+    }
+    __syncwarp();
+  }
+  bool ok = true;
+#pragma unroll 1
+  for (int p = 0; p < pairs; ++p) {
+    const int i = pair_i(p), j = pair_j(p);
+    ok = tc::mbar_wait(s_done, p & 1);
+    if (!__syncthreads_and((ok && *bad == 0) ? 1 : 0)) {
+      ok = false;
+      break;
+    }
+    tc::fence_after_sync();
+    const float lse = s_lse[i * kBlk + row], delta = s_delta[i * kBlk + row];
+    const int limit = i == j ? row : kBlk;   // keys after the query are masked
+#pragma unroll 1
+    for (int c0 = wg * 64; c0 < wg * 64 + 64; c0 += 32) {
+      uint32_t rs[32], rd[32];
+      tc::tmem_ld_32x32(tmem + lane_base + static_cast<uint32_t>(c0), rs);
+      tc::tmem_ld_32x32(tmem + lane_base + static_cast<uint32_t>(128 + c0), rd);
+      tc::tmem_ld_wait();
+      const int sub = wg * kTile;
 #pragma unroll
-        for (int c0 = 0; c0 < kHd; c0 += 32) {
-          float v[32];
-          tmem_ld32(base + static_cast<uint32_t>(i * kHd) + lane_base + static_cast<uint32_t>(c0), v);
+      for (int c8 = 0; c8 < 4; ++c8) {
+        uint4 pk, dk;
+        __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
+        __nv_bfloat162* hs = reinterpret_cast<__nv_bfloat162*>(&dk);
 #pragma unroll
-          for (int c8 = 0; c8 < 4; ++c8) {
-            uint4 pk;
-            __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-            for (int e2 = 0; e2 < 4; ++e2) hp[e2] = __floats2bfloat162_rn(v[c8 * 8 + 2 * e2], v[c8 * 8 + 2 * e2 + 1]);
-            reinterpret_cast<uint4*>(grow)[(c0 >> 3) + c8] = pk;
-          }
+        for (int e2 = 0; e2 < 4; ++e2) {
+          const int e = c8 * 8 + e2 * 2;
+          const float p0 = c0 + e <= limit ? exp2f(__uint_as_float(rs[e]) * a.scale_log2 - lse) : 0.f;
+          const float p1 = c0 + e + 1 <= limit ? exp2f(__uint_as_float(rs[e + 1]) * a.scale_log2 - lse) : 0.f;
+          hp[e2] = __floats2bfloat162_rn(p0, p1);
+          const float2 pr = __bfloat1622float2(hp[e2]);
+          hs[e2] = __floats2bfloat162_rn(pr.x * (__uint_as_float(rd[e]) - delta) * a.scale,
+                                         pr.y * (__uint_as_float(rd[e + 1]) - delta) * a.scale);
         }
+        const uint32_t off = sw128_offset(row, ((c0 & 63) >> 3) + c8);
+        *reinterpret_cast<uint4*>(sP + sub + off) = pk;
+        *reinterpret_cast<uint4*>(sDS + sub + off) = dk;
       }
+    }
+    fence_async_smem();
+    tc::fence_before_sync();
+    __syncthreads();   // P and dS are complete, and nobody reads the score columns any more
+    if (warp == 0) {
+      bool w = true;
+      if (p + 1 < pairs && p == 0) w = tc::mbar_wait(&in_full[0], 0);   // the second pair is the first to need block 0
+      w = __all_sync(0xffffffffu, w);
+      tc::fence_after_sync();
+      if (tc::elect_one()) {
+        if (!w) *bad = 1;
+        if (p + 1 < pairs) issue_scores(pair_i(p + 1), pair_j(p + 1));
+        const uint64_t dpt = tc::smem_desc_mn_sw128(sP, kTile), dst = tc::smem_desc_mn_sw128(sDS, kTile);
+        const uint64_t ddo = tc::smem_desc_mn_sw128(sDO + i * kTile, kTile), dq = tc::smem_desc_mn_sw128(sQ + i * kTile, kTile);
+        const uint64_t dk = tc::smem_desc_mn_sw128(sK + j * kTile, kTile), dsn = tc::smem_desc_k_sw128(sDS);
+        const bool add_kv = p == 2;                   // dK_0, dV_0: pairs (1,0), (0,0)
+        const bool add_q = p == 1;                    // dQ_1: pairs (1,1), (1,0)
+#pragma unroll
+        for (int kk = 0; kk < kBlk / UMMA_K; ++kk) tc::mma_bf16(tm_dv, dpt + 128 * kk, ddo + 128 * kk, idesc_tt, kk != 0 || add_kv);
+#pragma unroll
+        for (int kk = 0; kk < kBlk / UMMA_K; ++kk) tc::mma_bf16(tm_dk, dst + 128 * kk, dq + 128 * kk, idesc_tt, kk != 0 || add_kv);
+#pragma unroll
+        for (int kk = 0; kk < kBlk / UMMA_K; ++kk)
+          tc::mma_bf16(tm_dq + static_cast<uint32_t>(i * kHd), dsn + (kk >> 2) * (kTile >> 4) + 2 * (kk & 3), dk + 128 * kk, idesc_nt, kk != 0 || add_q);
+        tc::mma_commit(g_done);
+      }
+      __syncwarp();
+    }
+    ok = tc::mbar_wait(g_done, p & 1);   // P and dS may be overwritten, this pair's gradients are in tensor memory
+    ok = __all_sync(0xffffffffu, ok);
+    tc::fence_after_sync();
+    if (ok && *bad == 0 && (p + 1 == pairs || pair_j(p + 1) != j)) {   // last pair of this key block: its dK and dV leave
+      write_out(wg == 0 ? tm_dk : tm_dv, 1 + wg, j, 0);
+      write_out(wg == 0 ? tm_dk : tm_dv, 1 + wg, j, 32);
+      tc::fence_before_sync();
+    }
+  }
+  if (ok && *bad == 0) {
+    if (nblk == 2) {
+      write_out(tm_dq + static_cast<uint32_t>(wg * kHd), 0, wg, 0);
+      write_out(tm_dq + static_cast<uint32_t>(wg * kHd), 0, wg, 32);
+    } else {
+      write_out(tm_dq, 0, 0, wg * 32);
     }
   } else if (tid == 0) {
     atomicExch(a.err, 12);
-    tc::mbar_wait(in_full, 0, 1u << 20);   // the loads that were issued must land before the CTA retires
+    for (int i = 0; i < nblk; ++i) tc::mbar_wait(&in_full[i], 0, 1u << 20);   // issued loads must land before the CTA retires
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) {
+  if (warp == 1) {
     tc::fence_after_sync();
-    tc::tmem_dealloc(tmem0, 512);
+    tc::tmem_dealloc(tmem, 512);
   }
 }
 
-constexpr int kBwdSmem = 12 * kTile + 64 + 1024;   // 193 KiB
+constexpr int kBwdSmem = 12 * kTile + 2048 + 64 + 1024;   // 195 KiB
+
+// [B, S, slots, hd] with contiguous hd as boxes of 128 rows x 64 columns of one (batch, slot).
+bool encode_slots(CUtensorMap* map, const void* base, int B, int S, int slots, int hd) {
+  const CuDriver& cu = CuDriver::get();
+  if (!cu.loaded || !cu.TensorMapEncodeTiled) return false;
+  int device = 0;
+  cudaGetDevice(&device);
+  cu.ensure_context(device);
+  const cuuint64_t row = static_cast<cuuint64_t>(slots) * hd * 2;
+  cuuint64_t dims[4] = {static_cast<cuuint64_t>(hd), static_cast<cuuint64_t>(slots), static_cast<cuuint64_t>(S), static_cast<cuuint64_t>(B)};
+  cuuint64_t strides[3] = {static_cast<cuuint64_t>(hd) * 2, row, row * S};
+  cuuint32_t box[4] = {kHd, 1, kBlk, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return cu.TensorMapEncodeTiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <typename K>
+cudaError_t allow_smem(K kernel, int bytes, std::atomic<bool>& done) {
+  if (done.load(std::memory_order_acquire)) return cudaSuccess;
+  cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (rc == cudaSuccess) done.store(true, std::memory_order_release);
+  return rc;
+}
 
 }  // namespace
 
+bool attention_supported(int S, int hd) { return S >= 1 && S <= 2 * kBlk && hd >= 8 && hd <= kHd && hd % 8 == 0; }
+
 cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, const __nv_bfloat16* d_o, const float* lse,
-                          __nv_bfloat16* dqkv, int B, int S, int H, float softmax_scale, cudaStream_t stream) {
-  if ((S != kBlk && S != 2 * kBlk) || B <= 0 || H <= 0) return cudaErrorNotSupported;
+                          __nv_bfloat16* dqkv, float* colsum, int B, int S, int H, int hd, float softmax_scale, cudaStream_t stream) {
+  if (!attention_supported(S, hd) || B <= 0 || H <= 0) return cudaErrorNotSupported;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o) |
        reinterpret_cast<uintptr_t>(dqkv)) & 15u)
     return cudaErrorNotSupported;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t rc = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
-    if (rc != cudaSuccess) return rc;
-    configured = true;
-  }
+  static std::atomic<bool> configured{false};
+  cudaError_t rc = allow_smem(attn_bwd_kernel, kBwdSmem, configured);
+  if (rc != cudaSuccess) return rc;
   CUtensorMap tq, tdo;
-  if (!encode_map(&tq, qkv, B * S, 3 * H * kHd, 3 * H * kHd, kBlk)) return cudaErrorNotSupported;
-  if (!encode_map(&tdo, d_o, B * S, H * kHd, H * kHd, kBlk)) return cudaErrorNotSupported;
+  if (!encode_slots(&tq, qkv, B, S, 3 * H, hd) || !encode_slots(&tdo, d_o, B, S, H, hd)) return cudaErrorNotSupported;
   (void)cudaGetLastError();
-  AttnBwdDev a;
+  AttnArgs a = {};
   a.o = o;
   a.d_o = d_o;
-  a.lse = lse;
+  a.lse = const_cast<float*>(lse);
   a.dqkv = dqkv;
+  a.colsum = colsum;
   a.S = S;
   a.H = H;
+  a.hd = hd;
   a.scale = softmax_scale;
   a.scale_log2 = softmax_scale * 1.4426950408889634f;
   a.err = gemm_error_device_ptr();
   if (!a.err) return cudaErrorNotSupported;
-  MCCL_LAUNCH_PDL(attn_bwd_kernel, dim3(H, B), 128, kBwdSmem, stream, tq, tdo, a);
+  MCCL_LAUNCH_PDL(attn_bwd_kernel, dim3(H, B), 256, kBwdSmem, stream, tq, tdo, a);
   count_launch();
   return launch_status();
 }
 
-cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse, int B, int S, int H, float softmax_scale,
+cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse, int B, int S, int H, int hd, float softmax_scale,
                           cudaStream_t stream) {
-  if (S % kBlk != 0 || S <= 0 || B <= 0 || H <= 0) return cudaErrorNotSupported;
+  if (B <= 0 || H <= 0) return cudaErrorNotSupported;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(o)) & 15u) return cudaErrorNotSupported;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t rc = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
-    if (rc != cudaSuccess) return rc;
-    configured = true;
-  }
+  const float scale_log2 = softmax_scale * 1.4426950408889634f;
+  int* err = gemm_error_device_ptr();
+  if (!err) return cudaErrorNotSupported;
   CUtensorMap tm;
-  if (!encode_map(&tm, qkv, B * S, 3 * H * kHd, 3 * H * kHd, kBlk)) return cudaErrorNotSupported;
   (void)cudaGetLastError();
-  AttnDev a;
-  a.o = o;
-  a.lse = lse;
-  a.S = S;
-  a.H = H;
-  a.scale_log2 = softmax_scale * 1.4426950408889634f;
-  a.err = gemm_error_device_ptr();
-  if (!a.err) return cudaErrorNotSupported;
-  MCCL_LAUNCH_PDL(attn_fwd_kernel, dim3(S / kBlk, H, B), 128, kFwdSmem, stream, tm, a);
+  if (attention_supported(S, hd)) {
+    static std::atomic<bool> configured{false};
+    cudaError_t rc = allow_smem(attn_fwd_kernel, kFwdSmem, configured);
+    if (rc != cudaSuccess) return rc;
+    if (!encode_slots(&tm, qkv, B, S, 3 * H, hd)) return cudaErrorNotSupported;
+    AttnArgs a = {};
+    a.o_out = o;
+    a.lse = lse;
+    a.S = S;
+    a.H = H;
+    a.hd = hd;
+    a.scale = softmax_scale;
+    a.scale_log2 = scale_log2;
+    a.err = err;
+    MCCL_LAUNCH_PDL(attn_fwd_kernel, dim3((S + kBlk - 1) / kBlk, H, B), 256, kFwdSmem, stream, tm, a);
+  } else {
+    if (hd != kHd || S <= 0 || S % kBlk != 0) return cudaErrorNotSupported;
+    static std::atomic<bool> configured{false};
+    cudaError_t rc = allow_smem(attn_fwd_long_kernel, kLongSmem, configured);
+    if (rc != cudaSuccess) return rc;
+    if (!encode_map(&tm, qkv, B * S, 3 * H * kHd, 3 * H * kHd, kBlk)) return cudaErrorNotSupported;
+    AttnDev a;
+    a.o = o;
+    a.lse = lse;
+    a.S = S;
+    a.H = H;
+    a.scale_log2 = scale_log2;
+    a.err = err;
+    MCCL_LAUNCH_PDL(attn_fwd_long_kernel, dim3(S / kBlk, H, B), 128, kLongSmem, stream, tm, a);
+  }
   count_launch();
   return launch_status();
 }

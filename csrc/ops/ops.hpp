@@ -65,14 +65,16 @@ cudaError_t embed_fwd(const long long* ids, const float* tok, const float* pos, 
 cudaError_t embed_bwd(const long long* ids, const __nv_bfloat16* dy, float* dtok, float* dpos, int tokens, int seq, int dim,
                       int vocab, cudaStream_t stream, float scale = 1.f);
 
-// ---- causal self-attention, head dimension 64, straight from the fused QKV projection.
-// qkv: [B, S, 3, H, 64] bf16; o: [B, S, H, 64] bf16; lse: [B, H, S] fp32 (log2 domain, saved for backward).
-// Forward needs S % 128 == 0; backward S == 128 or 256 (cudaErrorNotSupported otherwise: the caller falls back).
-cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse, int B, int S, int H, float softmax_scale,
+// ---- causal self-attention straight from the fused QKV projection.
+// qkv: [B, S, 3, H, hd] bf16; o: [B, S, H, hd]; lse: [B, H, S] fp32 (log2 domain, saved for backward).
+// Both ways: S <= 256 and hd <= 64 (a multiple of 8); forward also head dimension 64 with S a multiple of 128.
+// cudaErrorNotSupported otherwise: the caller falls back.
+bool attention_supported(int S, int hd);
+cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse, int B, int S, int H, int hd, float softmax_scale,
                           cudaStream_t stream);
-// dqkv: [B, S, 3, H, 64] bf16, every element written.
+// dqkv: [B, S, 3, H, hd] bf16, every element written.  colsum (optional, fp32 [3 * H * hd]): its column sums are added here.
 cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, const __nv_bfloat16* d_o, const float* lse,
-                          __nv_bfloat16* dqkv, int B, int S, int H, float softmax_scale, cudaStream_t stream);
+                          __nv_bfloat16* dqkv, float* colsum, int B, int S, int H, int hd, float softmax_scale, cudaStream_t stream);
 
 // ---- rotary embedding of the fused QKV projection's output (pairs of even and odd elements; cos / sin: fp32
 // [>= seq, head_dim / 2]; token t has position t % seq).  qkv [tokens, 3, H, hd] -> qk [tokens, 2, H, hd].

@@ -167,7 +167,7 @@ class Block(nn.Module):
         qkv = self.qkv(h, native)
         if native and rope is None:
             from .. import ops
-            a = ops.causal_attention(qkv, cfg.n_heads)   # own kernels for head dimension 64, S in {128, 256}
+            a = ops.causal_attention(qkv, cfg.n_heads)   # own kernels for S <= 256, head dimension <= 64
         elif native:
             from .. import ops
             a = ops.rope_attention(qkv, cfg.n_heads, *rope)

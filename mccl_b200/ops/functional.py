@@ -54,13 +54,13 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias=None, act: str = "none", 
 
 
 def native_attention_supported(seq: int, head_dim: int) -> bool:
-    """Shapes the attention kernels cover: head dimension 64, sequences of 128 or 256 (training needs backward)."""
-    return bool(_HAS.get("attn_fwd")) and head_dim == 64 and seq in (128, 256) and os.environ.get("MCCL_NATIVE_ATTN", "1") != "0"
+    """Shapes the attention kernels cover: sequences of up to 256, head dimensions of up to 64 (multiples of 8)."""
+    return bool(_HAS.get("attn_fwd")) and _C.attention_supported(seq, head_dim) and os.environ.get("MCCL_NATIVE_ATTN", "1") != "0"
 
 
 def causal_attention(qkv: torch.Tensor, n_heads: int) -> torch.Tensor:
     """Causal self-attention.  qkv: [B, S, 3 * n_heads * head_dim] (or already [B, S, 3, H, Dh]), the output of a
-    fused QKV projection; returns [B, S, n_heads * head_dim].  On CUDA with head dimension 64 and S in {128, 256}
+    fused QKV projection; returns [B, S, n_heads * head_dim].  On CUDA with S <= 256 and a head dimension of up to 64
     this is one kernel each way; otherwise PyTorch's scaled_dot_product_attention on views of the same tensor."""
     B, S = qkv.shape[0], qkv.shape[1]
     hd = qkv.numel() // (B * S * 3 * n_heads)
