@@ -265,11 +265,7 @@ constexpr int kLongSmem = 6 * kTile + 64 + 1024;   // 97 KiB: two CTAs per SM
 
 // ------------------------------------------------- forward, up to 256 keys --
 struct AttnArgs {
-  const __nv_bfloat16* o;     // [B, S, H, hd]: backward reads it, forward writes through o_out
-  const __nv_bfloat16* d_o;   // [B, S, H, hd]
-  __nv_bfloat16* o_out;
   float* lse;                 // [B, H, S], log2 domain: m + log2(l)
-  __nv_bfloat16* dqkv;        // [B, S, 3, H, hd]
   float* colsum;              // optional: column sums of dqkv are added here, fp32 [3 * H * hd]
   int S, H, hd;
   float scale, scale_log2;
@@ -284,7 +280,18 @@ __device__ __forceinline__ void load_tile(void* dst, const CUtensorMap* map, uin
       : "memory");
 }
 
-__global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, AttnArgs a) {
+// Store of 32 rows x 64 columns of a part from a tile in shared memory (clipped past S and past hd).  A thread that stored
+// its own row touched 32 lines per instruction: 1.6 us for dK and dV of one block, 3.7 us for the rest.
+__device__ __forceinline__ void store_rows32(const CUtensorMap* map, const void* src, int slot, int row, int b) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(src)), "r"(0), "r"(slot), "r"(row), "r"(b)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void stores_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+__global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_o,
+                                                          AttnArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sK = smem;                // 2 tiles
@@ -349,20 +356,27 @@ __global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant_
   tc::fence_after_sync();
 
   const int wg = warp >> 2, row = (warp & 3) * 32 + lane;      // two threads per query row, half of the keys each
-  const int cols = nk >> 1, c_begin = wg * cols, limit = qi * kBlk + row;   // keys after `limit` are masked
+  // Groups of 32 keys before `diag` are seen by all of the warp's queries, those after it by none.
+  const int diag = qi * kBlk + (warp & 3) * 32, cols = nk >> 1, c_begin = wg * cols, c_end = min(c_begin + cols, diag + 32);
   const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
   float mx = -INFINITY;
 #pragma unroll 1
-  for (int c0 = c_begin; c0 < c_begin + cols; c0 += 32) {
-    float s[32];
-    tmem_ld32(lane_base + static_cast<uint32_t>(c0), s);
-    if (c0 + 31 <= limit) {
+  for (int c0 = c_begin; c0 < c_end; c0 += 64) {
+    uint32_t r0[32], r1[32];
+    tc::tmem_ld_32x32(lane_base + static_cast<uint32_t>(c0), r0);
+    tc::tmem_ld_32x32(lane_base + static_cast<uint32_t>(c0 + 32), r1);
+    tc::tmem_ld_wait();
+    auto group_max = [&](const uint32_t (&r)[32], int c) {
+      if (c < diag) {
 #pragma unroll
-      for (int e = 0; e < 32; ++e) mx = fmaxf(mx, s[e]);
-    } else {
+        for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(r[e]));
+      } else if (c == diag) {
 #pragma unroll
-      for (int e = 0; e < 32; ++e) mx = c0 + e <= limit ? fmaxf(mx, s[e]) : mx;
-    }
+        for (int e = 0; e < 32; ++e) mx = e <= lane ? fmaxf(mx, __uint_as_float(r[e])) : mx;
+      }
+    };
+    group_max(r0, c0);
+    group_max(r1, c0 + 32);
   }
   s_max[wg * 128 + row] = mx;
   __syncthreads();
@@ -370,24 +384,33 @@ __global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant_
   float sum = 0.f;
 #pragma unroll 1
   for (int c0 = c_begin; c0 < c_begin + cols; c0 += 32) {
+    uint8_t* sub = sP + (c0 >> 6) * kTile;
+    const int chunk0 = (c0 & 63) >> 3;
+    if (c0 > diag) {
+#pragma unroll
+      for (int c8 = 0; c8 < 4; ++c8) *reinterpret_cast<uint4*>(sub + sw128_offset(row, chunk0 + c8)) = make_uint4(0u, 0u, 0u, 0u);
+      continue;
+    }
     float s[32];
     tmem_ld32(lane_base + static_cast<uint32_t>(c0), s);
-    uint8_t* sub = sP + (c0 >> 6) * kTile;
+#pragma unroll
+    for (int e = 0; e < 32; ++e) s[e] = exp2f(s[e] * a.scale_log2 - m);
+    if (c0 == diag) {
+#pragma unroll
+      for (int e = 0; e < 32; ++e) s[e] = e <= lane ? s[e] : 0.f;
+    }
 #pragma unroll
     for (int c8 = 0; c8 < 4; ++c8) {
       uint4 pk;
       __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
       for (int e2 = 0; e2 < 4; ++e2) {
-        const int e = c8 * 8 + e2 * 2;
-        const float p0 = c0 + e <= limit ? exp2f(s[e] * a.scale_log2 - m) : 0.f;
-        const float p1 = c0 + e + 1 <= limit ? exp2f(s[e + 1] * a.scale_log2 - m) : 0.f;
-        hp[e2] = __floats2bfloat162_rn(p0, p1);
+        hp[e2] = __floats2bfloat162_rn(s[c8 * 8 + e2 * 2], s[c8 * 8 + e2 * 2 + 1]);
         // the sum uses the rounded values: they are what multiplies V
         const float2 back = __bfloat1622float2(hp[e2]);
         sum += back.x + back.y;
       }
-      *reinterpret_cast<uint4*>(sub + sw128_offset(row, ((c0 & 63) >> 3) + c8)) = pk;
+      *reinterpret_cast<uint4*>(sub + sw128_offset(row, chunk0 + c8)) = pk;
     }
   }
   s_sum[wg * 128 + row] = sum;
@@ -422,29 +445,32 @@ __global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant_
     tmem_ld32(lane_base + static_cast<uint32_t>(wg * 32), o);
     const int q_row = qi * kBlk + row;
     const float l = s_sum[row] + s_sum[128 + row], inv = 1.f / l;
-    if (q_row < a.S && ok && *bad == 0) {
-      __nv_bfloat16* orow = a.o_out + ((static_cast<size_t>(b) * a.S + q_row) * a.H + h) * a.hd + wg * 32;
 #pragma unroll
-      for (int c8 = 0; c8 < 4; ++c8) {
-        if (wg * 32 + c8 * 8 < a.hd) {
-          uint4 pk;
-          __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
+    for (int c8 = 0; c8 < 4; ++c8) {   // V has been read: its first tile takes the output on its way to memory
+      uint4 pk;
+      __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
-          for (int e2 = 0; e2 < 4; ++e2) hp[e2] = __floats2bfloat162_rn(o[c8 * 8 + 2 * e2] * inv, o[c8 * 8 + 2 * e2 + 1] * inv);
-          reinterpret_cast<uint4*>(orow)[c8] = pk;
-        }
-      }
-      if (wg == 0) a.lse[(static_cast<size_t>(b) * a.H + h) * a.S + q_row] = m + log2f(l);
+      for (int e2 = 0; e2 < 4; ++e2) hp[e2] = __floats2bfloat162_rn(o[c8 * 8 + 2 * e2] * inv, o[c8 * 8 + 2 * e2 + 1] * inv);
+      *reinterpret_cast<uint4*>(sV + sw128_offset(row, wg * 4 + c8)) = pk;
     }
+    if (wg == 0 && q_row < a.S && ok) a.lse[(static_cast<size_t>(b) * a.H + h) * a.S + q_row] = m + log2f(l);
+  }
+  fence_async_smem();
+  tc::fence_before_sync();
+  __syncthreads();
+  if (ok && *bad == 0 && warp < 4 && qi * kBlk + warp * 32 < a.S) {
+    if (tc::elect_one()) {
+      store_rows32(&tm_o, sV + warp * 4096, h, qi * kBlk + warp * 32, b);
+      stores_read();
+    }
+    __syncwarp();
   }
   if ((!ok || *bad) && tid == 0) {
     atomicExch(a.err, 11);
     tc::mbar_wait(qk_full, 0, 1u << 20);   // loads that were issued must land before the CTA retires
     tc::mbar_wait(v_full, 0, 1u << 20);
   }
-  tc::fence_before_sync();
-  __syncthreads();
-  if (warp == 1) {
+  if (warp == 1) {   // everybody's tensor-memory reads were before the barrier above
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, 256);
   }
@@ -469,7 +495,9 @@ __device__ __forceinline__ float column_sum32(float (&v)[32], int lane) {
 
 // Tensor memory, 512 columns: [0,128) S  [128,256) dP  [256,384) dQ_0, dQ_1  [384,448) dK_j  [448,512) dV_j
 __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv,
-                                                          const __grid_constant__ CUtensorMap tm_do, AttnArgs a) {
+                                                          const __grid_constant__ CUtensorMap tm_do,
+                                                          const __grid_constant__ CUtensorMap tm_o,
+                                                          const __grid_constant__ CUtensorMap tm_dqkv, AttnArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;                 // [2] tiles each
@@ -494,51 +522,29 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
     tc::mbar_init(&in_full[0], 1);
     tc::mbar_init(&in_full[1], 1);
     tc::mbar_init(s_done, 1);
-    tc::mbar_init(g_done, 1);
+    tc::mbar_init(g_done, 2);   // two issuing threads
     *bad = 0;
     tc::mbar_init_fence();
     tc::tma_prefetch_desc(&tm_qkv);
     tc::tma_prefetch_desc(&tm_do);
+    tc::tma_prefetch_desc(&tm_o);
+    tc::tma_prefetch_desc(&tm_dqkv);
     pdl_wait();
     for (int i = nblk - 1; i >= 0; --i) {   // the last block first: its pair is the first one computed
-      tc::mbar_expect_tx(&in_full[i], 4 * kTile);
+      tc::mbar_expect_tx(&in_full[i], 5 * kTile);
       load_tile(sQ + i * kTile, &tm_qkv, &in_full[i], h, i * kBlk, b);
       load_tile(sK + i * kTile, &tm_qkv, &in_full[i], a.H + h, i * kBlk, b);
       load_tile(sDO + i * kTile, &tm_do, &in_full[i], h, i * kBlk, b);
       load_tile(sV + i * kTile, &tm_qkv, &in_full[i], 2 * a.H + h, i * kBlk, b);
+      load_tile(sP + i * kTile, &tm_o, &in_full[i], h, i * kBlk, b);   // the output waits where P will go
     }
   }
   __syncwarp();
   if (warp == 1) tc::tmem_alloc(tmem_slot, 512);
-  pdl_wait();
-  {
-    // delta[row] = sum_d dO[row, d] * O[row, d] and the row's log-sum-exp.  Rows past the sequence get an infinite one: P = 0.
-    float acc = 0.f, l = INFINITY;
-    if (tid < a.S) {
-      const size_t r = (static_cast<size_t>(b) * a.S + tid) * a.H + h;
-      const uint4* po = reinterpret_cast<const uint4*>(a.o + r * a.hd);
-      const uint4* pd = reinterpret_cast<const uint4*>(a.d_o + r * a.hd);
-#pragma unroll
-      for (int c = 0; c < kHd / 8; ++c) {
-        if (c * 8 < a.hd) {
-          const uint4 vo = __ldg(po + c), vd = __ldg(pd + c);
-          const __nv_bfloat162* ho = reinterpret_cast<const __nv_bfloat162*>(&vo);
-          const __nv_bfloat162* hd = reinterpret_cast<const __nv_bfloat162*>(&vd);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 x = __bfloat1622float2(ho[e]), y = __bfloat1622float2(hd[e]);
-            acc += x.x * y.x + x.y * y.y;
-          }
-        }
-      }
-      l = a.lse[(static_cast<size_t>(b) * a.H + h) * a.S + tid];
-    }
-    s_delta[tid] = acc;
-    s_lse[tid] = l;
-  }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  pdl_wait();
   const uint32_t tmem = *tmem_slot;
   const uint32_t tm_dq = tmem + 256, tm_dk = tmem + 384, tm_dv = tmem + 448;
   const int wg = warp >> 2, row = (warp & 3) * 32 + lane;
@@ -560,28 +566,37 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
     for (int k4 = 0; k4 < kHd / UMMA_K; ++k4) tc::mma_bf16(tmem + 128, dd + 2 * k4, dv + 2 * k4, idesc_qk, k4 != 0);
     tc::mma_commit(s_done);
   };
-  // one row of 32 gradient columns [c0, c0 + 32) of part t (0: dQ, 1: dK, 2: dV), block blk, out of tensor memory
-  auto write_out = [&](uint32_t taddr, int t, int blk, int c0) {
+  // one row of 32 gradient columns [c0, c0 + 32) of part t (0: dQ, 1: dK, 2: dV) out of tensor memory into a tile that is
+  // no longer needed; then the warp's 32 rows leave for block blk
+  auto stage_out = [&](uint8_t* tile, uint32_t taddr, int t, int c0) {
     float v[32];
     tmem_ld32(taddr + lane_base + static_cast<uint32_t>(c0), v);
-    const int r = blk * kBlk + row;
-    if (r < a.S) {
-      uint4* grow = reinterpret_cast<uint4*>(a.dqkv + (((static_cast<size_t>(b) * a.S + r) * 3 + t) * a.H + h) * a.hd + c0);
 #pragma unroll
-      for (int c8 = 0; c8 < 4; ++c8) {
-        if (c0 + c8 * 8 < a.hd) {
-          uint4 pk;
-          __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
+    for (int c8 = 0; c8 < 4; ++c8) {
+      uint4 pk;
+      __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
-          for (int e2 = 0; e2 < 4; ++e2) hp[e2] = __floats2bfloat162_rn(v[c8 * 8 + 2 * e2], v[c8 * 8 + 2 * e2 + 1]);
-          grow[c8] = pk;
-        }
-      }
+      for (int e2 = 0; e2 < 4; ++e2) hp[e2] = __floats2bfloat162_rn(v[c8 * 8 + 2 * e2], v[c8 * 8 + 2 * e2 + 1]);
+      *reinterpret_cast<uint4*>(tile + sw128_offset(row, (c0 >> 3) + c8)) = pk;
     }
     if (a.colsum != nullptr && c0 < a.hd) {   // rows past the sequence are zero
       const float sum = column_sum32(v, lane);
       if (c0 + lane < a.hd) atomicAdd(a.colsum + (t * a.H + h) * a.hd + c0 + lane, sum);
     }
+  };
+  auto send_out = [&](const uint8_t* tile, int t, int blk) {
+    fence_async_smem();
+    __syncwarp();
+    const int q = warp & 3;
+    if (blk * kBlk + q * 32 < a.S && tc::elect_one()) store_rows32(&tm_dqkv, tile + q * 4096, t * a.H + h, blk * kBlk + q * 32, b);
+    __syncwarp();
+  };
+  auto key_block_out = [&](int j) {   // one warpgroup takes dK_j, the other dV_j; K_j and V_j have been read for the last time
+    uint8_t* tile = (wg == 0 ? sK : sV) + j * kTile;
+    stage_out(tile, wg == 0 ? tm_dk : tm_dv, 1 + wg, 0);
+    stage_out(tile, wg == 0 ? tm_dk : tm_dv, 1 + wg, 32);
+    tc::fence_before_sync();
+    send_out(tile, 1 + wg, j);
   };
 
   if (warp == 0) {
@@ -595,6 +610,31 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
     __syncwarp();
   }
   bool ok = true;
+  {
+    // delta[row] = sum_d dO[row, d] * O[row, d] and the row's log-sum-exp, one row per thread.  Rows past the sequence get an
+    // infinite one: P = 0.
+    const int blk = tid >> 7, r = tid & 127;
+    float acc = 0.f, l = INFINITY;
+    if (tid < a.S) l = a.lse[(static_cast<size_t>(b) * a.H + h) * a.S + tid];
+    if (blk < nblk) {
+      ok = tc::mbar_wait(&in_full[blk], 0);
+#pragma unroll
+      for (int c = 0; c < kHd / 8; ++c) {
+        const uint4 vo = *reinterpret_cast<const uint4*>(sP + blk * kTile + sw128_offset(r, c));
+        const uint4 vd = *reinterpret_cast<const uint4*>(sDO + blk * kTile + sw128_offset(r, c));
+        const __nv_bfloat162* ho = reinterpret_cast<const __nv_bfloat162*>(&vo);
+        const __nv_bfloat162* hd = reinterpret_cast<const __nv_bfloat162*>(&vd);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 x = __bfloat1622float2(ho[e]), y = __bfloat1622float2(hd[e]);
+          acc += x.x * y.x + x.y * y.y;
+        }
+      }
+    }
+    s_delta[tid] = acc;
+    s_lse[tid] = l;
+    if (!ok) *bad = 1;
+  }
 #pragma unroll 1
   for (int p = 0; p < pairs; ++p) {
     const int i = pair_i(p), j = pair_j(p);
@@ -604,38 +644,57 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
       break;
     }
     tc::fence_after_sync();
-    const float lse = s_lse[i * kBlk + row], delta = s_delta[i * kBlk + row];
-    const int limit = i == j ? row : kBlk;   // keys after the query are masked
-#pragma unroll 1
-    for (int c0 = wg * 64; c0 < wg * 64 + 64; c0 += 32) {
+    const float lse = s_lse[i * kBlk + row], delta = s_delta[i * kBlk + row] * a.scale;
+    // Groups of 32 keys before `diag` are seen by all of the warp's queries, those after it by none.
+    const int diag = i == j ? (warp & 3) * 32 : kBlk;
+    uint4 pk[8], dk[8];   // kept until the gradient products of the pair before have read the shared tiles
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      const int c0 = wg * 64 + g * 32;
+      if (c0 > diag) {
+#pragma unroll
+        for (int c8 = 0; c8 < 4; ++c8) pk[g * 4 + c8] = dk[g * 4 + c8] = make_uint4(0u, 0u, 0u, 0u);
+        continue;
+      }
       uint32_t rs[32], rd[32];
       tc::tmem_ld_32x32(tmem + lane_base + static_cast<uint32_t>(c0), rs);
       tc::tmem_ld_32x32(tmem + lane_base + static_cast<uint32_t>(128 + c0), rd);
       tc::tmem_ld_wait();
-      const int sub = wg * kTile;
+      float pr[32];
+#pragma unroll
+      for (int e = 0; e < 32; ++e) pr[e] = exp2f(__uint_as_float(rs[e]) * a.scale_log2 - lse);
+      if (c0 == diag) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) pr[e] = e <= lane ? pr[e] : 0.f;
+      }
 #pragma unroll
       for (int c8 = 0; c8 < 4; ++c8) {
-        uint4 pk, dk;
-        __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
-        __nv_bfloat162* hs = reinterpret_cast<__nv_bfloat162*>(&dk);
+        __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk[g * 4 + c8]);
+        __nv_bfloat162* hs = reinterpret_cast<__nv_bfloat162*>(&dk[g * 4 + c8]);
 #pragma unroll
         for (int e2 = 0; e2 < 4; ++e2) {
           const int e = c8 * 8 + e2 * 2;
-          const float p0 = c0 + e <= limit ? exp2f(__uint_as_float(rs[e]) * a.scale_log2 - lse) : 0.f;
-          const float p1 = c0 + e + 1 <= limit ? exp2f(__uint_as_float(rs[e + 1]) * a.scale_log2 - lse) : 0.f;
-          hp[e2] = __floats2bfloat162_rn(p0, p1);
-          const float2 pr = __bfloat1622float2(hp[e2]);
-          hs[e2] = __floats2bfloat162_rn(pr.x * (__uint_as_float(rd[e]) - delta) * a.scale,
-                                         pr.y * (__uint_as_float(rd[e + 1]) - delta) * a.scale);
+          hp[e2] = __floats2bfloat162_rn(pr[e], pr[e + 1]);
+          hs[e2] = __floats2bfloat162_rn(pr[e] * (__uint_as_float(rd[e]) * a.scale - delta), pr[e + 1] * (__uint_as_float(rd[e + 1]) * a.scale - delta));
         }
-        const uint32_t off = sw128_offset(row, ((c0 & 63) >> 3) + c8);
-        *reinterpret_cast<uint4*>(sP + sub + off) = pk;
-        *reinterpret_cast<uint4*>(sDS + sub + off) = dk;
       }
+    }
+    if (p > 0) {
+      ok = tc::mbar_wait(g_done, (p - 1) & 1);   // P and dS may be overwritten, the last pair's gradients are in tensor memory
+      ok = __all_sync(0xffffffffu, ok);
+      tc::fence_after_sync();
+      if (ok && *bad == 0 && pair_j(p - 1) != j) key_block_out(pair_j(p - 1));
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const uint32_t off = wg * kTile + sw128_offset(row, c);
+      *reinterpret_cast<uint4*>(sP + off) = pk[c];
+      *reinterpret_cast<uint4*>(sDS + off) = dk[c];
     }
     fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();   // P and dS are complete, and nobody reads the score columns any more
+    // Two threads issue: an MMA takes its issuer some 50 clocks, and these 24 would be 0.7 us of the chain for one.
     if (warp == 0) {
       bool w = true;
       if (p + 1 < pairs && p == 0) w = tc::mbar_wait(&in_full[0], 0);   // the second pair is the first to need block 0
@@ -644,38 +703,49 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
       if (tc::elect_one()) {
         if (!w) *bad = 1;
         if (p + 1 < pairs) issue_scores(pair_i(p + 1), pair_j(p + 1));
-        const uint64_t dpt = tc::smem_desc_mn_sw128(sP, kTile), dst = tc::smem_desc_mn_sw128(sDS, kTile);
-        const uint64_t ddo = tc::smem_desc_mn_sw128(sDO + i * kTile, kTile), dq = tc::smem_desc_mn_sw128(sQ + i * kTile, kTile);
-        const uint64_t dk = tc::smem_desc_mn_sw128(sK + j * kTile, kTile), dsn = tc::smem_desc_k_sw128(sDS);
-        const bool add_kv = p == 2;                   // dK_0, dV_0: pairs (1,0), (0,0)
-        const bool add_q = p == 1;                    // dQ_1: pairs (1,1), (1,0)
+        const uint64_t dpt = tc::smem_desc_mn_sw128(sP, kTile), ddo = tc::smem_desc_mn_sw128(sDO + i * kTile, kTile);
+        const bool add = p == 2;   // dV_0: pairs (1,0), (0,0)
 #pragma unroll
-        for (int kk = 0; kk < kBlk / UMMA_K; ++kk) tc::mma_bf16(tm_dv, dpt + 128 * kk, ddo + 128 * kk, idesc_tt, kk != 0 || add_kv);
+        for (int kk = 0; kk < kBlk / UMMA_K; ++kk) tc::mma_bf16(tm_dv, dpt + 128 * kk, ddo + 128 * kk, idesc_tt, kk != 0 || add);
+        tc::mma_commit(g_done);
+      }
+      __syncwarp();
+    } else if (warp == 4) {
+      tc::fence_after_sync();
+      if (tc::elect_one()) {
+        const uint64_t dst = tc::smem_desc_mn_sw128(sDS, kTile), dq = tc::smem_desc_mn_sw128(sQ + i * kTile, kTile);
+        const uint64_t dkm = tc::smem_desc_mn_sw128(sK + j * kTile, kTile), dsn = tc::smem_desc_k_sw128(sDS);
+        const bool add_k = p == 2, add_q = p == 1;   // dK_0: pairs (1,0), (0,0); dQ_1: pairs (1,1), (1,0)
 #pragma unroll
-        for (int kk = 0; kk < kBlk / UMMA_K; ++kk) tc::mma_bf16(tm_dk, dst + 128 * kk, dq + 128 * kk, idesc_tt, kk != 0 || add_kv);
+        for (int kk = 0; kk < kBlk / UMMA_K; ++kk) tc::mma_bf16(tm_dk, dst + 128 * kk, dq + 128 * kk, idesc_tt, kk != 0 || add_k);
 #pragma unroll
         for (int kk = 0; kk < kBlk / UMMA_K; ++kk)
-          tc::mma_bf16(tm_dq + static_cast<uint32_t>(i * kHd), dsn + (kk >> 2) * (kTile >> 4) + 2 * (kk & 3), dk + 128 * kk, idesc_nt, kk != 0 || add_q);
+          tc::mma_bf16(tm_dq + static_cast<uint32_t>(i * kHd), dsn + (kk >> 2) * (kTile >> 4) + 2 * (kk & 3), dkm + 128 * kk, idesc_nt, kk != 0 || add_q);
         tc::mma_commit(g_done);
       }
       __syncwarp();
     }
-    ok = tc::mbar_wait(g_done, p & 1);   // P and dS may be overwritten, this pair's gradients are in tensor memory
+  }
+  if (ok) {
+    ok = tc::mbar_wait(g_done, (pairs - 1) & 1);
     ok = __all_sync(0xffffffffu, ok);
     tc::fence_after_sync();
-    if (ok && *bad == 0 && (p + 1 == pairs || pair_j(p + 1) != j)) {   // last pair of this key block: its dK and dV leave
-      write_out(wg == 0 ? tm_dk : tm_dv, 1 + wg, j, 0);
-      write_out(wg == 0 ? tm_dk : tm_dv, 1 + wg, j, 32);
-      tc::fence_before_sync();
-    }
+    if (ok && *bad == 0) key_block_out(0);
   }
-  if (ok && *bad == 0) {
-    if (nblk == 2) {
-      write_out(tm_dq + static_cast<uint32_t>(wg * kHd), 0, wg, 0);
-      write_out(tm_dq + static_cast<uint32_t>(wg * kHd), 0, wg, 32);
-    } else {
-      write_out(tm_dq, 0, 0, wg * 32);
+  ok = __syncthreads_and((ok && *bad == 0) ? 1 : 0) != 0;
+  if (ok) {
+    if (nblk == 2) {   // one query block per warpgroup
+      stage_out(sQ + wg * kTile, tm_dq + static_cast<uint32_t>(wg * kHd), 0, 0);
+      stage_out(sQ + wg * kTile, tm_dq + static_cast<uint32_t>(wg * kHd), 0, 32);
+      send_out(sQ + wg * kTile, 0, wg);
+    } else {           // half of the columns per warpgroup
+      stage_out(sQ, tm_dq, 0, wg * 32);
+      fence_async_smem();
+      __syncthreads();
+      if (wg == 0) send_out(sQ, 0, 0);
     }
+    if (tc::elect_one()) stores_read();   // the thread that sent this warp's rows
+    __syncwarp();
   } else if (tid == 0) {
     atomicExch(a.err, 12);
     for (int i = 0; i < nblk; ++i) tc::mbar_wait(&in_full[i], 0, 1u << 20);   // issued loads must land before the CTA retires
@@ -690,8 +760,8 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
 
 constexpr int kBwdSmem = 12 * kTile + 2048 + 64 + 1024;   // 195 KiB
 
-// [B, S, slots, hd] with contiguous hd as boxes of 128 rows x 64 columns of one (batch, slot).
-bool encode_slots(CUtensorMap* map, const void* base, int B, int S, int slots, int hd) {
+// [B, S, slots, hd] with contiguous hd as boxes of box_rows rows x 64 columns of one (batch, slot).
+bool encode_slots(CUtensorMap* map, const void* base, int B, int S, int slots, int hd, int box_rows = kBlk) {
   const CuDriver& cu = CuDriver::get();
   if (!cu.loaded || !cu.TensorMapEncodeTiled) return false;
   int device = 0;
@@ -700,7 +770,7 @@ bool encode_slots(CUtensorMap* map, const void* base, int B, int S, int slots, i
   const cuuint64_t row = static_cast<cuuint64_t>(slots) * hd * 2;
   cuuint64_t dims[4] = {static_cast<cuuint64_t>(hd), static_cast<cuuint64_t>(slots), static_cast<cuuint64_t>(S), static_cast<cuuint64_t>(B)};
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(hd) * 2, row, row * S};
-  cuuint32_t box[4] = {kHd, 1, kBlk, 1};
+  cuuint32_t box[4] = {kHd, 1, static_cast<cuuint32_t>(box_rows), 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   return cu.TensorMapEncodeTiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -728,14 +798,13 @@ cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, cons
   static std::atomic<bool> configured{false};
   cudaError_t rc = allow_smem(attn_bwd_kernel, kBwdSmem, configured);
   if (rc != cudaSuccess) return rc;
-  CUtensorMap tq, tdo;
-  if (!encode_slots(&tq, qkv, B, S, 3 * H, hd) || !encode_slots(&tdo, d_o, B, S, H, hd)) return cudaErrorNotSupported;
+  CUtensorMap tq, tdo, to, tdqkv;
+  if (!encode_slots(&tq, qkv, B, S, 3 * H, hd) || !encode_slots(&tdo, d_o, B, S, H, hd) || !encode_slots(&to, o, B, S, H, hd) ||
+      !encode_slots(&tdqkv, dqkv, B, S, 3 * H, hd, 32))
+    return cudaErrorNotSupported;
   (void)cudaGetLastError();
   AttnArgs a = {};
-  a.o = o;
-  a.d_o = d_o;
   a.lse = const_cast<float*>(lse);
-  a.dqkv = dqkv;
   a.colsum = colsum;
   a.S = S;
   a.H = H;
@@ -744,7 +813,7 @@ cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, cons
   a.scale_log2 = softmax_scale * 1.4426950408889634f;
   a.err = gemm_error_device_ptr();
   if (!a.err) return cudaErrorNotSupported;
-  MCCL_LAUNCH_PDL(attn_bwd_kernel, dim3(H, B), 256, kBwdSmem, stream, tq, tdo, a);
+  MCCL_LAUNCH_PDL(attn_bwd_kernel, dim3(H, B), 256, kBwdSmem, stream, tq, tdo, to, tdqkv, a);
   count_launch();
   return launch_status();
 }
@@ -762,9 +831,9 @@ cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse
     static std::atomic<bool> configured{false};
     cudaError_t rc = allow_smem(attn_fwd_kernel, kFwdSmem, configured);
     if (rc != cudaSuccess) return rc;
-    if (!encode_slots(&tm, qkv, B, S, 3 * H, hd)) return cudaErrorNotSupported;
+    CUtensorMap to;
+    if (!encode_slots(&tm, qkv, B, S, 3 * H, hd) || !encode_slots(&to, o, B, S, H, hd, 32)) return cudaErrorNotSupported;
     AttnArgs a = {};
-    a.o_out = o;
     a.lse = lse;
     a.S = S;
     a.H = H;
@@ -772,7 +841,7 @@ cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse
     a.scale = softmax_scale;
     a.scale_log2 = scale_log2;
     a.err = err;
-    MCCL_LAUNCH_PDL(attn_fwd_kernel, dim3((S + kBlk - 1) / kBlk, H, B), 256, kFwdSmem, stream, tm, a);
+    MCCL_LAUNCH_PDL(attn_fwd_kernel, dim3((S + kBlk - 1) / kBlk, H, B), 256, kFwdSmem, stream, tm, to, a);
   } else {
     if (hd != kHd || S <= 0 || S % kBlk != 0) return cudaErrorNotSupported;
     static std::atomic<bool> configured{false};
