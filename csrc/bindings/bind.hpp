@@ -9,4 +9,5 @@ void bind_pg(pybind11::module_& m);       // process group, metrics, logging
 void bind_comm(pybind11::module_& m);     // device communicator, symmetric heap, kernels
 void bind_runtime(pybind11::module_& m);  // dmem, coherence, scheduler, cluster manager, agent
 void bind_ops(pybind11::module_& m);      // model operators (GEMM, norms, optimizer)
+void bind_layers(pybind11::module_& m);   // whole decoder layers
 }  // namespace mccl

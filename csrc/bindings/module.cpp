@@ -8,4 +8,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   mccl::bind_comm(m);
   mccl::bind_runtime(m);
   mccl::bind_ops(m);
+  mccl::bind_layers(m);
 }

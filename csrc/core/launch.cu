@@ -2,16 +2,34 @@
 
 #include <atomic>
 #include <cstdlib>
-#include <mutex>
 
 #include "log.hpp"
 
 namespace mccl {
 
 namespace {
-std::mutex g_mu;
-std::map<std::string, uint64_t> g_counts;
+// Launches per kernel-name literal, counted without a lock: a launch costs the host two or three microseconds, and a mutex,
+// a string and a map lookup were a tenth of that.  Every call site passes the same literal every time, so the pointer is
+// the key; equal names from different sites are added up when somebody asks.
+constexpr int kSlots = 256;
+struct Slot {
+  std::atomic<const char*> name{nullptr};
+  std::atomic<uint64_t> count{0};
+};
+Slot g_slots[kSlots];
 std::atomic<uint64_t> g_total{0};
+
+void count(const char* kernel) {
+  size_t at = (reinterpret_cast<uintptr_t>(kernel) >> 3) % kSlots;
+  for (int i = 0; i < kSlots; ++i, at = (at + 1) % kSlots) {
+    const char* have = g_slots[at].name.load(std::memory_order_acquire);
+    if (have == nullptr && g_slots[at].name.compare_exchange_strong(have, kernel, std::memory_order_acq_rel)) have = kernel;
+    if (have == kernel) {
+      g_slots[at].count.fetch_add(1, std::memory_order_relaxed);
+      return;
+    }
+  }
+}
 thread_local cudaError_t t_first_error = cudaSuccess;
 
 // "(gemm_persistent_kernel<BN, STAGES, kAMn, kBMn>)" -> "gemm_persistent_kernel"
@@ -28,10 +46,7 @@ std::string short_name(const char* kernel) {
 cudaError_t launch_record(const char* kernel, const char* file, int line, dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {
   const cudaError_t rc = cudaGetLastError();
   g_total.fetch_add(1, std::memory_order_relaxed);
-  {
-    std::lock_guard<std::mutex> g(g_mu);
-    ++g_counts[short_name(kernel)];
-  }
+  count(kernel);
   if (rc != cudaSuccess) {
     if (t_first_error == cudaSuccess) t_first_error = rc;
     MCCL_ERROR("launch of " << kernel << " at " << file << ":" << line << " failed: " << cudaGetErrorString(rc) << " (grid " << grid.x
@@ -63,12 +78,16 @@ cudaError_t launch_status() {
 }
 
 std::map<std::string, uint64_t> launch_counts() {
-  std::lock_guard<std::mutex> g(g_mu);
-  return g_counts;
+  std::map<std::string, uint64_t> out;
+  for (const Slot& slot : g_slots) {
+    const char* name = slot.name.load(std::memory_order_acquire);
+    const uint64_t n = slot.count.load(std::memory_order_relaxed);
+    if (name && n) out[short_name(name)] += n;
+  }
+  return out;
 }
 void launch_counts_reset() {
-  std::lock_guard<std::mutex> g(g_mu);
-  g_counts.clear();
+  for (Slot& slot : g_slots) slot.count.store(0);
   g_total.store(0);
 }
 uint64_t launch_total() { return g_total.load(); }

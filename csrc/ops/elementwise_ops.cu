@@ -45,8 +45,9 @@ uint64_t launch_count() { return g_launches.load(); }
 void count_launch(int n) { g_launches.fetch_add(static_cast<uint64_t>(n)); }
 
 // ------------------------------------------------------------------- norm --
-// One warp per row; dim must be a multiple of 8.
-template <bool kLayerNorm>
+// One warp per row; dim must be a multiple of 8.  kVecs > 0: the row is at most kVecs x 256 wide and stays in registers, so
+// it is read once with all of its loads in flight (4096 x 512: 5.0 us in three passes over the row, 3.2 us in one).
+template <bool kLayerNorm, int kVecs>
 __global__ void __launch_bounds__(256) norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
                                                        const float* __restrict__ b, __nv_bfloat16* __restrict__ y,
                                                        float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows,
@@ -57,41 +58,70 @@ __global__ void __launch_bounds__(256) norm_fwd_kernel(const __nv_bfloat16* __re
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= rows) return;
   const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(warp) * dim);
-  const int vecs = dim >> 3;
-  float sum = 0.f;
-  for (int v = lane; v < vecs; v += 32) {
-    float f[8];
-    unpack8(xr[v], f);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) sum += f[i];
-  }
-  const float mean = kLayerNorm ? warp_sum(sum) / dim : 0.f;
-  float sq = 0.f;
-  for (int v = lane; v < vecs; v += 32) {
-    float f[8];
-    unpack8(xr[v], f);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) sq += (f[i] - mean) * (f[i] - mean);
-  }
-  const float rstd = rsqrtf(warp_sum(sq) / dim + eps);
-  if (lane == 0) {
-    mean_out[warp] = mean;
-    rstd_out[warp] = rstd;
-  }
   uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(warp) * dim);
-  for (int v = lane; v < vecs; v += 32) {
-    float f[8], o[8];
-    unpack8(xr[v], f);
-    const float4 w0 = reinterpret_cast<const float4*>(w)[2 * v], w1 = reinterpret_cast<const float4*>(w)[2 * v + 1];
+  const int vecs = dim >> 3;
+  auto normalise = [&](int v, const float (&f)[8], float mean, float rstd) {
+    const float4 w0 = __ldg(reinterpret_cast<const float4*>(w) + 2 * v), w1 = __ldg(reinterpret_cast<const float4*>(w) + 2 * v + 1);
     const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-    float bb[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    float bb[8] = {0, 0, 0, 0, 0, 0, 0, 0}, o[8];
     if (kLayerNorm) {
-      const float4 b0 = reinterpret_cast<const float4*>(b)[2 * v], b1 = reinterpret_cast<const float4*>(b)[2 * v + 1];
+      const float4 b0 = __ldg(reinterpret_cast<const float4*>(b) + 2 * v), b1 = __ldg(reinterpret_cast<const float4*>(b) + 2 * v + 1);
       bb[0] = b0.x; bb[1] = b0.y; bb[2] = b0.z; bb[3] = b0.w; bb[4] = b1.x; bb[5] = b1.y; bb[6] = b1.z; bb[7] = b1.w;
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) o[i] = (f[i] - mean) * rstd * ww[i] + bb[i];
     yr[v] = pack8(o);
+  };
+  float sum = 0.f, sq = 0.f, mean, rstd;
+  if constexpr (kVecs > 0) {
+    uint4 raw[kVecs];
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) raw[k] = __ldg(xr + lane + 32 * k);
+    float f[kVecs][8];
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k) {
+      if (lane + 32 * k < vecs) {
+        unpack8(raw[k], f[k]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += f[k][i];
+      }
+    }
+    mean = kLayerNorm ? warp_sum(sum) / dim : 0.f;
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sq += (f[k][i] - mean) * (f[k][i] - mean);
+      }
+    rstd = rsqrtf(warp_sum(sq) / dim + eps);
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) normalise(lane + 32 * k, f[k], mean, rstd);
+  } else {
+    for (int v = lane; v < vecs; v += 32) {
+      float f[8];
+      unpack8(xr[v], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sum += f[i];
+    }
+    mean = kLayerNorm ? warp_sum(sum) / dim : 0.f;
+    for (int v = lane; v < vecs; v += 32) {
+      float f[8];
+      unpack8(xr[v], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sq += (f[i] - mean) * (f[i] - mean);
+    }
+    rstd = rsqrtf(warp_sum(sq) / dim + eps);
+    for (int v = lane; v < vecs; v += 32) {
+      float f[8];
+      unpack8(xr[v], f);
+      normalise(v, f, mean, rstd);
+    }
+  }
+  if (lane == 0 && mean_out != nullptr) {
+    mean_out[warp] = mean;
+    rstd_out[warp] = rstd;
   }
 }
 
@@ -143,6 +173,111 @@ __global__ void __launch_bounds__(256) norm_bwd_dx_kernel(const __nv_bfloat16* _
       for (int i = 0; i < 8; ++i) o[i] += a[i];
     }
     dr[v] = pack8(o);
+  }
+}
+
+// The whole backward of a norm in one pass: dx, and added into fp32 buffers the weight and bias gradients and (optional) the
+// column sums of dx_add and of dx, which are bias gradients of the projections around the norm.  One warp per row, several
+// rows per warp; a lane keeps the sums of its 8 x kVecs columns in registers until the CTA adds them up at the end.
+// (dx alone and the column sums in a pass of their own: 6.6 + 5.2 us at 4096 x 512, and 4.1 us for each further bias.)
+template <bool kLayerNorm, int kVecs, bool kSums>
+__global__ void __launch_bounds__(256) norm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                                                             const float* __restrict__ w, const float* __restrict__ mean,
+                                                             const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx,
+                                                             const __nv_bfloat16* __restrict__ dx_add, float* __restrict__ dw,
+                                                             float* __restrict__ db, float* __restrict__ sum_add,
+                                                             float* __restrict__ sum_dx, int rows, int dim) {
+  ::mccl::pdl_trigger();
+  extern __shared__ float red[];   // [8 warps][kVecs * 256]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, vecs = dim >> 3;
+  float aw[kVecs][8], ab[kVecs][8], sa[kSums ? kVecs : 1][8], sd[kSums ? kVecs : 1][8];
+#pragma unroll
+  for (int k = 0; k < kVecs; ++k)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      aw[k][i] = ab[k][i] = 0.f;
+      if (kSums) sa[k][i] = sd[k][i] = 0.f;
+    }
+  ::mccl::pdl_wait();
+  for (int row = blockIdx.x * 8 + warp; row < rows; row += gridDim.x * 8) {
+    const size_t at = static_cast<size_t>(row) * vecs + lane;
+    uint4 rx[kVecs], rg[kVecs], ra[kVecs];
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) {
+        rx[k] = __ldg(reinterpret_cast<const uint4*>(x) + at + 32 * k);
+        rg[k] = __ldg(reinterpret_cast<const uint4*>(dy) + at + 32 * k);
+        if (dx_add != nullptr) ra[k] = __ldg(reinterpret_cast<const uint4*>(dx_add) + at + 32 * k);
+      }
+    const float mu = kLayerNorm ? mean[row] : 0.f, rs = rstd[row];
+    float c1 = 0.f, c2 = 0.f;  // sum(dy * w * xhat), sum(dy * w)
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) {
+        float f[8], g[8];
+        unpack8(rx[k], f);
+        unpack8(rg[k], g);
+        const float4 w0 = __ldg(reinterpret_cast<const float4*>(w) + 2 * (lane + 32 * k)), w1 = __ldg(reinterpret_cast<const float4*>(w) + 2 * (lane + 32 * k) + 1);
+        const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float xhat = (f[i] - mu) * rs, gw = g[i] * ww[i];
+          aw[k][i] += g[i] * xhat;
+          if (kLayerNorm) ab[k][i] += g[i];
+          c1 += gw * xhat;
+          c2 += gw;
+        }
+      }
+    c1 = warp_sum(c1) / dim;
+    c2 = kLayerNorm ? warp_sum(c2) / dim : 0.f;
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) {
+        float f[8], g[8], o[8];
+        unpack8(rx[k], f);
+        unpack8(rg[k], g);
+        const float4 w0 = __ldg(reinterpret_cast<const float4*>(w) + 2 * (lane + 32 * k)), w1 = __ldg(reinterpret_cast<const float4*>(w) + 2 * (lane + 32 * k) + 1);
+        const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = rs * (g[i] * ww[i] - c2 - (f[i] - mu) * rs * c1);
+        if (dx_add != nullptr) {
+          float a[8];
+          unpack8(ra[k], a);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            o[i] += a[i];
+            if (kSums) sa[k][i] += a[i];
+          }
+        }
+        if (kSums) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sd[k][i] += o[i];
+        }
+        reinterpret_cast<uint4*>(dx)[at + 32 * k] = pack8(o);
+      }
+  }
+  auto reduce = [&](const auto& acc, float* out) {
+    if (out == nullptr) return;   // uniform over the block
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k) {
+      float4* p = reinterpret_cast<float4*>(red + (warp * kVecs + k) * 256 + lane * 8);
+      p[0] = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+      p[1] = make_float4(acc[k][4], acc[k][5], acc[k][6], acc[k][7]);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < dim; c += 256) {
+      float t = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t += red[i * kVecs * 256 + c];
+      atomicAdd(out + c, t);
+    }
+  };
+  reduce(aw, dw);
+  if (kLayerNorm) reduce(ab, db);
+  if constexpr (kSums) {
+    reduce(sa, sum_add);
+    reduce(sd, sum_dx);
   }
 }
 
@@ -247,9 +382,18 @@ int colsum_slabs(int rows) { return (rows + kSlabRows - 1) / kSlabRows; }
 cudaError_t norm_fwd(const __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y, float* mean, float* rstd,
                      int rows, int dim, float eps, cudaStream_t stream) {
   if (dim % 8 != 0) return cudaErrorNotSupported;
-  const int blocks = (rows + 7) / 8;
-  if (b) MCCL_LAUNCH_PDL(norm_fwd_kernel<true>, blocks, 256, 0, stream, x, w, b, y, mean, rstd, rows, dim, eps);
-  else MCCL_LAUNCH_PDL(norm_fwd_kernel<false>, blocks, 256, 0, stream, x, w, b, y, mean, rstd, rows, dim, eps);
+  const int blocks = (rows + 7) / 8, vecs = (dim + 255) / 256;
+#define MCCL_NORM_FWD(LN, V) MCCL_LAUNCH_PDL((norm_fwd_kernel<LN, V>), blocks, 256, 0, stream, x, w, b, y, mean, rstd, rows, dim, eps)
+#define MCCL_NORM_FWD_V(LN)                              \
+  (vecs == 1   ? MCCL_NORM_FWD(LN, 1)                    \
+   : vecs == 2 ? MCCL_NORM_FWD(LN, 2)                    \
+   : vecs <= 4 ? MCCL_NORM_FWD(LN, 4)                    \
+   : vecs <= 8 ? MCCL_NORM_FWD(LN, 8)                    \
+               : MCCL_NORM_FWD(LN, 0))
+  if (b) MCCL_NORM_FWD_V(true);
+  else MCCL_NORM_FWD_V(false);
+#undef MCCL_NORM_FWD_V
+#undef MCCL_NORM_FWD
   count_launch();
   return ::mccl::launch_status();
 }
@@ -258,6 +402,10 @@ cudaError_t norm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const floa
                      __nv_bfloat16* dx, float* dw, float* db, float* scratch, int rows, int dim, bool layernorm,
                      cudaStream_t stream, const __nv_bfloat16* dx_add, int parts) {
   if (dim % 8 != 0) return cudaErrorNotSupported;
+  if (parts == 3 && !scratch) {   // everything is added into dw / db: one pass, where the sums fit registers
+    cudaError_t rc = norm_bwd_fused(dy, x, w, mean, rstd, dx, dx_add, dw, layernorm ? db : nullptr, nullptr, nullptr, rows, dim, layernorm, stream);
+    if (rc != cudaErrorNotSupported) return rc;
+  }
   const int blocks = (rows + 7) / 8;
   if (parts & 1) {
     if (layernorm) MCCL_LAUNCH_PDL(norm_bwd_dx_kernel<true>, blocks, 256, 0, stream, dy, x, w, mean, rstd, dx, dx_add, rows, dim);
@@ -278,6 +426,43 @@ cudaError_t norm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const floa
   MCCL_LAUNCH_PDL(colsum_partial_kernel<true>, grid, 256, 0, stream, dy, x, mean, rstd, part_w, part_b, rows, dim, 0);
   MCCL_LAUNCH_PDL(colsum_final_kernel, (dim + 31) / 32, 256, 0, stream, part_w, part_b, dw, layernorm ? db : nullptr, slabs, dim);
   count_launch(2);
+  return ::mccl::launch_status();
+}
+
+cudaError_t norm_bwd_fused(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* w, const float* mean, const float* rstd,
+                           __nv_bfloat16* dx, const __nv_bfloat16* dx_add, float* dw, float* db, float* sum_add, float* sum_dx, int rows,
+                           int dim, bool layernorm, cudaStream_t stream) {
+  const int vecs = (dim + 255) / 256;
+  const bool sums = sum_add != nullptr || sum_dx != nullptr;
+  // the sums of a lane's columns live in registers: four sets of up to 32 or one of up to 64
+  if (dim % 8 != 0 || vecs > (layernorm || sums ? 4 : 8) || (sum_add != nullptr && dx_add == nullptr)) return cudaErrorNotSupported;
+  int blocks = (rows + 7) / 8;
+  const int most = vecs <= 2 ? 2 * 148 : 148;
+  if (blocks > most) blocks = most;
+  if (blocks < 1) return cudaSuccess;
+#define MCCL_NORM_BWD(LN, V, S)                                                                                                  \
+  MCCL_LAUNCH_PDL((norm_bwd_fused_kernel<LN, V, S>), blocks, 256, 8 * V * 256 * sizeof(float), stream, dy, x, w, mean, rstd, dx, \
+                  dx_add, dw, db, sum_add, sum_dx, rows, dim)
+#define MCCL_NORM_BWD_V(LN, S) \
+  (vecs == 1 ? MCCL_NORM_BWD(LN, 1, S) : vecs == 2 ? MCCL_NORM_BWD(LN, 2, S) : vecs == 3 ? MCCL_NORM_BWD(LN, 3, S) : MCCL_NORM_BWD(LN, 4, S))
+  if (vecs > 4) {
+    static std::atomic<bool> configured{false};
+    if (!configured.load(std::memory_order_acquire)) {
+      cudaError_t rc = cudaFuncSetAttribute(norm_bwd_fused_kernel<false, 8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536);
+      if (rc != cudaSuccess) return rc;
+      configured.store(true, std::memory_order_release);
+    }
+    MCCL_NORM_BWD(false, 8, false);
+  } else if (layernorm) {
+    if (sums) MCCL_NORM_BWD_V(true, true);
+    else MCCL_NORM_BWD_V(true, false);
+  } else {
+    if (sums) MCCL_NORM_BWD_V(false, true);
+    else MCCL_NORM_BWD_V(false, false);
+  }
+#undef MCCL_NORM_BWD_V
+#undef MCCL_NORM_BWD
+  count_launch();
   return ::mccl::launch_status();
 }
 
@@ -510,6 +695,69 @@ cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cuda
   if (blocks < 1) blocks = 1;
   MCCL_LAUNCH_PDL(cast_kernel, static_cast<int>(blocks), 256, 0, stream, in, out, n);
   count_launch();
+  return ::mccl::launch_status();
+}
+
+// Casts of many tensors into one buffer: a block takes kCastChunk consecutive elements of the concatenation.  64 weights of
+// a 70M model one by one: 182 us, most of it launches that leave most SMs idle; together: 75 us (6 bytes per element).
+constexpr int kCastMax = 128, kCastChunk = 8192;
+struct CastTable {
+  const float* src[kCastMax];
+  long long dst[kCastMax];      // first element in the output
+  long long numel[kCastMax];
+  int block[kCastMax + 1];      // first block of each tensor
+  int count;
+};
+
+__global__ void __launch_bounds__(256) cast_many_kernel(const __grid_constant__ CastTable t, __nv_bfloat16* __restrict__ out) {
+  ::mccl::pdl_trigger();
+  ::mccl::pdl_wait();
+  int lo = 0, hi = t.count - 1;   // the tensor this block belongs to
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (t.block[mid] <= static_cast<int>(blockIdx.x)) lo = mid;
+    else hi = mid - 1;
+  }
+  const long long first = static_cast<long long>(blockIdx.x - t.block[lo]) * kCastChunk;
+  const float* src = t.src[lo] + first;
+  __nv_bfloat16* dst = out + t.dst[lo] + first;
+  const long long left = t.numel[lo] - first;
+  if (left >= kCastChunk) {
+    float4 f[kCastChunk / 2048][2];
+#pragma unroll
+    for (int k = 0; k < kCastChunk / 2048; ++k) {
+      f[k][0] = __ldg(reinterpret_cast<const float4*>(src) + (k * 256 + threadIdx.x) * 2);
+      f[k][1] = __ldg(reinterpret_cast<const float4*>(src) + (k * 256 + threadIdx.x) * 2 + 1);
+    }
+#pragma unroll
+    for (int k = 0; k < kCastChunk / 2048; ++k) {
+      const float v[8] = {f[k][0].x, f[k][0].y, f[k][0].z, f[k][0].w, f[k][1].x, f[k][1].y, f[k][1].z, f[k][1].w};
+      reinterpret_cast<uint4*>(dst)[k * 256 + threadIdx.x] = pack8(v);
+    }
+  } else {
+    for (int i = threadIdx.x; i < left; i += 256) dst[i] = __float2bfloat16_rn(src[i]);
+  }
+}
+
+cudaError_t cast_many(const float* const* src, const long long* numel, const long long* dst_offset, int count, __nv_bfloat16* out,
+                      cudaStream_t stream) {
+  for (int p = 0; p < count; p += kCastMax) {
+    CastTable t;
+    t.count = count - p < kCastMax ? count - p : kCastMax;
+    int blocks = 0;
+    for (int i = 0; i < t.count; ++i) {
+      if ((reinterpret_cast<uintptr_t>(src[p + i]) & 15u) || (reinterpret_cast<uintptr_t>(out + dst_offset[p + i]) & 15u)) return cudaErrorNotSupported;
+      t.src[i] = src[p + i];
+      t.dst[i] = dst_offset[p + i];
+      t.numel[i] = numel[p + i];
+      t.block[i] = blocks;
+      blocks += static_cast<int>((numel[p + i] + kCastChunk - 1) / kCastChunk);
+    }
+    t.block[t.count] = blocks;
+    if (blocks == 0) continue;
+    MCCL_LAUNCH_PDL(cast_many_kernel, blocks, 256, 0, stream, t, out);
+    count_launch();
+  }
   return ::mccl::launch_status();
 }
 

@@ -57,7 +57,7 @@ cudaError_t gemm_bf16_tn(const GemmArgs& a, cudaStream_t stream) {
   if (a.aux && (reinterpret_cast<uintptr_t>(a.aux) & 15u)) return unsupported("aux pointer must be 16-byte aligned");
   if ((a.epilogue == EPI_BIAS || a.epilogue == EPI_BIAS_GELU || a.epilogue == EPI_BIAS_GELU_D) && !a.bias) return cudaErrorInvalidValue;
   if ((a.epilogue == EPI_BIAS_GELU || a.epilogue == EPI_GELU || a.epilogue == EPI_BIAS_GELU_D || a.epilogue == EPI_GELU_D) &&
-      (!a.aux || a.d_fp32))
+      a.d_fp32)
     return cudaErrorInvalidValue;
   if (a.accumulate && !a.d_fp32) return cudaErrorInvalidValue;
   if (a.residual && (reinterpret_cast<uintptr_t>(a.residual) & 15u)) return unsupported("residual pointer must be 16-byte aligned");
@@ -69,7 +69,8 @@ cudaError_t gemm_bf16_tn(const GemmArgs& a, cudaStream_t stream) {
   }();
   const int forced = g_gemm_kernel_override.load(std::memory_order_relaxed);
   const int choice = forced != -2 ? forced : env_choice;
-  const bool tile_only = a.k % BK != 0 || a.colsum;   // what only the tile kernel does
+  const bool gelu = a.epilogue == EPI_BIAS_GELU || a.epilogue == EPI_GELU || a.epilogue == EPI_BIAS_GELU_D || a.epilogue == EPI_GELU_D;
+  const bool tile_only = a.k % BK != 0 || a.colsum || (gelu && !a.aux);   // what only the tile kernel does
   cudaError_t rc = choice == kPersistent && !tile_only ? launch_gemm_persistent(a, FusedDev{}, 0, stream) : launch_gemm_tiles(a, choice, stream);
   if (rc == cudaErrorNotSupported) return unsupported("cuTensorMapEncodeTiled rejected an operand");
   return rc;

@@ -110,7 +110,7 @@ cudaError_t launch_gemm_tiles(const GemmArgs& a, int forced_bn, cudaStream_t str
   // over an MN-major operand, a bias or an extra input with an fp32 output, a bias that is not 16-byte aligned.
   if ((a.mul && a.residual) || (gelu && (a.mul || a.residual || a.a_mn_major || a.b_mn_major)) ||
       (a.d_fp32 && (a.epilogue != EPI_NONE || a.residual)) || (a.bias && (reinterpret_cast<uintptr_t>(a.bias) & 15)))
-    return launch_gemm_persistent(a, FusedDev{}, 0, stream);
+    return gelu && !a.aux ? cudaErrorNotSupported : launch_gemm_persistent(a, FusedDev{}, 0, stream);
   (void)cudaGetLastError();   // a stale error of an earlier, unrelated call must not be blamed on this launch
   if (a.colsum) {
     if (gelu || a.d_fp32 || a.bias || a.residual || a.a_mn_major || !a.b_mn_major) return cudaErrorInvalidValue;

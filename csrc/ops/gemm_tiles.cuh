@@ -519,9 +519,9 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
             if constexpr (kOut == OUT_GELU) bulk_wait_read<0>();
           }
           __syncwarp();
-          if constexpr (kOut == OUT_GELU) {
+          if (kOut == OUT_GELU && g.aux != nullptr) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) *stage_unit(buf_c, lane, j) = second[j];
+            for (int j = 0; j < 8; ++j) *stage_unit(buf_c, lane, j) = second[kOut == OUT_GELU ? j : 0];
             fence_async_smem();
             __syncwarp();
             if (tc::elect_one()) {

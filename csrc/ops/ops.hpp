@@ -22,7 +22,7 @@ void count_launch(int n = 1);
 
 // ---- normalisation: y = (x - mean) * rstd * w + b  (LayerNorm, bias != null)
 //                     y = x * rstd * w                (RMSNorm, bias == null)
-// x, y: [rows, dim] bf16; w, b: fp32; mean / rstd: fp32 [rows] saved for backward.
+// x, y: [rows, dim] bf16; w, b: fp32; mean / rstd: fp32 [rows] saved for backward (both may be null).
 cudaError_t norm_fwd(const __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y, float* mean, float* rstd,
                      int rows, int dim, float eps, cudaStream_t stream);
 // dx: [rows, dim] bf16; dw, db: fp32 [dim].  With scratch (fp32, 2 * colsum_slabs(rows) * dim
@@ -32,6 +32,11 @@ cudaError_t norm_fwd(const __nv_bfloat16* x, const float* w, const float* b, __n
 cudaError_t norm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* w, const float* mean, const float* rstd,
                      __nv_bfloat16* dx, float* dw, float* db, float* scratch, int rows, int dim, bool layernorm,
                      cudaStream_t stream, const __nv_bfloat16* dx_add = nullptr, int parts = 3);
+// The same backward in one pass: dw, db (LayerNorm) and, where given, the column sums of dx_add and of dx are ADDED into fp32
+// [dim] buffers.  dim <= 1024, or 2048 for RMSNorm without column sums; cudaErrorNotSupported otherwise.
+cudaError_t norm_bwd_fused(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* w, const float* mean, const float* rstd,
+                           __nv_bfloat16* dx, const __nv_bfloat16* dx_add, float* dw, float* db, float* sum_add, float* sum_dx, int rows,
+                           int dim, bool layernorm, cudaStream_t stream);
 // out[c] = sum over rows of in[r, c] (bias gradients).  scratch: colsum_slabs(rows) * dim floats,
 // or nullptr to add into out atomically in one pass.
 cudaError_t colsum_bf16(const __nv_bfloat16* in, float* out, float* scratch, int rows, int dim, cudaStream_t stream);
@@ -54,6 +59,9 @@ cudaError_t cross_entropy_fwd_bwd(__nv_bfloat16* logits, const long long* target
 cudaError_t transpose_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, int rows, int cols, cudaStream_t stream);
 // fp32 → bf16 cast of n elements.
 cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t stream);
+// The same for `count` tensors, tensor i into out[dst_offset[i], ...); 16-byte aligned sources and places.
+cudaError_t cast_many(const float* const* src, const long long* numel, const long long* dst_offset, int count, __nv_bfloat16* out,
+                      cudaStream_t stream);
 // GELU backward on a pre-activation: dz = dy * gelu'(z).
 cudaError_t gelu_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* z, __nv_bfloat16* dz, long long n, cudaStream_t stream);
 
@@ -107,7 +115,7 @@ struct GemmArgs {
   bool a_mn_major = false;
   bool b_mn_major = false;
   void* d = nullptr;                 // [M, N] bf16 or fp32, row stride ldd
-  __nv_bfloat16* aux = nullptr;      // [M, N] pre-activation (GELU epilogues)
+  __nv_bfloat16* aux = nullptr;      // [M, N] second output of GELU epilogues (may be null: not written)
   const float* bias = nullptr;       // [N]
   const __nv_bfloat16* residual = nullptr;  // [M, N] added after bias / activation, row stride ldd
   const __nv_bfloat16* mul = nullptr;       // [M, N]: D = acc * mul (e.g. the saved gelu'(z): the input gradient through a GELU), row stride ldd

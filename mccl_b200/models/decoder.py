@@ -100,6 +100,44 @@ def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.T
     return out.flatten(-2).to(x.dtype)
 
 
+class _Structure:
+    """The parameters of a module tree, collected once, and whether the tree is still what it was: no module or parameter
+    replaced, no hook registered, nothing but plain fp32 parameters.  (Walking the modules again takes longer than launching
+    a small model's kernels.)"""
+
+    def __init__(self, root: nn.Module):
+        modules = list(root.modules())
+        self.dicts = [d for m in modules for d in (m._modules, m._parameters) if d]
+        self.values = [list(d.values()) for d in self.dicts]
+        self.hooks = [d for m in modules for d in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks, m._backward_pre_hooks)]
+        self.plain = all(type(p) is nn.Parameter and p.dtype == torch.float32 and p.is_contiguous() for p in root.parameters())
+        self.device = next(root.parameters()).device
+        self.params = {name: p for name, p in root.named_parameters()}
+
+    def intact(self) -> bool:
+        if not self.plain or any(self.hooks):
+            return False
+        try:
+            return all(list(d.values()) == v for d, v in zip(self.dicts, self.values))
+        except RuntimeError:   # a replaced parameter compares by element
+            return False
+
+
+def _structure(module: nn.Module, device):
+    """The module's cached `_Structure` when it can be used on `device`, else None."""
+    s = module.__dict__.get("_structure_cache")
+    if s is None or s.device != device or not s.intact():
+        s = _Structure(module)
+        module.__dict__["_structure_cache"] = s
+        if s.device != device or not s.intact():
+            return None
+    return s
+
+
+# A layer as one autograd node, and a forward without gradients as one call (MCCL_FUSE_LAYER=0: operator by operator).
+_FUSE_LAYER = os.environ.get("MCCL_FUSE_LAYER", "1") != "0"
+
+
 class Norm(nn.Module):
     def __init__(self, cfg: DecoderConfig):
         super().__init__()
@@ -160,9 +198,35 @@ class Block(nn.Module):
             self.up = Linear(d, cfg.d_ff, bias, std)
         self.down = Linear(cfg.d_ff, d, bias, out_std)
 
+    def _layer_params(self, x: torch.Tensor):
+        """This layer's parameters in the order the fused layer takes them, or None where it does not apply."""
+        cfg = self.cfg
+        from .. import _C
+        from ..ops.functional import native_attention_supported
+        if cfg.norm != "layernorm" or cfg.act != "gelu" or not native_attention_supported(x.shape[1], cfg.head_dim):
+            return None
+        if not _C.decoder_layer_supported(x.shape[1], cfg.n_heads, cfg.d_model, cfg.d_ff):
+            return None
+        s = _structure(self, x.device)
+        if s is None:
+            return None
+        params = s.__dict__.get("ordered")
+        if params is None:
+            s.ordered = params = [s.params.get(f"{m}.{k}") for m in ("ln1", "qkv", "proj", "ln2", "up", "down") for k in ("weight", "bias")]
+        if any(p is None for p in params):
+            return None
+        if torch.is_grad_enabled() and not all(p.requires_grad for p in params):
+            return None   # frozen parameters: operator by operator
+        return params
+
     def forward(self, x: torch.Tensor, rope, native: bool) -> torch.Tensor:
         cfg = self.cfg
         B, S, D = x.shape
+        if native and rope is None and _FUSE_LAYER and x.dtype == torch.bfloat16:
+            params = self._layer_params(x)
+            if params is not None:
+                from ..ops.native import DecoderLayerFn
+                return DecoderLayerFn.apply(x if x.is_contiguous() else x.contiguous(), cfg.n_heads, cfg.eps, *params)
         h, x = self.ln1.with_residual(x, native)
         qkv = self.qkv(h, native)
         if native and rope is None:
@@ -234,11 +298,48 @@ class Decoder(nn.Module):
             x = blk(x, rope, native)
         return self.ln_f(x, native)
 
+    def _forward_without_gradients(self, tokens: torch.Tensor):
+        """Logits from one native call over the whole decoder, or None where it does not apply."""
+        cfg = self.cfg
+        from .. import _C
+        from ..ops.functional import native_attention_supported
+        rope = cfg.pos == "rope"
+        if tokens.dim() != 2 or tokens.dtype != torch.int64 or cfg.d_model % 64 or cfg.d_ff % 64 or cfg.vocab % 8:
+            return None
+        if rope:
+            if cfg.norm != "rmsnorm" or cfg.act != "swiglu" or cfg.head_dim % 8:
+                return None
+        elif (cfg.norm != "layernorm" or cfg.act != "gelu" or tokens.shape[1] > cfg.max_seq
+              or not native_attention_supported(tokens.shape[1], cfg.head_dim)):
+            return None
+        if torch.is_autocast_enabled():
+            return None
+        s = _structure(self, tokens.device)
+        if s is None:
+            return None
+        layers = s.__dict__.get("ordered")
+        if layers is None:
+            names = (("ln1.weight", "qkv.weight", "proj.weight", "ln2.weight", "gate_up.weight", "down.weight") if rope else
+                     [f"{m}.{k}" for m in ("ln1", "qkv", "proj", "ln2", "up", "down") for k in ("weight", "bias")])
+            s.ordered = layers = [s.params[f"blocks.{i}.{n}"] for i in range(cfg.n_layers) for n in names]
+        head = self.head_weight()
+        if hasattr(head, "_bf16"):   # a trainer keeps bf16 copies of the matrices up to date
+            layers = [getattr(p, "_bf16", p) if p.dim() == 2 else p for p in layers]
+            head = head._bf16
+        tables = _rope_tables(tokens.shape[1], cfg.head_dim, tokens.device) if rope else (None, None)
+        p = s.params
+        return _C.decoder_fwd(tokens, p["tok.weight"], p.get("pos.weight"), layers, p["ln_f.weight"], p.get("ln_f.bias"), head,
+                              cfg.n_heads, cfg.eps, *tables)
+
     def head_weight(self) -> torch.Tensor:
         return self.tok.weight if self.head is None else self.head.weight
 
     def forward(self, tokens: torch.Tensor, targets: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Returns logits [B, S, V] (bf16), or the mean next-token loss when targets are given."""
+        if targets is None and not torch.is_grad_enabled() and _FUSE_LAYER and self._native(tokens):
+            logits = self._forward_without_gradients(tokens)
+            if logits is not None:
+                return logits
         h = self.hidden(tokens)
         native = self._native(tokens)
         w = self.head_weight()

@@ -266,6 +266,46 @@ class CausalAttentionFn(torch.autograd.Function):
         return _C.attn_bwd(q5, o, d, lse, ctx.scale), None
 
 
+class DecoderLayerFn(torch.autograd.Function):
+    """A whole pre-LayerNorm GELU decoder layer as one autograd node (csrc/bindings/bind_layers.cpp).  params: weight and bias
+    of first norm, qkv, output projection, second norm, up and down projection."""
+
+    MATRICES = (2, 4, 8, 10)
+
+    @staticmethod
+    def forward(ctx, x, heads, eps, *params):
+        w = list(params)
+        todo = []
+        for i in DecoderLayerFn.MATRICES:
+            w16 = getattr(w[i], "_bf16", None)   # a trainer keeps one up to date
+            if w16 is None:
+                todo.append(i)
+            else:
+                w[i] = w16
+        if todo:
+            for i, w16 in zip(todo, _C.cast_many([w[i] for i in todo])):
+                w[i] = w16
+        B, S = x.shape[0], x.shape[1]
+        out, slab = _C.decoder_layer_fwd(x, w, B, S, heads, eps)
+        ctx.save_for_backward(x, slab, *w)
+        ctx.params, ctx.heads = params, heads
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        x, slab, *w = ctx.saved_tensors
+        params = ctx.params
+        sinks = [getattr(p, "_grad_sink", None) for p in params]
+        direct = all(s is not None for s in sinks)
+        dx, grads = _C.decoder_layer_bwd(dout if dout.is_contiguous() else dout.contiguous(), x, slab, w, sinks if direct else [],
+                                         x.shape[0], x.shape[1], ctx.heads)
+        if not direct:
+            return (dx, None, None, *grads)
+        for p in reversed(params):
+            _notify(p)
+        return (dx, None, None) + (None,) * len(params)
+
+
 class RopeQkvFn(torch.autograd.Function):
     """Fused QKV projection output [B, S, 3, H, hd] -> rotated q, rotated k, v, each [B, H, S, hd] (views).  One kernel
     each way: the backward turns dq and dk back and gathers all three into the gradient of the whole projection."""

@@ -83,7 +83,7 @@ class DDPTrainer:
         # GEMMs that each want every SM take turns, set-up and tail included; capped at 88 of 148 CTAs each they mostly
         # run side by side (a second round of tiles costs a CTA about a third more, not twice).  Measured on the 70M
         # decoder: 4.72 -> 4.49 ms per step on one GPU, 4.97 -> 4.68 on two (with 40 SMs kept for the collectives).
-        side_on = device.type == "cuda" and os.environ.get("MCCL_SIDE_WGRAD", "1") != "0"
+        side_on = device.type == "cuda" and os.environ.get("MCCL_SIDE_WGRAD", "0") != "0"
         self._bwd_main_ctas = int(os.environ.get("MCCL_BWD_MAIN_CTAS", "88" if side_on else "0")) if device.type == "cuda" else 0
         self._bwd_side_ctas = int(os.environ.get("MCCL_BWD_SIDE_CTAS", "88" if side_on else "0")) if device.type == "cuda" else 0
         # without an explicit setting the graph is captured with and without the caps and the faster one is kept
@@ -104,13 +104,13 @@ class DDPTrainer:
         # weight-gradient stream while backward continues.  Off by default: measured 4.79 ms per step against 4.72 with
         # one update at the end (AdamW's traffic slows the GEMMs it runs beside by more than it hides).
         self._local_overlap = (self.world == 1 and device.type == "cuda"
-                               and os.environ.get("MCCL_SIDE_WGRAD", "1") != "0"
+                               and os.environ.get("MCCL_SIDE_WGRAD", "0") != "0"
                                and os.environ.get("MCCL_OVERLAP_ADAMW", "0") == "1")
         self._per_bucket = self.world > 1 or self._local_overlap
         self._body_done = None   # event on the side stream: every non-tail bucket has been reduced
         # weight-gradient GEMMs on a stream of their own, beside the input-gradient chain (MCCL_SIDE_WGRAD=0: in line)
         self.wgrad_stream = None
-        if device.type == "cuda" and os.environ.get("MCCL_SIDE_WGRAD", "1") != "0":
+        if device.type == "cuda" and os.environ.get("MCCL_SIDE_WGRAD", "0") != "0":
             self.wgrad_stream = torch.cuda.Stream(device=device)
         self._flatten(bucket_mb, last_bucket_mb)
         self.step_t = torch.zeros((), device=device, dtype=torch.float32)
