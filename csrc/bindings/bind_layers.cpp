@@ -144,6 +144,24 @@ ops::GemmArgs weight_gradient(const bf16* dy, const bf16* x, float* dw, int toke
   return g;
 }
 
+// What the weight gradients of a layer are made of.
+struct Pending {
+  const bf16 *dout, *dz, *dqkv, *dy;
+  Slab s;
+  float *down, *up, *qkv, *proj;
+};
+void weight_gradients(const std::vector<Pending>& layers, const Dims& d, cudaStream_t stream) {
+  const int T = d.tokens(), D = d.D, F = d.F;
+  std::vector<ops::GemmArgs> args;
+  for (const Pending& p : layers) {
+    args.push_back(weight_gradient(p.dout, p.s.act, p.down, T, D, F));
+    args.push_back(weight_gradient(p.dz, p.s.h2, p.up, T, F, D));
+    args.push_back(weight_gradient(p.dqkv, p.s.h1, p.qkv, T, 3 * D, D));
+    args.push_back(weight_gradient(p.dy, p.s.o, p.proj, T, D, D));
+  }
+  check(ops::gemm_group(args.data(), static_cast<int>(args.size()), stream), "weight gradients");
+}
+
 void layer_forward(const bf16* x, bf16* out, const Weights& w, const Slab& s, const Dims& d, float eps, bool keep, cudaStream_t st) {
   const int T = d.tokens(), D = d.D, F = d.F;
   const float scale = 1.f / std::sqrt(static_cast<float>(d.head_dim()));
@@ -184,10 +202,11 @@ void bind_layers(py::module_& m) {
     layer_forward(bf(x), bf(out), w, s, d, static_cast<float>(eps), true, at::cuda::getCurrentCUDAStream(x.get_device()).stream());
     return std::make_pair(out, slab);
   });
-  // (gradient of x, gradients of the parameters).  The latter are ADDED into `grads` (fp32, one per parameter, same order)
-  // where given, else returned as views of one new buffer.
+  // (gradient of x, gradients of the parameters, see decoder_layer_wgrads).  The gradients of the parameters are ADDED into `grads` (fp32, one per parameter, same order)
+  // where given, else returned as views of one new buffer.  With defer, those of the four matrices are left for
+  // decoder_layer_wgrads.
   m.def("decoder_layer_bwd", [](const at::Tensor& dout, const at::Tensor& x, const at::Tensor& slab, const std::vector<at::Tensor>& params,
-                                std::vector<at::Tensor> grads, int64_t B, int64_t S, int64_t H) {
+                                std::vector<at::Tensor> grads, int64_t B, int64_t S, int64_t H, bool defer) {
     const Dims d = dims_of(x, B, S, H, params.at(UP_B).numel());
     c10::cuda::CUDAGuard guard(x.device());
     const Weights w = weights_of(params, d);
@@ -227,11 +246,40 @@ void bind_layers(py::module_& m) {
     input_gradient(dqkv, w.qkv, dh, T, 3 * D, D, nullptr, nullptr, st, "qkv projection backward");
     check(ops::norm_bwd_fused(dh, bf(x), w.ln1_w, s.mean1, s.rstd1, bf(dx), dy, g[LN1_W], g[LN1_B], nullptr, nullptr, T, D, true, st),
           "first norm backward");
-    const ops::GemmArgs wg[4] = {
-        weight_gradient(bf(dout), s.act, g[DOWN_W], T, D, F), weight_gradient(dz, s.h2, g[UP_W], T, F, D),
-        weight_gradient(dqkv, s.h1, g[QKV_W], T, 3 * D, D), weight_gradient(dy, s.o, g[PROJ_W], T, D, D)};
-    check(ops::gemm_group(wg, 4, st), "weight gradients");
-    return std::make_pair(dx, grads);
+    if (!defer) {
+      const Pending p = {bf(dout), dz, dqkv, dy, s, g[DOWN_W], g[UP_W], g[QKV_W], g[PROJ_W]};
+      weight_gradients({p}, d, st);
+    }
+    return std::make_tuple(dx, grads, defer ? tmp : at::Tensor());
+  });
+  // The weight gradients of layers whose backward was called with defer: (output gradient, slab, the third result of
+  // decoder_layer_bwd, gradient buffers) of each; the buffers are added into.
+  m.def("decoder_layer_wgrads", [](const std::vector<std::tuple<at::Tensor, at::Tensor, at::Tensor, std::vector<at::Tensor>>>& layers, int64_t B,
+                                   int64_t S, int64_t H) {
+    if (layers.empty()) return;
+    const at::Tensor& first = std::get<0>(layers[0]);
+    const Dims d = dims_of(first, B, S, H, std::get<3>(layers[0]).at(UP_B).numel());
+    c10::cuda::CUDAGuard guard(first.device());
+    const int64_t TD = static_cast<int64_t>(d.tokens()) * d.D;
+    std::vector<Pending> pending;
+    for (const auto& [dout, slab, tmp, grads] : layers) {
+      Pending p;
+      need(dout, at::kBFloat16, TD, "output gradient");
+      need(tmp, at::kBFloat16, TD * 6 + static_cast<int64_t>(d.tokens()) * d.F, "gradients between the kernels");
+      MCCL_CHECK_TENSOR(slab.is_cuda() && slab.numel() == Slab::place(&p.s, nullptr, d) && grads.size() == kParams, "decoder layer: layers of one size expected");
+      Slab::place(&p.s, slab.data_ptr<uint8_t>(), d);
+      for (int i = 0; i < kParams; ++i) need(grads[i], at::kFloat, param_numel(d, i), "gradient buffer");
+      p.dout = bf(dout);
+      p.dy = bf(tmp) + TD;
+      p.dqkv = bf(tmp) + 3 * TD;
+      p.dz = bf(tmp) + 6 * TD;
+      p.down = grads[DOWN_W].data_ptr<float>();
+      p.up = grads[UP_W].data_ptr<float>();
+      p.qkv = grads[QKV_W].data_ptr<float>();
+      p.proj = grads[PROJ_W].data_ptr<float>();
+      pending.push_back(p);
+    }
+    weight_gradients(pending, d, at::cuda::getCurrentCUDAStream(first.get_device()).stream());
   });
   // bf16 copies of fp32 tensors: views of one buffer, made by one launch (or few).
   m.def("cast_many", [](const std::vector<at::Tensor>& in) {

@@ -160,7 +160,18 @@ void bind_ops(py::module_& m) {
                             "gemm: colsum must have N elements and goes with a bf16 output, an MN-major B and no bias, activation or residual");
           g.colsum = colsum->data_ptr<float>();
         }
+        // A contraction far longer than the output is wide (the input gradient of an LM head: 32000 against 512) has too few
+        // tiles for the SMs; its fp32 partial sums go through a workspace (4096 x 512 x 32000: 123 -> 108 us).
+        at::Tensor partial;
+        if (!out_fp32 && !out.has_value() && g.epilogue == ops::EPI_NONE && !g.residual && !g.mul && !g.colsum && K >= 8 * N && K >= 4096 &&
+            ((M + 127) / 128) * ((N + 127) / 128) < 4 * ops::gemm_sm_count()) {
+          partial = at::zeros({M, N}, a.options().dtype(at::kFloat));
+          g.d = partial.data_ptr();
+          g.d_fp32 = g.accumulate = true;
+          g.ldd = static_cast<int>(N);
+        }
         cudaError_t rc = ops::gemm_bf16_tn(g, stream_of(a));
+        if (rc == cudaSuccess && partial.defined()) rc = ops::cast_f32_bf16(partial.data_ptr<float>(), bf(d), M * N, stream_of(a));
         MCCL_CHECK_T(rc == cudaSuccess, CudaError,
                      "gemm_bf16 [" << M << "x" << N << "x" << K << ", lda " << g.lda << ", ldb " << g.ldb << ", ldd " << g.ldd
                                    << "] failed: " << cudaGetErrorString(rc) << " " << ops::gemm_last_reason());
@@ -170,7 +181,7 @@ void bind_ops(py::module_& m) {
       py::arg("out") = py::none(), py::arg("accumulate") = false, py::arg("a_t") = false, py::arg("b_t") = false,
       py::arg("residual") = py::none(), py::arg("mul") = py::none(), py::arg("colsum") = py::none());
 
-  // dW_i[N_i, K_i] = dY_i[tokens, N_i]^T · X_i[tokens, K_i], four products per launch.  items: (dY, X, dW or None); with
+  // dW_i[N_i, K_i] = dY_i[tokens, N_i]^T · X_i[tokens, K_i], sixteen products per launch.  items: (dY, X, dW or None); with
   // accumulate every dW is given and added into.  Returns the dW.
   m.def(
       "gemm_group",

@@ -256,28 +256,35 @@ __global__ void __launch_bounds__(256) norm_bwd_fused_kernel(const __nv_bfloat16
         reinterpret_cast<uint4*>(dx)[at + 32 * k] = pack8(o);
       }
   }
-  auto reduce = [&](const auto& acc, float* out) {
-    if (out == nullptr) return;   // uniform over the block
-    __syncthreads();
+  // [set][warp][column]: every set of sums at once, one barrier, then a column's eight parts to one thread
+  constexpr int kSets = 1 + (kLayerNorm ? 1 : 0) + (kSums ? 2 : 0);
+  auto park = [&](const auto& acc, int set) {
 #pragma unroll
     for (int k = 0; k < kVecs; ++k) {
-      float4* p = reinterpret_cast<float4*>(red + (warp * kVecs + k) * 256 + lane * 8);
+      float4* p = reinterpret_cast<float4*>(red + ((set * 8 + warp) * kVecs + k) * 256 + lane * 8);
       p[0] = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
       p[1] = make_float4(acc[k][4], acc[k][5], acc[k][6], acc[k][7]);
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < dim; c += 256) {
+  };
+  park(aw, 0);
+  if (kLayerNorm) park(ab, 1);
+  if constexpr (kSums) {
+    park(sa, kSets - 2);
+    park(sd, kSets - 1);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int set = 0; set < kSets; ++set) {
+    float* out = set == 0 ? dw : (kLayerNorm && set == 1 ? db : (set == kSets - 2 ? sum_add : sum_dx));
+    if (out == nullptr) continue;
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k) {
+      const int c = k * 256 + threadIdx.x;
       float t = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) t += red[i * kVecs * 256 + c];
-      atomicAdd(out + c, t);
+      for (int i = 0; i < 8; ++i) t += red[(set * 8 + i) * kVecs * 256 + c];
+      if (c < dim) atomicAdd(out + c, t);
     }
-  };
-  reduce(aw, dw);
-  if (kLayerNorm) reduce(ab, db);
-  if constexpr (kSums) {
-    reduce(sa, sum_add);
-    reduce(sd, sum_dx);
   }
 }
 
@@ -440,30 +447,36 @@ cudaError_t norm_bwd_fused(const __nv_bfloat16* dy, const __nv_bfloat16* x, cons
   const int most = vecs <= 2 ? 2 * 148 : 148;
   if (blocks > most) blocks = most;
   if (blocks < 1) return cudaSuccess;
-#define MCCL_NORM_BWD(LN, V, S)                                                                                                  \
-  MCCL_LAUNCH_PDL((norm_bwd_fused_kernel<LN, V, S>), blocks, 256, 8 * V * 256 * sizeof(float), stream, dy, x, w, mean, rstd, dx, \
-                  dx_add, dw, db, sum_add, sum_dx, rows, dim)
-#define MCCL_NORM_BWD_V(LN, S) \
-  (vecs == 1 ? MCCL_NORM_BWD(LN, 1, S) : vecs == 2 ? MCCL_NORM_BWD(LN, 2, S) : vecs == 3 ? MCCL_NORM_BWD(LN, 3, S) : MCCL_NORM_BWD(LN, 4, S))
-  if (vecs > 4) {
-    static std::atomic<bool> configured{false};
-    if (!configured.load(std::memory_order_acquire)) {
-      cudaError_t rc = cudaFuncSetAttribute(norm_bwd_fused_kernel<false, 8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536);
+  auto go = [&](auto kernel, int v, int sets, std::atomic<bool>& configured) -> cudaError_t {
+    const int smem = sets * 8 * v * 256 * static_cast<int>(sizeof(float));
+    if (smem > 48 * 1024 && !configured.load(std::memory_order_acquire)) {
+      cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       if (rc != cudaSuccess) return rc;
       configured.store(true, std::memory_order_release);
     }
-    MCCL_NORM_BWD(false, 8, false);
-  } else if (layernorm) {
-    if (sums) MCCL_NORM_BWD_V(true, true);
-    else MCCL_NORM_BWD_V(true, false);
-  } else {
-    if (sums) MCCL_NORM_BWD_V(false, true);
-    else MCCL_NORM_BWD_V(false, false);
+    MCCL_LAUNCH_PDL(kernel, blocks, 256, smem, stream, dy, x, w, mean, rstd, dx, dx_add, dw, db, sum_add, sum_dx, rows, dim);
+    count_launch();
+    return ::mccl::launch_status();
+  };
+#define MCCL_NORM_BWD(LN, V, S)                                                                                     \
+  {                                                                                                                 \
+    static std::atomic<bool> configured{false};                                                                     \
+    return go(norm_bwd_fused_kernel<LN, V, S>, V, 1 + (LN ? 1 : 0) + (S ? 2 : 0), configured);                      \
   }
+#define MCCL_NORM_BWD_V(LN, S)              \
+  switch (vecs) {                           \
+    case 1: MCCL_NORM_BWD(LN, 1, S)         \
+    case 2: MCCL_NORM_BWD(LN, 2, S)         \
+    case 3: MCCL_NORM_BWD(LN, 3, S)         \
+    default: MCCL_NORM_BWD(LN, 4, S)        \
+  }
+  if (vecs > 4) MCCL_NORM_BWD(false, 8, false)
+  if (layernorm && sums) MCCL_NORM_BWD_V(true, true)
+  if (layernorm) MCCL_NORM_BWD_V(true, false)
+  if (sums) MCCL_NORM_BWD_V(false, true)
+  MCCL_NORM_BWD_V(false, false)
 #undef MCCL_NORM_BWD_V
 #undef MCCL_NORM_BWD
-  count_launch();
-  return ::mccl::launch_status();
 }
 
 cudaError_t colsum_bf16(const __nv_bfloat16* in, float* out, float* scratch, int rows, int dim, cudaStream_t stream) {

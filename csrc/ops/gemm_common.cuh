@@ -50,6 +50,52 @@ __device__ __forceinline__ void gelu_value_grad(float x, float& value, float& gr
   grad = fmaf(x * 0.39894228f, e, cdf);
 }
 
+// The same for two values at once in packed fp32 arithmetic (fma.rn.f32x2 and friends: two results per issue slot), with the
+// factor one half of the distribution function folded into the coefficients: 11 instructions per value instead of 19.
+struct Packed2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ Packed2 pack2(float lo, float hi) {
+  Packed2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(Packed2 p, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p.v)); }
+__device__ __forceinline__ Packed2 fma2(Packed2 a, Packed2 b, Packed2 c) {
+  Packed2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ Packed2 mul2(Packed2 a, Packed2 b) {
+  Packed2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+template <bool kGrad>
+__device__ __forceinline__ void gelu_two(float& x0, float& x1, float& d0, float& d1) {
+  const Packed2 x = pack2(x0, x1);
+  const Packed2 den = fma2(pack2(fabsf(x0), fabsf(x1)), pack2(0.231641888f, 0.231641888f), pack2(1.f, 1.f));
+  float a, b;
+  unpack2(den, a, b);
+  const Packed2 t = pack2(rcp_approx(a), rcp_approx(b));
+  unpack2(mul2(mul2(x, x), pack2(-0.72134752f, -0.72134752f)), a, b);
+  const Packed2 e = pack2(exp2f(a), exp2f(b));
+  Packed2 h = fma2(t, pack2(0.5307027145f, 0.5307027145f), pack2(-0.7265760135f, -0.7265760135f));
+  h = fma2(t, h, pack2(0.7107068705f, 0.7107068705f));
+  h = fma2(t, h, pack2(-0.142248368f, -0.142248368f));
+  h = fma2(t, h, pack2(0.127414796f, 0.127414796f));
+  h = mul2(mul2(t, h), e);   // half of erfc(|x| / sqrt(2))
+  unpack2(h, a, b);
+  const Packed2 cdf = pack2(0.5f + copysignf(0.5f - a, x0), 0.5f + copysignf(0.5f - b, x1));
+  if (kGrad) unpack2(fma2(mul2(x, pack2(0.39894228f, 0.39894228f)), e, cdf), d0, d1);
+  unpack2(mul2(x, cdf), x0, x1);
+}
+
 __device__ __forceinline__ float gelu_erf(float x) {
   float v, d;
   gelu_value_grad(x, v, d);
@@ -185,6 +231,11 @@ __device__ __forceinline__ uint4* stage_unit(uint8_t* stage, int r, int u) {
   return reinterpret_cast<uint4*>(stage + r * 128 + ((u ^ (r & 7)) << 4));
 }
 
+// The same for rows of 64 bytes (32 bf16 columns, 64-byte swizzle).
+__device__ __forceinline__ uint4* stage_unit64(uint8_t* stage, int r, int u) {
+  return reinterpret_cast<uint4*>(stage + r * 64 + ((u ^ ((r >> 1) & 3)) << 4));
+}
+
 __device__ __forceinline__ uint2 pack4(const float4& v) {
   uint2 pk;
   *reinterpret_cast<__nv_bfloat162*>(&pk.x) = __floats2bfloat162_rn(v.x, v.y);
@@ -288,7 +339,8 @@ inline bool encode_map(CUtensorMap* map, const void* base, int rows, int cols, i
 
 // Output matrix [rows, cols] (bf16, or fp32 when `fp32`) as the target of TMA stores of 32-row boxes whose rows are
 // 128 bytes (64 bf16 or 32 fp32 columns), 128-byte swizzle: the layout of an epilogue warp's staging buffer.
-inline bool encode_out_map(CUtensorMap* map, const void* base, int rows, int cols, int ld_elems, bool fp32) {
+// With `half`, boxes of 32 bf16 columns (64-byte rows and swizzle).
+inline bool encode_out_map(CUtensorMap* map, const void* base, int rows, int cols, int ld_elems, bool fp32, bool half = false) {
   const CuDriver& cu = CuDriver::get();
   if (!cu.loaded || !cu.TensorMapEncodeTiled) return false;
   int device = 0;
@@ -297,11 +349,11 @@ inline bool encode_out_map(CUtensorMap* map, const void* base, int rows, int col
   const int es = fp32 ? 4 : 2;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld_elems) * es};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / es), 32u};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>((half ? 64 : 128) / es), 32u};
   cuuint32_t estr[2] = {1, 1};
   CUresult rc = cu.TensorMapEncodeTiled(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                                         const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                        half ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return rc == CUDA_SUCCESS;
 }

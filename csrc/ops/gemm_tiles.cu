@@ -35,27 +35,32 @@ struct Plan {
   int splits = 1;
 };
 
+constexpr double kRunsBytes = 80e6;   // of 126 MB of L2, which also holds the output
 constexpr int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// Clocks of a product on one kind of tile.  Fitted to graphs of back-to-back launches (70M to 1.3B shapes):
-// per 64 of K a 128 x 64 tile takes 260 clocks, a 128 x 128 tile 350 and a 256 x 256 pair tile 515; an epilogue 1500 /
-// 2000 / 4000, hidden behind the next tile's main loop when there is one; launch and set-up 3500, a pair's two cluster
-// barriers 2000 more.
-double cost(int bn, int tiles, int k, int workers, int splits, bool gelu) {
-  const bool pair = bn == 256;
+// Clocks of a product on one kind of tile, fitted to graphs of back-to-back launches (70M to 1.3B shapes) and the kernel's
+// timeline: per 64 of K a 128 x 64 tile takes 260 clocks, a 128 x 128 tile 350 and a 256 x 256 pair tile 515 (its MMAs
+// need 512); an epilogue 1500 / 2000 / 4000, fp32 sums added into memory 1800 / 2600 / 7000, hidden behind the next tile's
+// main loop when there is one; launch and set-up 3500, a pair's two cluster barriers 2000 more.
+constexpr double kPer64[3] = {260, 350, 515}, kEpilogue[3] = {1500, 2000, 4000}, kAdding[3] = {1800, 2600, 7000};
+int kind_of(int bn) { return bn == 64 ? 0 : (bn == 128 ? 1 : 2); }
+
+double cost(int bn, int tiles, int k, int workers, int splits, bool gelu, bool adding) {
+  const int kind = kind_of(bn);
   const int rounds = ceil_div(tiles * splits, workers);
-  const double per64 = pair ? 515 : (bn == 128 ? 350 : 260);
-  double epilogue = pair ? 4000 : (bn == 128 ? 2000 : 1500);
+  double epilogue = adding ? kAdding[kind] : kEpilogue[kind];
   if (gelu) epilogue *= 2.5;
-  const double main_loop = per64 * ceil_div(k, 64) / splits;
+  const double main_loop = kPer64[kind] * ceil_div(k, 64) / splits;
   const double round = main_loop > epilogue ? main_loop : epilogue;
-  return 3500 + (pair ? 2000 : 0) + (rounds - 1) * round + main_loop + epilogue + (splits > 1 ? 1500 : 0);
+  return 3500 + (kind == 2 ? 2000 : 0) + (rounds - 1) * round + main_loop + epilogue;
 }
 
 Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, bool gelu, bool splittable) {
   Plan best;
   double best_cost = 0;
   const int k = args[0].k;
+  double operand_bytes = 0;
+  for (int p = 0; p < count; ++p) operand_bytes += 2.0 * k * (static_cast<double>(args[p].m) + args[p].n);
   for (int bn : {64, 128, 256}) {
     if (forced ? bn != forced : false) continue;
     if (bn == 256 && (gelu || pairs < 1)) continue;
@@ -63,9 +68,22 @@ Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, boo
     int tiles = 0;
     for (int p = 0; p < count; ++p) tiles += ceil_div(args[p].m, bn == 256 ? 256 : 128) * ceil_div(args[p].n, bn);
     const int num_kb = ceil_div(k, 64);
+    if (splittable && operand_bytes < kRunsBytes && static_cast<long long>(tiles) * num_kb >= 8ll * workers) {
+      // Equal runs of k-blocks for every worker: no last round that leaves SMs idle, at the price of up to two more partial
+      // tiles per worker.  Workers are then at different places of K, so operands that do not stay in L2 are read several
+      // times (the 262 MB of an LM head's gradient: 4096 x 512 x 32000 131 us against 123).
+      const double run = kPer64[kind_of(bn)] * (static_cast<double>(tiles) * num_kb / workers);
+      const double c = 3500 + (bn == 256 ? 2000 : 0) + run + 1.5 * kAdding[kind_of(bn)];
+      if (best.bn == 0 || c < best_cost) {
+        best_cost = c;
+        best.bn = bn;
+        best.splits = 0;
+        best.workers = workers;
+      }
+    }
     for (int s = 1; s <= 16; s = s < 4 ? s + 1 : s + 2) {
       if (s > 1 && (!splittable || num_kb / s < 4 || tiles * (s - 1) >= 2 * workers)) break;
-      const double c = cost(bn, tiles, k, workers, s, gelu);
+      const double c = cost(bn, tiles, k, workers, s, gelu, splittable && (s > 1 || args[0].accumulate));
       if (best.bn == 0 || c < best_cost) {
         best_cost = c;
         best.bn = bn;

@@ -40,9 +40,9 @@ namespace tiles {
 // OUT_BF16_SUM: the bf16 output and, added into GemmDev::colsum, its column sums (a bias gradient).
 enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3 };
 
-// One product, or several with the same K whose tiles one launch works through (the weight gradients of a layer: alone,
-// a 512 x 2048 gradient is 64 tiles and leaves half the SMs without one; together they fill two rounds).
-constexpr int kMaxGroup = 4;
+// One product, or several with the same K whose tiles one launch works through (the weight gradients of one or more layers:
+// alone, a 512 x 2048 gradient is 64 tiles and leaves half the SMs without one).
+constexpr int kMaxGroup = 16;
 template <int kMax>
 struct Problems {
   CUtensorMap a[kMax], b[kMax], d[kMax];
@@ -50,20 +50,23 @@ struct Problems {
   int m[kMax], n[kMax];
   int first[kMax + 1];        // first tile of each product
   int n_tiles[kMax];
+  int atoms[kMax];            // bit 0 / 1: the MN-major A / B has whole groups of 64 columns and is fetched by one load
   int count;
 };
 
-template <int BN, bool kPair>
+template <int BN, bool kPair, bool kGelu = false>
 struct Shape {
-  static constexpr int kStages = kPair ? 5 : (BN == 64 ? 8 : 6);
+  static constexpr int kStages = kPair ? 5 : (BN == 64 ? 8 : (kGelu ? 5 : 6));
   static constexpr int kRowsB = kPair ? BN / 2 : BN;   // rows of the B tile this CTA loads
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBBytes = kRowsB * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kEpiWarps = BN == 64 ? 4 : 8;
+  // GELU: 11 instructions per value and two of them long; twice the warps, half the columns each, so that more chains are in
+  // flight per scheduler, and a staging buffer per output
+  static constexpr int kEpiWarps = (BN == 64 ? 4 : 8) * (kGelu ? 2 : 1);
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
   static constexpr int kCols = BN / (kEpiWarps / 4);   // accumulator columns per epilogue warp
-  static constexpr int kBufs = kCols / 64;             // 4 KB staging buffers per epilogue warp
+  static constexpr int kBufs = kGelu ? 1 : kCols / 64;             // 4 KB staging buffers per epilogue warp
   static constexpr int kTiles = kStages * kStageBytes;
   static constexpr int kStagingOff = kTiles;
   static constexpr int kBarOff = kStagingOff + kEpiWarps * kBufs * 4096;
@@ -112,6 +115,19 @@ __device__ __forceinline__ void load_2d_pair(void* dst, const CUtensorMap* map, 
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y)
+      : "memory");
+}
+// All 64-column groups of an MN-major tile at once: the matrix [K, MN] seen as [MN / 64][K][64].
+__device__ __forceinline__ void load_groups(void* dst, const CUtensorMap* map, uint64_t* bar, int group, int k) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(bar)), "r"(0), "r"(k), "r"(group)
+      : "memory");
+}
+__device__ __forceinline__ void load_groups_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int group, int k) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(tc::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(0), "r"(k), "r"(group)
       : "memory");
 }
 __device__ __forceinline__ void mma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
@@ -168,10 +184,10 @@ __device__ __forceinline__ void unpack8(const uint4& pk, float (&v)[8]) {
 }
 
 template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut, int kMax>
-__global__ void __launch_bounds__(Shape<BN, kPair>::kThreads, 1)
+__global__ void __launch_bounds__(Shape<BN, kPair, kOut == OUT_GELU>::kThreads, 1)
 gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits) {
   constexpr bool kBf16 = kOut == OUT_BF16 || kOut == OUT_BF16_SUM;
-  using S = Shape<BN, kPair>;
+  using S = Shape<BN, kPair, kOut == OUT_GELU>;
   constexpr int kStages = S::kStages, kTileM = kPair ? 2 * BM : BM;
   extern __shared__ uint8_t smem_raw[];
   // the same offset in both CTAs of a pair: the MMA addresses the peer's operands by this CTA's offsets
@@ -189,8 +205,13 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = kPair ? cluster_ctarank() : 0u;
   const int worker = static_cast<int>(kPair ? blockIdx.x >> 1 : blockIdx.x), workers = static_cast<int>(kPair ? gridDim.x >> 1 : gridDim.x);
-  const int total = P.first[P.count] * splits;
   const int all_kb = (g.k + BK - 1) / BK;
+  // splits >= 1: work items are (tile, part of K), taken in turn.  splits == 0: every worker gets an equal run of k-blocks,
+  // across tile borders, and adds what it has of each tile into D.
+  const int tiles = P.first[P.count];
+  const bool runs = kOut == OUT_F32 && splits == 0;
+  const int work_begin = runs ? static_cast<int>(static_cast<long long>(tiles) * all_kb * worker / workers) : worker;
+  const int work_end = runs ? static_cast<int>(static_cast<long long>(tiles) * all_kb * (worker + 1) / workers) : tiles * splits;
 
   if (warp == 0 && tc::elect_one()) {
     for (int s = 0; s < kStages; ++s) {
@@ -228,16 +249,25 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
   pdl_wait();   // set-up done: from here on operands are read and outputs written
   if (tl_t0 != 0ull && tl_detail(g.tl)) tl_mark(g.tl, tl_t0, tl_now(), TL_GEMM_PHASE, 0u);
 
-  // product, tile row, tile column and range of k-blocks of work item w
+  // product, tile row, tile column and range of k-blocks of the work item at w, and where the next one is
   struct Item {
-    int p, m_blk, n_blk, kb0, kb1;
+    int p, m_blk, n_blk, kb0, kb1, next;
   };
   auto item = [&](int w) {
     Item it;
-    int t = splits > 1 ? w / splits : w;
-    const int s = w - t * splits;
-    it.kb0 = splits > 1 ? all_kb * s / splits : 0;
-    it.kb1 = splits > 1 ? all_kb * (s + 1) / splits : all_kb;
+    int t;
+    if (runs) {
+      t = w / all_kb;
+      it.kb0 = w - t * all_kb;
+      it.kb1 = work_end - w < all_kb - it.kb0 ? it.kb0 + work_end - w : all_kb;
+      it.next = w + it.kb1 - it.kb0;
+    } else {
+      t = splits > 1 ? w / splits : w;
+      const int s = w - t * splits;
+      it.kb0 = splits > 1 ? all_kb * s / splits : 0;
+      it.kb1 = splits > 1 ? all_kb * (s + 1) / splits : all_kb;
+      it.next = w + workers;
+    }
     it.p = 0;
     if constexpr (kMax > 1) {
       while (it.p + 1 < P.count && t >= P.first[it.p + 1]) ++it.p;
@@ -254,8 +284,9 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
       bool ok = true;
       int s = 0;
       uint32_t parity = 1;   // a fresh barrier counts as the phase before the first: the first round does not wait
-      for (int w = worker; w < total && ok; w += workers) {
+      for (int w = work_begin; w < work_end && ok;) {
         const Item it = item(w);
+        w = it.next;
         const CUtensorMap* map_a = &P.a[it.p];
         const CUtensorMap* map_b = &P.b[it.p];
         const int a_row = it.m_blk * kTileM + static_cast<int>(rank) * BM;
@@ -269,13 +300,17 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           if constexpr (kPair) {
             if (rank == 0) tc::mbar_expect_tx(&full[s], 2 * S::kStageBytes);
             const uint32_t bar = leader_addr(&full[s]);
-            if (kAMn) {
+            if (kAMn && (P.atoms[it.p] & 1)) {
+              load_groups_pair(a_dst, map_a, bar, a_row / 64, k0);
+            } else if (kAMn) {
 #pragma unroll
               for (int q = 0; q < BM / 64; ++q) load_2d_pair(a_dst + q * (BK * 128), map_a, bar, a_row + q * 64, k0);
             } else {
               load_2d_pair(a_dst, map_a, bar, k0, a_row);
             }
-            if (kBMn) {
+            if (kBMn && (P.atoms[it.p] & 2)) {
+              load_groups_pair(b_dst, map_b, bar, b_row / 64, k0);
+            } else if (kBMn) {
 #pragma unroll
               for (int q = 0; q < S::kRowsB / 64; ++q) load_2d_pair(b_dst + q * (BK * 128), map_b, bar, b_row + q * 64, k0);
             } else {
@@ -283,13 +318,17 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
             }
           } else {
             tc::mbar_expect_tx(&full[s], S::kStageBytes);
-            if (kAMn) {
+            if (kAMn && (P.atoms[it.p] & 1)) {
+              load_groups(a_dst, map_a, &full[s], a_row / 64, k0);
+            } else if (kAMn) {
 #pragma unroll
               for (int q = 0; q < BM / 64; ++q) tc::tma_load_2d(a_dst + q * (BK * 128), map_a, &full[s], a_row + q * 64, k0);
             } else {
               tc::tma_load_2d(a_dst, map_a, &full[s], k0, a_row);
             }
-            if (kBMn) {
+            if (kBMn && (P.atoms[it.p] & 2)) {
+              load_groups(b_dst, map_b, &full[s], b_row / 64, k0);
+            } else if (kBMn) {
 #pragma unroll
               for (int q = 0; q < S::kRowsB / 64; ++q) tc::tma_load_2d(b_dst + q * (BK * 128), map_b, &full[s], b_row + q * 64, k0);
             } else {
@@ -317,8 +356,9 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
       bool ok = true;
       int s = 0, i = 0;
       uint32_t parity = 0;
-      for (int w = worker; w < total; w += workers, ++i) {
+      for (int w = work_begin; w < work_end; ++i) {
         const Item it = item(w);
+        w = it.next;
         const int kb0 = it.kb0, kb1 = it.kb1, buf = i & 1;
         if (i >= 2) {
           ok = wait(&acc_empty[buf], ((i >> 1) - 1) & 1, abort_flag);
@@ -367,8 +407,9 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
     bool ok = true;
     int i = 0;
     uint32_t xparity = 0;   // one bit per staging buffer
-    for (int w = worker; w < total; w += workers, ++i) {
+    for (int w = work_begin; w < work_end; ++i) {
       const Item it = item(w);
+      w = it.next;
       const CUtensorMap* map_d = &P.d[it.p];
       const int m = P.m[it.p], n = P.n[it.p];
       const int buf = i & 1;
@@ -431,8 +472,46 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           }
           __syncwarp();
         }
+      } else if constexpr (kOut == OUT_GELU) {
+        uint32_t r[32];
+        tc::tmem_ld_32x32(taddr, r);
+        tc::tmem_ld_wait();
+        last_read();
+        if (inside) {
+          uint8_t* stage2 = stage + 2048;
+          const bool second = g.aux != nullptr;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float v[8], dv[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(r[j * 8 + q]);
+            if (has_bias) {
+              v[0] += __shfl_sync(0xffffffffu, bias4.x, 2 * j);
+              v[1] += __shfl_sync(0xffffffffu, bias4.y, 2 * j);
+              v[2] += __shfl_sync(0xffffffffu, bias4.z, 2 * j);
+              v[3] += __shfl_sync(0xffffffffu, bias4.w, 2 * j);
+              v[4] += __shfl_sync(0xffffffffu, bias4.x, 2 * j + 1);
+              v[5] += __shfl_sync(0xffffffffu, bias4.y, 2 * j + 1);
+              v[6] += __shfl_sync(0xffffffffu, bias4.z, 2 * j + 1);
+              v[7] += __shfl_sync(0xffffffffu, bias4.w, 2 * j + 1);
+            }
+            if (!gelu_d && second) *stage_unit64(stage2, lane, j) = pack8(v);
+            // value and derivative share one exponential; the derivative is what backward needs, so it is saved instead of z
+#pragma unroll
+            for (int q = 0; q < 8; q += 2) gelu_two<true>(v[q], v[q + 1], dv[q], dv[q + 1]);
+            *stage_unit64(stage, lane, j) = pack8(v);
+            if (gelu_d && second) *stage_unit64(stage2, lane, j) = pack8(dv);
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (tc::elect_one()) {
+            store_2d(map_d, stage, col0, row0);
+            if (second) store_2d(&P.x, stage2, col0, row0);
+            bulk_commit();
+          }
+          __syncwarp();
+        }
       } else {
-        uint4 second[kOut == OUT_GELU ? 8 : 1];   // the second output waits here until the first has left the staging buffer
 #pragma unroll 1
         for (int c = 0; c < S::kCols; c += 64) {
           const int cg = col0 + c;
@@ -467,19 +546,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
                 v[6] += __shfl_sync(0xffffffffu, bias4.z, src + 1);
                 v[7] += __shfl_sync(0xffffffffu, bias4.w, src + 1);
               }
-              if constexpr (kOut == OUT_GELU) {
-                if (gelu_d) {
-                  // value and derivative share one exponential; the derivative is what backward needs, so it is saved instead of z
-                  float dv[8];
-#pragma unroll
-                  for (int q = 0; q < 8; ++q) gelu_value_grad(v[q], v[q], dv[q]);
-                  second[j] = pack8(dv);
-                } else {
-                  second[j] = pack8(v);
-#pragma unroll
-                  for (int q = 0; q < 8; ++q) v[q] = gelu_erf(v[q]);
-                }
-              } else if (has_extra) {
+              if (has_extra) {
                 float x[8];
                 unpack8(*stage_unit(buf_c, lane, j), x);
                 if (multiply) {
@@ -516,20 +583,8 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           if (tc::elect_one()) {
             store_2d(map_d, buf_c, cg, row0);
             bulk_commit();
-            if constexpr (kOut == OUT_GELU) bulk_wait_read<0>();
           }
           __syncwarp();
-          if (kOut == OUT_GELU && g.aux != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) *stage_unit(buf_c, lane, j) = second[kOut == OUT_GELU ? j : 0];
-            fence_async_smem();
-            __syncwarp();
-            if (tc::elect_one()) {
-              store_2d(&P.x, buf_c, cg, row0);
-              bulk_commit();
-            }
-            __syncwarp();
-          }
         }
         if (!ok) break;
       }
@@ -560,14 +615,31 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
     if constexpr (kPair) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * BN) : "memory");
     else tc::tmem_dealloc(tmem_base, 2 * BN);
   }
-  tl_end(g.tl, tl_t0, TL_GEMM, (static_cast<uint32_t>(total / (P.n_tiles[0] * splits) * (kPair ? 2 : 1)) << 16) | static_cast<uint32_t>(P.n_tiles[0] * splits));
+  tl_end(g.tl, tl_t0, TL_GEMM, (static_cast<uint32_t>(tiles / P.n_tiles[0] * (kPair ? 2 : 1)) << 16) | static_cast<uint32_t>(P.n_tiles[0]));
 }
 
-// Launches `workers` CTAs (pairs) over the tiles of `count` products with the same K, which is cut into `splits` (fp32
-// sums added into D).
+// MN-major operand [K, cols] as [cols / 64][K][64], a box being `groups` groups x BK rows.  (A load costs the TMA unit 50 clocks
+// and its bytes 80 per 8 KB: with one load per group an MN-major 256 x 256 k-block took 650-730 clocks against 515.)
+inline bool encode_groups(CUtensorMap* map, const void* base, int k, int cols, int ld_elems, int groups) {
+  const CuDriver& cu = CuDriver::get();
+  if (!cu.loaded || !cu.TensorMapEncodeTiled) return false;
+  int device = 0;
+  cudaGetDevice(&device);
+  cu.ensure_context(device);
+  cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(cols / 64)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld_elems) * 2, 128};
+  cuuint32_t box[3] = {64, static_cast<cuuint32_t>(BK), static_cast<cuuint32_t>(groups)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return cu.TensorMapEncodeTiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Launches `workers` CTAs (pairs) over the tiles of `count` products with the same K, which is cut into `splits` (0: equal
+// runs of k-blocks; with anything but 1, fp32 sums are added into D).
 template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut, int kMax>
 cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int splits, cudaStream_t stream) {
-  using S = Shape<BN, kPair>;
+  using S = Shape<BN, kPair, kOut == OUT_GELU>;
   auto kernel = gemm_tile_kernel<BN, kPair, kAMn, kBMn, kOut, kMax>;
   static std::atomic<bool> configured{false};
   if (!configured.load(std::memory_order_acquire)) {
@@ -581,15 +653,18 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
   for (int p = 0; p < count; ++p) {
     const GemmArgs& a = args[p];
     // K-major: boxes of 64 of K x the tile's rows; MN-major: boxes of 64 columns x 64 of K (zero fill past K)
-    const bool oka = kAMn ? encode_map(&P.a[p], a.a, a.k, a.m, a.lda, BK) : encode_map(&P.a[p], a.a, a.m, a.k, a.lda, BM);
-    const bool okb = kBMn ? encode_map(&P.b[p], a.b, a.k, a.n, a.ldb, BK) : encode_map(&P.b[p], a.b, a.n, a.k, a.ldb, S::kRowsB);
-    if (!oka || !okb || !encode_out_map(&P.d[p], a.d, a.m, a.n, a.ldd, kOut == OUT_F32)) return cudaErrorNotSupported;
+    P.atoms[p] = (kAMn && a.m % 64 == 0 ? 1 : 0) | (kBMn && a.n % 64 == 0 && S::kRowsB > 64 ? 2 : 0);
+    const bool oka = P.atoms[p] & 1 ? encode_groups(&P.a[p], a.a, a.k, a.m, a.lda, BM / 64)
+                     : kAMn ? encode_map(&P.a[p], a.a, a.k, a.m, a.lda, BK) : encode_map(&P.a[p], a.a, a.m, a.k, a.lda, BM);
+    const bool okb = P.atoms[p] & 2 ? encode_groups(&P.b[p], a.b, a.k, a.n, a.ldb, S::kRowsB / 64)
+                     : kBMn ? encode_map(&P.b[p], a.b, a.k, a.n, a.ldb, BK) : encode_map(&P.b[p], a.b, a.n, a.k, a.ldb, S::kRowsB);
+    if (!oka || !okb || !encode_out_map(&P.d[p], a.d, a.m, a.n, a.ldd, kOut == OUT_F32, kOut == OUT_GELU)) return cudaErrorNotSupported;
     P.m[p] = a.m;
     P.n[p] = a.n;
     P.n_tiles[p] = (a.n + BN - 1) / BN;
     P.first[p + 1] = P.first[p] + P.n_tiles[p] * ((a.m + (kPair ? 2 * BM : BM) - 1) / (kPair ? 2 * BM : BM));
     // partial sums are added into the output: start from zero unless the caller accumulates anyway
-    if (splits > 1 && !a.accumulate) {
+    if (splits != 1 && !a.accumulate) {
       cudaError_t rc = cudaMemsetAsync(a.d, 0, static_cast<size_t>(a.m) * a.n * sizeof(float), stream);
       if (rc != cudaSuccess) return rc;
     }
@@ -597,7 +672,7 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
   const GemmArgs& a = args[0];
   const void* x = kOut == OUT_GELU ? a.aux : (kOut == OUT_F32 ? nullptr : (a.mul ? a.mul : a.residual));
   if (x == nullptr) P.x = P.d[0];   // never used
-  else if (!encode_out_map(&P.x, x, a.m, a.n, a.ldd, false)) return cudaErrorNotSupported;
+  else if (!encode_out_map(&P.x, x, a.m, a.n, a.ldd, false, kOut == OUT_GELU)) return cudaErrorNotSupported;
   GemmDev g;
   g.d = a.d;
   g.aux = a.aux;
@@ -612,7 +687,7 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
   g.d_fp32 = kOut == OUT_F32 ? 1 : 0;
   g.accumulate = a.accumulate ? 1 : 0;
   g.epilogue = a.epilogue;
-  g.atomic_add = splits > 1 ? 1 : 0;
+  g.atomic_add = splits != 1 ? 1 : 0;
   g.err = gemm_error_device_ptr();
   if (!g.err) return cudaErrorNotSupported;
   g.tl = timeline_device_ptr();

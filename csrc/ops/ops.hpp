@@ -130,7 +130,7 @@ struct GemmArgs {
 // (K % 64 != 0, N % 8 != 0, unaligned pointers); the caller falls back.
 cudaError_t gemm_bf16_tn(const GemmArgs& args, cudaStream_t stream);
 // Up to any number of weight gradients dW[N, K] = dY[tokens, N]^T · X[tokens, K] over the same tokens, worked through together
-// (four products per launch).  A product is a GemmArgs with both operands MN-major, fp32 output, no epilogue; all of them
+// (sixteen products per launch).  A product is a GemmArgs with both operands MN-major, fp32 output, no epilogue; all of them
 // accumulate, or none.
 cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream);
 // Caps the number of CTAs (= SMs) plain GEMM launches occupy from now on; 0 restores one CTA per SM.  A

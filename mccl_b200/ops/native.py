@@ -1,6 +1,8 @@
 """autograd Functions over the native kernels (CUDA tensors only)."""
 from __future__ import annotations
 
+import threading
+
 import torch
 import torch.nn.functional as F
 
@@ -55,6 +57,7 @@ def mark_wgrad_pending() -> None:
 
 def join_wgrad(stream=None) -> None:
     """Makes ``stream`` (default: the current one) wait for the weight gradients queued on the side stream."""
+    _deferred.flush_all()
     s = _wgrad["stream"]
     if s is not None and _wgrad["pending"]:
         (stream if stream is not None else torch.cuda.current_stream()).wait_stream(s)
@@ -297,13 +300,65 @@ class DecoderLayerFn(torch.autograd.Function):
         params = ctx.params
         sinks = [getattr(p, "_grad_sink", None) for p in params]
         direct = all(s is not None for s in sinks)
-        dx, grads = _C.decoder_layer_bwd(dout if dout.is_contiguous() else dout.contiguous(), x, slab, w, sinks if direct else [],
-                                         x.shape[0], x.shape[1], ctx.heads)
+        dout = dout if dout.is_contiguous() else dout.contiguous()
+        B, S = x.shape[0], x.shape[1]
+        dx, grads, between = _C.decoder_layer_bwd(dout, x, slab, w, sinks if direct else [], B, S, ctx.heads, direct)
         if not direct:
             return (dx, None, None, *grads)
-        for p in reversed(params):
-            _notify(p)
+        _deferred.add((dout, slab, between, sinks), (B, S, ctx.heads), params, x.device)
         return (dx, None, None) + (None,) * len(params)
+
+
+class _Deferred:
+    """Weight gradients of decoder layers that go straight into a trainer's buffers, kept back until several layers can share a
+    launch: a layer's four products fill the SMs for 20 us and pay 8 us of set-up, first loads and last epilogue, so at 4096
+    tokens four layers together take 23 us each instead of 25, at 1600 tokens 12 instead of 18, and a small model's 2
+    instead of 6.  Flushed at the end of backward at the latest (by an engine callback), and before anybody looks at the
+    gradients of a bucket."""
+
+    #: multiply-adds that keep the GPU busy for some 60 us: enough for the fixed part to be small
+    ENOUGH = 5e10
+    MOST = 4
+
+    def __init__(self):
+        self._lock = threading.Lock()
+        self._pending = {}   # device -> (sizes, stream, [items], [params], multiply-adds)
+
+    def add(self, item, sizes, params, device) -> None:
+        stream = torch.cuda.current_stream(device)
+        with self._lock:
+            entry = self._pending.get(device)
+        if entry is not None and (entry["sizes"] != sizes or entry["stream"] != stream or entry["shape"] != item[3][8].shape):
+            self.flush(device)
+            entry = None
+        if entry is None:
+            entry = {"sizes": sizes, "stream": stream, "shape": item[3][8].shape, "items": [], "params": [], "work": 0.0}
+            with self._lock:
+                self._pending[device] = entry
+            torch.autograd.Variable._execution_engine.queue_callback(lambda: self.flush(device))
+        entry["items"].append(item)
+        entry["params"].append(params)
+        entry["work"] += sizes[0] * sizes[1] * float(sum(item[3][i].numel() for i in DecoderLayerFn.MATRICES))
+        if len(entry["items"]) >= self.MOST or entry["work"] >= self.ENOUGH:
+            self.flush(device)
+
+    def flush(self, device) -> None:
+        with self._lock:
+            entry = self._pending.pop(device, None)
+        if entry is None:
+            return
+        with torch.cuda.stream(entry["stream"]):
+            _C.decoder_layer_wgrads(entry["items"], *entry["sizes"])
+            for params in entry["params"]:
+                for p in reversed(params):
+                    _notify(p)
+
+    def flush_all(self) -> None:
+        for device in list(self._pending):
+            self.flush(device)
+
+
+_deferred = _Deferred()
 
 
 class RopeQkvFn(torch.autograd.Function):

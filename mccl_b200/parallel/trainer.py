@@ -312,7 +312,7 @@ class DDPTrainer:
         _native.set_wgrad_stream(self.wgrad_stream, main_ctas, self._bwd_side_ctas)
         try:
             loss.backward()
-            if self.wgrad_stream is not None:
+            if self.device.type == "cuda":
                 _native.join_wgrad(torch.cuda.current_stream(self.device))
         finally:
             _native.set_wgrad_stream(None)
