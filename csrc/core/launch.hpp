@@ -34,10 +34,10 @@ uint64_t launch_total();
 // it in the stream is still draining: its CTAs become resident, do their set-up (barrier init, tensor-memory
 // allocation, descriptor prefetch, index arithmetic) and then block in pdl_wait() until every earlier kernel of the
 // stream has finished and its memory is visible.  Such a kernel must call pdl_wait() before its first access to
-// global memory, read or write.  pdl_trigger() tells the hardware that the kernels after this one may start their
-// set-up; kernels that never call it release their dependents when they exit.  The launch attribute is only set with
-// MCCL_PDL=1 (without it the device calls are no-ops and the stream serialises as usual): measured on the training
-// step it did not pay, so it is an option, not the default.
+// global memory, read or write.  pdl_trigger() tells the hardware that the kernel after this one may start its
+// set-up; it comes AFTER pdl_wait(), so that no more than one kernel is ever resident ahead of its turn (triggered on
+// entry, several queued up and held the shared memory and registers that the running one's remaining CTAs needed: a
+// training step in a graph was slower with dependent launches than without).
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {

@@ -79,7 +79,6 @@ __global__ void __launch_bounds__(128) attn_fwd_long_kernel(const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_bar + 1);
   volatile int* bad = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  pdl_trigger();
   const int tid = threadIdx.x, warp = tid >> 5;
   const int nblk = a.S / kBlk;
   const int qi = nblk - 1 - static_cast<int>(blockIdx.x);   // long rows first
@@ -102,6 +101,7 @@ __global__ void __launch_bounds__(128) attn_fwd_long_kernel(const __grid_constan
   const uint32_t tmem_s = *tmem_slot, tmem_o = tmem_s + 128;
   const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
   pdl_wait();
+  pdl_trigger();
 
   const int row0 = b * a.S;
   auto load_k = [&](int j) {
@@ -307,7 +307,6 @@ __global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
   volatile int* bad = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  pdl_trigger();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qi = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);   // long rows first
   const int h = blockIdx.y, b = blockIdx.z, nblk = qi + 1, nk = nblk * kBlk;
@@ -355,6 +354,7 @@ __global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant_
   ok = __all_sync(0xffffffffu, ok);
   tc::fence_after_sync();
 
+  pdl_trigger();
   const int wg = warp >> 2, row = (warp & 3) * 32 + lane;      // two threads per query row, half of the keys each
   // Groups of 32 keys before `diag` are seen by all of the warp's queries, those after it by none.
   const int diag = qi * kBlk + (warp & 3) * 32, cols = nk >> 1, c_begin = wg * cols, c_end = min(c_begin + cols, diag + 32);
@@ -514,7 +514,6 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(g_done + 1);
   volatile int* bad = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  pdl_trigger();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nblk = (a.S + kBlk - 1) / kBlk;   // 1 or 2
   const int h = blockIdx.x, b = blockIdx.y;
@@ -609,6 +608,7 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
     }
     __syncwarp();
   }
+  pdl_trigger();
   bool ok = true;
   {
     // delta[row] = sum_d dO[row, d] * O[row, d] and the row's log-sum-exp, one row per thread.  Rows past the sequence get an

@@ -53,8 +53,8 @@ __global__ void __launch_bounds__(256) norm_fwd_kernel(const __nv_bfloat16* __re
                                                        float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows,
                                                        int dim, float eps) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= rows) return;
   const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(warp) * dim);
@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(256) norm_bwd_dx_kernel(const __nv_bfloat16* _
                                                           const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx,
                                                           const __nv_bfloat16* __restrict__ dx_add, int rows, int dim) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= rows) return;
   const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(warp) * dim);
@@ -187,7 +187,6 @@ __global__ void __launch_bounds__(256) norm_bwd_fused_kernel(const __nv_bfloat16
                                                              const __nv_bfloat16* __restrict__ dx_add, float* __restrict__ dw,
                                                              float* __restrict__ db, float* __restrict__ sum_add,
                                                              float* __restrict__ sum_dx, int rows, int dim) {
-  ::mccl::pdl_trigger();
   extern __shared__ float red[];   // [8 warps][kVecs * 256]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, vecs = dim >> 3;
   float aw[kVecs][8], ab[kVecs][8], sa[kSums ? kVecs : 1][8], sd[kSums ? kVecs : 1][8];
@@ -199,6 +198,7 @@ __global__ void __launch_bounds__(256) norm_bwd_fused_kernel(const __nv_bfloat16
       if (kSums) sa[k][i] = sd[k][i] = 0.f;
     }
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   for (int row = blockIdx.x * 8 + warp; row < rows; row += gridDim.x * 8) {
     const size_t at = static_cast<size_t>(row) * vecs + lane;
     uint4 rx[kVecs], rg[kVecs], ra[kVecs];
@@ -302,8 +302,8 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
                                                              float* __restrict__ part_w, float* __restrict__ part_b, int rows,
                                                              int dim, int atomic) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   __shared__ float sw[8][32][9], sb[8][32][9];
   const int cg = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int col = blockIdx.x * 256 + cg * 8;
@@ -357,8 +357,8 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
 __global__ void __launch_bounds__(256) colsum_final_kernel(const float* __restrict__ part_w, const float* __restrict__ part_b,
                                                            float* __restrict__ dw, float* __restrict__ db, int slabs, int dim) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   __shared__ float sw[8][33], sb[8][33];
   const int cx = threadIdx.x & 31, ly = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
@@ -500,8 +500,8 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p, float
                                                     float lr, float b1, float b2, float eps, float wd,
                                                     const float* __restrict__ step_ptr, float gscale, int zero_grad) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   const float step = *step_ptr;
   const float bc1 = 1.f - powf(b1, step), bc2 = 1.f - powf(b2, step);
   const float inv_bc1 = 1.f / bc1, inv_sqrt_bc2 = rsqrtf(bc2), decay = 1.f - lr * wd;
@@ -572,8 +572,8 @@ cudaError_t adamw_flat(float* p, float* g, float* m, float* v, __nv_bfloat16* p1
 __global__ void __launch_bounds__(512) ce_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
                                                  float* __restrict__ loss_rows, int vocab, float scale) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   __shared__ float s_max[16], s_sum[16];
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   __nv_bfloat16* lr = logits + static_cast<size_t>(row) * vocab;
@@ -650,8 +650,8 @@ cudaError_t cross_entropy_fwd_bwd(__nv_bfloat16* logits, const long long* target
 __global__ void __launch_bounds__(256) transpose_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
                                                         int rows, int cols) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   __shared__ __nv_bfloat16 tile[64][66];
   const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -684,8 +684,8 @@ cudaError_t transpose_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, int rows
 // ------------------------------------------------------------------ casts --
 __global__ void __launch_bounds__(256) cast_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   const long long n4 = n / 4;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -723,8 +723,8 @@ struct CastTable {
 };
 
 __global__ void __launch_bounds__(256) cast_many_kernel(const __grid_constant__ CastTable t, __nv_bfloat16* __restrict__ out) {
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   int lo = 0, hi = t.count - 1;   // the tensor this block belongs to
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -778,8 +778,8 @@ cudaError_t cast_many(const float* const* src, const long long* numel, const lon
 __global__ void __launch_bounds__(256) gelu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ z,
                                                        __nv_bfloat16* __restrict__ dz, long long n8) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n8;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float g[8], zz[8], o[8];
@@ -812,8 +812,8 @@ __global__ void __launch_bounds__(256) embed_fwd_kernel(const long long* __restr
                                                         const float* __restrict__ pos, __nv_bfloat16* __restrict__ y, long long n8,
                                                         int seq, int dim8, int vocab) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n8;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long t = i / dim8;
@@ -837,8 +837,8 @@ __global__ void __launch_bounds__(256) embed_bwd_kernel(const long long* __restr
                                                         float* __restrict__ dtok, float* __restrict__ dpos, long long n8, int seq,
                                                         int dim8, int vocab, float scale) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n8;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long t = i / dim8;

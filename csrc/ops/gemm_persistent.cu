@@ -393,8 +393,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_persistent_kernel(const 
   // Dependent launch: this CTA may be resident while the previous kernel of the stream is still draining.  Barrier
   // init, tensor-memory allocation and descriptor prefetch below touch no global data; pdl_wait() comes before the
   // first access that does (at once for the fused roles, which read their call number from global memory).
-  pdl_trigger();
-  if (f.mode != FUSE_NONE) pdl_wait();
+  if (f.mode != FUSE_NONE) {
+    pdl_wait();
+    pdl_trigger();
+  }
   const unsigned long long tl_t0 = tl_begin(g.tl);
   const uint32_t epoch = f.mode != FUSE_NONE ? *f.epoch_ptr : 0u;
   if (f.mode != FUSE_NONE && static_cast<int>(blockIdx.x) < f.copy_ctas) {
@@ -440,7 +442,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_persistent_kernel(const 
   tc::fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   if (tl_t0 != 0ull && tl_detail(g.tl)) tl_mark(g.tl, tl_t0, tl_now(), TL_GEMM_PHASE, 0u);
-  if (f.mode == FUSE_NONE) pdl_wait();   // set-up done: from here on operands are read and outputs written
+  if (f.mode == FUSE_NONE) {   // set-up done: from here on operands are read and outputs written
+    pdl_wait();
+    pdl_trigger();
+  }
 
   // Reduce-scatter fusion: phase-major order; inside a phase the chunks of the other ranks come first
   // (rank + 1, rank + 2, ...) and this rank's own chunk last, so what peers wait for is ready earliest.

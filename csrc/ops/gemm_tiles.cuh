@@ -200,7 +200,6 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(extra_full + S::kEpiWarps * S::kBufs);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  pdl_trigger();
   const unsigned long long tl_t0 = tl_begin(g.tl);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = kPair ? cluster_ctarank() : 0u;
@@ -341,6 +340,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           }
         }
       }
+      pdl_trigger();   // the last loads are on their way: the next kernel may set up beside this one's tail
       if (!ok) {
         *abort_flag = 1;
         atomicExch(g.err, 11);

@@ -59,8 +59,8 @@ __device__ __forceinline__ void rotate8(float (&f)[8], const float* cos_row, con
 __global__ void __launch_bounds__(kThreads) rope_qk_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
                                                                const float* __restrict__ sin_t, __nv_bfloat16* __restrict__ qk,
                                                                long long units, int seq, int row_units, int hd8) {
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   for (long long i = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x; i < units; i += static_cast<long long>(gridDim.x) * kThreads) {
     const long long t = i / (2 * row_units);
     const int u = static_cast<int>(i - t * (2 * row_units));   // unit within the token's q and k
@@ -83,8 +83,8 @@ struct GradView {
 __global__ void __launch_bounds__(kThreads) rope_qkv_bwd_kernel(GradView dq, GradView dk, GradView dv, const float* __restrict__ cos_t,
                                                                 const float* __restrict__ sin_t, __nv_bfloat16* __restrict__ dqkv,
                                                                 long long units, int seq, int row_units, int hd8) {
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   for (long long i = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x; i < units; i += static_cast<long long>(gridDim.x) * kThreads) {
     const long long t = i / (3 * row_units);
     const int u = static_cast<int>(i - t * (3 * row_units));
@@ -109,8 +109,8 @@ __global__ void __launch_bounds__(kThreads) rope_qkv_bwd_kernel(GradView dq, Gra
 // as the two separate operators do, so results do not depend on which path ran.
 __global__ void __launch_bounds__(kThreads) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h,
                                                               long long units, int f8) {
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   for (long long i = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x; i < units; i += static_cast<long long>(gridDim.x) * kThreads) {
     const long long row = i / f8;
     const uint4* g_row = reinterpret_cast<const uint4*>(gu) + row * f8 + i;   // row * 2 f8 + (i - row * f8)
@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(kThreads) swiglu_fwd_kernel(const __nv_bfloat1
 // d(gate) = dh * up * silu'(gate), d(up) = dh * silu(gate), written side by side as the gradient of gu.
 __global__ void __launch_bounds__(kThreads) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ gu,
                                                               __nv_bfloat16* __restrict__ dgu, long long units, int f8) {
-  ::mccl::pdl_trigger();
   ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
   for (long long i = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x; i < units; i += static_cast<long long>(gridDim.x) * kThreads) {
     const long long row = i / f8;
     const long long at = row * f8 + i;
