@@ -10,4 +10,5 @@ void bind_comm(pybind11::module_& m);     // device communicator, symmetric heap
 void bind_runtime(pybind11::module_& m);  // dmem, coherence, scheduler, cluster manager, agent
 void bind_ops(pybind11::module_& m);      // model operators (GEMM, norms, optimizer)
 void bind_layers(pybind11::module_& m);   // whole decoder layers
+void bind_decoder_autograd(pybind11::module_& m);   // a decoder's loss as C++ autograd nodes
 }  // namespace mccl

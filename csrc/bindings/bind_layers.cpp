@@ -5,183 +5,14 @@
 // Here the launches of a layer follow each other from C++ over one slab of saved activations (one allocation), and
 // what only a view of the whole layer allows is taken: bias gradients come out of the kernels that produce or read the
 // tensors they sum (norm backward, attention backward, the GELU product), and the four weight gradients are one launch.
-#include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDAGuard.h>
-#include <torch/extension.h>
-
-#include <cmath>
-
-#include "../core/errors.hpp"
-#include "../ops/ops.hpp"
 #include "bind.hpp"
+#include "decoder_layer.hpp"
 
 namespace py = pybind11;
 
 namespace mccl {
 
-namespace {
-
-using bf16 = __nv_bfloat16;
-
-void check(cudaError_t rc, const char* what) {
-  MCCL_CHECK_T(rc == cudaSuccess, CudaError, "decoder layer: " << what << " failed: " << cudaGetErrorString(rc) << " " << ops::gemm_last_reason());
-}
-bf16* bf(const at::Tensor& t) { return reinterpret_cast<bf16*>(t.data_ptr()); }
-void need(const at::Tensor& t, at::ScalarType dt, int64_t numel, const char* what) {
-  MCCL_CHECK_TENSOR(t.defined() && t.is_cuda() && t.is_contiguous() && t.scalar_type() == dt && t.numel() == numel,
-                    "decoder layer: " << what << ": a contiguous CUDA tensor of " << numel << " " << c10::toString(dt) << " elements expected");
-}
-
-// Order of a layer's parameters everywhere below.
-enum Param { LN1_W, LN1_B, QKV_W, QKV_B, PROJ_W, PROJ_B, LN2_W, LN2_B, UP_W, UP_B, DOWN_W, DOWN_B, kParams };
-
-struct Dims {
-  int B, S, H, D, F;
-  int tokens() const { return B * S; }
-  int head_dim() const { return D / H; }
-};
-
-int64_t param_numel(const Dims& d, int p) {
-  const int64_t D = d.D, F = d.F;
-  switch (p) {
-    case QKV_W: return 3 * D * D;
-    case QKV_B: return 3 * D;
-    case PROJ_W: return D * D;
-    case UP_W:
-    case DOWN_W: return D * F;
-    case UP_B: return F;
-    default: return D;
-  }
-}
-
-struct Weights {
-  const float *ln1_w, *ln1_b, *qkv_b, *proj_b, *ln2_w, *ln2_b, *up_b, *down_b;
-  const bf16 *qkv, *proj, *up, *down;
-};
-Weights weights_of(const std::vector<at::Tensor>& p, const Dims& d) {
-  MCCL_CHECK_TENSOR(p.size() == kParams, "decoder layer: " << static_cast<int>(kParams) << " parameters expected");
-  for (int i = 0; i < kParams; ++i) {
-    const bool matrix = i == QKV_W || i == PROJ_W || i == UP_W || i == DOWN_W;
-    need(p[i], matrix ? at::kBFloat16 : at::kFloat, param_numel(d, i), "parameter");
-  }
-  auto f = [&](int i) { return p[i].data_ptr<float>(); };
-  return {f(LN1_W), f(LN1_B), f(QKV_B), f(PROJ_B), f(LN2_W), f(LN2_B), f(UP_B), f(DOWN_B), bf(p[QKV_W]), bf(p[PROJ_W]), bf(p[UP_W]), bf(p[DOWN_W])};
-}
-
-// Activations of a layer that backward reads, in one allocation.
-struct Slab {
-  bf16 *h1, *qkv, *o, *y, *h2, *act, *gelu_grad;
-  float *mean1, *rstd1, *mean2, *rstd2, *lse;
-  static int64_t place(Slab* s, uint8_t* base, const Dims& d) {
-    int64_t at = 0;
-    const int64_t T = d.tokens();
-    auto take = [&](auto*& p, int64_t elems) {
-      p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
-      at += (elems * static_cast<int64_t>(sizeof(*p)) + 255) / 256 * 256;
-    };
-    take(s->h1, T * d.D);
-    take(s->qkv, T * 3 * d.D);
-    take(s->o, T * d.D);
-    take(s->y, T * d.D);
-    take(s->h2, T * d.D);
-    take(s->act, T * d.F);
-    take(s->gelu_grad, T * d.F);
-    take(s->mean1, T);
-    take(s->rstd1, T);
-    take(s->mean2, T);
-    take(s->rstd2, T);
-    take(s->lse, T * d.H);
-    return at;
-  }
-};
-
-// y[M, N] = x[M, K] · w[N, K]^T + bias (+ residual), or GELU with its derivative in `aux` (null: not wanted)
-void product(const bf16* x, const bf16* w, const float* bias, bf16* y, int M, int N, int K, const bf16* residual, bool gelu, bf16* aux,
-             cudaStream_t stream, const char* what) {
-  ops::GemmArgs g;
-  g.a = x;
-  g.b = w;
-  g.d = y;
-  g.aux = aux;
-  g.bias = bias;
-  g.residual = residual;
-  g.m = M;
-  g.n = N;
-  g.k = K;
-  g.lda = g.ldb = K;
-  g.ldd = N;
-  g.epilogue = gelu ? (aux ? ops::EPI_BIAS_GELU_D : ops::EPI_BIAS_GELU) : (bias ? ops::EPI_BIAS : ops::EPI_NONE);
-  check(ops::gemm_bf16_tn(g, stream), what);
-}
-// dx[M, K] = dy[M, N] · w[N, K] (times mul, with its column sums added to colsum)
-void input_gradient(const bf16* dy, const bf16* w, bf16* dx, int M, int N, int K, const bf16* mul, float* colsum, cudaStream_t stream,
-                    const char* what) {
-  ops::GemmArgs g;
-  g.a = dy;
-  g.b = w;
-  g.b_mn_major = true;
-  g.d = dx;
-  g.mul = mul;
-  g.colsum = colsum;
-  g.m = M;
-  g.n = K;
-  g.k = N;
-  g.lda = N;
-  g.ldb = g.ldd = K;
-  check(ops::gemm_bf16_tn(g, stream), what);
-}
-ops::GemmArgs weight_gradient(const bf16* dy, const bf16* x, float* dw, int tokens, int N, int K) {
-  ops::GemmArgs g;
-  g.a = dy;
-  g.b = x;
-  g.d = dw;
-  g.a_mn_major = g.b_mn_major = g.d_fp32 = g.accumulate = true;
-  g.m = N;
-  g.n = K;
-  g.k = tokens;
-  g.lda = N;
-  g.ldb = g.ldd = K;
-  return g;
-}
-
-// What the weight gradients of a layer are made of.
-struct Pending {
-  const bf16 *dout, *dz, *dqkv, *dy;
-  Slab s;
-  float *down, *up, *qkv, *proj;
-};
-void weight_gradients(const std::vector<Pending>& layers, const Dims& d, cudaStream_t stream) {
-  const int T = d.tokens(), D = d.D, F = d.F;
-  std::vector<ops::GemmArgs> args;
-  for (const Pending& p : layers) {
-    args.push_back(weight_gradient(p.dout, p.s.act, p.down, T, D, F));
-    args.push_back(weight_gradient(p.dz, p.s.h2, p.up, T, F, D));
-    args.push_back(weight_gradient(p.dqkv, p.s.h1, p.qkv, T, 3 * D, D));
-    args.push_back(weight_gradient(p.dy, p.s.o, p.proj, T, D, D));
-  }
-  check(ops::gemm_group(args.data(), static_cast<int>(args.size()), stream), "weight gradients");
-}
-
-void layer_forward(const bf16* x, bf16* out, const Weights& w, const Slab& s, const Dims& d, float eps, bool keep, cudaStream_t st) {
-  const int T = d.tokens(), D = d.D, F = d.F;
-  const float scale = 1.f / std::sqrt(static_cast<float>(d.head_dim()));
-  check(ops::norm_fwd(x, w.ln1_w, w.ln1_b, s.h1, keep ? s.mean1 : nullptr, keep ? s.rstd1 : nullptr, T, D, eps, st), "first norm");
-  product(s.h1, w.qkv, w.qkv_b, s.qkv, T, 3 * D, D, nullptr, false, nullptr, st, "qkv projection");
-  check(ops::attention_fwd(s.qkv, s.o, s.lse, d.B, d.S, d.H, d.head_dim(), scale, st), "attention");
-  product(s.o, w.proj, w.proj_b, s.y, T, D, D, x, false, nullptr, st, "output projection");
-  check(ops::norm_fwd(s.y, w.ln2_w, w.ln2_b, s.h2, keep ? s.mean2 : nullptr, keep ? s.rstd2 : nullptr, T, D, eps, st), "second norm");
-  product(s.h2, w.up, w.up_b, s.act, T, F, D, nullptr, true, keep ? s.gelu_grad : nullptr, st, "up projection");
-  product(s.act, w.down, w.down_b, out, T, D, F, s.y, false, nullptr, st, "down projection");
-}
-
-Dims dims_of(const at::Tensor& x, int64_t B, int64_t S, int64_t H, int64_t F) {
-  MCCL_CHECK_TENSOR(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.dim() >= 2, "decoder layer: a contiguous bf16 CUDA activation expected");
-  const int64_t D = x.size(-1);
-  MCCL_CHECK_TENSOR(B > 0 && S > 0 && H > 0 && D % H == 0 && x.numel() == B * S * D && B * S < (1ll << 31), "decoder layer: bad sizes");
-  return {static_cast<int>(B), static_cast<int>(S), static_cast<int>(H), static_cast<int>(D), static_cast<int>(F)};
-}
-
-}  // namespace
+using namespace layers;
 
 void bind_layers(py::module_& m) {
   // Whether decoder_layer_fwd / _bwd cover these sizes.
@@ -202,8 +33,8 @@ void bind_layers(py::module_& m) {
     layer_forward(bf(x), bf(out), w, s, d, static_cast<float>(eps), true, at::cuda::getCurrentCUDAStream(x.get_device()).stream());
     return std::make_pair(out, slab);
   });
-  // (gradient of x, gradients of the parameters, see decoder_layer_wgrads).  The gradients of the parameters are ADDED into `grads` (fp32, one per parameter, same order)
-  // where given, else returned as views of one new buffer.  With defer, those of the four matrices are left for
+  // (gradient of x, gradients of the parameters, see decoder_layer_wgrads).  The gradients of the parameters are
+  // ADDED into `grads` (fp32, one per parameter, same order) where given, else returned as views of one new buffer.  With defer, those of the four matrices are left for
   // decoder_layer_wgrads.
   m.def("decoder_layer_bwd", [](const at::Tensor& dout, const at::Tensor& x, const at::Tensor& slab, const std::vector<at::Tensor>& params,
                                 std::vector<at::Tensor> grads, int64_t B, int64_t S, int64_t H, bool defer) {
@@ -229,27 +60,7 @@ void bind_layers(py::module_& m) {
     Slab s;
     MCCL_CHECK_TENSOR(slab.is_cuda() && slab.numel() == Slab::place(&s, nullptr, d), "decoder layer: not the slab of this forward");
     Slab::place(&s, slab.data_ptr<uint8_t>(), d);
-    const int T = d.tokens(), D = d.D, F = d.F;
-    const float scale = 1.f / std::sqrt(static_cast<float>(d.head_dim()));
-    cudaStream_t st = at::cuda::getCurrentCUDAStream(x.get_device()).stream();
-    // gradients between the kernels: dz [T, F], dqkv [T, 3 D], and three of [T, D]
-    const int64_t TD = static_cast<int64_t>(T) * D;
-    at::Tensor tmp = at::empty({TD * 6 + static_cast<int64_t>(T) * F}, x.options());
-    bf16 *dh = bf(tmp), *dy = dh + TD, *d_o = dy + TD, *dqkv = d_o + TD, *dz = dqkv + 3 * TD;
-    at::Tensor dx = at::empty_like(x);
-    input_gradient(bf(dout), w.down, dz, T, D, F, s.gelu_grad, g[UP_B], st, "down projection backward");
-    input_gradient(dz, w.up, dh, T, F, D, nullptr, nullptr, st, "up projection backward");
-    check(ops::norm_bwd_fused(dh, s.y, w.ln2_w, s.mean2, s.rstd2, dy, bf(dout), g[LN2_W], g[LN2_B], g[DOWN_B], g[PROJ_B], T, D, true, st),
-          "second norm backward");
-    input_gradient(dy, w.proj, d_o, T, D, D, nullptr, nullptr, st, "output projection backward");
-    check(ops::attention_bwd(s.qkv, s.o, d_o, s.lse, dqkv, g[QKV_B], d.B, d.S, d.H, d.head_dim(), scale, st), "attention backward");
-    input_gradient(dqkv, w.qkv, dh, T, 3 * D, D, nullptr, nullptr, st, "qkv projection backward");
-    check(ops::norm_bwd_fused(dh, bf(x), w.ln1_w, s.mean1, s.rstd1, bf(dx), dy, g[LN1_W], g[LN1_B], nullptr, nullptr, T, D, true, st),
-          "first norm backward");
-    if (!defer) {
-      const Pending p = {bf(dout), dz, dqkv, dy, s, g[DOWN_W], g[UP_W], g[QKV_W], g[PROJ_W]};
-      weight_gradients({p}, d, st);
-    }
+    const auto [dx, tmp] = layer_backward(dout, x, w, s, g, d, defer);
     return std::make_tuple(dx, grads, defer ? tmp : at::Tensor());
   });
   // The weight gradients of layers whose backward was called with defer: (output gradient, slab, the third result of

@@ -9,4 +9,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   mccl::bind_runtime(m);
   mccl::bind_ops(m);
   mccl::bind_layers(m);
+  mccl::bind_decoder_autograd(m);
 }

@@ -127,7 +127,7 @@ struct GemmArgs {
   int epilogue = EPI_NONE;
 };
 // Returns cudaErrorNotSupported for shapes the kernel does not cover
-// (K % 64 != 0, N % 8 != 0, unaligned pointers); the caller falls back.
+// (N % 8 != 0, unaligned pointers or row strides); the caller falls back.
 cudaError_t gemm_bf16_tn(const GemmArgs& args, cudaStream_t stream);
 // Up to any number of weight gradients dW[N, K] = dY[tokens, N]^T · X[tokens, K] over the same tokens, worked through together
 // (sixteen products per launch).  A product is a GemmArgs with both operands MN-major, fp32 output, no epilogue; all of them

@@ -298,30 +298,52 @@ class Decoder(nn.Module):
             x = blk(x, rope, native)
         return self.ln_f(x, native)
 
-    def _forward_without_gradients(self, tokens: torch.Tensor):
-        """Logits from one native call over the whole decoder, or None where it does not apply."""
-        cfg = self.cfg
-        from .. import _C
-        from ..ops.functional import native_attention_supported
-        rope = cfg.pos == "rope"
-        if tokens.dim() != 2 or tokens.dtype != torch.int64 or cfg.d_model % 64 or cfg.d_ff % 64 or cfg.vocab % 8:
-            return None
-        if rope:
-            if cfg.norm != "rmsnorm" or cfg.act != "swiglu" or cfg.head_dim % 8:
-                return None
-        elif (cfg.norm != "layernorm" or cfg.act != "gelu" or tokens.shape[1] > cfg.max_seq
-              or not native_attention_supported(tokens.shape[1], cfg.head_dim)):
-            return None
-        if torch.is_autocast_enabled():
-            return None
-        s = _structure(self, tokens.device)
-        if s is None:
-            return None
+    def _ordered(self, s, rope: bool):
+        """The layers' parameters in the order the native calls take them."""
         layers = s.__dict__.get("ordered")
         if layers is None:
             names = (("ln1.weight", "qkv.weight", "proj.weight", "ln2.weight", "gate_up.weight", "down.weight") if rope else
                      [f"{m}.{k}" for m in ("ln1", "qkv", "proj", "ln2", "up", "down") for k in ("weight", "bias")])
-            s.ordered = layers = [s.params[f"blocks.{i}.{n}"] for i in range(cfg.n_layers) for n in names]
+            s.ordered = layers = [s.params[f"blocks.{i}.{n}"] for i in range(self.cfg.n_layers) for n in names]
+        return layers
+
+    def _fused_gelu(self, tokens: torch.Tensor) -> bool:
+        cfg = self.cfg
+        from .. import _C
+        from ..ops.functional import native_attention_supported
+        return (cfg.pos == "learned" and cfg.norm == "layernorm" and cfg.act == "gelu" and tokens.dim() == 2 and tokens.dtype == torch.int64
+                and cfg.vocab % 8 == 0 and tokens.shape[1] <= cfg.max_seq and not torch.is_autocast_enabled()
+                and native_attention_supported(tokens.shape[1], cfg.head_dim)
+                and _C.decoder_layer_supported(tokens.shape[1], cfg.n_heads, cfg.d_model, cfg.d_ff))
+
+    def _loss_in_one_call(self, tokens: torch.Tensor, targets: torch.Tensor):
+        """The training loss through C++ autograd nodes, or None where that does not apply (a trainer's gradient buffers, frozen
+        or replaced parameters, hooks)."""
+        if not self._fused_gelu(tokens) or targets.dtype != torch.int64 or targets.numel() != tokens.numel():
+            return None
+        s = _structure(self, tokens.device)
+        if s is None or hasattr(self.tok.weight, "_grad_sink") or not all(p.requires_grad for p in s.params.values()):
+            return None
+        from .. import _C
+        p = s.params
+        return _C.decoder_loss(tokens, targets, p["tok.weight"], p["pos.weight"], self._ordered(s, False), p["ln_f.weight"], p["ln_f.bias"],
+                               self.head_weight(), self.cfg.n_heads, self.cfg.eps)
+
+    def _forward_without_gradients(self, tokens: torch.Tensor):
+        """Logits from one native call over the whole decoder, or None where it does not apply."""
+        cfg = self.cfg
+        from .. import _C
+        rope = cfg.pos == "rope"
+        if rope:
+            if (tokens.dim() != 2 or tokens.dtype != torch.int64 or cfg.d_model % 64 or cfg.d_ff % 64 or cfg.vocab % 8 or cfg.norm != "rmsnorm"
+                    or cfg.act != "swiglu" or cfg.head_dim % 8 or torch.is_autocast_enabled()):
+                return None
+        elif not self._fused_gelu(tokens):
+            return None
+        s = _structure(self, tokens.device)
+        if s is None:
+            return None
+        layers = self._ordered(s, rope)
         head = self.head_weight()
         if hasattr(head, "_bf16"):   # a trainer keeps bf16 copies of the matrices up to date
             layers = [getattr(p, "_bf16", p) if p.dim() == 2 else p for p in layers]
@@ -340,6 +362,10 @@ class Decoder(nn.Module):
             logits = self._forward_without_gradients(tokens)
             if logits is not None:
                 return logits
+        if targets is not None and torch.is_grad_enabled() and _FUSE_LAYER and self._native(tokens):
+            loss = self._loss_in_one_call(tokens, targets)
+            if loss is not None:
+                return loss
         h = self.hidden(tokens)
         native = self._native(tokens)
         w = self.head_weight()

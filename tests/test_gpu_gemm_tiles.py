@@ -70,11 +70,14 @@ def test_long_contraction_is_split(C):
 
 
 @pytest.mark.parametrize("K", [8, 72, 1000])
-def test_ragged_contraction_of_row_major_operands(C, K):
-    """Weight gradients over any number of tokens: past the last row the loads are zeros."""
+def test_ragged_contraction(C, K):
+    """Contractions that end inside a k-block: past the end the loads are zeros."""
     torch.manual_seed(K)
     a, b = torch.randn(K, 264, device="cuda").bfloat16(), torch.randn(K, 136, device="cuda").bfloat16()
-    assert _rel(C.gemm_bf16(a, b, None, "none", True, None, False, True, True)[0], a.float().t() @ b.float()) < 1e-5
+    ref = a.float().t() @ b.float()
+    assert _rel(C.gemm_bf16(a, b, None, "none", True, None, False, True, True)[0], ref) < 1e-5
+    assert _rel(C.gemm_bf16(a.t().contiguous(), b, None, "none", False, None, False, False, True)[0], ref) < 1e-2
+    assert _rel(C.gemm_bf16(a.t().contiguous(), b.t().contiguous())[0], ref) < 1e-2
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 8, 64), (300, 200, 128), (4096, 2048, 512)])
