@@ -54,7 +54,7 @@ void bind_ops(py::module_& m) {
   m.def("launch_counts_reset", [] { launch_counts_reset(); });
   m.def("launch_total", [] { return launch_total(); });
   m.def("set_gemm_kernel", &ops::set_gemm_kernel, py::arg("name"),
-        "Kernel for plain products from now on: 'pair' or 'tile' (the default: tile chosen by size), 'tile64', 'tile128', "
+        "Kernel for plain products from now on: 'pair' or 'tile' (the default: tile chosen by size), 'tile64', 'tile128', 'tile192', "
         "'pair256' (that tile), 'persistent' (one CTA per SM); '' returns to MCCL_GEMM_KERNEL / the default.");
   m.def("set_gemm_cta_limit", &ops::set_gemm_cta_limit, py::arg("ctas"),
         "Caps the CTAs (SMs) of plain GEMM launches from now on; 0 = one per SM.");
@@ -163,8 +163,7 @@ void bind_ops(py::module_& m) {
         // A contraction far longer than the output is wide (the input gradient of an LM head: 32000 against 512) has too few
         // tiles for the SMs; its fp32 partial sums go through a workspace (4096 x 512 x 32000: 123 -> 108 us).
         at::Tensor partial;
-        if (!out_fp32 && !out.has_value() && g.epilogue == ops::EPI_NONE && !g.residual && !g.mul && !g.colsum && K >= 8 * N && K >= 4096 &&
-            ((M + 127) / 128) * ((N + 127) / 128) < 4 * ops::gemm_sm_count()) {
+        if (!out_fp32 && !out.has_value() && g.epilogue == ops::EPI_NONE && !g.residual && !g.mul && !g.colsum && ops::gemm_wants_partial_sums(g)) {
           partial = at::zeros({M, N}, a.options().dtype(at::kFloat));
           g.d = partial.data_ptr();
           g.d_fp32 = g.accumulate = true;

@@ -133,25 +133,27 @@ struct CrossEntropyNode : torch::autograd::Function<CrossEntropyNode> {
     cudaStream_t st = stream_on(h);
     at::Tensor dh = at::empty_like(h);
     const bf16* w = bf(flat) + ctx->saved_data["off"].toInt();
-    if (V >= 8 * D && V >= 4096) {   // far longer than it is wide: fp32 partial sums (see gemm_bf16)
+    ops::GemmArgs g;
+    g.a = bf(dlogits);
+    g.b = w;
+    g.b_mn_major = true;
+    g.d = dh.data_ptr();
+    g.m = T;
+    g.n = g.ldb = g.ldd = D;
+    g.k = g.lda = V;
+    if (ops::gemm_wants_partial_sums(g)) {
       at::Tensor partial = at::zeros({T, D}, head.options());
-      ops::GemmArgs g;
-      g.a = bf(dlogits);
-      g.b = w;
-      g.b_mn_major = g.d_fp32 = g.accumulate = true;
+      g.d_fp32 = g.accumulate = true;
       g.d = partial.data_ptr();
-      g.m = T;
-      g.n = g.ldb = g.ldd = D;
-      g.k = g.lda = V;
       check(ops::gemm_bf16_tn(g, st), "head backward");
       check(ops::cast_f32_bf16(partial.data_ptr<float>(), bf(dh), static_cast<long long>(T) * D, st), "head backward");
     } else {
-      input_gradient(bf(dlogits), w, bf(dh), T, V, D, nullptr, nullptr, st, "head backward");
+      check(ops::gemm_bf16_tn(g, st), "head backward");
     }
     at::Tensor dw = at::empty({V, D}, head.options());
-    ops::GemmArgs g = weight_gradient(bf(dlogits), bf(h), dw.data_ptr<float>(), T, V, D);
-    g.accumulate = false;
-    check(ops::gemm_bf16_tn(g, st), "head weight gradient");
+    ops::GemmArgs wg = weight_gradient(bf(dlogits), bf(h), dw.data_ptr<float>(), T, V, D);
+    wg.accumulate = false;
+    check(ops::gemm_bf16_tn(wg, st), "head weight gradient");
     return {dh, dw, at::Tensor(), at::Tensor(), at::Tensor()};
   }
 };

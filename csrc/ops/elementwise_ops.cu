@@ -45,9 +45,77 @@ uint64_t launch_count() { return g_launches.load(); }
 void count_launch(int n) { g_launches.fetch_add(static_cast<uint64_t>(n)); }
 
 // ------------------------------------------------------------------- norm --
-// One warp per row; dim must be a multiple of 8.  kVecs > 0: the row is at most kVecs x 256 wide and stays in registers, so
-// it is read once with all of its loads in flight (4096 x 512: 5.0 us in three passes over the row, 3.2 us in one).
+// One warp per row and, where the row is at most kVecs x 256 wide, in registers: a warp works through several rows, keeps its
+// columns' weights and has the next row's loads in flight while it reduces this one.  (Three passes over a row: 5.0 us at
+// 4096 x 512; one row per warp, weights loaded when they are needed: 3.7 us, and 15 us at 16384 rows, where the row's
+// bytes take 5.)
 template <bool kLayerNorm, int kVecs>
+__global__ void __launch_bounds__(256) norm_fwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
+                                                            const float* __restrict__ b, __nv_bfloat16* __restrict__ y,
+                                                            float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows,
+                                                            int dim, float eps) {
+  const int lane = threadIdx.x & 31, vecs = dim >> 3, stride = gridDim.x * 8;
+  int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  float ww[kVecs][8], bb[kLayerNorm ? kVecs : 1][8];
+  // parameters are not written by the kernels just before this one in any program, but nothing says so: they wait too
+  ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
+  uint4 next[kVecs];
+  auto fetch = [&](int r) {
+    const uint4* xr = reinterpret_cast<const uint4*>(x) + static_cast<size_t>(r) * vecs + lane;
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) next[k] = __ldg(xr + 32 * k);
+  };
+  if (row < rows) fetch(row);
+#pragma unroll
+  for (int k = 0; k < kVecs; ++k) {
+    const int v = lane + 32 * k;
+    if (v < vecs) {
+      const float4 w0 = __ldg(reinterpret_cast<const float4*>(w) + 2 * v), w1 = __ldg(reinterpret_cast<const float4*>(w) + 2 * v + 1);
+      ww[k][0] = w0.x; ww[k][1] = w0.y; ww[k][2] = w0.z; ww[k][3] = w0.w; ww[k][4] = w1.x; ww[k][5] = w1.y; ww[k][6] = w1.z; ww[k][7] = w1.w;
+      if constexpr (kLayerNorm) {
+        const float4 b0 = __ldg(reinterpret_cast<const float4*>(b) + 2 * v), b1 = __ldg(reinterpret_cast<const float4*>(b) + 2 * v + 1);
+        bb[k][0] = b0.x; bb[k][1] = b0.y; bb[k][2] = b0.z; bb[k][3] = b0.w; bb[k][4] = b1.x; bb[k][5] = b1.y; bb[k][6] = b1.z; bb[k][7] = b1.w;
+      }
+    }
+  }
+  for (; row < rows; row += stride) {
+    float f[kVecs][8], sum = 0.f, sq = 0.f;
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) {
+        unpack8(next[k], f[k]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += f[k][i];
+      }
+    if (row + stride < rows) fetch(row + stride);
+    const float mean = kLayerNorm ? warp_sum(sum) / dim : 0.f;
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sq += (f[k][i] - mean) * (f[k][i] - mean);
+      }
+    const float rstd = rsqrtf(warp_sum(sq) / dim + eps);
+    uint4* yr = reinterpret_cast<uint4*>(y) + static_cast<size_t>(row) * vecs + lane;
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (lane + 32 * k < vecs) {
+        float o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = (f[k][i] - mean) * rstd * ww[k][i] + (kLayerNorm ? bb[kLayerNorm ? k : 0][i] : 0.f);
+        yr[32 * k] = pack8(o);
+      }
+    if (lane == 0 && mean_out != nullptr) {
+      mean_out[row] = mean;
+      rstd_out[row] = rstd;
+    }
+  }
+}
+
+// Rows of any length: three passes over the row, the second and third from cache.
+template <bool kLayerNorm>
 __global__ void __launch_bounds__(256) norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
                                                        const float* __restrict__ b, __nv_bfloat16* __restrict__ y,
                                                        float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows,
@@ -60,10 +128,27 @@ __global__ void __launch_bounds__(256) norm_fwd_kernel(const __nv_bfloat16* __re
   const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(warp) * dim);
   uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(warp) * dim);
   const int vecs = dim >> 3;
-  auto normalise = [&](int v, const float (&f)[8], float mean, float rstd) {
+  float sum = 0.f, sq = 0.f;
+  for (int v = lane; v < vecs; v += 32) {
+    float f[8];
+    unpack8(xr[v], f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sum += f[i];
+  }
+  const float mean = kLayerNorm ? warp_sum(sum) / dim : 0.f;
+  for (int v = lane; v < vecs; v += 32) {
+    float f[8];
+    unpack8(xr[v], f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sq += (f[i] - mean) * (f[i] - mean);
+  }
+  const float rstd = rsqrtf(warp_sum(sq) / dim + eps);
+  for (int v = lane; v < vecs; v += 32) {
+    float f[8], o[8];
+    unpack8(xr[v], f);
     const float4 w0 = __ldg(reinterpret_cast<const float4*>(w) + 2 * v), w1 = __ldg(reinterpret_cast<const float4*>(w) + 2 * v + 1);
     const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-    float bb[8] = {0, 0, 0, 0, 0, 0, 0, 0}, o[8];
+    float bb[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (kLayerNorm) {
       const float4 b0 = __ldg(reinterpret_cast<const float4*>(b) + 2 * v), b1 = __ldg(reinterpret_cast<const float4*>(b) + 2 * v + 1);
       bb[0] = b0.x; bb[1] = b0.y; bb[2] = b0.z; bb[3] = b0.w; bb[4] = b1.x; bb[5] = b1.y; bb[6] = b1.z; bb[7] = b1.w;
@@ -71,53 +156,6 @@ __global__ void __launch_bounds__(256) norm_fwd_kernel(const __nv_bfloat16* __re
 #pragma unroll
     for (int i = 0; i < 8; ++i) o[i] = (f[i] - mean) * rstd * ww[i] + bb[i];
     yr[v] = pack8(o);
-  };
-  float sum = 0.f, sq = 0.f, mean, rstd;
-  if constexpr (kVecs > 0) {
-    uint4 raw[kVecs];
-#pragma unroll
-    for (int k = 0; k < kVecs; ++k)
-      if (lane + 32 * k < vecs) raw[k] = __ldg(xr + lane + 32 * k);
-    float f[kVecs][8];
-#pragma unroll
-    for (int k = 0; k < kVecs; ++k) {
-      if (lane + 32 * k < vecs) {
-        unpack8(raw[k], f[k]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) sum += f[k][i];
-      }
-    }
-    mean = kLayerNorm ? warp_sum(sum) / dim : 0.f;
-#pragma unroll
-    for (int k = 0; k < kVecs; ++k)
-      if (lane + 32 * k < vecs) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) sq += (f[k][i] - mean) * (f[k][i] - mean);
-      }
-    rstd = rsqrtf(warp_sum(sq) / dim + eps);
-#pragma unroll
-    for (int k = 0; k < kVecs; ++k)
-      if (lane + 32 * k < vecs) normalise(lane + 32 * k, f[k], mean, rstd);
-  } else {
-    for (int v = lane; v < vecs; v += 32) {
-      float f[8];
-      unpack8(xr[v], f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) sum += f[i];
-    }
-    mean = kLayerNorm ? warp_sum(sum) / dim : 0.f;
-    for (int v = lane; v < vecs; v += 32) {
-      float f[8];
-      unpack8(xr[v], f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) sq += (f[i] - mean) * (f[i] - mean);
-    }
-    rstd = rsqrtf(warp_sum(sq) / dim + eps);
-    for (int v = lane; v < vecs; v += 32) {
-      float f[8];
-      unpack8(xr[v], f);
-      normalise(v, f, mean, rstd);
-    }
   }
   if (lane == 0 && mean_out != nullptr) {
     mean_out[warp] = mean;
@@ -179,7 +217,8 @@ __global__ void __launch_bounds__(256) norm_bwd_dx_kernel(const __nv_bfloat16* _
 // The whole backward of a norm in one pass: dx, and added into fp32 buffers the weight and bias gradients and (optional) the
 // column sums of dx_add and of dx, which are bias gradients of the projections around the norm.  One warp per row, several
 // rows per warp; a lane keeps the sums of its 8 x kVecs columns in registers until the CTA adds them up at the end.
-// (dx alone and the column sums in a pass of their own: 6.6 + 5.2 us at 4096 x 512, and 4.1 us for each further bias.)
+// (dx alone and the column sums in a pass of their own: 6.6 + 5.2 us at 4096 x 512, and 4.1 us for each further bias.)  With 8 or
+// 16 warps per SM, which is what the sums leave room for, the next row has to be in flight while a row is reduced.
 template <bool kLayerNorm, int kVecs, bool kSums>
 __global__ void __launch_bounds__(256) norm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                              const float* __restrict__ w, const float* __restrict__ mean,
@@ -199,17 +238,33 @@ __global__ void __launch_bounds__(256) norm_bwd_fused_kernel(const __nv_bfloat16
     }
   ::mccl::pdl_wait();
   ::mccl::pdl_trigger();
-  for (int row = blockIdx.x * 8 + warp; row < rows; row += gridDim.x * 8) {
+  uint4 nx[kVecs], ng[kVecs], na[kVecs];
+  float nmu = 0.f, nrs = 0.f;
+  auto fetch = [&](int row) {
     const size_t at = static_cast<size_t>(row) * vecs + lane;
-    uint4 rx[kVecs], rg[kVecs], ra[kVecs];
 #pragma unroll
     for (int k = 0; k < kVecs; ++k)
       if (lane + 32 * k < vecs) {
-        rx[k] = __ldg(reinterpret_cast<const uint4*>(x) + at + 32 * k);
-        rg[k] = __ldg(reinterpret_cast<const uint4*>(dy) + at + 32 * k);
-        if (dx_add != nullptr) ra[k] = __ldg(reinterpret_cast<const uint4*>(dx_add) + at + 32 * k);
+        nx[k] = __ldg(reinterpret_cast<const uint4*>(x) + at + 32 * k);
+        ng[k] = __ldg(reinterpret_cast<const uint4*>(dy) + at + 32 * k);
+        if (dx_add != nullptr) na[k] = __ldg(reinterpret_cast<const uint4*>(dx_add) + at + 32 * k);
       }
-    const float mu = kLayerNorm ? mean[row] : 0.f, rs = rstd[row];
+    nmu = kLayerNorm ? __ldg(mean + row) : 0.f;
+    nrs = __ldg(rstd + row);
+  };
+  int row = blockIdx.x * 8 + warp;
+  if (row < rows) fetch(row);
+  for (; row < rows; row += gridDim.x * 8) {
+    const size_t at = static_cast<size_t>(row) * vecs + lane;
+    uint4 rx[kVecs], rg[kVecs], ra[kVecs];
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k) {
+      rx[k] = nx[k];
+      rg[k] = ng[k];
+      ra[k] = na[k];
+    }
+    const float mu = nmu, rs = nrs;
+    if (row + static_cast<int>(gridDim.x) * 8 < rows) fetch(row + gridDim.x * 8);   // in flight while this row is reduced
     float c1 = 0.f, c2 = 0.f;  // sum(dy * w * xhat), sum(dy * w)
 #pragma unroll
     for (int k = 0; k < kVecs; ++k)
@@ -389,14 +444,19 @@ int colsum_slabs(int rows) { return (rows + kSlabRows - 1) / kSlabRows; }
 cudaError_t norm_fwd(const __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y, float* mean, float* rstd,
                      int rows, int dim, float eps, cudaStream_t stream) {
   if (dim % 8 != 0) return cudaErrorNotSupported;
-  const int blocks = (rows + 7) / 8, vecs = (dim + 255) / 256;
-#define MCCL_NORM_FWD(LN, V) MCCL_LAUNCH_PDL((norm_fwd_kernel<LN, V>), blocks, 256, 0, stream, x, w, b, y, mean, rstd, rows, dim, eps)
+  const int vecs = (dim + 255) / 256;
+  int blocks = (rows + 7) / 8;
+  // more rows per warp once every warp that registers leave room for has one
+  const int most = 148 * (vecs == 1 ? 5 : (vecs == 2 ? 3 : (vecs <= 4 ? 2 : 1)));
+  if (vecs <= 8 && blocks > most) blocks = most;
+#define MCCL_NORM_FWD(LN, V) MCCL_LAUNCH_PDL((norm_fwd_rows_kernel<LN, V>), blocks, 256, 0, stream, x, w, b, y, mean, rstd, rows, dim, eps)
 #define MCCL_NORM_FWD_V(LN)                              \
   (vecs == 1   ? MCCL_NORM_FWD(LN, 1)                    \
    : vecs == 2 ? MCCL_NORM_FWD(LN, 2)                    \
+   : vecs == 3 ? MCCL_NORM_FWD(LN, 3)                    \
    : vecs <= 4 ? MCCL_NORM_FWD(LN, 4)                    \
    : vecs <= 8 ? MCCL_NORM_FWD(LN, 8)                    \
-               : MCCL_NORM_FWD(LN, 0))
+               : MCCL_LAUNCH_PDL(norm_fwd_kernel<LN>, blocks, 256, 0, stream, x, w, b, y, mean, rstd, rows, dim, eps))
   if (b) MCCL_NORM_FWD_V(true);
   else MCCL_NORM_FWD_V(false);
 #undef MCCL_NORM_FWD_V
@@ -444,7 +504,7 @@ cudaError_t norm_bwd_fused(const __nv_bfloat16* dy, const __nv_bfloat16* x, cons
   // the sums of a lane's columns live in registers: four sets of up to 32 or one of up to 64
   if (dim % 8 != 0 || vecs > (layernorm || sums ? 4 : 8) || (sum_add != nullptr && dx_add == nullptr)) return cudaErrorNotSupported;
   int blocks = (rows + 7) / 8;
-  const int most = vecs <= 2 ? 2 * 148 : 148;
+  const int most = vecs == 1 ? 2 * 148 : 148;
   if (blocks > most) blocks = most;
   if (blocks < 1) return cudaSuccess;
   auto go = [&](auto kernel, int v, int sets, std::atomic<bool>& configured) -> cudaError_t {
@@ -580,9 +640,9 @@ __global__ void __launch_bounds__(512) ce_kernel(__nv_bfloat16* __restrict__ log
   uint4* lv = reinterpret_cast<uint4*>(lr);
   const int vecs = vocab >> 3;
   float mx = -INFINITY, sm = 0.f;
-  for (int v = tid; v < vecs; v += blockDim.x) {
+  auto take = [&](const uint4& raw) {
     float f[8];
-    unpack8(lv[v], f);
+    unpack8(raw, f);
     float local = f[0];
 #pragma unroll
     for (int i = 1; i < 8; ++i) local = fmaxf(local, f[i]);
@@ -592,7 +652,16 @@ __global__ void __launch_bounds__(512) ce_kernel(__nv_bfloat16* __restrict__ log
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) sm += __expf(f[i] - mx);
+  };
+  int v0 = tid;
+  for (; v0 + 3 * 512 < vecs; v0 += 4 * 512) {   // four loads in flight
+    const uint4 r0 = lv[v0], r1 = lv[v0 + 512], r2 = lv[v0 + 1024], r3 = lv[v0 + 1536];
+    take(r0);
+    take(r1);
+    take(r2);
+    take(r3);
   }
+  for (; v0 < vecs; v0 += 512) take(lv[v0]);
   for (int c = vecs * 8 + tid; c < vocab; c += blockDim.x) {
     const float f = __bfloat162float(lr[c]);
     if (f > mx) {
@@ -619,16 +688,28 @@ __global__ void __launch_bounds__(512) ce_kernel(__nv_bfloat16* __restrict__ log
   if (tid == 0) loss_rows[row] = ignore ? 0.f : (logf(bsum) + bmx - __bfloat162float(lr[tgt]));
   __syncthreads();  // the target logit is read before anyone overwrites it
   const float inv = ignore ? 0.f : scale / bsum;
-  for (int v = tid; v < vecs; v += blockDim.x) {
+  const int tgt_vec = ignore ? -1 : static_cast<int>(tgt >> 3), tgt_lane = static_cast<int>(tgt & 7);
+  const float log2e = 1.4426950408889634f, shift = bmx * log2e - log2f(fmaxf(inv, 1e-38f));   // inv * exp(f - bmx) as one exponential
+  auto gradient = [&](const uint4& raw, int v) {
     float f[8], o[8];
-    unpack8(lv[v], f);
+    unpack8(raw, f);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      o[i] = __expf(f[i] - bmx) * inv;
-      if (!ignore && v * 8 + i == tgt) o[i] -= scale;
+    for (int i = 0; i < 8; ++i) o[i] = ignore ? 0.f : exp2f(fmaf(f[i], log2e, -shift));
+    if (v == tgt_vec) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] -= i == tgt_lane ? scale : 0.f;
     }
     lv[v] = pack8(o);
+  };
+  int v1 = tid;
+  for (; v1 + 3 * 512 < vecs; v1 += 4 * 512) {
+    const uint4 r0 = lv[v1], r1 = lv[v1 + 512], r2 = lv[v1 + 1024], r3 = lv[v1 + 1536];
+    gradient(r0, v1);
+    gradient(r1, v1 + 512);
+    gradient(r2, v1 + 1024);
+    gradient(r3, v1 + 1536);
   }
+  for (; v1 < vecs; v1 += 512) gradient(lv[v1], v1);
   for (int c = vecs * 8 + tid; c < vocab; c += blockDim.x) {
     float o = __expf(__bfloat162float(lr[c]) - bmx) * inv;
     if (!ignore && c == tgt) o -= scale;

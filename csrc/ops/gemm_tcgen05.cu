@@ -25,13 +25,14 @@ cudaError_t unsupported(const char* why) {
 }  // namespace
 
 namespace {
-// The tile kernel with a tile of its choosing (0) or a given one (64, 128, 256), or the one-CTA persistent kernel.
+// The tile kernel with a tile of its choosing (0) or a given one (64, 128, 192, 256), or the one-CTA persistent kernel.
 constexpr int kPersistent = -1;
 std::atomic<int> g_gemm_kernel_override{-2};
 int kernel_index(const std::string& s) {
   if (s == "persistent") return kPersistent;
   if (s == "tile64") return 64;
   if (s == "tile128") return 128;
+  if (s == "tile192") return 192;
   if (s == "pair256") return 256;
   return 0;
 }

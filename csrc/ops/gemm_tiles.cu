@@ -11,6 +11,7 @@ namespace tiles {
   extern template cudaError_t launch_tiles<128, false, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t);
 #define MCCL_TILES_EXTERN_PAIR(A, B, OUT, MAX)                                                                                \
   MCCL_TILES_EXTERN(A, B, OUT, MAX)                                                                                           \
+  extern template cudaError_t launch_tiles<192, false, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t);         \
   extern template cudaError_t launch_tiles<256, true, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t);          \
   extern template int max_pairs<256, A, B, OUT, MAX>();
 MCCL_TILES_EXTERN(false, false, OUT_GELU, 1)
@@ -30,7 +31,7 @@ MCCL_TILES_EXTERN_PAIR(true, true, OUT_F32, kMaxGroup)
 namespace {
 
 struct Plan {
-  int bn = 0;         // 64, 128 (one CTA) or 256 (CTA pair)
+  int bn = 0;         // 64, 128, 192 (one CTA) or 256 (CTA pair)
   int workers = 0;
   int splits = 1;
 };
@@ -39,11 +40,11 @@ constexpr double kRunsBytes = 80e6;   // of 126 MB of L2, which also holds the o
 constexpr int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Clocks of a product on one kind of tile, fitted to graphs of back-to-back launches (70M to 1.3B shapes) and the kernel's
-// timeline: per 64 of K a 128 x 64 tile takes 260 clocks, a 128 x 128 tile 350 and a 256 x 256 pair tile 515 (its MMAs
-// need 512); an epilogue 1500 / 2000 / 4000, fp32 sums added into memory 1800 / 2600 / 7000, hidden behind the next tile's
+// timeline: per 64 of K a 128 x 64 tile takes 260 clocks, a 128 x 128 tile 350, a 128 x 192 tile 520 and a 256 x 256
+// pair tile 515 (its MMAs need 512); an epilogue 1500 / 2000 / 2500 / 3000, fp32 sums added into memory 1800 / 2600 / 3900 / 7000, hidden behind the next tile's
 // main loop when there is one; launch and set-up 3500, a pair's two cluster barriers 2000 more.
-constexpr double kPer64[3] = {260, 350, 515}, kEpilogue[3] = {1500, 2000, 4000}, kAdding[3] = {1800, 2600, 7000};
-int kind_of(int bn) { return bn == 64 ? 0 : (bn == 128 ? 1 : 2); }
+constexpr double kPer64[4] = {260, 350, 520, 515}, kEpilogue[4] = {1500, 2000, 2500, 3000}, kAdding[4] = {1800, 2600, 3900, 7000};
+int kind_of(int bn) { return bn / 64 - 1; }
 
 double cost(int bn, int tiles, int k, int workers, int splits, bool gelu, bool adding) {
   const int kind = kind_of(bn);
@@ -52,7 +53,7 @@ double cost(int bn, int tiles, int k, int workers, int splits, bool gelu, bool a
   if (gelu) epilogue *= 2.5;
   const double main_loop = kPer64[kind] * ceil_div(k, 64) / splits;
   const double round = main_loop > epilogue ? main_loop : epilogue;
-  return 3500 + (kind == 2 ? 2000 : 0) + (rounds - 1) * round + main_loop + epilogue;
+  return 3500 + (kind == 3 ? 2000 : 0) + (rounds - 1) * round + main_loop + epilogue;
 }
 
 Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, bool gelu, bool splittable) {
@@ -61,9 +62,9 @@ Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, boo
   const int k = args[0].k;
   double operand_bytes = 0;
   for (int p = 0; p < count; ++p) operand_bytes += 2.0 * k * (static_cast<double>(args[p].m) + args[p].n);
-  for (int bn : {64, 128, 256}) {
+  for (int bn : {64, 128, 192, 256}) {
     if (forced ? bn != forced : false) continue;
-    if (bn == 256 && (gelu || pairs < 1)) continue;
+    if ((bn == 256 && (gelu || pairs < 1)) || (bn == 192 && gelu)) continue;
     const int workers = bn == 256 ? pairs : sms;
     int tiles = 0;
     for (int p = 0; p < count; ++p) tiles += ceil_div(args[p].m, bn == 256 ? 256 : 128) * ceil_div(args[p].n, bn);
@@ -109,6 +110,8 @@ cudaError_t run(const GemmArgs* a, int count, int forced, cudaStream_t stream) {
   const Plan plan = choose(a, count, forced, sms, pairs, kOut == OUT_GELU, splittable);
   if (plan.bn == 64) return launch_tiles<64, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
   if constexpr (kOut != OUT_GELU)
+    if (plan.bn == 192) return launch_tiles<192, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
+  if constexpr (kOut != OUT_GELU)
     if (plan.bn == 256) return launch_tiles<256, true, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
   return launch_tiles<128, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
 }
@@ -134,9 +137,15 @@ cudaError_t launch_gemm_tiles(const GemmArgs& a, int forced_bn, cudaStream_t str
     if (gelu || a.d_fp32 || a.bias || a.residual || a.a_mn_major || !a.b_mn_major) return cudaErrorInvalidValue;
     return tiles::run<false, true, tiles::OUT_BF16_SUM>(&a, 1, forced_bn, stream);
   }
-  if (gelu) return tiles::run<false, false, tiles::OUT_GELU>(&a, 1, forced_bn == 256 ? 128 : forced_bn, stream);
+  if (gelu) return tiles::run<false, false, tiles::OUT_GELU>(&a, 1, forced_bn > 128 ? 128 : forced_bn, stream);
   if (a.d_fp32) return tiles::run_majors<tiles::OUT_F32>(a, forced_bn, stream);
   return tiles::run_majors<tiles::OUT_BF16>(a, forced_bn, stream);
+}
+
+// Measured on an LM head's input gradient (K 32000): 32 pair tiles (4096 x 512) 108 against 123 us, 48 (4096 x 768) 145 against
+// 152; with 64 tiles (4096 x 1024, K 8192) the zeroing, adding and casting cost more than the idle SMs, 67 against 43.
+bool gemm_wants_partial_sums(const GemmArgs& a) {
+  return a.k >= 4096 && tiles::ceil_div(a.m, 256) * tiles::ceil_div(a.n, 256) * 10 <= gemm_sm_count() / 2 * 7;
 }
 
 cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream) {

@@ -1,7 +1,7 @@
 // The bf16 GEMM of the model operators: D[M, N] = A[M, K] * B[N, K]^T on tcgen05, one persistent kernel template.
 //
 // Two shapes of tile:
-//   one CTA    128 x BN (BN 64 or 128): cta_group::1; every SM works alone, no cluster launch, no cluster barriers
+//   one CTA    128 x BN (BN 64, 128 or 192): cta_group::1; every SM works alone, no cluster launch, no cluster barriers
 //   CTA pair   256 x 256: cta_group::2; each CTA loads its 128 rows of A and half of the B tile and the even CTA issues
 //              the MMAs for both, so a 128 x 256 block costs 32 KB of operands per 64 of K instead of 48
 //
@@ -21,7 +21,7 @@
 //
 //   warp 0        producer: one elected thread issues the TMA loads
 //   warp 1        MMA issuer (even CTA of a pair), tensor-memory allocation
-//   warps 2..     epilogue, two per tensor-memory lane quarter (one where BN is 64); the accumulator is double buffered
+//   warps 2..     epilogue, one per tensor-memory lane quarter and 64 columns; the accumulator is double buffered
 //
 // No load uses cluster multicast.  Every wait is bounded (two seconds); a wait that runs out sets the error word the
 // host checks, the roles leave their loops, and the CTAs of a pair still meet before tensor memory is freed.
@@ -56,21 +56,21 @@ struct Problems {
 
 template <int BN, bool kPair, bool kGelu = false>
 struct Shape {
-  static constexpr int kStages = kPair ? 5 : (BN == 64 ? 8 : (kGelu ? 5 : 6));
+  static constexpr int kStages = kPair ? 5 : (BN == 64 ? 8 : (BN == 192 ? 4 : (kGelu ? 5 : 6)));
   static constexpr int kRowsB = kPair ? BN / 2 : BN;   // rows of the B tile this CTA loads
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBBytes = kRowsB * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   // GELU: 11 instructions per value and two of them long; twice the warps, half the columns each, so that more chains are in
   // flight per scheduler, and a staging buffer per output
-  static constexpr int kEpiWarps = (BN == 64 ? 4 : 8) * (kGelu ? 2 : 1);
+  static constexpr int kEpiWarps = BN / 16 * (kGelu ? 2 : 1);   // 64 (GELU: 32) accumulator columns each
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
-  static constexpr int kCols = BN / (kEpiWarps / 4);   // accumulator columns per epilogue warp
-  static constexpr int kBufs = kGelu ? 1 : kCols / 64;             // 4 KB staging buffers per epilogue warp
+  static constexpr int kCols = BN / (kEpiWarps / 4);
   static constexpr int kTiles = kStages * kStageBytes;
   static constexpr int kStagingOff = kTiles;
-  static constexpr int kBarOff = kStagingOff + kEpiWarps * kBufs * 4096;
-  static constexpr int kBarriers = 2 * kStages + 4 + kEpiWarps * kBufs;
+  static constexpr int kBarOff = kStagingOff + kEpiWarps * 4096;
+  static constexpr int kTmem = BN > 128 ? 512 : 4 * BN / 2;       // two accumulators; allocations are powers of two
+  static constexpr int kBarriers = 2 * kStages + 4 + kEpiWarps;
   static constexpr int kTotal = kBarOff + kBarriers * 8 + 16 + 1024;
   static_assert(kTotal <= 227 * 1024, "shared memory of one CTA");
 };
@@ -197,7 +197,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
   uint64_t* acc_full = empty + kStages;   // [2]
   uint64_t* acc_empty = acc_full + 2;     // [2]
   uint64_t* extra_full = acc_empty + 2;   // [epilogue warp][buffer]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(extra_full + S::kEpiWarps * S::kBufs);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(extra_full + S::kEpiWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const unsigned long long tl_t0 = tl_begin(g.tl);
@@ -221,7 +221,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
       tc::mbar_init(&acc_full[b], 1);
       tc::mbar_init(&acc_empty[b], (kPair ? 2 : 1) * S::kEpiWarps);
     }
-    for (int b = 0; b < S::kEpiWarps * S::kBufs; ++b) tc::mbar_init(&extra_full[b], 1);
+    for (int b = 0; b < S::kEpiWarps; ++b) tc::mbar_init(&extra_full[b], 1);
     *abort_flag = 0;
     tc::mbar_init_fence();
     for (int p = 0; p < P.count; ++p) {
@@ -233,10 +233,10 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
   }
   if (warp == 1) {
     if constexpr (kPair) {
-      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(2 * BN) : "memory");
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(S::kTmem) : "memory");
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     } else {
-      tc::tmem_alloc(tmem_slot, 2 * BN);
+      tc::tmem_alloc(tmem_slot, S::kTmem);
     }
   }
   tc::fence_before_sync();
@@ -365,7 +365,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           if (!ok) break;
           tc::fence_after_sync();
         }
-        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * BN);
+        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * (S::kTmem / 2));
         for (int kb = kb0; kb < kb1; ++kb) {
           ok = wait(&full[s], parity, abort_flag);
           if (!ok) break;
@@ -398,15 +398,15 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
   } else {
     // ----------------------------------------------------------- epilogue --
     const int e = warp - 2, quarter = warp & 3, part = e >> 2;
-    uint8_t* stage = smem + S::kStagingOff + e * S::kBufs * 4096;
-    uint64_t* xfull = extra_full + e * S::kBufs;
+    uint8_t* stage = smem + S::kStagingOff + e * 4096;
+    uint64_t* xfull = extra_full + e;
     const bool has_bias = kOut != OUT_F32 && (g.epilogue == EPI_BIAS || g.epilogue == EPI_BIAS_GELU || g.epilogue == EPI_BIAS_GELU_D);
     const bool has_extra = kBf16 && (g.mul != nullptr || g.residual != nullptr);
     const bool multiply = g.mul != nullptr;
     const bool gelu_d = g.epilogue == EPI_BIAS_GELU_D || g.epilogue == EPI_GELU_D;
     bool ok = true;
     int i = 0;
-    uint32_t xparity = 0;   // one bit per staging buffer
+    uint32_t xparity = 0;
     for (int w = work_begin; w < work_end; ++i) {
       const Item it = item(w);
       w = it.next;
@@ -422,13 +422,8 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
       if (tc::elect_one()) {
         bulk_wait_read<0>();
         if (has_extra && inside) {
-#pragma unroll
-          for (int b = 0; b < S::kBufs; ++b) {
-            if (col0 + b * 64 < n) {
-              tc::mbar_expect_tx(&xfull[b], 4096);
-              tc::tma_load_2d(stage + b * 4096, &P.x, &xfull[b], col0 + b * 64, row0);
-            }
-          }
+          tc::mbar_expect_tx(xfull, 4096);
+          tc::tma_load_2d(stage, &P.x, xfull, col0, row0);
         }
       }
       // lane l keeps the bias of columns [col0 + 4 l, col0 + 4 l + 4); the loop below spreads it by shuffles
@@ -440,7 +435,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
       if (!ok) break;
       tc::fence_after_sync();
       const unsigned long long ts1 = stamp ? tl_now() : 0ull;
-      const uint32_t taddr = tmem_base + static_cast<uint32_t>(buf * BN + part * S::kCols) + (static_cast<uint32_t>(quarter * 32) << 16);
+      const uint32_t taddr = tmem_base + static_cast<uint32_t>(buf * (S::kTmem / 2) + part * S::kCols) + (static_cast<uint32_t>(quarter * 32) << 16);
       auto last_read = [&]() {
         // every column of this warp's part is in registers: hand the buffer back to the MMA thread
         tc::fence_before_sync();
@@ -458,16 +453,15 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           tc::tmem_ld_wait();
           if (c + 32 >= S::kCols) last_read();
           if (row0 >= m || col0 + c >= n) continue;
-          uint8_t* dst = stage + (S::kBufs > 1 ? ((c >> 5) & 1) * 4096 : 0);
-          if (tc::elect_one()) bulk_wait_read<S::kBufs - 1>();
+          if (tc::elect_one()) bulk_wait_read<0>();
           __syncwarp();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) *stage_unit(dst, lane, j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          for (int j = 0; j < 8; ++j) *stage_unit(stage, lane, j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
           fence_async_smem();
           __syncwarp();
           if (tc::elect_one()) {
-            if (add) reduce_add_2d(map_d, dst, col0 + c, row0);
-            else store_2d(map_d, dst, col0 + c, row0);
+            if (add) reduce_add_2d(map_d, stage, col0 + c, row0);
+            else store_2d(map_d, stage, col0 + c, row0);
             bulk_commit();
           }
           __syncwarp();
@@ -512,76 +506,71 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           __syncwarp();
         }
       } else {
-#pragma unroll 1
-        for (int c = 0; c < S::kCols; c += 64) {
-          const int cg = col0 + c;
-          const bool active = row0 < m && cg < n;   // uniform over the warp
-          uint8_t* buf_c = stage + (c >> 6) * 4096;
-          if (has_extra && active) {
-            ok = wait(&xfull[c >> 6], (xparity >> (c >> 6)) & 1u, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            xparity ^= 1u << (c >> 6);
-          }
+        if (has_extra && inside) {
+          ok = wait(xfull, xparity, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          xparity ^= 1u;
+        }
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t r[32];
-            tc::tmem_ld_32x32(taddr + static_cast<uint32_t>(c + 32 * h), r);
-            tc::tmem_ld_wait();
-            if (h == 1 && c + 64 >= S::kCols) last_read();
-            if (!active) continue;
+        for (int h = 0; h < 2; ++h) {
+          uint32_t r[32];
+          tc::tmem_ld_32x32(taddr + static_cast<uint32_t>(32 * h), r);
+          tc::tmem_ld_wait();
+          if (h == 1) last_read();
+          if (!inside) continue;
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-              const int j = 4 * h + jj;
-              float v[8];
+          for (int jj = 0; jj < 4; ++jj) {
+            const int j = 4 * h + jj;
+            float v[8];
 #pragma unroll
-              for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(r[jj * 8 + q]);
-              if (has_bias) {
-                const int src = (c >> 2) + 2 * j;
-                v[0] += __shfl_sync(0xffffffffu, bias4.x, src);
-                v[1] += __shfl_sync(0xffffffffu, bias4.y, src);
-                v[2] += __shfl_sync(0xffffffffu, bias4.z, src);
-                v[3] += __shfl_sync(0xffffffffu, bias4.w, src);
-                v[4] += __shfl_sync(0xffffffffu, bias4.x, src + 1);
-                v[5] += __shfl_sync(0xffffffffu, bias4.y, src + 1);
-                v[6] += __shfl_sync(0xffffffffu, bias4.z, src + 1);
-                v[7] += __shfl_sync(0xffffffffu, bias4.w, src + 1);
-              }
-              if (has_extra) {
-                float x[8];
-                unpack8(*stage_unit(buf_c, lane, j), x);
-                if (multiply) {
+            for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(r[jj * 8 + q]);
+            if (has_bias) {
+              const int src = 2 * j;
+              v[0] += __shfl_sync(0xffffffffu, bias4.x, src);
+              v[1] += __shfl_sync(0xffffffffu, bias4.y, src);
+              v[2] += __shfl_sync(0xffffffffu, bias4.z, src);
+              v[3] += __shfl_sync(0xffffffffu, bias4.w, src);
+              v[4] += __shfl_sync(0xffffffffu, bias4.x, src + 1);
+              v[5] += __shfl_sync(0xffffffffu, bias4.y, src + 1);
+              v[6] += __shfl_sync(0xffffffffu, bias4.z, src + 1);
+              v[7] += __shfl_sync(0xffffffffu, bias4.w, src + 1);
+            }
+            if (has_extra) {
+              float x[8];
+              unpack8(*stage_unit(stage, lane, j), x);
+              if (multiply) {
 #pragma unroll
-                  for (int q = 0; q < 8; ++q) v[q] *= x[q];
-                } else {
+                for (int q = 0; q < 8; ++q) v[q] *= x[q];
+              } else {
 #pragma unroll
-                  for (int q = 0; q < 8; ++q) v[q] += x[q];
-                }
-              }
-              *stage_unit(buf_c, lane, j) = pack8(v);
-              if constexpr (kOut == OUT_BF16_SUM) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) r[jj * 8 + q] = __float_as_uint(v[q]);
+                for (int q = 0; q < 8; ++q) v[q] += x[q];
               }
             }
+            *stage_unit(stage, lane, j) = pack8(v);
             if constexpr (kOut == OUT_BF16_SUM) {
-              // sums of 32 columns over the warp's 32 rows by halving: 31 shuffles, lane l ends up with column l
 #pragma unroll
-              for (int o = 16; o >= 1; o >>= 1) {
-#pragma unroll
-                for (int q = 0; q < o; ++q) {
-                  const float lo = __uint_as_float(r[q]), hi = __uint_as_float(r[q + o]);
-                  const float other = __shfl_xor_sync(0xffffffffu, (lane & o) ? lo : hi, o);
-                  r[q] = __float_as_uint(((lane & o) ? hi : lo) + other);
-                }
-              }
-              if (cg + 32 * h + lane < n) atomicAdd(g.colsum + cg + 32 * h + lane, __uint_as_float(r[0]));
+              for (int q = 0; q < 8; ++q) r[jj * 8 + q] = __float_as_uint(v[q]);
             }
           }
-          if (!active) continue;
+          if constexpr (kOut == OUT_BF16_SUM) {
+            // sums of 32 columns over the warp's 32 rows by halving: 31 shuffles, lane l ends up with column l
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) {
+#pragma unroll
+              for (int q = 0; q < o; ++q) {
+                const float lo = __uint_as_float(r[q]), hi = __uint_as_float(r[q + o]);
+                const float other = __shfl_xor_sync(0xffffffffu, (lane & o) ? lo : hi, o);
+                r[q] = __float_as_uint(((lane & o) ? hi : lo) + other);
+              }
+            }
+            if (col0 + 32 * h + lane < n) atomicAdd(g.colsum + col0 + 32 * h + lane, __uint_as_float(r[0]));
+          }
+        }
+        if (inside) {
           fence_async_smem();
           __syncwarp();
           if (tc::elect_one()) {
-            store_2d(map_d, buf_c, cg, row0);
+            store_2d(map_d, stage, col0, row0);
             bulk_commit();
           }
           __syncwarp();
@@ -612,8 +601,8 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
   if constexpr (kPair) cluster_sync_all();
   if (warp == 1) {
     tc::fence_after_sync();
-    if constexpr (kPair) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * BN) : "memory");
-    else tc::tmem_dealloc(tmem_base, 2 * BN);
+    if constexpr (kPair) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S::kTmem) : "memory");
+    else tc::tmem_dealloc(tmem_base, S::kTmem);
   }
   tl_end(g.tl, tl_t0, TL_GEMM, (static_cast<uint32_t>(tiles / P.n_tiles[0] * (kPair ? 2 : 1)) << 16) | static_cast<uint32_t>(P.n_tiles[0]));
 }

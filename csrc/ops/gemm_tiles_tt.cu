@@ -7,14 +7,17 @@ namespace tiles {
 
 template cudaError_t launch_tiles<64, false, true, true, OUT_BF16, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template cudaError_t launch_tiles<128, false, true, true, OUT_BF16, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+template cudaError_t launch_tiles<192, false, true, true, OUT_BF16, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template cudaError_t launch_tiles<256, true, true, true, OUT_BF16, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template int max_pairs<256, true, true, OUT_BF16, 1>();
 template cudaError_t launch_tiles<64, false, true, true, OUT_F32, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template cudaError_t launch_tiles<128, false, true, true, OUT_F32, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+template cudaError_t launch_tiles<192, false, true, true, OUT_F32, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template cudaError_t launch_tiles<256, true, true, true, OUT_F32, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template int max_pairs<256, true, true, OUT_F32, 1>();
 template cudaError_t launch_tiles<64, false, true, true, OUT_F32, kMaxGroup>(const GemmArgs*, int, int, int, cudaStream_t);
 template cudaError_t launch_tiles<128, false, true, true, OUT_F32, kMaxGroup>(const GemmArgs*, int, int, int, cudaStream_t);
+template cudaError_t launch_tiles<192, false, true, true, OUT_F32, kMaxGroup>(const GemmArgs*, int, int, int, cudaStream_t);
 template cudaError_t launch_tiles<256, true, true, true, OUT_F32, kMaxGroup>(const GemmArgs*, int, int, int, cudaStream_t);
 template int max_pairs<256, true, true, OUT_F32, kMaxGroup>();
 

@@ -133,12 +133,15 @@ cudaError_t gemm_bf16_tn(const GemmArgs& args, cudaStream_t stream);
 // (sixteen products per launch).  A product is a GemmArgs with both operands MN-major, fp32 output, no epilogue; all of them
 // accumulate, or none.
 cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream);
+// Whether a bf16 product without epilogue is better computed as fp32 partial sums, added into a zeroed fp32 [M, N], and cast:
+// a long contraction whose tiles leave much of the GPU idle.
+bool gemm_wants_partial_sums(const GemmArgs& args);
 // Caps the number of CTAs (= SMs) plain GEMM launches occupy from now on; 0 restores one CTA per SM.  A
 // data-parallel trainer lowers it during backward so that a few SMs stay free for the gradient collectives
 // that run beside the GEMMs.  The value is read at launch time, so it is baked into a captured CUDA graph.
 void set_gemm_cta_limit(int ctas);
-// Which kernel plain products use: "pair" / "tile" (the default: tile chosen by size), "tile64", "tile128", "pair256" (that
-// tile), "persistent" (one CTA per SM); "" = default.
+// Which kernel plain products use: "pair" / "tile" (the default: tile chosen by size), "tile64", "tile128", "tile192",
+// "pair256" (that tile), "persistent" (one CTA per SM); "" = default.
 void set_gemm_kernel(const std::string& name);
 int gemm_cta_limit();
 int gemm_sm_count();

@@ -10,7 +10,7 @@ def _rel(a, b):
     return ((a.double() - b.double()).abs().max() / b.double().abs().max().clamp_min(1e-6)).item()
 
 
-@pytest.fixture(params=["tile64", "tile128", "pair256", ""])
+@pytest.fixture(params=["tile64", "tile128", "tile192", "pair256", ""])
 def C(request):
     from mccl_b200 import _C
     _C.set_gemm_kernel(request.param)
