@@ -50,11 +50,6 @@ def set_wgrad_stream(stream, main_ctas: int = 0, side_ctas: int = 0) -> None:
     _wgrad["main_ctas"], _wgrad["side_ctas"] = main_ctas, side_ctas
 
 
-def mark_wgrad_pending() -> None:
-    """A trainer queued work of its own on the weight-gradient stream."""
-    _wgrad["pending"] = True
-
-
 def join_wgrad(stream=None) -> None:
     """Makes ``stream`` (default: the current one) wait for the weight gradients queued on the side stream."""
     _deferred.flush_all()

@@ -92,20 +92,20 @@ class DDPTrainer:
             comm_threads = int(os.environ.get("MCCL_DDP_COMM_THREADS", "512" if self.comm_sms > 0 else "0"))
         self.comm_threads = comm_threads
         # The optimizer pass over the already reduced buckets runs while the tail buckets' collectives are still
-        # in flight.  (Running the optimizer bucket by bucket during backward was measured too: its CTAs delay
-        # the GEMMs by as much as the pass saves, 6.71 against 6.64 ms per step of the 70M decoder on one GPU.)
+        # in flight.
         if overlap_optimizer is None:
             overlap_optimizer = os.environ.get("MCCL_DDP_OVERLAP_OPTIMIZER", "1") != "0"
         self.overlap_optimizer = bool(overlap_optimizer and overlap and self.world > 1 and device.type == "cuda"
                                       and ops.native_ops_available().get("adamw_flat"))
         self._fused_zero = device.type == "cuda" and bool(ops.native_ops_available().get("adamw_flat"))
+        # One GPU: the optimizer update of a bucket whose gradients are complete runs on a stream of its own while backward
+        # continues (MCCL_OVERLAP_ADAMW=0: one update at the end).  It is bound by memory and the GEMMs beside it are not;
+        # with two CTAs per SM it takes little of what they use.  Measured: SwiGLU decoder 2948 -> 2812 us per step, 70M
+        # decoder with 64 x 256 tokens 10492 -> 10423 us, the 70M and 110M decoders at 16 x 256 the same within noise.
+        self._opt_ctas = int(os.environ.get("MCCL_OVERLAP_ADAMW_CTAS", "2"))
+        self._local_overlap = (self.world == 1 and self._fused_zero and os.environ.get("MCCL_OVERLAP_ADAMW", "1") != "0")
+        self.opt_stream = torch.cuda.Stream(device=device) if self._local_overlap else None
         # Hooks are needed whenever something happens per bucket.
-        # One GPU, MCCL_OVERLAP_ADAMW=1: the optimizer update of a bucket whose gradients are complete runs on the
-        # weight-gradient stream while backward continues.  Off by default: measured 4.79 ms per step against 4.72 with
-        # one update at the end (AdamW's traffic slows the GEMMs it runs beside by more than it hides).
-        self._local_overlap = (self.world == 1 and device.type == "cuda"
-                               and os.environ.get("MCCL_SIDE_WGRAD", "0") != "0"
-                               and os.environ.get("MCCL_OVERLAP_ADAMW", "0") == "1")
         self._per_bucket = self.world > 1 or self._local_overlap
         self._body_done = None   # event on the side stream: every non-tail bucket has been reduced
         # weight-gradient GEMMs on a stream of their own, beside the input-gradient chain (MCCL_SIDE_WGRAD=0: in line)
@@ -241,7 +241,7 @@ class DDPTrainer:
         self.buckets[self._param_bucket[p]].late = True
         self._on_grad_ready(p)
 
-    def _adamw(self, start: int, numel: int) -> None:
+    def _adamw(self, start: int, numel: int, ctas_per_sm: int = 8) -> None:
         end = start + numel
         ops.adamw_step(self.flat_p[start:end], self.flat_g[start:end], self.m[start:end], self.v[start:end], self.lr,
                        self.betas[0], self.betas[1], self.eps, self.wd, self.step_t,
@@ -252,13 +252,15 @@ class DDPTrainer:
         b.fired = self._step_id
         main = torch.cuda.current_stream(self.device)
         if self.comm is None and self.world == 1:
-            if self._local_overlap and self._in_backward and self.wgrad_stream is not None and not b.late:
+            if self._local_overlap and self._in_backward and not b.late and not b.tail:
                 # every kernel that reads this bucket's weights in backward is already queued on the main stream
-                self.wgrad_stream.wait_stream(main)
-                with torch.cuda.stream(self.wgrad_stream):
-                    self._adamw(b.start, b.numel)
-                _native.mark_wgrad_pending()
+                if self.wgrad_stream is not None:
+                    _native.join_wgrad(self.opt_stream)
+                self.opt_stream.wait_stream(main)
+                with torch.cuda.stream(self.opt_stream):
+                    self._adamw(b.start, b.numel, self._opt_ctas)
                 b.applied = self._step_id
+                self._opt_used = True
             return
         stream = self.comm_stream if (self.overlap and self.comm_stream is not None) else main
         if stream is not main:
@@ -299,6 +301,7 @@ class DDPTrainer:
             b.pending = 0
         self.step_t.add_(1.0)
         self._body_recorded = False
+        self._opt_used = False
         if not self._fused_zero:
             self.flat_g.zero_()   # otherwise the optimizer cleared what it consumed
         loss = self.model(tokens, targets)
@@ -341,8 +344,7 @@ class DDPTrainer:
             if self.comm_stream is not None and self.overlap:
                 main.wait_stream(self.comm_stream)
             if self._local_overlap:
-                # buckets updated during backward are done (the streams were joined after backward); the rest now,
-                # neighbouring ranges merged into one launch
+                # what backward did not update, neighbouring ranges merged into one launch
                 start = None
                 for b in self.buckets + [None]:
                     todo = b is not None and b.applied != self._step_id
@@ -352,6 +354,8 @@ class DDPTrainer:
                         end = b.start if b is not None else self.total
                         self._adamw(start, end - start)
                         start = None
+                if self._opt_used:
+                    main.wait_stream(self.opt_stream)
             else:
                 self._adamw(0, self.total)
         return loss.detach()
