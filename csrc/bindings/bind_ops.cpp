@@ -328,6 +328,14 @@ void bind_ops(py::module_& m) {
       py::arg("logits"), py::arg("targets"), py::arg("grad_scale") = 1.0,
       "Returns per-row losses; overwrites logits with (softmax - onehot) * grad_scale.");
 
+  m.def("mean_f32", [](const at::Tensor& x) {
+    need(x, at::kFloat, "mean");
+    c10::cuda::CUDAGuard guard(x.device());
+    at::Tensor out = at::empty({}, x.options());
+    check_launch(ops::mean_f32(x.data_ptr<float>(), out.data_ptr<float>(), x.numel(), stream_of(x)), "mean");
+    return out;
+  });
+
   // ---- causal self-attention (head dimension 64) on the fused QKV projection ----
   m.def(
       "attn_fwd",

@@ -55,6 +55,9 @@ cudaError_t adamw_flat(float* p, float* g, float* m, float* v, __nv_bfloat16* p1
 cudaError_t cross_entropy_fwd_bwd(__nv_bfloat16* logits, const long long* targets, float* loss_rows, int rows, int vocab,
                                   float grad_scale, cudaStream_t stream);
 
+// out = mean of n fp32 values, always added in the same order.
+cudaError_t mean_f32(const float* in, float* out, long long n, cudaStream_t stream);
+
 // ---- out[c, r] = in[r, c] for a bf16 matrix [rows, cols].
 cudaError_t transpose_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, int rows, int cols, cudaStream_t stream);
 // fp32 → bf16 cast of n elements.

@@ -469,7 +469,7 @@ class LinearCrossEntropyFn(torch.autograd.Function):
         loss_rows = _C.ce_fwd_bwd(logits, targets.contiguous(), 1.0 / T)
         ctx.save_for_backward(hc, w16, logits)   # logits now hold d(loss)/d(logits)
         ctx.weight = weight
-        return loss_rows.mean()
+        return _C.mean_f32(loss_rows)
 
     @staticmethod
     def backward(ctx, gout):

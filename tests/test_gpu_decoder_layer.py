@@ -117,3 +117,11 @@ def test_cast_many():
     ts = [torch.randn(n, device="cuda") for n in (1, 7, 8192, 8193, 100_001)] + [torch.randn(130, 70, device="cuda") for _ in range(150)]
     for t, c in zip(ts, _C.cast_many(ts)):
         assert torch.equal(c, t.bfloat16())
+
+
+@pytest.mark.parametrize("n", [1, 3, 192, 1027, 16384, 100_001])
+def test_mean(n):
+    from mccl_b200 import _C
+    x = torch.randn(n + 1, device="cuda") + 3
+    for t in (x[:n].clone(), x[1:]):   # the second does not start on 16 bytes
+        assert torch.allclose(_C.mean_f32(t), t.double().mean().float(), rtol=1e-6)
