@@ -104,7 +104,7 @@ class DDPTrainer:
         # decoder with 64 x 256 tokens 10492 -> 10423 us, the 70M and 110M decoders at 16 x 256 the same within noise.
         self._opt_ctas = int(os.environ.get("MCCL_OVERLAP_ADAMW_CTAS", "2"))
         self._local_overlap = (self.world == 1 and self._fused_zero and os.environ.get("MCCL_OVERLAP_ADAMW", "1") != "0")
-        self.opt_stream = torch.cuda.Stream(device=device) if self._local_overlap else None
+        self.opt_stream = None   # made on first use
         # Hooks are needed whenever something happens per bucket.
         self._per_bucket = self.world > 1 or self._local_overlap
         self._body_done = None   # event on the side stream: every non-tail bucket has been reduced
@@ -254,6 +254,8 @@ class DDPTrainer:
         if self.comm is None and self.world == 1:
             if self._local_overlap and self._in_backward and not b.late and not b.tail:
                 # every kernel that reads this bucket's weights in backward is already queued on the main stream
+                if self.opt_stream is None:
+                    self.opt_stream = torch.cuda.Stream(device=self.device)
                 if self.wgrad_stream is not None:
                     _native.join_wgrad(self.opt_stream)
                 self.opt_stream.wait_stream(main)
