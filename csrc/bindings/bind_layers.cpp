@@ -209,7 +209,7 @@ void bind_layers(py::module_& m) {
           need(*sin_t, at::kFloat, cos_t->numel(), "sin");
           MCCL_CHECK_TENSOR(cos_t->numel() >= static_cast<int64_t>(d.S) * hd / 2, "decoder_fwd: rotary tables too small");
           at::Tensor h = at::empty({T, D}, opt16), y = at::empty({T, D}, opt16), qkv = at::empty({d.B, d.S, 3, d.H, hd}, opt16);
-          at::Tensor qk = at::empty({d.B, d.S, 2, d.H, hd}, opt16), gu = at::empty({T, 2 * static_cast<int64_t>(F)}, opt16), act = at::empty({T, F}, opt16);
+          at::Tensor qk = at::empty({d.B, d.S, 2, d.H, hd}, opt16), gu, act = at::empty({T, F}, opt16);
           const at::Tensor q = qk.select(2, 0).transpose(1, 2), k = qk.select(2, 1).transpose(1, 2), v = qkv.select(2, 2).transpose(1, 2);
           for (int l = 0; l < L; ++l) {
             check(ops::norm_fwd(bf(x), f32(l, 0, D), nullptr, bf(h), nullptr, nullptr, T, D, eps, st), "first norm");
@@ -218,8 +218,13 @@ void bind_layers(py::module_& m) {
             const at::Tensor o = at::scaled_dot_product_attention(q, k, v, {}, 0.0, true).transpose(1, 2).contiguous();
             product(bf(o), w16[l * 4 + 1], nullptr, bf(y), T, D, D, bf(x), false, nullptr, st, "output projection");
             check(ops::norm_fwd(bf(y), f32(l, 3, D), nullptr, bf(h), nullptr, nullptr, T, D, eps, st), "second norm");
-            product(bf(h), w16[l * 4 + 2], nullptr, bf(gu), T, 2 * F, D, nullptr, false, nullptr, st, "gate and up projection");
-            check(ops::swiglu_fwd(bf(gu), bf(act), T, F, st), "activation");
+            const cudaError_t fused = gated(bf(h), w16[l * 4 + 2], bf(act), nullptr, T, F, D, st);
+            if (fused != cudaSuccess) {
+              if (fused != cudaErrorNotSupported) check(fused, "gate and up projection");
+              if (!gu.defined()) gu = at::empty({T, 2 * static_cast<int64_t>(F)}, opt16);
+              product(bf(h), w16[l * 4 + 2], nullptr, bf(gu), T, 2 * F, D, nullptr, false, nullptr, st, "gate and up projection");
+              check(ops::swiglu_fwd(bf(gu), bf(act), T, F, st), "activation");
+            }
             product(bf(act), w16[l * 4 + 3], nullptr, bf(x2), T, D, F, bf(y), false, nullptr, st, "down projection");
             std::swap(x, x2);
           }

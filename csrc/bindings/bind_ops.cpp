@@ -584,6 +584,33 @@ void bind_ops(py::module_& m) {
     check_launch(ops::swiglu_fwd(bf(gu), bf(h), h.numel() / f, static_cast<int>(f), stream_of(gu)), "swiglu_fwd");
     return h;
   });
+  // (silu(gate) * up, [gate | up]) of [gate | up] = x [T, K] · w [2 F, K]^T
+  m.def("gate_up_swiglu", [](const at::Tensor& x, const at::Tensor& w) {
+    need(x, at::kBFloat16, "gate_up_swiglu(x)");
+    need(w, at::kBFloat16, "gate_up_swiglu(w)");
+    MCCL_CHECK_TENSOR(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && w.size(0) % 16 == 0 && x.size(0) > 0, "gate_up_swiglu: x [T, K], w [2 F, K]");
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t T = x.size(0), K = x.size(1), F = w.size(0) / 2;
+    at::Tensor h = at::empty({T, F}, x.options()), gu = at::empty({T, 2 * F}, x.options());
+    ops::GemmArgs g;
+    g.a = bf(x);
+    g.b = bf(w);
+    g.d = h.data_ptr();
+    g.aux = bf(gu);
+    g.m = static_cast<int>(T);
+    g.n = g.ldd = static_cast<int>(F);
+    g.k = g.lda = g.ldb = static_cast<int>(K);
+    cudaError_t rc = ops::gemm_swiglu(g, stream_of(x));
+    if (rc == cudaErrorNotSupported) {
+      g.d = gu.data_ptr();
+      g.aux = nullptr;
+      g.n = g.ldd = static_cast<int>(2 * F);
+      check_launch(ops::gemm_bf16_tn(g, stream_of(x)), "gate_up_swiglu");
+      rc = ops::swiglu_fwd(bf(gu), bf(h), T, static_cast<int>(F), stream_of(x));
+    }
+    check_launch(rc, "gate_up_swiglu");
+    return std::make_pair(h, gu);
+  });
   m.def("swiglu_bwd", [](const at::Tensor& dh, const at::Tensor& gu) {
     need(dh, at::kBFloat16, "swiglu_bwd(dh)");
     need(gu, at::kBFloat16, "swiglu_bwd(gate_up)");

@@ -105,6 +105,18 @@ inline void product(const bf16* x, const bf16* w, const float* bias, bf16* y, in
   g.epilogue = gelu ? (aux ? ops::EPI_BIAS_GELU_D : ops::EPI_BIAS_GELU) : (bias ? ops::EPI_BIAS : ops::EPI_NONE);
   check(ops::gemm_bf16_tn(g, stream), what);
 }
+// h[M, N] = silu(gate) * up of [gate | up] = x[M, K] · w[2 N, K]^T, which goes to gu where given; not supported: product and swiglu_fwd
+inline cudaError_t gated(const bf16* x, const bf16* w, bf16* h, bf16* gu, int M, int N, int K, cudaStream_t stream) {
+  ops::GemmArgs g;
+  g.a = x;
+  g.b = w;
+  g.d = h;
+  g.aux = gu;
+  g.m = M;
+  g.n = g.ldd = N;
+  g.k = g.lda = g.ldb = K;
+  return ops::gemm_swiglu(g, stream);
+}
 // dx[M, K] = dy[M, N] · w[N, K] (times mul, with its column sums added to colsum)
 inline void input_gradient(const bf16* dy, const bf16* w, bf16* dx, int M, int N, int K, const bf16* mul, float* colsum, cudaStream_t stream,
                     const char* what) {

@@ -132,6 +132,9 @@ struct GemmArgs {
 // Returns cudaErrorNotSupported for shapes the kernel does not cover
 // (N % 8 != 0, unaligned pointers or row strides); the caller falls back.
 cudaError_t gemm_bf16_tn(const GemmArgs& args, cudaStream_t stream);
+// d[M, N] = silu(gate) * up of [gate | up] = A · B^T, B [2 N, K]; `aux` [M, 2 N] (may be null) takes [gate | up] itself.  N % 32 == 0.
+// cudaErrorNotSupported also where a product and swiglu_fwd are the better choice.
+cudaError_t gemm_swiglu(const GemmArgs& args, cudaStream_t stream);
 // Up to any number of weight gradients dW[N, K] = dY[tokens, N]^T · X[tokens, K] over the same tokens, worked through together
 // (sixteen products per launch).  A product is a GemmArgs with both operands MN-major, fp32 output, no epilogue; all of them
 // accumulate, or none.

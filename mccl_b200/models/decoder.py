@@ -245,12 +245,15 @@ class Block(nn.Module):
         x = self.proj(a, native, residual=x)
         h, x = self.ln2.with_residual(x, native)
         if cfg.act == "swiglu":
-            gu = self.gate_up(h, native)
             if native:
                 from .. import ops
-                h = ops.swiglu(gu)
+                lin = self.gate_up
+                if lin._forward_hooks or lin._forward_pre_hooks or lin._backward_hooks or lin._backward_pre_hooks:
+                    h = ops.swiglu(lin(h, native))   # somebody wants to see the projection's own call
+                else:
+                    h = ops.gate_up_swiglu(h, lin.weight)
             else:
-                g, u = gu.chunk(2, dim=-1)
+                g, u = self.gate_up(h, native).chunk(2, dim=-1)
                 h = F.silu(g) * u
         elif native:
             from .. import ops

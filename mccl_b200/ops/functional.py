@@ -99,6 +99,15 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     return F.silu(g) * u
 
 
+def gate_up_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """silu(gate) * up of [gate | up] = x @ W^T; on CUDA the activation is part of the product's kernel."""
+    if (x.is_cuda and x.dtype == torch.bfloat16 and _HAS["swiglu_fwd"] and _HAS["gemm_bf16"] and weight.shape[0] % 16 == 0 and weight.shape[1] % 64 == 0
+            and x.numel() > 0):
+        from .native import GateUpFn
+        return GateUpFn.apply(x, weight)
+    return swiglu(linear(x, weight))
+
+
 def mlp_gelu(x: torch.Tensor, w1: torch.Tensor, b1, w2: torch.Tensor, b2, residual=None) -> torch.Tensor:
     """gelu(x @ w1^T + b1) @ w2^T + b2 (+ residual).  On CUDA the whole block is one autograd node whose backward
     fuses the GELU derivative into the input-gradient GEMM of the second layer."""

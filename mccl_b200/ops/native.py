@@ -107,6 +107,31 @@ def _gemm_ok(m: int, n: int, k: int) -> bool:
     return k % 64 == 0 and n % 8 == 0 and m > 0
 
 
+def _linear_grads(dz, x2, w16, weight, need_dx: bool, need_dw: bool):
+    """Gradients of x2 [M, K] and of weight [N, K] (None where it goes into the weight's own buffer), from dz [M, N]."""
+    N, K = w16.shape
+    M = x2.shape[0]
+    dx = dw = None
+    if need_dx:
+        if _gemm_ok(M, K, N):
+            # dx[M,K] = dz[M,N] · W[N,K]: W is the B operand stored [contraction, K], read MN-major
+            dx, _ = _C.gemm_bf16(dz, w16, None, "none", False, None, False, False, True)
+        else:
+            dx = dz @ w16
+    if need_dw:
+        sink = _sink(weight)
+        if _gemm_ok(N, K, M) and N % 8 == 0:
+            # dW[N,K] = dz^T · x: both operands stored [tokens, features], read MN-major
+            if sink is not None:
+                _wgrad_gemm(dz, x2, sink)
+                _notify(weight)
+            else:
+                dw, _ = _C.gemm_bf16(dz, x2, None, "none", True, None, False, True, True)
+        else:
+            dw = (dz.t() @ x2).float()
+    return dx, dw
+
+
 class LinearFn(torch.autograd.Function):
     """y = act(x @ W^T + b); W [N, K] fp32 master, x [..., K] bf16."""
 
@@ -147,25 +172,10 @@ class LinearFn(torch.autograd.Function):
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         dz = _C.gelu_bwd(dy2, z) if ctx.act == "gelu" else dy2
-        dx = dw = db = None
-        if ctx.needs_input_grad[0]:
-            if _gemm_ok(M, K, N):
-                # dx[M,K] = dz[M,N] · W[N,K]: W is the B operand stored [contraction, K], read MN-major
-                dx, _ = _C.gemm_bf16(dz, w16, None, "none", False, None, False, False, True)
-            else:
-                dx = dz @ w16
+        db = None
+        dx, dw = _linear_grads(dz, x2, w16, weight, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        if dx is not None:
             dx = dx.view(*dy.shape[:-1], K)
-        if ctx.needs_input_grad[1]:
-            sink = _sink(weight)
-            if _gemm_ok(N, K, M) and N % 8 == 0:
-                # dW[N,K] = dz^T · x: both operands stored [tokens, features], read MN-major
-                if sink is not None:
-                    _wgrad_gemm(dz, x2, sink)
-                    _notify(weight)
-                else:
-                    dw, _ = _C.gemm_bf16(dz, x2, None, "none", True, None, False, True, True)
-            else:
-                dw = (dz.t() @ x2).float()
         if ctx.has_bias and ctx.needs_input_grad[2]:
             bsink = _sink(ctx.bias)
             if N % 8 == 0:
@@ -387,6 +397,29 @@ class SwigluFn(torch.autograd.Function):
     def backward(ctx, dh):
         (gu,) = ctx.saved_tensors
         return _C.swiglu_bwd(dh if dh.is_contiguous() else dh.contiguous(), gu)
+
+
+class GateUpFn(torch.autograd.Function):
+    """silu(gate) * up of [gate | up] = x @ W^T, W [2 F, K] fp32 master: the activation is the product's epilogue."""
+
+    @staticmethod
+    def forward(ctx, x, weight):
+        K, N = weight.shape[1], weight.shape[0]
+        x2 = x.reshape(-1, K)
+        if not x2.is_contiguous():
+            x2 = x2.contiguous()
+        w16 = _bf16_weight(weight)
+        h, gu = _C.gate_up_swiglu(x2, w16)
+        ctx.save_for_backward(x2, w16, gu)
+        ctx.weight = weight
+        return h.view(*x.shape[:-1], N // 2)
+
+    @staticmethod
+    def backward(ctx, dh):
+        x2, w16, gu = ctx.saved_tensors
+        dgu = _C.swiglu_bwd(dh.reshape(-1, dh.shape[-1]).contiguous(), gu)
+        dx, dw = _linear_grads(dgu, x2, w16, ctx.weight, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        return None if dx is None else dx.view(*dh.shape[:-1], x2.shape[1]), dw
 
 
 class NormFn(torch.autograd.Function):

@@ -47,3 +47,26 @@ def test_swiglu(rows, f):
     g, u = r.chunk(2, dim=-1)
     (F.silu(g) * u).backward(d.float())
     assert _rel(a.grad, r.grad) < 1e-2
+
+
+@pytest.mark.parametrize("rows,f,k,fused", [(4096, 4096, 1024, True), (2040, 4128, 1024, True), (1537, 8160, 2048, True), (37, 4096, 1024, False), (1, 24, 64, False)])
+def test_gate_up_swiglu(rows, f, k, fused):
+    from mccl_b200 import _C, ops
+    torch.manual_seed(rows)
+    x = torch.randn(rows, k, device="cuda").bfloat16().requires_grad_(True)
+    w = (torch.randn(2 * f, k, device="cuda") * k ** -0.5).requires_grad_(True)
+    separate = _C.launch_counts().get("swiglu_fwd_kernel", 0)
+    out = ops.gate_up_swiglu(x, w)
+    assert (_C.launch_counts().get("swiglu_fwd_kernel", 0) == separate) == fused
+    gu = _C.gate_up_swiglu(x.detach(), w.detach().bfloat16())[1]
+    z, _ = _C.gemm_bf16(x.detach(), w.detach().bfloat16())
+    assert _rel(gu, z) < 1e-2 and _rel(out, _C.swiglu_fwd(gu)) < 1e-2
+    assert (gu.float() - z.float()).norm() < 2e-3 * z.float().norm() and (out.float() - _C.swiglu_fwd(z).float()).norm() < 5e-3 * out.float().norm()
+    d = torch.randn_like(out)
+    out.backward(d)
+    xr, wr = x.detach().float().requires_grad_(True), w.detach().bfloat16().float().requires_grad_(True)
+    g, u = (xr @ wr.t()).chunk(2, dim=-1)
+    (F.silu(g) * u).backward(d.float())
+    for a, b in ((x.grad, xr.grad), (w.grad, wr.grad)):
+        assert ((a.float() - b).norm() / b.norm()).item() < 1e-2
+    assert _C.gemm_error_flag() == 0
