@@ -611,6 +611,39 @@ void bind_ops(py::module_& m) {
     check_launch(rc, "gate_up_swiglu");
     return std::make_pair(h, gu);
   });
+  // Gradient of [gate | up] from dy [T, D], w [D, F] of the product behind the activation, and [gate | up] itself.
+  m.def("down_swiglu_bwd", [](const at::Tensor& dy, const at::Tensor& w, const at::Tensor& gu) {
+    need(dy, at::kBFloat16, "down_swiglu_bwd(dy)");
+    need(w, at::kBFloat16, "down_swiglu_bwd(w)");
+    need(gu, at::kBFloat16, "down_swiglu_bwd(gate_up)");
+    MCCL_CHECK_TENSOR(dy.dim() == 2 && w.dim() == 2 && gu.dim() == 2 && dy.size(1) == w.size(0) && gu.size(1) == 2 * w.size(1) && gu.size(0) == dy.size(0) &&
+                          w.size(1) % 8 == 0 && dy.size(0) > 0,
+                      "down_swiglu_bwd: dy [T, D], w [D, F], gate_up [T, 2 F]");
+    c10::cuda::CUDAGuard guard(dy.device());
+    const int64_t T = dy.size(0), D = w.size(0), F = w.size(1);
+    at::Tensor dgu = at::empty_like(gu);
+    ops::GemmArgs g;
+    g.a = bf(dy);
+    g.b = bf(w);
+    g.b_mn_major = true;
+    g.d = dgu.data_ptr();
+    g.aux = bf(gu);
+    g.m = static_cast<int>(T);
+    g.n = g.ldb = static_cast<int>(F);
+    g.k = g.lda = static_cast<int>(D);
+    g.ldd = static_cast<int>(2 * F);
+    cudaError_t rc = ops::gemm_swiglu_grad(g, stream_of(dy));
+    if (rc == cudaErrorNotSupported) {
+      at::Tensor dh = at::empty({T, F}, gu.options());
+      g.d = dh.data_ptr();
+      g.aux = nullptr;
+      g.ldd = g.n;
+      check_launch(ops::gemm_bf16_tn(g, stream_of(dy)), "down_swiglu_bwd");
+      rc = ops::swiglu_bwd(bf(dh), bf(gu), bf(dgu), T, static_cast<int>(F), stream_of(dy));
+    }
+    check_launch(rc, "down_swiglu_bwd");
+    return dgu;
+  });
   m.def("swiglu_bwd", [](const at::Tensor& dh, const at::Tensor& gu) {
     need(dh, at::kBFloat16, "swiglu_bwd(dh)");
     need(gu, at::kBFloat16, "swiglu_bwd(gate_up)");

@@ -27,6 +27,8 @@ MCCL_TILES_EXTERN_PAIR(true, true, OUT_F32, 1)
 MCCL_TILES_EXTERN_PAIR(true, true, OUT_F32, kMaxGroup)
 extern template cudaError_t launch_tiles<256, true, false, false, OUT_SWIGLU, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 extern template int max_pairs<256, false, false, OUT_SWIGLU, 1>();
+extern template cudaError_t launch_tiles<256, true, false, true, OUT_SWIGLU_GRAD, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+extern template int max_pairs<256, false, true, OUT_SWIGLU_GRAD, 1>();
 #undef MCCL_TILES_EXTERN
 #undef MCCL_TILES_EXTERN_PAIR
 
@@ -150,26 +152,36 @@ bool gemm_wants_partial_sums(const GemmArgs& a) {
   return a.k >= 4096 && tiles::ceil_div(a.m, 256) * tiles::ceil_div(a.n, 256) * 10 <= gemm_sm_count() / 2 * 7;
 }
 
-// Only on the pair tile: where the product alone would take another, its 128 output columns per tile would leave SMs idle.
-cudaError_t gemm_swiglu(const GemmArgs& a, cudaStream_t stream) {
-  if (a.m <= 0 || a.n <= 0 || a.k <= 0 || a.d_fp32 || a.accumulate || a.bias || a.residual || a.mul || a.colsum || a.a_mn_major || a.b_mn_major ||
+namespace {
+// SwiGLU around a product of n (grad) or 2 n columns, on the pair tile only: where the product alone takes another one, tiles of
+// 256 rows would leave SMs idle.
+template <bool kBMn, int kOut>
+cudaError_t run_swiglu(const GemmArgs& a, cudaStream_t stream) {
+  if (a.m <= 0 || a.n <= 0 || a.k <= 0 || a.d_fp32 || a.accumulate || a.bias || a.residual || a.mul || a.colsum || a.a_mn_major || a.b_mn_major != kBMn ||
       a.epilogue != EPI_NONE)
     return cudaErrorInvalidValue;
   if (a.n % 32 != 0 || a.lda % 8 != 0 || a.ldb % 8 != 0 || a.ldd % 8 != 0 ||
       ((reinterpret_cast<uintptr_t>(a.a) | reinterpret_cast<uintptr_t>(a.b) | reinterpret_cast<uintptr_t>(a.d) | reinterpret_cast<uintptr_t>(a.aux)) & 15u))
     return cudaErrorNotSupported;
-  int sms = gemm_sm_count(), pairs = tiles::max_pairs<256, false, false, tiles::OUT_SWIGLU, 1>();
+  int sms = gemm_sm_count(), pairs = tiles::max_pairs<256, false, kBMn, kOut, 1>();
   const int limit = gemm_cta_limit();
   if (limit > 0) {
     sms = limit < sms ? limit : sms;
     pairs = limit / 2 < pairs ? limit / 2 : pairs;
   }
-  GemmArgs whole = a;
-  whole.n = 2 * a.n;
-  if (tiles::choose(&whole, 1, 0, sms, pairs, false, false).bn != 256) return cudaErrorNotSupported;
-  const int tiles = tiles::ceil_div(a.m, 256) * tiles::ceil_div(a.n, 128);
+  constexpr int kTileN = kOut == tiles::OUT_SWIGLU ? 128 : 256;
+  GemmArgs alone = a;
+  alone.n = a.n * (256 / kTileN);
+  if (tiles::choose(&alone, 1, 0, sms, pairs, false, false).bn != 256) return cudaErrorNotSupported;
+  const int tiles = tiles::ceil_div(a.m, 256) * tiles::ceil_div(a.n, kTileN);
   (void)cudaGetLastError();
-  return tiles::launch_tiles<256, true, false, false, tiles::OUT_SWIGLU, 1>(&a, 1, tiles < pairs ? tiles : pairs, 1, stream);
+  return tiles::launch_tiles<256, true, false, kBMn, kOut, 1>(&a, 1, tiles < pairs ? tiles : pairs, 1, stream);
+}
+}  // namespace
+
+cudaError_t gemm_swiglu(const GemmArgs& a, cudaStream_t stream) { return run_swiglu<false, tiles::OUT_SWIGLU>(a, stream); }
+cudaError_t gemm_swiglu_grad(const GemmArgs& a, cudaStream_t stream) {
+  return a.aux ? run_swiglu<true, tiles::OUT_SWIGLU_GRAD>(a, stream) : cudaErrorInvalidValue;
 }
 
 cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream) {

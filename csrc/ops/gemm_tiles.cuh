@@ -42,7 +42,11 @@ namespace tiles {
 // so that a tile's accumulator holds both factors of 128 outputs and silu(gate) * up is the epilogue.  The [m, 2 n] product
 // itself, which backward reads, is written too where `aux` is given.  As a kernel of its own the activation read it back:
 // 1537 x 16384 x 2048 (no aux) 86 + 17.6 us against 86, 4096 x 8192 x 1024 53 + 22 us against 54.
-enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3, OUT_SWIGLU = 4 };
+// OUT_SWIGLU_GRAD (pair tile only): the input gradient of the product behind the activation, turned into the gradient of
+// [gate | up] (D, [m, 2 n]) with the saved [gate | up] (`aux`) on its way out; the [m, n] tensor between the two is neither
+// written nor read.
+enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3, OUT_SWIGLU = 4, OUT_SWIGLU_GRAD = 5 };
+constexpr bool half_boxes(int out) { return out == OUT_GELU || out == OUT_SWIGLU || out == OUT_SWIGLU_GRAD; }   // 32-column output boxes
 
 // One product, or several with the same K whose tiles one launch works through (the weight gradients of one or more layers:
 // alone, a 512 x 2048 gradient is 64 tiles and leaves half the SMs without one).
@@ -425,6 +429,11 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
       const int col0 = it.n_blk * kTileN + part * kCols;
       const int row0 = it.m_blk * kTileM + static_cast<int>(rank) * BM + quarter * 32;
       const bool inside = row0 < m && col0 < n;   // uniform over the warp
+      auto load_gate_up = [&](int col) {
+        tc::mbar_expect_tx(xfull, 4096);
+        tc::tma_load_2d(stage, &P.x, xfull, col, row0);
+        tc::tma_load_2d(stage + 2048, &P.x, xfull, n + col, row0);
+      };
       // the staging buffers are free again; fetch what the epilogue will need while the MMAs of the tile still run
       if (tc::elect_one()) {
         bulk_wait_read<0>();
@@ -432,6 +441,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           tc::mbar_expect_tx(xfull, 4096);
           tc::tma_load_2d(stage, &P.x, xfull, col0, row0);
         }
+        if (kOut == OUT_SWIGLU_GRAD && inside) load_gate_up(col0);
       }
       // lane l keeps the bias of columns [col0 + 4 l, col0 + 4 l + 4); the loop below spreads it by shuffles
       float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -559,6 +569,57 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           }
           __syncwarp();
         }
+      } else if constexpr (kOut == OUT_SWIGLU_GRAD) {
+#pragma unroll 1
+        for (int c = 0; c < S::kCols; c += 32) {   // gate and up of 32 columns fill the staging buffer
+          const int col = col0 + c;
+          const bool here = row0 < m && col < n;
+          if (here) {
+            if (c > 0) {
+              if (tc::elect_one()) {
+                bulk_wait_read<0>();
+                load_gate_up(col);
+              }
+              __syncwarp();
+            }
+            ok = wait(xfull, xparity, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            xparity ^= 1u;
+            if (!ok) break;
+          }
+          uint32_t r[32];
+          tc::tmem_ld_32x32(taddr + static_cast<uint32_t>(c), r);
+          tc::tmem_ld_wait();
+          if (c + 32 >= S::kCols) last_read();
+          if (!here) continue;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float d[8], gate[8], up[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) d[q] = __uint_as_float(r[j * 8 + q]);
+            unpack8(pack8(d), d);   // rounded where a product of its own would round
+            unpack8(*stage_unit64(stage, lane, j), gate);
+            unpack8(*stage_unit64(stage + 2048, lane, j), up);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const float s = __fdividef(1.f, 1.f + __expf(-gate[q]));
+              const float dg = d[q] * up[q] * s * (1.f + gate[q] * (1.f - s));
+              up[q] = d[q] * gate[q] * s;
+              gate[q] = dg;
+            }
+            *stage_unit64(stage, lane, j) = pack8(gate);
+            *stage_unit64(stage + 2048, lane, j) = pack8(up);
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (tc::elect_one()) {
+            store_2d(map_d, stage, col, row0);
+            store_2d(map_d, stage + 2048, n + col, row0);
+            bulk_commit();
+          }
+          __syncwarp();
+        }
+        if (!ok) break;
       } else {
         if (has_extra && inside) {
           ok = wait(xfull, xparity, abort_flag);
@@ -701,7 +762,7 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
                      : kAMn ? encode_map(&P.a[p], a.a, a.k, a.m, a.lda, BK) : encode_map(&P.a[p], a.a, a.m, a.k, a.lda, BM);
     const bool okb = P.atoms[p] & 2 ? encode_groups(&P.b[p], a.b, a.k, a.n, a.ldb, S::kRowsB / 64)
                      : kBMn ? encode_map(&P.b[p], a.b, a.k, a.n, a.ldb, BK) : encode_map(&P.b[p], a.b, kOut == OUT_SWIGLU ? 2 * a.n : a.n, a.k, a.ldb, S::kRowsB);
-    if (!oka || !okb || !encode_out_map(&P.d[p], a.d, a.m, a.n, a.ldd, kOut == OUT_F32, kOut == OUT_GELU || kOut == OUT_SWIGLU)) return cudaErrorNotSupported;
+    if (!oka || !okb || !encode_out_map(&P.d[p], a.d, a.m, kOut == OUT_SWIGLU_GRAD ? 2 * a.n : a.n, a.ldd, kOut == OUT_F32, half_boxes(kOut))) return cudaErrorNotSupported;
     P.m[p] = a.m;
     P.n[p] = a.n;
     constexpr int kTileN = kOut == OUT_SWIGLU ? BN / 2 : BN;
@@ -714,9 +775,10 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
     }
   }
   const GemmArgs& a = args[0];
-  const void* x = kOut == OUT_GELU || kOut == OUT_SWIGLU ? a.aux : (kOut == OUT_F32 ? nullptr : (a.mul ? a.mul : a.residual));
+  const void* x = half_boxes(kOut) ? a.aux : (kOut == OUT_F32 ? nullptr : (a.mul ? a.mul : a.residual));
   if (x == nullptr) P.x = P.d[0];   // never used
-  else if (kOut == OUT_SWIGLU ? !encode_out_map(&P.x, x, a.m, 2 * a.n, 2 * a.n, false, true) : !encode_out_map(&P.x, x, a.m, a.n, a.ldd, false, kOut == OUT_GELU)) return cudaErrorNotSupported;
+  else if (kOut == OUT_SWIGLU || kOut == OUT_SWIGLU_GRAD ? !encode_out_map(&P.x, x, a.m, 2 * a.n, 2 * a.n, false, true)
+                                                         : !encode_out_map(&P.x, x, a.m, a.n, a.ldd, false, half_boxes(kOut))) return cudaErrorNotSupported;
   GemmDev g;
   g.d = a.d;
   g.aux = a.aux;

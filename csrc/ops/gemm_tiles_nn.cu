@@ -31,6 +31,9 @@ template cudaError_t launch_tiles<192, false, true, false, OUT_F32, 1>(const Gem
 template cudaError_t launch_tiles<256, true, true, false, OUT_F32, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template int max_pairs<256, true, false, OUT_F32, 1>();
 
+template cudaError_t launch_tiles<256, true, false, true, OUT_SWIGLU_GRAD, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+template int max_pairs<256, false, true, OUT_SWIGLU_GRAD, 1>();
+
 }  // namespace tiles
 }  // namespace ops
 }  // namespace mccl

@@ -135,6 +135,8 @@ cudaError_t gemm_bf16_tn(const GemmArgs& args, cudaStream_t stream);
 // d[M, N] = silu(gate) * up of [gate | up] = A · B^T, B [2 N, K]; `aux` [M, 2 N] (may be null) takes [gate | up] itself.  N % 32 == 0.
 // cudaErrorNotSupported also where a product and swiglu_fwd are the better choice.
 cudaError_t gemm_swiglu(const GemmArgs& args, cudaStream_t stream);
+// d[M, 2 N] = gradient of [gate | up] (`aux`, [M, 2 N]) for dh = A · B, B [K, N] (b_mn_major, rows ldb): swiglu_bwd on a product's way out.
+cudaError_t gemm_swiglu_grad(const GemmArgs& args, cudaStream_t stream);
 // Up to any number of weight gradients dW[N, K] = dY[tokens, N]^T · X[tokens, K] over the same tokens, worked through together
 // (sixteen products per launch).  A product is a GemmArgs with both operands MN-major, fp32 output, no epilogue; all of them
 // accumulate, or none.

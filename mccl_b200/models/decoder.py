@@ -247,11 +247,9 @@ class Block(nn.Module):
         if cfg.act == "swiglu":
             if native:
                 from .. import ops
-                lin = self.gate_up
-                if lin._forward_hooks or lin._forward_pre_hooks or lin._backward_hooks or lin._backward_pre_hooks:
-                    h = ops.swiglu(lin(h, native))   # somebody wants to see the projection's own call
-                else:
-                    h = ops.gate_up_swiglu(h, lin.weight)
+                if not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (self.gate_up, self.down)):
+                    return ops.mlp_swiglu(h, self.gate_up.weight, self.down.weight, residual=x)
+                h = ops.swiglu(self.gate_up(h, native))   # somebody wants to see the projections' own calls
             else:
                 g, u = self.gate_up(h, native).chunk(2, dim=-1)
                 h = F.silu(g) * u

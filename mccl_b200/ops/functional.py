@@ -99,13 +99,14 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     return F.silu(g) * u
 
 
-def gate_up_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """silu(gate) * up of [gate | up] = x @ W^T; on CUDA the activation is part of the product's kernel."""
-    if (x.is_cuda and x.dtype == torch.bfloat16 and _HAS["swiglu_fwd"] and _HAS["gemm_bf16"] and weight.shape[0] % 16 == 0 and weight.shape[1] % 64 == 0
-            and x.numel() > 0):
-        from .native import GateUpFn
-        return GateUpFn.apply(x, weight)
-    return swiglu(linear(x, weight))
+def mlp_swiglu(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, residual=None) -> torch.Tensor:
+    """(silu(gate) * up) @ w2^T (+ residual) with [gate | up] = x @ w1^T.  On CUDA one autograd node whose products carry the
+    activation and its backward in their epilogues."""
+    if (x.is_cuda and x.dtype == torch.bfloat16 and _HAS["swiglu_fwd"] and _HAS["gemm_bf16"] and w1.shape[1] % 64 == 0 and w2.shape[1] % 64 == 0
+            and w2.shape[0] % 64 == 0 and x.numel() > 0 and os.environ.get("MCCL_FUSE_MLP", "1") != "0"):
+        from .native import MlpSwigluFn
+        return MlpSwigluFn.apply(x, w1, w2, residual)
+    return linear(swiglu(linear(x, w1)), w2, residual=residual)
 
 
 def mlp_gelu(x: torch.Tensor, w1: torch.Tensor, b1, w2: torch.Tensor, b2, residual=None) -> torch.Tensor:

@@ -399,27 +399,42 @@ class SwigluFn(torch.autograd.Function):
         return _C.swiglu_bwd(dh if dh.is_contiguous() else dh.contiguous(), gu)
 
 
-class GateUpFn(torch.autograd.Function):
-    """silu(gate) * up of [gate | up] = x @ W^T, W [2 F, K] fp32 master: the activation is the product's epilogue."""
+class MlpSwigluFn(torch.autograd.Function):
+    """y = (silu(gate) * up) @ W2^T (+ residual), [gate | up] = x @ W1^T, as one autograd node: the activation is the first
+    product's epilogue, its backward that of the second product's input gradient."""
 
     @staticmethod
-    def forward(ctx, x, weight):
-        K, N = weight.shape[1], weight.shape[0]
-        x2 = x.reshape(-1, K)
+    def forward(ctx, x, w1, w2, residual=None):
+        x2 = x.reshape(-1, w1.shape[1])
         if not x2.is_contiguous():
             x2 = x2.contiguous()
-        w16 = _bf16_weight(weight)
-        h, gu = _C.gate_up_swiglu(x2, w16)
-        ctx.save_for_backward(x2, w16, gu)
-        ctx.weight = weight
-        return h.view(*x.shape[:-1], N // 2)
+        w1_16, w2_16 = _bf16_weight(w1), _bf16_weight(w2)
+        h, gu = _C.gate_up_swiglu(x2, w1_16)
+        res2 = None
+        if residual is not None:
+            res2 = residual.reshape(-1, w2.shape[0])
+            if not res2.is_contiguous():
+                res2 = res2.contiguous()
+        y, _ = _C.gemm_bf16(h, w2_16, None, "none", False, None, False, False, False, res2)
+        ctx.save_for_backward(x2, w1_16, w2_16, gu, h)
+        ctx.params = (w1, w2)
+        ctx.has_residual = residual is not None
+        return y.view(*x.shape[:-1], w2.shape[0])
 
     @staticmethod
-    def backward(ctx, dh):
-        x2, w16, gu = ctx.saved_tensors
-        dgu = _C.swiglu_bwd(dh.reshape(-1, dh.shape[-1]).contiguous(), gu)
-        dx, dw = _linear_grads(dgu, x2, w16, ctx.weight, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
-        return None if dx is None else dx.view(*dh.shape[:-1], x2.shape[1]), dw
+    def backward(ctx, dy):
+        x2, w1_16, w2_16, gu, h = ctx.saved_tensors
+        w1, w2 = ctx.params
+        dy2 = dy.reshape(-1, w2_16.shape[0])
+        if not dy2.is_contiguous():
+            dy2 = dy2.contiguous()
+        dgu = _C.down_swiglu_bwd(dy2, w2_16, gu)
+        # each weight's gradient once nothing reads the weight any more (see MlpGeluFn)
+        _, dw2 = _linear_grads(dy2, h, w2_16, w2, False, ctx.needs_input_grad[2])
+        dx, dw1 = _linear_grads(dgu, x2, w1_16, w1, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        if dx is not None:
+            dx = dx.view(*dy.shape[:-1], x2.shape[1])
+        return dx, dw1, dw2, (dy if ctx.has_residual else None)
 
 
 class NormFn(torch.autograd.Function):

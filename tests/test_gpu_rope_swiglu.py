@@ -49,24 +49,30 @@ def test_swiglu(rows, f):
     assert _rel(a.grad, r.grad) < 1e-2
 
 
-@pytest.mark.parametrize("rows,f,k,fused", [(4096, 4096, 1024, True), (2040, 4128, 1024, True), (1537, 8160, 2048, True), (37, 4096, 1024, False), (1, 24, 64, False)])
-def test_gate_up_swiglu(rows, f, k, fused):
+@pytest.mark.parametrize("rows,f,k,fused", [(4096, 4096, 1024, (1, 1)), (2040, 4128, 1024, (1, 1)), (1537, 8160, 2048, (1, 1)), (37, 4096, 1024, (0, 0)), (1, 64, 64, (0, 0))])
+def test_mlp_swiglu(rows, f, k, fused):
     from mccl_b200 import _C, ops
     torch.manual_seed(rows)
-    x = torch.randn(rows, k, device="cuda").bfloat16().requires_grad_(True)
-    w = (torch.randn(2 * f, k, device="cuda") * k ** -0.5).requires_grad_(True)
-    separate = _C.launch_counts().get("swiglu_fwd_kernel", 0)
-    out = ops.gate_up_swiglu(x, w)
-    assert (_C.launch_counts().get("swiglu_fwd_kernel", 0) == separate) == fused
-    gu = _C.gate_up_swiglu(x.detach(), w.detach().bfloat16())[1]
-    z, _ = _C.gemm_bf16(x.detach(), w.detach().bfloat16())
-    assert _rel(gu, z) < 1e-2 and _rel(out, _C.swiglu_fwd(gu)) < 1e-2
-    assert (gu.float() - z.float()).norm() < 2e-3 * z.float().norm() and (out.float() - _C.swiglu_fwd(z).float()).norm() < 5e-3 * out.float().norm()
-    d = torch.randn_like(out)
-    out.backward(d)
-    xr, wr = x.detach().float().requires_grad_(True), w.detach().bfloat16().float().requires_grad_(True)
-    g, u = (xr @ wr.t()).chunk(2, dim=-1)
-    (F.silu(g) * u).backward(d.float())
-    for a, b in ((x.grad, xr.grad), (w.grad, wr.grad)):
-        assert ((a.float() - b).norm() / b.norm()).item() < 1e-2
+    x, r = (torch.randn(rows, k, device="cuda").bfloat16().requires_grad_(True) for _ in range(2))
+    w1, w2 = ((torch.randn(*s, device="cuda") * s[1] ** -0.5).requires_grad_(True) for s in ((2 * f, k), (k, f)))
+    x16, w16, v16 = x.detach(), w1.detach().bfloat16(), w2.detach().bfloat16()
+
+    def separate(name, call):
+        before = _C.launch_counts().get(name, 0)
+        return call(), _C.launch_counts().get(name, 0) - before
+    (h, gu), one = separate("swiglu_fwd_kernel", lambda: _C.gate_up_swiglu(x16, w16))
+    z, _ = _C.gemm_bf16(x16, w16)
+    d = torch.randn_like(x16)
+    dgu, two = separate("swiglu_bwd_kernel", lambda: _C.down_swiglu_bwd(d, v16, gu))
+    dh, _ = _C.gemm_bf16(d, v16, None, "none", False, None, False, False, True)
+    for a, b in ((gu, z), (h, _C.swiglu_fwd(gu)), (dgu, _C.swiglu_bwd(dh, gu))):
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 3e-3
+    if f % 64 == 0:
+        assert (1 - one, 1 - two) == fused
+    ops.mlp_swiglu(x, w1, w2, residual=r).backward(d)
+    xr, ar, br = (t.detach().bfloat16().float().requires_grad_(True) for t in (x, w1, w2))
+    g, u = (xr @ ar.t()).chunk(2, dim=-1)
+    ((F.silu(g) * u) @ br.t()).backward(d.float())
+    for a, b in ((x.grad, xr.grad), (w1.grad, ar.grad), (w2.grad, br.grad), (r.grad, d)):
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 1e-2
     assert _C.gemm_error_flag() == 0
