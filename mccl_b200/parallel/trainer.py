@@ -103,7 +103,10 @@ class DDPTrainer:
         # with two CTAs per SM it takes little of what they use.  Measured: SwiGLU decoder 2948 -> 2812 us per step, 70M
         # decoder with 64 x 256 tokens 10492 -> 10423 us, the 70M and 110M decoders at 16 x 256 the same within noise.
         self._opt_ctas = int(os.environ.get("MCCL_OVERLAP_ADAMW_CTAS", "2"))
-        self._local_overlap = (self.world == 1 and self._fused_zero and os.environ.get("MCCL_OVERLAP_ADAMW", "1") != "0")
+        # Only in a captured step, and only if the first warm-up step shows that every gradient is written by a native operator,
+        # which reports it: what autograd accumulates arrives after such a report, if the same parameter has one.
+        self._local_overlap = (self.world == 1 and self._fused_zero and use_graph and os.environ.get("MCCL_OVERLAP_ADAMW", "1") != "0")
+        self._all_native = False
         self.opt_stream = None   # made on first use
         # Hooks are needed whenever something happens per bucket.
         self._per_bucket = self.world > 1 or self._local_overlap
@@ -203,7 +206,8 @@ class DDPTrainer:
             if self._per_bucket:
                 # ... and say so; gradients that come back through autograd fire its hook instead
                 p._grad_ready = (lambda q=p: self._on_grad_ready(q))
-                p.register_post_accumulate_grad_hook(self._on_autograd_grad)
+                if self.world > 1:
+                    p.register_post_accumulate_grad_hook(self._on_autograd_grad)
         # bf16 working copies of the parameters, refreshed by the optimizer kernel (the GEMMs
         # read them in either orientation, so no transposed copies are kept).
         self.flat_p16 = None
@@ -252,7 +256,7 @@ class DDPTrainer:
         b.fired = self._step_id
         main = torch.cuda.current_stream(self.device)
         if self.comm is None and self.world == 1:
-            if self._local_overlap and self._in_backward and not b.late and not b.tail:
+            if self._local_overlap and self._all_native and self._in_backward and not b.tail:
                 # every kernel that reads this bucket's weights in backward is already queued on the main stream
                 if self.opt_stream is None:
                     self.opt_stream = torch.cuda.Stream(device=self.device)
@@ -307,6 +311,7 @@ class DDPTrainer:
         if not self._fused_zero:
             self.flat_g.zero_()   # otherwise the optimizer cleared what it consumed
         loss = self.model(tokens, targets)
+        version = self.flat_g._version   # shared by every gradient, and moved by whatever PyTorch itself adds into one
         free_sms = self.comm_sms if self.comm_sms > 0 else self._bwd_free_sms
         main_ctas = max(_C.gemm_sm_count() - free_sms, 2) if free_sms > 0 else 0
         if self._bwd_main_ctas > 0:
@@ -324,6 +329,8 @@ class DDPTrainer:
             self._in_backward = False
             if main_ctas > 0 or self._bwd_side_ctas > 0:
                 _C.set_gemm_cta_limit(0)
+        if self._local_overlap and not self._all_native:
+            self._all_native = self._local_overlap = self.flat_g._version == version
         for b in self._late:
             self._reduce_bucket(b)
         self._late.clear()

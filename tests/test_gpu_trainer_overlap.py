@@ -1,0 +1,40 @@
+"""Optimizer updates during backward on one GPU against one update at the end."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+class _Mixed(torch.nn.Module):
+    """A decoder whose layer weight is also used by a plain PyTorch operator: that share arrives after the native one's report."""
+
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def forward(self, tokens, targets):
+        return self.inner(tokens, targets) + self.inner.blocks[1].up.weight.square().mean()
+
+
+@pytest.mark.parametrize("name,changes,mixed", [("tiny", {"n_layers": 6}, False), ("tiny", {"n_layers": 6}, True),
+                                                ("1.3b", {"vocab": 512, "d_model": 256, "n_layers": 3, "n_heads": 4, "d_ff": 512, "max_seq": 256}, False)])
+def test_updates_during_backward(monkeypatch, name, changes, mixed):
+    from mccl_b200.models import build_decoder
+    from mccl_b200.parallel import DDPTrainer
+    dev = torch.device("cuda", 0)
+    got = []
+    for overlap in ("0", "1"):
+        monkeypatch.setenv("MCCL_OVERLAP_ADAMW", overlap)
+        torch.manual_seed(0)
+        with dev:
+            model = build_decoder(name, **changes)
+        trainer = DDPTrainer(_Mixed(model) if mixed else model, dev, lr=1e-3, bucket_mb=0.25, last_bucket_mb=0.05)
+        ids = torch.randint(0, model.cfg.vocab, (4, 65), device=dev, generator=torch.Generator(dev).manual_seed(1))
+        for _ in range(4):
+            loss = trainer.step(ids[:, :-1].contiguous(), ids[:, 1:].contiguous())
+        torch.cuda.synchronize()
+        if overlap == "1":
+            assert trainer._local_overlap == (not mixed) and (trainer.opt_stream is not None) == (not mixed)
+        got.append((float(loss), trainer.flat_p.clone(), trainer.m.clone()))
+    (l0, p0, m0), (l1, p1, m1) = got
+    assert abs(l0 - l1) < 2e-2 and (p0 - p1).norm() < 1e-3 * p0.norm() and (m0 - m1).norm() < 3e-2 * m0.norm()
