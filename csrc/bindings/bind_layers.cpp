@@ -189,6 +189,16 @@ void bind_layers(py::module_& m) {
         check(ops::embed_fwd(reinterpret_cast<const long long*>(ids.data_ptr<int64_t>()), tok.data_ptr<float>(), pos.has_value() ? pos->data_ptr<float>() : nullptr,
                              bf(x), T, d.S, D, static_cast<int>(tok.size(0)), st),
               "embedding");
+        // few tokens: the down projections as sums, all layers' zeroed at once, which the norm behind each finishes
+        const bool as_sums = L > 0 && down_as_sums(d);
+        const int64_t TD = static_cast<int64_t>(T) * D;
+        at::Tensor sums;
+        if (as_sums) {
+          sums = at::empty({L, TD}, opt16.dtype(at::kFloat));
+          check(cudaMemsetAsync(sums.data_ptr(), 0, static_cast<size_t>(L * TD) * 4, st), "sums");
+        }
+        Unfinished before = {nullptr, nullptr, nullptr};
+        at::Tensor kept;   // what `before` points into
         auto f32 = [&](int l, int p, int64_t n) {
           const at::Tensor& t = layers[l * per + p];
           need(t, at::kFloat, n, "parameter");
@@ -198,11 +208,14 @@ void bind_layers(py::module_& m) {
           Slab s;
           at::Tensor slab = at::empty({Slab::place(&s, nullptr, d)}, opt16.dtype(at::kByte));
           Slab::place(&s, slab.data_ptr<uint8_t>(), d);
+          kept = slab;
           for (int l = 0; l < L; ++l) {
             const Weights w = {f32(l, LN1_W, D), f32(l, LN1_B, D), f32(l, QKV_B, 3 * D), f32(l, PROJ_B, D), f32(l, LN2_W, D), f32(l, LN2_B, D),
                                f32(l, UP_B, F), f32(l, DOWN_B, D), w16[l * 4], w16[l * 4 + 1], w16[l * 4 + 2], w16[l * 4 + 3]};
-            layer_forward(bf(x), bf(x2), w, s, d, eps, false, st);
-            std::swap(x, x2);
+            float* to = as_sums ? sums.data_ptr<float>() + l * TD : nullptr;
+            layer_forward(bf(x), bf(x2), w, s, d, eps, false, st, to, as_sums && l > 0 ? &before : nullptr);
+            before = {to, w.down_b, s.y};
+            if (!as_sums) std::swap(x, x2);
           }
         } else {
           need(*cos_t, at::kFloat, cos_t->numel(), "cos");
@@ -210,9 +223,11 @@ void bind_layers(py::module_& m) {
           MCCL_CHECK_TENSOR(cos_t->numel() >= static_cast<int64_t>(d.S) * hd / 2, "decoder_fwd: rotary tables too small");
           at::Tensor h = at::empty({T, D}, opt16), y = at::empty({T, D}, opt16), qkv = at::empty({d.B, d.S, 3, d.H, hd}, opt16);
           at::Tensor qk = at::empty({d.B, d.S, 2, d.H, hd}, opt16), gu, act = at::empty({T, F}, opt16);
+          kept = y;
           const at::Tensor q = qk.select(2, 0).transpose(1, 2), k = qk.select(2, 1).transpose(1, 2), v = qkv.select(2, 2).transpose(1, 2);
           for (int l = 0; l < L; ++l) {
-            check(ops::norm_fwd(bf(x), f32(l, 0, D), nullptr, bf(h), nullptr, nullptr, T, D, eps, st), "first norm");
+            if (as_sums && l > 0) check(ops::norm_sum_fwd(before.sums, nullptr, before.residual, bf(x), f32(l, 0, D), nullptr, bf(h), T, D, eps, st), "first norm");
+            else check(ops::norm_fwd(bf(x), f32(l, 0, D), nullptr, bf(h), nullptr, nullptr, T, D, eps, st), "first norm");
             product(bf(h), w16[l * 4], nullptr, bf(qkv), T, 3 * D, D, nullptr, false, nullptr, st, "qkv projection");
             check(ops::rope_qk_fwd(bf(qkv), cos_t->data_ptr<float>(), sin_t->data_ptr<float>(), bf(qk), T, d.S, d.H, hd, st), "rotary embedding");
             const at::Tensor o = at::scaled_dot_product_attention(q, k, v, {}, 0.0, true).transpose(1, 2).contiguous();
@@ -225,12 +240,18 @@ void bind_layers(py::module_& m) {
               product(bf(h), w16[l * 4 + 2], nullptr, bf(gu), T, 2 * F, D, nullptr, false, nullptr, st, "gate and up projection");
               check(ops::swiglu_fwd(bf(gu), bf(act), T, F, st), "activation");
             }
-            product(bf(act), w16[l * 4 + 3], nullptr, bf(x2), T, D, F, bf(y), false, nullptr, st, "down projection");
-            std::swap(x, x2);
+            if (as_sums) {
+              before = {sums.data_ptr<float>() + l * TD, nullptr, bf(y)};
+              product_sums(bf(act), w16[l * 4 + 3], sums.data_ptr<float>() + l * TD, T, D, F, st, "down projection");
+            } else {
+              product(bf(act), w16[l * 4 + 3], nullptr, bf(x2), T, D, F, bf(y), false, nullptr, st, "down projection");
+              std::swap(x, x2);
+            }
           }
         }
-        check(ops::norm_fwd(bf(x), lnf_w.data_ptr<float>(), lnf_b.has_value() ? lnf_b->data_ptr<float>() : nullptr, bf(x2), nullptr, nullptr, T, D, eps, st),
-              "final norm");
+        const float* final_b = lnf_b.has_value() ? lnf_b->data_ptr<float>() : nullptr;
+        if (as_sums) check(ops::norm_sum_fwd(before.sums, before.bias, before.residual, bf(x), lnf_w.data_ptr<float>(), final_b, bf(x2), T, D, eps, st), "final norm");
+        else check(ops::norm_fwd(bf(x), lnf_w.data_ptr<float>(), final_b, bf(x2), nullptr, nullptr, T, D, eps, st), "final norm");
         at::Tensor logits = at::empty({d.B, d.S, V}, opt16);
         product(bf(x2), w16[L * 4], nullptr, bf(logits), T, V, D, nullptr, false, nullptr, st, "head");
         return logits;

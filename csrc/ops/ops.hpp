@@ -25,6 +25,9 @@ void count_launch(int n = 1);
 // x, y: [rows, dim] bf16; w, b: fp32; mean / rstd: fp32 [rows] saved for backward (both may be null).
 cudaError_t norm_fwd(const __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y, float* mean, float* rstd,
                      int rows, int dim, float eps, cudaStream_t stream);
+// x = bf16(sum + bias + residual) and y = norm(x), for a product left as fp32 sums [rows, dim]; bias may be null; dim up to 2048.
+cudaError_t norm_sum_fwd(const float* sum, const float* bias, const __nv_bfloat16* residual, __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y,
+                         int rows, int dim, float eps, cudaStream_t stream);
 // dx: [rows, dim] bf16; dw, db: fp32 [dim].  With scratch (fp32, 2 * colsum_slabs(rows) * dim
 // elements) dw / db are overwritten by a two-stage, order-fixed reduction; with scratch == nullptr
 // the slab sums are added to dw / db atomically in one pass.  dx_add (optional, [rows, dim] bf16) is a

@@ -125,3 +125,22 @@ def test_mean(n):
     x = torch.randn(n + 1, device="cuda") + 3
     for t in (x[:n].clone(), x[1:]):   # the second does not start on 16 bytes
         assert torch.allclose(_C.mean_f32(t), t.double().mean().float(), rtol=1e-6)
+
+
+@pytest.mark.parametrize("name,changes,B,S,sums", [("70m", {"n_layers": 1, "vocab": 1000}, 1, 1, True), ("70m", {"n_layers": 3, "vocab": 1000}, 1, 37, True),
+                                                   ("110m", {"n_layers": 2, "vocab": 1000}, 4, 32, True), ("110m", {"n_layers": 2, "vocab": 1000}, 1, 129, False),
+                                                   ("1.3b", {**SWIGLU, "d_ff": 1088}, 1, 100, True), ("1.3b", {**SWIGLU, "d_model": 2048, "n_heads": 16, "d_ff": 2112}, 2, 3, True)])
+def test_few_tokens(name, changes, B, S, sums):
+    """The down projections of a short forward are fp32 sums that the next norm finishes."""
+    from mccl_b200 import _C
+    a, b = _pair(name, **changes)
+    tok = torch.randint(0, a.cfg.vocab, (B, S), device="cuda")
+
+    def count():
+        return sum(n for k, n in _C.launch_counts().items() if "norm_sum_kernel" in k)
+    before = count()
+    with torch.no_grad():
+        got, want = a(tok), b(tok)
+    assert count() - before == (a.cfg.n_layers if sums else 0)
+    assert _rel(got, want) < 2e-2
+    assert _C.gemm_error_flag() == 0
