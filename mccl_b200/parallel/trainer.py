@@ -79,10 +79,9 @@ class DDPTrainer:
         self.comm_sms = comm_sms if (self.world > 1 and overlap) else 0
         # SMs every backward GEMM leaves free when no collectives need them (one GPU): room for the weight-gradient stream
         self._bwd_free_sms = int(os.environ.get("MCCL_BWD_FREE_SMS", "0")) if device.type == "cuda" else 0
-        # CTA caps of the backward GEMMs on the main stream and of the weight-gradient GEMMs on the side stream.  Two
-        # GEMMs that each want every SM take turns, set-up and tail included; capped at 88 of 148 CTAs each they mostly
-        # run side by side (a second round of tiles costs a CTA about a third more, not twice).  Measured on the 70M
-        # decoder: 4.72 -> 4.49 ms per step on one GPU, 4.97 -> 4.68 on two (with 40 SMs kept for the collectives).
+        # With MCCL_SIDE_WGRAD=1 only: CTA caps of the backward GEMMs on the main stream and of the weight-gradient GEMMs on
+        # the side stream.  Two GEMMs that each want every SM take turns, set-up and tail included; capped at 88 of 148 CTAs
+        # each they mostly run side by side.  Off by default: four layers' weight gradients in one launch leave no SMs idle.
         side_on = device.type == "cuda" and os.environ.get("MCCL_SIDE_WGRAD", "0") != "0"
         self._bwd_main_ctas = int(os.environ.get("MCCL_BWD_MAIN_CTAS", "88" if side_on else "0")) if device.type == "cuda" else 0
         self._bwd_side_ctas = int(os.environ.get("MCCL_BWD_SIDE_CTAS", "88" if side_on else "0")) if device.type == "cuda" else 0
