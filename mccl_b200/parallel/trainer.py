@@ -27,7 +27,9 @@ B200-first form of the same job:
 """
 from __future__ import annotations
 
+import gc
 import os
+import weakref
 from typing import List, Optional
 
 import torch
@@ -191,6 +193,18 @@ class DDPTrainer:
             self.flat_g = torch.zeros(total, device=self.device, dtype=torch.float32)
         self.flat_g.zero_()
         self._param_bucket = {}
+        # the parameters outlive their trainer, or die with it: no reference back, which would leave both (and their CUDA graph)
+        # to the garbage collector
+        me = weakref.ref(self)
+
+        def report(q):
+            q = weakref.ref(q)
+
+            def ready():
+                trainer, param = me(), q()
+                if trainer is not None and param is not None:
+                    trainer._on_grad_ready(param)
+            return ready
         bi = 0
         for p, off in zip(order, offsets):
             while off >= self.buckets[bi].start + self.buckets[bi].numel:
@@ -204,7 +218,7 @@ class DDPTrainer:
             p._grad_sink = p.grad
             if self._per_bucket:
                 # ... and say so; gradients that come back through autograd fire its hook instead
-                p._grad_ready = (lambda q=p: self._on_grad_ready(q))
+                p._grad_ready = report(p)
                 if self.world > 1:
                     p.register_post_accumulate_grad_hook(self._on_autograd_grad)
         # bf16 working copies of the parameters, refreshed by the optimizer kernel (the GEMMs
@@ -375,8 +389,14 @@ class DDPTrainer:
         # the step is captured on a high-priority stream: its kernels are placed before those of the weight-gradient
         # stream (default priority), which then only fills what the main chain leaves free
         capture_stream = torch.cuda.Stream(device=self.device, priority=-1)
-        with torch.cuda.graph(graph, stream=capture_stream):
-            self.static_loss = self._step_body(self.static_tokens, self.static_targets)
+        collecting = gc.isenabled()
+        gc.disable()   # a CUDA graph or an allocation that the collector destroys meanwhile would invalidate the capture
+        try:
+            with torch.cuda.graph(graph, stream=capture_stream):
+                self.static_loss = self._step_body(self.static_tokens, self.static_targets)
+        finally:
+            if collecting:
+                gc.enable()
         return graph
 
     def _capture(self, tokens: torch.Tensor, targets: torch.Tensor) -> None:

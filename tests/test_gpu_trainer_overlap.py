@@ -38,3 +38,53 @@ def test_updates_during_backward(monkeypatch, name, changes, mixed):
         got.append((float(loss), trainer.flat_p.clone(), trainer.m.clone()))
     (l0, p0, m0), (l1, p1, m1) = got
     assert abs(l0 - l1) < 2e-2 and (p0 - p1).norm() < 1e-3 * p0.norm() and (m0 - m1).norm() < 3e-2 * m0.norm()
+
+
+@pytest.mark.parametrize("sizes,tokens", [([(1024, 1024), (3072, 1024), (1024, 1024)], 512), ([(256, 64), (64, 256), (128, 128), (8, 64), (512, 512)], 192), ([(64, 8192), (8192, 8192)], 128)])
+def test_weight_gradients_that_share_a_launch(sizes, tokens):
+    """Linear layers with gradient buffers, in turn, against each layer's own product."""
+    from mccl_b200 import ops
+    torch.manual_seed(tokens)
+    got, want, ready = [], [], []
+    total = 0
+    for i, (n, k) in enumerate(sizes):
+        x = torch.randn(tokens, k, device="cuda").bfloat16()
+        w = torch.nn.Parameter(torch.randn(n, k, device="cuda") * 0.02)
+        w._grad_sink = torch.ones(n, k, device="cuda")
+        w._grad_ready = lambda i=i: ready.append(i)
+        d = torch.randn(tokens, n, device="cuda").bfloat16()
+        total = total + (ops.linear(x, w) * d).sum()
+        got.append(w)
+        want.append(d.float().t() @ x.float() + 1)
+    total.backward()
+    torch.cuda.synchronize()
+    assert sorted(ready) == list(range(len(sizes)))
+    for w, r in zip(got, want):
+        assert ((w._grad_sink - r).norm() / r.norm()).item() < 1e-2 and w.grad is None
+
+
+def test_trainers_come_and_go():
+    """A dropped trainer is gone at once, and what the garbage collector finds does not disturb the next one's capture."""
+    import gc
+    import weakref
+    from mccl_b200.models import build_decoder
+    from mccl_b200.parallel import DDPTrainer
+    dev = torch.device("cuda", 0)
+    ids = torch.randint(0, 512, (2, 65), device=dev)
+    threshold = gc.get_threshold()
+    gc.collect()
+    gc.set_threshold(20, 2, 2)
+    try:
+        for _ in range(3):
+            with dev:
+                model = build_decoder("tiny")
+            trainer = DDPTrainer(model, dev, lr=1e-3)
+            trainer.cycle = trainer   # one that only the collector frees
+            trainer.step(ids[:, :-1].contiguous(), ids[:, 1:].contiguous())
+            torch.cuda.synchronize()
+    finally:
+        gc.set_threshold(*threshold)
+    del trainer.cycle
+    gone = weakref.ref(trainer)
+    del trainer
+    assert gone() is None
