@@ -100,10 +100,12 @@ class DDPTrainer:
                                       and ops.native_ops_available().get("adamw_flat"))
         self._fused_zero = device.type == "cuda" and bool(ops.native_ops_available().get("adamw_flat"))
         # One GPU: the optimizer update of a bucket whose gradients are complete runs on a stream of its own while backward
-        # continues (MCCL_OVERLAP_ADAMW=0: one update at the end).  It is bound by memory and the GEMMs beside it are not;
-        # with two CTAs per SM it takes little of what they use.  Measured: SwiGLU decoder 2948 -> 2812 us per step, 70M
-        # decoder with 64 x 256 tokens 10492 -> 10423 us, the 70M and 110M decoders at 16 x 256 the same within noise.
-        self._opt_ctas = int(os.environ.get("MCCL_OVERLAP_ADAMW_CTAS", "2"))
+        # continues (MCCL_OVERLAP_ADAMW=0: one update at the end).  It is bound by memory and the GEMMs beside it are not.
+        # MCCL_OVERLAP_ADAMW_CTAS caps its CTAs per SM (256 threads each, eight fill an SM).  No cap is best: 1 / 2 / 4 / 8 take
+        # 2980 / 2856 / 2779 / 2784 us per step on the 4-layer SwiGLU decoder, 4664 / 4551 / 4525 / 4504 on the 110M one,
+        # 3457 / 3405 / 3422 / 3413 on the 70M one at 16 x 256 and 10610 / 10566 / 10559 / 10470 at 64 x 256: a GEMM that waits for
+        # thread slots loses less than an update that no longer keeps memory busy.
+        self._opt_ctas = int(os.environ.get("MCCL_OVERLAP_ADAMW_CTAS", "8"))
         # Only in a captured step, and only if the first warm-up step shows that every gradient is written by a native operator,
         # which reports it: what autograd accumulates arrives after such a report, if the same parameter has one.
         self._local_overlap = (self.world == 1 and self._fused_zero and use_graph and os.environ.get("MCCL_OVERLAP_ADAMW", "1") != "0")
@@ -262,7 +264,8 @@ class DDPTrainer:
         end = start + numel
         ops.adamw_step(self.flat_p[start:end], self.flat_g[start:end], self.m[start:end], self.v[start:end], self.lr,
                        self.betas[0], self.betas[1], self.eps, self.wd, self.step_t,
-                       p_bf16=None if self.flat_p16 is None else self.flat_p16[start:end], zero_grad=self._fused_zero)
+                       p_bf16=None if self.flat_p16 is None else self.flat_p16[start:end], zero_grad=self._fused_zero,
+                       ctas_per_sm=ctas_per_sm)
 
     def _reduce_bucket(self, b: _Bucket) -> None:
         """Collective (world > 1) and optimizer slice (overlap_optimizer) of one bucket, on the side stream."""
