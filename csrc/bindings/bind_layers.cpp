@@ -118,13 +118,15 @@ void bind_layers(py::module_& m) {
   });
   // Logits [B, S, V] of a whole decoder, no gradients.  `layers`: per layer the 12 parameters above, or for the RMSNorm / RoPE /
   // SwiGLU family (cos / sin given) ln1 w, qkv w, proj w, ln2 w, gate_up w, down w.  Matrices are fp32 and cast here (one
-  // launch for all), or bf16 copies the caller keeps up to date.
+  // launch for all), or bf16 copies the caller keeps up to date.  None when a parameter is laid out in another order: the operators
+  // copy such a weight first.
   m.def(
       "decoder_fwd",
       [](const at::Tensor& tokens, const at::Tensor& tok, const c10::optional<at::Tensor>& pos, std::vector<at::Tensor> layers,
          const at::Tensor& lnf_w, const c10::optional<at::Tensor>& lnf_b, at::Tensor head, int64_t H, double eps_in,
-         const c10::optional<at::Tensor>& cos_t, const c10::optional<at::Tensor>& sin_t) {
+         const c10::optional<at::Tensor>& cos_t, const c10::optional<at::Tensor>& sin_t) -> c10::optional<at::Tensor> {
         at::NoGradGuard no_grad;
+        if (!all_contiguous(layers) || !all_contiguous({tok, lnf_w, head})) return c10::nullopt;
         MCCL_CHECK_TENSOR(tokens.is_cuda() && tokens.dim() == 2 && tokens.scalar_type() == at::kLong, "decoder_fwd: int64 CUDA tokens [B, S] expected");
         c10::cuda::CUDAGuard guard(tokens.device());
         cudaStream_t st = at::cuda::getCurrentCUDAStream(tokens.get_device()).stream();

@@ -173,11 +173,12 @@ struct CrossEntropyNode : torch::autograd::Function<CrossEntropyNode> {
 
 void bind_decoder_autograd(py::module_& m) {
   // Mean next-token loss of a GELU / LayerNorm decoder with learned positions.  layers: 12 fp32 parameters per layer in the order
-  // of decoder_layer_fwd; head: the fp32 output table (tok itself where they are tied).
+  // of decoder_layer_fwd; head: the fp32 output table (tok itself where they are tied).  None when a parameter is laid out in another order.
   m.def(
       "decoder_loss",
       [](const at::Tensor& tokens, const at::Tensor& targets, const at::Tensor& tok, const at::Tensor& pos, const std::vector<at::Tensor>& layers,
-         const at::Tensor& lnf_w, const at::Tensor& lnf_b, const at::Tensor& head, int64_t heads, double eps) {
+         const at::Tensor& lnf_w, const at::Tensor& lnf_b, const at::Tensor& head, int64_t heads, double eps) -> c10::optional<at::Tensor> {
+        if (!all_contiguous(layers) || !all_contiguous({tok, pos, lnf_w, lnf_b, head})) return c10::nullopt;
         MCCL_CHECK_TENSOR(tokens.is_cuda() && tokens.dim() == 2 && tokens.scalar_type() == at::kLong && targets.is_cuda() &&
                               targets.scalar_type() == at::kLong && targets.numel() == tokens.numel(),
                           "decoder_loss: int64 CUDA tokens [B, S] and as many targets expected");

@@ -24,6 +24,12 @@ inline void need(const at::Tensor& t, at::ScalarType dt, int64_t numel, const ch
                     "decoder layer: " << what << ": a contiguous CUDA tensor of " << numel << " " << c10::toString(dt) << " elements expected");
 }
 
+inline bool all_contiguous(at::TensorList tensors) {
+  for (const at::Tensor& t : tensors)
+    if (!t.is_contiguous()) return false;
+  return true;
+}
+
 // Order of a layer's parameters everywhere below.
 enum Param { LN1_W, LN1_B, QKV_W, QKV_B, PROJ_W, PROJ_B, LN2_W, LN2_B, UP_W, UP_B, DOWN_W, DOWN_B, kParams };
 

@@ -18,8 +18,10 @@ is also the numerics reference in the tests.
 from __future__ import annotations
 
 import dataclasses
-import os
+import itertools
 import math
+import operator
+import os
 from typing import Optional
 
 import torch
@@ -100,34 +102,64 @@ def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.T
     return out.flatten(-2).to(x.dtype)
 
 
-class _Structure:
-    """The parameters of a module tree, collected once, and whether the tree is still what it was: no module or parameter
-    replaced, no hook registered, nothing but plain fp32 parameters.  (Walking the modules again takes longer than launching
-    a small model's kernels.)"""
+# What applies to every module of the process (torch.nn.modules.module.register_module_forward_hook and friends).
+_GLOBAL_HOOKS = tuple(getattr(nn.modules.module, f"_global_{kind}_hooks") for kind in ("forward", "forward_pre", "backward", "backward_pre"))
 
-    def __init__(self, root: nn.Module):
-        modules = list(root.modules())
-        self.dicts = [d for m in modules for d in (m._modules, m._parameters) if d]
-        self.values = [list(d.values()) for d in self.dicts]
-        self.hooks = [d for m in modules for d in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks, m._backward_pre_hooks)]
-        self.plain = all(type(p) is nn.Parameter and p.dtype == torch.float32 and p.is_contiguous() for p in root.parameters())
-        self.device = next(root.parameters()).device
-        self.params = {name: p for name, p in root.named_parameters()}
+
+def _stock(m: nn.Module) -> bool:
+    """Whether a native call may stand in for m: a module of this file, or of a class derived from one that leaves its
+    methods alone."""
+    return type(m).__call__ is nn.Module.__call__ and any(
+        isinstance(m, cls) and all(getattr(type(m), name) is f for name, f in methods.items()) for cls, methods in _STOCK.items())
+
+
+def _untouched(m: nn.Module) -> bool:
+    """The same, and nobody wants to see the module's own calls."""
+    return (_stock(m) and "forward" not in m.__dict__ and not any(_GLOBAL_HOOKS)
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks))
+
+
+class _Structure:
+    """The parameters of some of a module's children, collected once, and whether the tree is still what it was: modules of this
+    file whose methods nobody replaced, no module or parameter exchanged, no hook registered, nothing but plain fp32
+    parameters.  (Walking the modules again takes longer than launching a small model's kernels.)"""
+
+    def __init__(self, root: nn.Module, children):
+        # the root itself is not among them: it keeps this object
+        self.modules = list(dict.fromkeys(m for c in children if c is not None for m in c.modules()))
+        self.types = [type(m) for m in self.modules]
+        self.own = [m.__dict__ for m in self.modules]
+        self.eps = [m.eps for m in self.modules if isinstance(m, Norm)]
+        self.norms = [m.__dict__ for m in self.modules if isinstance(m, Norm)]
+        self.dicts = [d for m in (root, *self.modules) for d in (m._modules, m._parameters) if d]
+        self.values = [v for d in self.dicts for v in d.values()]
+        self.sizes = [len(d) for d in self.dicts]
+        self.hooks = [d for m in (root, *self.modules) for d in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks, m._backward_pre_hooks)]
+        self.params = list(dict.fromkeys(p for m in self.modules for p in m._parameters.values() if p is not None))
+        self.plain = (bool(self.params) and all(type(p) is nn.Parameter and p.dtype == torch.float32 and p.is_contiguous() for p in self.params)
+                      and all(_stock(m) for m in self.modules) and len(set(self.eps)) <= 1)
+        self.device = self.params[0].device if self.params else None
+        self.layers = None   # the layers' parameters in order, once somebody has asked for them (False: not applicable)
+
+    def __reduce__(self):
+        return type(None), ()   # a copied or stored model collects its own
 
     def intact(self) -> bool:
-        if not self.plain or any(self.hooks):
-            return False
-        try:
-            return all(list(d.values()) == v for d, v in zip(self.dicts, self.values))
-        except RuntimeError:   # a replaced parameter compares by element
-            return False
+        # (maps over built-in functions: half the time of comprehensions)
+        return (self.plain and not any(self.hooks) and not any(_GLOBAL_HOOKS)
+                and list(map(len, self.dicts)) == self.sizes
+                and all(map(operator.is_, itertools.chain.from_iterable(map(dict.values, self.dicts)), self.values))
+                and list(map(type, self.modules)) == self.types
+                and not any(map(dict.__contains__, self.own, itertools.repeat("forward")))
+                and list(map(operator.itemgetter("eps"), self.norms)) == self.eps
+                and all(getattr(cls, name) is f for cls, methods in _STOCK.items() for name, f in methods.items()))
 
 
-def _structure(module: nn.Module, device):
-    """The module's cached `_Structure` when it can be used on `device`, else None."""
+def _structure(module: nn.Module, device, children):
+    """The module's cached `_Structure` of these children when it can be used on `device`, else None."""
     s = module.__dict__.get("_structure_cache")
     if s is None or s.device != device or not s.intact():
-        s = _Structure(module)
+        s = _Structure(module, children)
         module.__dict__["_structure_cache"] = s
         if s.device != device or not s.intact():
             return None
@@ -158,7 +190,7 @@ class Norm(nn.Module):
         """(norm(x), x as it should be fed to the residual connection).  The native path hands x through the
         norm operator so that backward adds the residual gradient in the norm-backward kernel
         (MCCL_FUSE_RESIDUAL_GRAD=0: x is returned untouched)."""
-        if native and _FUSE_RESIDUAL_GRAD:
+        if native and _FUSE_RESIDUAL_GRAD and _stock(self) and "forward" not in self.__dict__:
             from .. import ops
             return ops.norm_residual(x, self.weight, self.bias, self.eps)
         return self.forward(x, native), x
@@ -207,17 +239,34 @@ class Block(nn.Module):
             return None
         if not _C.decoder_layer_supported(x.shape[1], cfg.n_heads, cfg.d_model, cfg.d_ff):
             return None
-        s = _structure(self, x.device)
+        s = _structure(self, x.device, self._modules.values())
         if s is None:
             return None
-        params = s.__dict__.get("ordered")
-        if params is None:
-            s.ordered = params = [s.params.get(f"{m}.{k}") for m in ("ln1", "qkv", "proj", "ln2", "up", "down") for k in ("weight", "bias")]
-        if any(p is None for p in params):
+        if s.layers is None:
+            s.layers = self._ordered() or False
+        if not s.layers or s.eps[0] != cfg.eps or not all(p.is_contiguous() for p in s.layers):
             return None
-        if torch.is_grad_enabled() and not all(p.requires_grad for p in params):
+        if torch.is_grad_enabled() and not all(p.requires_grad for p in s.layers):
             return None   # frozen parameters: operator by operator
-        return params
+        return s.layers
+
+    def _ordered(self):
+        """This layer's parameters in the order the native calls take them, or None when they are not the ones its sizes ask for."""
+        cfg = self.cfg
+        D, FF, bias = cfg.d_model, cfg.d_ff, cfg.norm == "layernorm"
+        swiglu = cfg.act == "swiglu"
+        want = [("ln1", (D,), bias), ("qkv", (3 * D, D), bias), ("proj", (D, D), bias), ("ln2", (D,), bias)]
+        want += [("gate_up", (2 * FF, D), False), ("down", (D, FF), bias)] if swiglu else [("up", (FF, D), bias), ("down", (D, FF), bias)]
+        out = []
+        for name, shape, with_bias in want:
+            m = self._modules.get(name)
+            if not isinstance(m, Norm if name.startswith("ln") else Linear):
+                return None
+            w, b = m._parameters.get("weight"), m._parameters.get("bias")
+            if w is None or w.shape != shape or (b is None) == with_bias or (with_bias and b.shape != shape[:1]):
+                return None
+            out += [w, b] if with_bias else [w]
+        return out
 
     def forward(self, x: torch.Tensor, rope, native: bool) -> torch.Tensor:
         cfg = self.cfg
@@ -247,18 +296,23 @@ class Block(nn.Module):
         if cfg.act == "swiglu":
             if native:
                 from .. import ops
-                if not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (self.gate_up, self.down)):
+                if all(_untouched(m) and m.bias is None for m in (self.gate_up, self.down)):
                     return ops.mlp_swiglu(h, self.gate_up.weight, self.down.weight, residual=x)
-                h = ops.swiglu(self.gate_up(h, native))   # somebody wants to see the projections' own calls
+                h = ops.swiglu(self.gate_up(h, native))   # not what the fused call computes, or somebody wants to see the calls
             else:
                 g, u = self.gate_up(h, native).chunk(2, dim=-1)
                 h = F.silu(g) * u
-        elif native:
+        elif native and _untouched(self.up) and _untouched(self.down):
             from .. import ops
             return ops.mlp_gelu(h, self.up.weight, self.up.bias, self.down.weight, self.down.bias, residual=x)
         else:
             h = self.up(h, native, act="gelu")
         return self.down(h, native, residual=x)
+
+
+#: Modules that the native calls can stand for, and the methods whose work they do.
+_STOCK = {cls: {name: getattr(cls, name) for name in ("forward", "with_residual") if hasattr(cls, name)}
+          for cls in (Block, Norm, Linear, nn.Embedding, nn.ModuleList)}
 
 
 class Decoder(nn.Module):
@@ -299,35 +353,52 @@ class Decoder(nn.Module):
             x = blk(x, rope, native)
         return self.ln_f(x, native)
 
-    def _ordered(self, s, rope: bool):
-        """The layers' parameters in the order the native calls take them."""
-        layers = s.__dict__.get("ordered")
-        if layers is None:
-            names = (("ln1.weight", "qkv.weight", "proj.weight", "ln2.weight", "gate_up.weight", "down.weight") if rope else
-                     [f"{m}.{k}" for m in ("ln1", "qkv", "proj", "ln2", "up", "down") for k in ("weight", "bias")])
-            s.ordered = layers = [s.params[f"blocks.{i}.{n}"] for i in range(self.cfg.n_layers) for n in names]
-        return layers
+    def _layers(self, device):
+        """(structure, the layers' parameters in the order the native calls take them), or None where those calls do not stand for
+        this model: a module or a method was replaced, parameters are missing or of other sizes, somebody watches the calls."""
+        cls = type(self)
+        if cls.hidden is not Decoder.hidden or cls.head_weight is not Decoder.head_weight or "hidden" in self.__dict__ or "head_weight" in self.__dict__:
+            return None
+        m = self._modules
+        s = _structure(self, device, (m.get("tok"), m.get("pos"), m.get("blocks"), m.get("ln_f"), m.get("head")))
+        if s is None:
+            return None
+        if s.layers is None:
+            cfg, layers = self.cfg, []
+            for blk in self.blocks:
+                own = blk._ordered() if isinstance(blk, Block) and blk.cfg == cfg else None
+                if own is None:
+                    layers = None
+                    break
+                layers += own
+            tables = [t._parameters.get("weight") for t in (self.tok, self.pos, self.head) if t is not None]
+            lnf = self.ln_f._parameters if isinstance(self.ln_f, Norm) else {}
+            fits = (layers is not None and all(t is not None and t.dim() == 2 and t.shape[1] == cfg.d_model for t in tables)
+                    and lnf.get("weight") is not None and lnf["weight"].numel() == cfg.d_model and (lnf.get("bias") is None) == (cfg.norm != "layernorm")
+                    and getattr(self.head, "bias", None) is None and (self.pos is None) == (cfg.pos == "rope") and s.eps[0] == cfg.eps)
+            s.layers = layers if fits else False
+        return None if s.layers is False else (s, s.layers)
 
     def _fused_gelu(self, tokens: torch.Tensor) -> bool:
         cfg = self.cfg
         from .. import _C
         from ..ops.functional import native_attention_supported
         return (cfg.pos == "learned" and cfg.norm == "layernorm" and cfg.act == "gelu" and tokens.dim() == 2 and tokens.dtype == torch.int64
-                and cfg.vocab % 8 == 0 and tokens.shape[1] <= cfg.max_seq and not torch.is_autocast_enabled()
+                and self.head_weight().shape[0] % 8 == 0 and tokens.shape[1] <= cfg.max_seq and not torch.is_autocast_enabled()
                 and native_attention_supported(tokens.shape[1], cfg.head_dim)
                 and _C.decoder_layer_supported(tokens.shape[1], cfg.n_heads, cfg.d_model, cfg.d_ff))
 
     def _loss_in_one_call(self, tokens: torch.Tensor, targets: torch.Tensor):
         """The training loss through C++ autograd nodes, or None where that does not apply (a trainer's gradient buffers, frozen
         or replaced parameters, hooks)."""
-        if not self._fused_gelu(tokens) or targets.dtype != torch.int64 or targets.numel() != tokens.numel():
+        found = self._layers(tokens.device)
+        if found is None or not self._fused_gelu(tokens) or targets.dtype != torch.int64 or targets.numel() != tokens.numel():
             return None
-        s = _structure(self, tokens.device)
-        if s is None or hasattr(self.tok.weight, "_grad_sink") or not all(p.requires_grad for p in s.params.values()):
+        s, layers = found
+        if hasattr(self.tok.weight, "_grad_sink") or not all(p.requires_grad for p in s.params):
             return None
         from .. import _C
-        p = s.params
-        return _C.decoder_loss(tokens, targets, p["tok.weight"], p["pos.weight"], self._ordered(s, False), p["ln_f.weight"], p["ln_f.bias"],
+        return _C.decoder_loss(tokens, targets, self.tok.weight, self.pos.weight, layers, self.ln_f.weight, self.ln_f.bias,
                                self.head_weight(), self.cfg.n_heads, self.cfg.eps)
 
     def _forward_without_gradients(self, tokens: torch.Tensor):
@@ -335,23 +406,21 @@ class Decoder(nn.Module):
         cfg = self.cfg
         from .. import _C
         rope = cfg.pos == "rope"
+        found = self._layers(tokens.device)
+        if found is None:
+            return None
         if rope:
-            if (tokens.dim() != 2 or tokens.dtype != torch.int64 or cfg.d_model % 64 or cfg.d_ff % 64 or cfg.vocab % 8 or cfg.norm != "rmsnorm"
-                    or cfg.act != "swiglu" or cfg.head_dim % 8 or torch.is_autocast_enabled()):
+            if (tokens.dim() != 2 or tokens.dtype != torch.int64 or cfg.d_model % 64 or cfg.d_ff % 64 or self.head_weight().shape[0] % 8
+                    or cfg.norm != "rmsnorm" or cfg.act != "swiglu" or cfg.head_dim % 8 or torch.is_autocast_enabled()):
                 return None
         elif not self._fused_gelu(tokens):
             return None
-        s = _structure(self, tokens.device)
-        if s is None:
-            return None
-        layers = self._ordered(s, rope)
-        head = self.head_weight()
+        layers, head = found[1], self.head_weight()
         if hasattr(head, "_bf16"):   # a trainer keeps bf16 copies of the matrices up to date
             layers = [getattr(p, "_bf16", p) if p.dim() == 2 else p for p in layers]
             head = head._bf16
         tables = _rope_tables(tokens.shape[1], cfg.head_dim, tokens.device) if rope else (None, None)
-        p = s.params
-        return _C.decoder_fwd(tokens, p["tok.weight"], p.get("pos.weight"), layers, p["ln_f.weight"], p.get("ln_f.bias"), head,
+        return _C.decoder_fwd(tokens, self.tok.weight, None if self.pos is None else self.pos.weight, layers, self.ln_f.weight, self.ln_f.bias, head,
                               cfg.n_heads, cfg.eps, *tables)
 
     def head_weight(self) -> torch.Tensor:
