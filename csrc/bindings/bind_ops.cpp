@@ -95,7 +95,8 @@ void bind_ops(py::module_& m) {
       "gemm_bf16",
       [](const at::Tensor& a, const at::Tensor& b, const c10::optional<at::Tensor>& bias, const std::string& epilogue,
          bool out_fp32, const c10::optional<at::Tensor>& out, bool accumulate, bool a_t, bool b_t,
-         const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& mul, const c10::optional<at::Tensor>& colsum) {
+         const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& mul, const c10::optional<at::Tensor>& colsum,
+         const c10::optional<at::Tensor>& alpha) {
         need_cuda(a, "gemm(a)");
         need_cuda(b, "gemm(b)");
         MCCL_CHECK_TENSOR(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16, "gemm: operands must be bf16");
@@ -160,6 +161,12 @@ void bind_ops(py::module_& m) {
                             "gemm: colsum must have N elements and goes with a bf16 output, an MN-major B and no bias, activation or residual");
           g.colsum = colsum->data_ptr<float>();
         }
+        if (alpha.has_value() && alpha->defined()) {
+          need(*alpha, at::kFloat, "gemm(alpha)");
+          MCCL_CHECK_TENSOR(alpha->numel() == 1 && !g.bias && !g.residual && !g.mul && !g.colsum && g.epilogue == ops::EPI_NONE && b_t && a_t == out_fp32,
+                            "gemm: alpha is one value for a weight gradient (fp32, both operands MN-major) or an input gradient (bf16, MN-major B) alone");
+          g.alpha = alpha->data_ptr<float>();
+        }
         // A contraction far longer than the output is wide (the input gradient of an LM head: 32000 against 512) has too few
         // tiles for the SMs; its fp32 partial sums go through a workspace (4096 x 512 x 32000: 123 -> 108 us).
         at::Tensor partial;
@@ -168,9 +175,10 @@ void bind_ops(py::module_& m) {
           g.d = partial.data_ptr();
           g.d_fp32 = g.accumulate = true;
           g.ldd = static_cast<int>(N);
+          g.alpha = nullptr;   // the cast multiplies
         }
         cudaError_t rc = ops::gemm_bf16_tn(g, stream_of(a));
-        if (rc == cudaSuccess && partial.defined()) rc = ops::cast_f32_bf16(partial.data_ptr<float>(), bf(d), M * N, stream_of(a));
+        if (rc == cudaSuccess && partial.defined()) rc = ops::cast_f32_bf16(partial.data_ptr<float>(), bf(d), M * N, stream_of(a), alpha.has_value() ? alpha->data_ptr<float>() : nullptr);
         MCCL_CHECK_T(rc == cudaSuccess, CudaError,
                      "gemm_bf16 [" << M << "x" << N << "x" << K << ", lda " << g.lda << ", ldb " << g.ldb << ", ldd " << g.ldd
                                    << "] failed: " << cudaGetErrorString(rc) << " " << ops::gemm_last_reason());
@@ -178,7 +186,7 @@ void bind_ops(py::module_& m) {
       },
       py::arg("a"), py::arg("b"), py::arg("bias") = py::none(), py::arg("epilogue") = "none", py::arg("out_fp32") = false,
       py::arg("out") = py::none(), py::arg("accumulate") = false, py::arg("a_t") = false, py::arg("b_t") = false,
-      py::arg("residual") = py::none(), py::arg("mul") = py::none(), py::arg("colsum") = py::none());
+      py::arg("residual") = py::none(), py::arg("mul") = py::none(), py::arg("colsum") = py::none(), py::arg("alpha") = py::none());
 
   // dW_i[N_i, K_i] = dY_i[tokens, N_i]^T · X_i[tokens, K_i], sixteen products per launch.  items: (dY, X, dW or None); with
   // accumulate every dW is given and added into.  Returns the dW.

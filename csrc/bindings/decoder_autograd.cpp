@@ -123,7 +123,7 @@ struct NormNode : torch::autograd::Function<NormNode> {
 };
 
 // Mean cross entropy of h · head^T against targets; the gradient of the logits replaces them in the forward pass, for an
-// upstream gradient of one (the loss is what backward() is called on).
+// upstream gradient of one.  Backward's two products multiply by the one that comes (a scaled loss, a sum of several).
 struct CrossEntropyNode : torch::autograd::Function<CrossEntropyNode> {
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& h, const at::Tensor& head, const at::Tensor& flat, int64_t off, const at::Tensor& targets) {
     const int D = static_cast<int>(h.size(-1)), T = static_cast<int>(h.numel() / D), V = static_cast<int>(head.size(0));
@@ -136,10 +136,11 @@ struct CrossEntropyNode : torch::autograd::Function<CrossEntropyNode> {
     check(ops::mean_f32(rows.data_ptr<float>(), loss.data_ptr<float>(), T, stream_on(h)), "mean loss");
     return loss;
   }
-  static variable_list backward(AutogradContext* ctx, variable_list) {
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const at::Tensor &h = saved[0], &head = saved[1], &flat = saved[2], &dlogits = saved[3];
     c10::cuda::CUDAGuard guard(h.device());
+    const at::Tensor upstream = grads[0].to(head.options());
     const int D = static_cast<int>(h.size(-1)), T = static_cast<int>(h.numel() / D), V = static_cast<int>(head.size(0));
     cudaStream_t st = stream_on(h);
     at::Tensor dh = at::empty_like(h);
@@ -157,13 +158,15 @@ struct CrossEntropyNode : torch::autograd::Function<CrossEntropyNode> {
       g.d_fp32 = g.accumulate = true;
       g.d = partial.data_ptr();
       check(ops::gemm_bf16_tn(g, st), "head backward");
-      check(ops::cast_f32_bf16(partial.data_ptr<float>(), bf(dh), static_cast<long long>(T) * D, st), "head backward");
+      check(ops::cast_f32_bf16(partial.data_ptr<float>(), bf(dh), static_cast<long long>(T) * D, st, upstream.data_ptr<float>()), "head backward");
     } else {
+      g.alpha = upstream.data_ptr<float>();
       check(ops::gemm_bf16_tn(g, st), "head backward");
     }
     at::Tensor dw = at::empty({V, D}, head.options());
     ops::GemmArgs wg = weight_gradient(bf(dlogits), bf(h), dw.data_ptr<float>(), T, V, D);
     wg.accumulate = false;
+    wg.alpha = upstream.data_ptr<float>();
     check(ops::gemm_bf16_tn(wg, st), "head weight gradient");
     return {dh, dw, at::Tensor(), at::Tensor(), at::Tensor()};
   }

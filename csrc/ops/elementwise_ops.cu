@@ -859,31 +859,33 @@ cudaError_t transpose_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, int rows
 }
 
 // ------------------------------------------------------------------ casts --
-__global__ void __launch_bounds__(256) cast_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n) {
+__global__ void __launch_bounds__(256) cast_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n,
+                                                   const float* __restrict__ alpha) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
   ::mccl::pdl_wait();
   ::mccl::pdl_trigger();
+  const float s = alpha != nullptr ? __ldg(alpha) : 1.f;
   const long long n4 = n / 4;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const float4 f = reinterpret_cast<const float4*>(in)[i];
-    __nv_bfloat162 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
+    __nv_bfloat162 lo = __floats2bfloat162_rn(f.x * s, f.y * s), hi = __floats2bfloat162_rn(f.z * s, f.w * s);
     uint2 packed;
     packed.x = *reinterpret_cast<uint32_t*>(&lo);
     packed.y = *reinterpret_cast<uint32_t*>(&hi);
     reinterpret_cast<uint2*>(out)[i] = packed;
   }
   if (blockIdx.x == 0)
-    for (long long i = n4 * 4 + threadIdx.x; i < n; i += blockDim.x) out[i] = __float2bfloat16_rn(in[i]);
+    for (long long i = n4 * 4 + threadIdx.x; i < n; i += blockDim.x) out[i] = __float2bfloat16_rn(in[i] * s);
 }
 
-cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t stream) {
+cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t stream, const float* alpha) {
   if (n <= 0) return cudaSuccess;
   if ((reinterpret_cast<uintptr_t>(in) & 15u) || (reinterpret_cast<uintptr_t>(out) & 7u)) return cudaErrorNotSupported;
   long long blocks = (n / 4 + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
   if (blocks < 1) blocks = 1;
-  MCCL_LAUNCH_PDL(cast_kernel, static_cast<int>(blocks), 256, 0, stream, in, out, n);
+  MCCL_LAUNCH_PDL(cast_kernel, static_cast<int>(blocks), 256, 0, stream, in, out, n, alpha);
   count_launch();
   return ::mccl::launch_status();
 }

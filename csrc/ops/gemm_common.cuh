@@ -23,6 +23,7 @@ struct GemmDev {
   const __nv_bfloat16* residual;
   const __nv_bfloat16* mul;       // when set: D = acc * mul, e.g. the backward of a GELU (mul = saved gelu'(z)) fused into the producing GEMM
   float* colsum = nullptr;        // when set: column sums of D (bf16 output) are added here, fp32 [N]
+  const float* alpha = nullptr;   // when set: the product is multiplied by this scalar before it is rounded or added
   int m, n, k;
   int ldd;
   int d_fp32;

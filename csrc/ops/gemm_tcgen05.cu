@@ -70,7 +70,8 @@ cudaError_t gemm_bf16_tn(const GemmArgs& a, cudaStream_t stream) {
   const int forced = g_gemm_kernel_override.load(std::memory_order_relaxed);
   const int choice = forced != -2 ? forced : env_choice;
   const bool gelu = a.epilogue == EPI_BIAS_GELU || a.epilogue == EPI_GELU || a.epilogue == EPI_BIAS_GELU_D || a.epilogue == EPI_GELU_D;
-  const bool tile_only = a.k % BK != 0 || a.colsum || (gelu && !a.aux);   // what only the tile kernel does
+  if (a.alpha && (gelu || a.bias || a.residual || a.mul || a.colsum)) return cudaErrorInvalidValue;
+  const bool tile_only = a.k % BK != 0 || a.colsum || a.alpha || (gelu && !a.aux);   // what only the tile kernel does
   cudaError_t rc = choice == kPersistent && !tile_only ? launch_gemm_persistent(a, FusedDev{}, 0, stream) : launch_gemm_tiles(a, choice, stream);
   if (rc == cudaErrorNotSupported) return unsupported("cuTensorMapEncodeTiled rejected an operand");
   return rc;

@@ -19,6 +19,8 @@ MCCL_TILES_EXTERN_PAIR(false, false, OUT_BF16, 1)
 MCCL_TILES_EXTERN_PAIR(false, false, OUT_F32, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16_SUM, 1)
+MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16_SCALED, 1)
+MCCL_TILES_EXTERN_PAIR(true, true, OUT_F32_SCALED, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_F32, 1)
 MCCL_TILES_EXTERN_PAIR(true, false, OUT_BF16, 1)
 MCCL_TILES_EXTERN_PAIR(true, false, OUT_F32, 1)
@@ -109,7 +111,7 @@ cudaError_t run(const GemmArgs* a, int count, int forced, cudaStream_t stream) {
     if (limit < sms) sms = limit;
     if (limit / 2 < pairs) pairs = limit / 2;
   }
-  bool splittable = kOut == OUT_F32;
+  bool splittable = fp32_out(kOut);
   for (int p = 0; p < count; ++p) splittable = splittable && (a[p].accumulate || a[p].ldd == a[p].n);
   const Plan plan = choose(a, count, forced, sms, pairs, kOut == OUT_GELU, splittable);
   if (plan.bn == 64) return launch_tiles<64, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
@@ -140,6 +142,11 @@ cudaError_t launch_gemm_tiles(const GemmArgs& a, int forced_bn, cudaStream_t str
   if (a.colsum) {
     if (gelu || a.d_fp32 || a.bias || a.residual || a.a_mn_major || !a.b_mn_major) return cudaErrorInvalidValue;
     return tiles::run<false, true, tiles::OUT_BF16_SUM>(&a, 1, forced_bn, stream);
+  }
+  if (a.alpha) {
+    if (a.d_fp32 && a.a_mn_major && a.b_mn_major) return tiles::run<true, true, tiles::OUT_F32_SCALED>(&a, 1, forced_bn, stream);
+    if (!a.d_fp32 && !a.a_mn_major && a.b_mn_major) return tiles::run<false, true, tiles::OUT_BF16_SCALED>(&a, 1, forced_bn, stream);
+    return cudaErrorInvalidValue;
   }
   if (gelu) return tiles::run<false, false, tiles::OUT_GELU>(&a, 1, forced_bn > 128 ? 128 : forced_bn, stream);
   if (a.d_fp32) return tiles::run_majors<tiles::OUT_F32>(a, forced_bn, stream);

@@ -37,6 +37,9 @@ namespace mccl {
 namespace ops {
 namespace tiles {
 
+// OUT_BF16_SCALED, OUT_F32_SCALED: times the scalar at GemmDev::alpha (the upstream gradient of a loss).  Instantiations of their own: the
+// multiplications in the other epilogues, even where they were skipped, cost 2 us of a 134 us training step (instruction
+// fetch, and fewer loads in flight).
 // OUT_BF16_SUM: the bf16 output and, added into GemmDev::colsum, its column sums (a bias gradient).
 // OUT_SWIGLU (pair tile only): B is [gate | up], 2 n rows; the even CTA brings 128 rows of gate and the odd one the same 128 of up,
 // so that a tile's accumulator holds both factors of 128 outputs and silu(gate) * up is the epilogue.  The [m, 2 n] product
@@ -45,7 +48,8 @@ namespace tiles {
 // OUT_SWIGLU_GRAD (pair tile only): the input gradient of the product behind the activation, turned into the gradient of
 // [gate | up] (D, [m, 2 n]) with the saved [gate | up] (`aux`) on its way out; the [m, n] tensor between the two is neither
 // written nor read.
-enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3, OUT_SWIGLU = 4, OUT_SWIGLU_GRAD = 5 };
+enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3, OUT_SWIGLU = 4, OUT_SWIGLU_GRAD = 5, OUT_BF16_SCALED = 6, OUT_F32_SCALED = 7 };
+constexpr bool fp32_out(int out) { return out == OUT_F32 || out == OUT_F32_SCALED; }
 constexpr bool half_boxes(int out) { return out == OUT_GELU || out == OUT_SWIGLU || out == OUT_SWIGLU_GRAD; }   // 32-column output boxes
 
 // One product, or several with the same K whose tiles one launch works through (the weight gradients of one or more layers:
@@ -194,7 +198,7 @@ __device__ __forceinline__ void unpack8(const uint4& pk, float (&v)[8]) {
 template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut, int kMax>
 __global__ void __launch_bounds__(Shape<BN, kPair, kOut == OUT_GELU>::kThreads, 1)
 gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits) {
-  constexpr bool kBf16 = kOut == OUT_BF16 || kOut == OUT_BF16_SUM;
+  constexpr bool kBf16 = kOut == OUT_BF16 || kOut == OUT_BF16_SUM, kF32 = fp32_out(kOut), kScaled = kOut == OUT_BF16_SCALED || kOut == OUT_F32_SCALED;
   using S = Shape<BN, kPair, kOut == OUT_GELU>;
   constexpr int kStages = S::kStages, kTileM = kPair ? 2 * BM : BM;
   constexpr bool kGated = kOut == OUT_SWIGLU;
@@ -219,7 +223,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
   // splits >= 1: work items are (tile, part of K), taken in turn.  splits == 0: every worker gets an equal run of k-blocks,
   // across tile borders, and adds what it has of each tile into D.
   const int tiles = P.first[P.count];
-  const bool runs = kOut == OUT_F32 && splits == 0;
+  const bool runs = kF32 && splits == 0;
   const int work_begin = runs ? static_cast<int>(static_cast<long long>(tiles) * all_kb * worker / workers) : worker;
   const int work_end = runs ? static_cast<int>(static_cast<long long>(tiles) * all_kb * (worker + 1) / workers) : tiles * splits;
 
@@ -411,13 +415,15 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
     const int e = warp - 2, quarter = warp & 3, part = e >> 2;
     uint8_t* stage = smem + S::kStagingOff + e * 4096;
     uint64_t* xfull = extra_full + e;
-    const bool has_bias = kOut != OUT_F32 && (g.epilogue == EPI_BIAS || g.epilogue == EPI_BIAS_GELU || g.epilogue == EPI_BIAS_GELU_D);
+    const bool has_bias = !kF32 && !kScaled && (g.epilogue == EPI_BIAS || g.epilogue == EPI_BIAS_GELU || g.epilogue == EPI_BIAS_GELU_D);
     const bool has_extra = kBf16 && (g.mul != nullptr || g.residual != nullptr);
     const bool multiply = g.mul != nullptr;
     const bool gelu_d = g.epilogue == EPI_BIAS_GELU_D || g.epilogue == EPI_GELU_D;
     bool ok = true;
     int i = 0;
     uint32_t xparity = 0;
+    float alpha = 1.f;
+    if constexpr (kScaled) alpha = __ldg(g.alpha);
     for (int w = work_begin; w < work_end; ++i) {
       const Item it = item(w);
       w = it.next;
@@ -461,7 +467,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           else tc::mbar_arrive(&acc_empty[buf]);
         }
       };
-      if constexpr (kOut == OUT_F32) {
+      if constexpr (kF32) {
         const bool add = g.atomic_add || g.accumulate;
 #pragma unroll 1
         for (int c = 0; c < S::kCols; c += 32) {
@@ -472,6 +478,10 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           if (row0 >= m || col0 + c >= n) continue;
           if (tc::elect_one()) bulk_wait_read<0>();
           __syncwarp();
+          if constexpr (kScaled) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
+          }
 #pragma unroll
           for (int j = 0; j < 8; ++j) *stage_unit(stage, lane, j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
           fence_async_smem();
@@ -638,7 +648,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
             const int j = 4 * h + jj;
             float v[8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(r[jj * 8 + q]);
+            for (int q = 0; q < 8; ++q) v[q] = kScaled ? __uint_as_float(r[jj * 8 + q]) * alpha : __uint_as_float(r[jj * 8 + q]);
             if (has_bias) {
               const int src = 2 * j;
               v[0] += __shfl_sync(0xffffffffu, bias4.x, src);
@@ -762,7 +772,7 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
                      : kAMn ? encode_map(&P.a[p], a.a, a.k, a.m, a.lda, BK) : encode_map(&P.a[p], a.a, a.m, a.k, a.lda, BM);
     const bool okb = P.atoms[p] & 2 ? encode_groups(&P.b[p], a.b, a.k, a.n, a.ldb, S::kRowsB / 64)
                      : kBMn ? encode_map(&P.b[p], a.b, a.k, a.n, a.ldb, BK) : encode_map(&P.b[p], a.b, kOut == OUT_SWIGLU ? 2 * a.n : a.n, a.k, a.ldb, S::kRowsB);
-    if (!oka || !okb || !encode_out_map(&P.d[p], a.d, a.m, kOut == OUT_SWIGLU_GRAD ? 2 * a.n : a.n, a.ldd, kOut == OUT_F32, half_boxes(kOut))) return cudaErrorNotSupported;
+    if (!oka || !okb || !encode_out_map(&P.d[p], a.d, a.m, kOut == OUT_SWIGLU_GRAD ? 2 * a.n : a.n, a.ldd, fp32_out(kOut), half_boxes(kOut))) return cudaErrorNotSupported;
     P.m[p] = a.m;
     P.n[p] = a.n;
     constexpr int kTileN = kOut == OUT_SWIGLU ? BN / 2 : BN;
@@ -775,7 +785,7 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
     }
   }
   const GemmArgs& a = args[0];
-  const void* x = half_boxes(kOut) ? a.aux : (kOut == OUT_F32 ? nullptr : (a.mul ? a.mul : a.residual));
+  const void* x = half_boxes(kOut) ? a.aux : (fp32_out(kOut) ? nullptr : (a.mul ? a.mul : a.residual));
   if (x == nullptr) P.x = P.d[0];   // never used
   else if (kOut == OUT_SWIGLU || kOut == OUT_SWIGLU_GRAD ? !encode_out_map(&P.x, x, a.m, 2 * a.n, 2 * a.n, false, true)
                                                          : !encode_out_map(&P.x, x, a.m, a.n, a.ldd, false, half_boxes(kOut))) return cudaErrorNotSupported;
@@ -786,11 +796,12 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
   g.residual = a.residual;
   g.mul = a.mul;
   g.colsum = a.colsum;
+  g.alpha = a.alpha;
   g.m = a.m;
   g.n = a.n;
   g.k = a.k;
   g.ldd = a.ldd;
-  g.d_fp32 = kOut == OUT_F32 ? 1 : 0;
+  g.d_fp32 = fp32_out(kOut) ? 1 : 0;
   g.accumulate = a.accumulate ? 1 : 0;
   g.epilogue = a.epilogue;
   g.atomic_add = splits != 1 ? 1 : 0;

@@ -63,8 +63,8 @@ cudaError_t mean_f32(const float* in, float* out, long long n, cudaStream_t stre
 
 // ---- out[c, r] = in[r, c] for a bf16 matrix [rows, cols].
 cudaError_t transpose_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, int rows, int cols, cudaStream_t stream);
-// fp32 → bf16 cast of n elements.
-cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t stream);
+// fp32 → bf16 cast of n elements, times the device scalar alpha (null: one).
+cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t stream, const float* alpha = nullptr);
 // The same for `count` tensors, tensor i into out[dst_offset[i], ...); 16-byte aligned sources and places.
 cudaError_t cast_many(const float* const* src, const long long* numel, const long long* dst_offset, int count, __nv_bfloat16* out,
                       cudaStream_t stream);
@@ -130,6 +130,8 @@ struct GemmArgs {
   int lda = 0, ldb = 0, ldd = 0;
   bool d_fp32 = false;
   bool accumulate = false;           // D += result (fp32 output only)
+  const float* alpha = nullptr;      // device scalar: the product is multiplied by it.  A weight gradient (fp32, both operands MN-major) or an input
+                                     // gradient (bf16, MN-major B) without bias, activation, residual, multiplier or column sums
   int epilogue = EPI_NONE;
 };
 // Returns cudaErrorNotSupported for shapes the kernel does not cover

@@ -59,21 +59,21 @@ def join_wgrad(stream=None) -> None:
         (stream if stream is not None else torch.cuda.current_stream()).wait_stream(s)
 
 
-def _wgrad_gemm(a_mat: torch.Tensor, b_mat: torch.Tensor, sink: torch.Tensor) -> None:
-    """sink += a_mat^T . b_mat (both [tokens, features]) on the weight-gradient stream."""
+def _wgrad_gemm(a_mat: torch.Tensor, b_mat: torch.Tensor, sink: torch.Tensor, alpha=None) -> None:
+    """sink += alpha * a_mat^T . b_mat (both [tokens, features]; alpha: a device scalar) on the weight-gradient stream."""
     s = _wgrad["stream"]
     if s is None:
-        _C.gemm_bf16(a_mat, b_mat, None, "none", True, sink, True, True, True)
+        _C.gemm_bf16(a_mat, b_mat, None, "none", True, sink, True, True, True, alpha=alpha)
         return
     s.wait_stream(torch.cuda.current_stream())
     if _wgrad["side_ctas"]:
         _C.set_gemm_cta_limit(_wgrad["side_ctas"])
     with torch.cuda.stream(s):
-        _C.gemm_bf16(a_mat, b_mat, None, "none", True, sink, True, True, True)
+        _C.gemm_bf16(a_mat, b_mat, None, "none", True, sink, True, True, True, alpha=alpha)
     if _wgrad["side_ctas"]:
         _C.set_gemm_cta_limit(_wgrad["main_ctas"])
-    a_mat.record_stream(s)
-    b_mat.record_stream(s)
+    for t in (a_mat, b_mat) if alpha is None else (a_mat, b_mat, alpha):
+        t.record_stream(s)
     _wgrad["pending"] = True
 
 
@@ -558,8 +558,8 @@ class NormResidualFn(torch.autograd.Function):
 
 class LinearCrossEntropyFn(torch.autograd.Function):
     """mean CE(h @ W^T, targets).  The backward of the loss with respect to the logits is
-    produced in the same pass that computes the loss, in place of the logits, assuming the
-    loss is what ``backward()`` is called on (upstream gradient 1)."""
+    produced in the same pass that computes the loss, in place of the logits, for an upstream
+    gradient of one; the products of backward multiply by the one that comes."""
 
     @staticmethod
     def forward(ctx, h, weight, targets):
@@ -582,22 +582,23 @@ class LinearCrossEntropyFn(torch.autograd.Function):
         weight = ctx.weight
         T, D = h.shape
         V = w16.shape[0]
+        up = gout.float().contiguous()
         dh = dw = None
         if ctx.needs_input_grad[0]:
             if _gemm_ok(T, D, V):
-                dh, _ = _C.gemm_bf16(dlogits, w16, None, "none", False, None, False, False, True)
+                dh, _ = _C.gemm_bf16(dlogits, w16, None, "none", False, None, False, False, True, alpha=up)
             else:
-                dh = dlogits @ w16
+                dh = ((dlogits @ w16).float() * up).to(h.dtype)
         if ctx.needs_input_grad[1]:
             sink = _sink(weight)
             if _gemm_ok(V, D, T) and V % 8 == 0:
                 if sink is not None:
-                    _wgrad_gemm(dlogits, h, sink)
+                    _wgrad_gemm(dlogits, h, sink, up)
                     _notify(weight)
                 else:
-                    dw, _ = _C.gemm_bf16(dlogits, h, None, "none", True, None, False, True, True)
+                    dw, _ = _C.gemm_bf16(dlogits, h, None, "none", True, None, False, True, True, alpha=up)
             else:
-                dw = (dlogits.t() @ h).float()
+                dw = (dlogits.t() @ h).float() * up
         return dh, dw, None
 
 
