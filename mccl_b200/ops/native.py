@@ -1,7 +1,10 @@
 """autograd Functions over the native kernels (CUDA tensors only)."""
 from __future__ import annotations
 
+import functools
+import itertools
 import threading
+import weakref
 
 import torch
 import torch.nn.functional as F
@@ -317,107 +320,108 @@ class DecoderLayerFn(torch.autograd.Function):
         return (dx, None, None) + (None,) * len(params)
 
 
-class _Deferred:
-    """Weight gradients of decoder layers that go straight into a trainer's buffers, kept back until several layers can share a
-    launch: a layer's four products fill the SMs for 20 us and pay 8 us of set-up, first loads and last epilogue, so at 4096
-    tokens four layers together take 23 us each instead of 25, at 1600 tokens 12 instead of 18, and a small model's 2
-    instead of 6.  Flushed at the end of backward at the latest (by an engine callback), and before anybody looks at the
-    gradients of a bucket."""
+class _Entry:
+    """Products of one backward pass that wait for others: like ones only, on one stream."""
+
+    __slots__ = ("kind", "stream", "items", "params", "size", "__weakref__")
+
+    def __init__(self, kind, stream):
+        self.kind, self.stream = kind, stream
+        self.items, self.params, self.size = [], [], 0.0
+
+
+class _Shared:
+    """Weight gradients that go straight into a trainer's buffers, kept back until several can share a launch.  Flushed at the end
+    of backward at the latest (by an engine callback), and before anybody looks at the gradients of a bucket.
+
+    The callback owns the entry and this table only knows it: the engine drops its callbacks when a pass fails, and what
+    was kept back goes with them instead of joining the next pass's products."""
+
+    def __init__(self):
+        self._lock = threading.Lock()
+        self._pending = weakref.WeakValueDictionary()   # (device, backward pass) -> _Entry
+
+    def _enter(self, device, kind, item, params, size) -> _Entry:
+        """Adds an item to the current pass's entry; one of another kind is flushed first."""
+        key = (device, torch._C._current_graph_task_id())
+        stream = torch.cuda.current_stream(device)
+        entry = self._pending.get(key)
+        if entry is not None and (entry.kind != kind or entry.stream != stream):
+            self._flush(entry)
+            entry = None
+        if entry is None:
+            entry = _Entry(kind, stream)
+            torch.autograd.Variable._execution_engine.queue_callback(functools.partial(self._flush, entry))
+            self._pending[key] = entry
+        with self._lock:
+            entry.items.append(item)
+            entry.params.append(params)
+            entry.size += size
+        return entry
+
+    def _flush(self, entry) -> None:
+        with self._lock:
+            items, params = entry.items, entry.params
+            entry.items, entry.params, entry.size = [], [], 0.0
+        if not items:
+            return
+        with torch.cuda.stream(entry.stream):
+            self._launch(entry.kind, items)
+            for p in itertools.chain.from_iterable(params):
+                _notify(p)
+
+    def flush_all(self) -> None:
+        for entry in list(self._pending.values()):
+            self._flush(entry)
+
+
+class _Deferred(_Shared):
+    """Weight gradients of decoder layers: a layer's four products fill the SMs for 20 us and pay 8 us of set-up, first loads and
+    last epilogue, so at 4096 tokens four layers together take 23 us each instead of 25, at 1600 tokens 12 instead of 18, and a
+    small model's 2 instead of 6."""
 
     #: multiply-adds that keep the GPU busy for some 60 us: enough for the fixed part to be small
     ENOUGH = 5e10
     MOST = 4
 
-    def __init__(self):
-        self._lock = threading.Lock()
-        self._pending = {}   # device -> (sizes, stream, [items], [params], multiply-adds)
-
     def add(self, item, sizes, params, device) -> None:
-        stream = torch.cuda.current_stream(device)
-        with self._lock:
-            entry = self._pending.get(device)
-        if entry is not None and (entry["sizes"] != sizes or entry["stream"] != stream or entry["shape"] != item[3][8].shape):
-            self.flush(device)
-            entry = None
-        if entry is None:
-            entry = {"sizes": sizes, "stream": stream, "shape": item[3][8].shape, "items": [], "params": [], "work": 0.0}
-            with self._lock:
-                self._pending[device] = entry
-            torch.autograd.Variable._execution_engine.queue_callback(lambda: self.flush(device))
-        entry["items"].append(item)
-        entry["params"].append(params)
-        entry["work"] += sizes[0] * sizes[1] * float(sum(item[3][i].numel() for i in DecoderLayerFn.MATRICES))
-        if len(entry["items"]) >= self.MOST or entry["work"] >= self.ENOUGH:
-            self.flush(device)
+        work = sizes[0] * sizes[1] * float(sum(item[3][i].numel() for i in DecoderLayerFn.MATRICES))
+        entry = self._enter(device, (sizes, item[3][8].shape), item, params[::-1], work)
+        if len(entry.items) >= self.MOST or entry.size >= self.ENOUGH:
+            self._flush(entry)
 
-    def flush(self, device) -> None:
-        with self._lock:
-            entry = self._pending.pop(device, None)
-        if entry is None:
-            return
-        with torch.cuda.stream(entry["stream"]):
-            _C.decoder_layer_wgrads(entry["items"], *entry["sizes"])
-            for params in entry["params"]:
-                for p in reversed(params):
-                    _notify(p)
-
-    def flush_all(self) -> None:
-        for device in list(self._pending):
-            self.flush(device)
+    def _launch(self, kind, items) -> None:
+        _C.decoder_layer_wgrads(items, *kind[0])
 
 
 _deferred = _Deferred()
 
 
-class _Products:
-    """Weight gradients of single linear layers that go straight into a trainer's buffers.  One whose tiles leave half the SMs
-    idle waits for the next ones over the same tokens and shares a launch with them (1024 x 1024 and 3072 x 1024 over 4096 tokens:
-    two launches of 28 and 33 us beside the optimizer, one of 35); at the latest it goes when backward ends."""
+class _Products(_Shared):
+    """Weight gradients of single linear layers.  One whose tiles leave half the SMs idle waits for the next ones over the same
+    tokens and shares a launch with them (1024 x 1024 and 3072 x 1024 over 4096 tokens: two launches of 28 and 33 us beside the
+    optimizer, one of 35)."""
 
     SMALL = 37    # 256 x 256 tiles: half of what the GPU works on at a time
     MOST = 64     # beyond that a product is better alone
 
-    def __init__(self):
-        self._lock = threading.Lock()
-        self._pending = {}   # device -> {"tokens", "stream", "tiles", "items": [(dz, x, sink)], "weights"}
-
     def add(self, dz, x2, sink, weight) -> None:
         device, tokens = dz.device, dz.shape[0]
         tiles = -(-dz.shape[1] // 256) * -(-x2.shape[1] // 256)
-        stream = torch.cuda.current_stream(device)
-        with self._lock:
-            entry = self._pending.get(device)
-        if entry is not None and (entry["tokens"] != tokens or entry["stream"] != stream or tiles > self.MOST):
-            self.flush(device)
-            entry = None
-        if entry is None and (tiles > self.SMALL or not dz.is_contiguous()):
+        entry = self._pending.get((device, torch._C._current_graph_task_id()))
+        waiting = entry is not None and entry.items and entry.kind == tokens and entry.stream == torch.cuda.current_stream(device)
+        if tiles > (self.MOST if waiting else self.SMALL) or (not waiting and not dz.is_contiguous()):
+            if entry is not None:
+                self._flush(entry)
             _wgrad_gemm(dz, x2, sink)
             _notify(weight)
             return
-        if entry is None:
-            entry = {"tokens": tokens, "stream": stream, "tiles": 0, "items": [], "weights": []}
-            with self._lock:
-                self._pending[device] = entry
-            torch.autograd.Variable._execution_engine.queue_callback(lambda: self.flush(device))
-        entry["items"].append((dz.contiguous(), x2, sink))
-        entry["weights"].append(weight)
-        entry["tiles"] += tiles
-        if entry["tiles"] > self.SMALL or len(entry["items"]) >= 4:
-            self.flush(device)
+        entry = self._enter(device, tokens, (dz.contiguous(), x2, sink), (weight,), tiles)
+        if entry.size > self.SMALL or len(entry.items) >= 4:
+            self._flush(entry)
 
-    def flush(self, device) -> None:
-        with self._lock:
-            entry = self._pending.pop(device, None)
-        if entry is None:
-            return
-        with torch.cuda.stream(entry["stream"]):
-            _C.gemm_group(entry["items"], True)
-            for w in entry["weights"]:
-                _notify(w)
-
-    def flush_all(self) -> None:
-        for device in list(self._pending):
-            self.flush(device)
+    def _launch(self, kind, items) -> None:
+        _C.gemm_group(items, True)
 
 
 _products = _Products()

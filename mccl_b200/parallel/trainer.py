@@ -340,6 +340,11 @@ class DDPTrainer:
             loss.backward()
             if self.device.type == "cuda":
                 _native.join_wgrad(torch.cuda.current_stream(self.device))
+        except BaseException:
+            # what this backward has added already is not part of the next step's gradients
+            if self._fused_zero and not torch.cuda.is_current_stream_capturing():
+                self.flat_g.zero_()
+            raise
         finally:
             _native.set_wgrad_stream(None)
             self._in_backward = False

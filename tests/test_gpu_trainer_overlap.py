@@ -88,3 +88,30 @@ def test_trainers_come_and_go():
     gone = weakref.ref(trainer)
     del trainer
     assert gone() is None
+
+
+@pytest.mark.parametrize("name,changes", [("tiny", {"n_layers": 3}), ("1.3b", {"vocab": 512, "d_model": 256, "n_layers": 3, "n_heads": 4, "d_ff": 512, "max_seq": 256})])
+def test_a_step_that_failed_in_backward(name, changes):
+    """Nothing of it is in the next step's gradients."""
+    from mccl_b200.models import build_decoder
+    from mccl_b200.parallel import DDPTrainer
+    dev = torch.device("cuda", 0)
+    ids = torch.randint(0, 512, (4, 65), device=dev)
+    tok, tgt = ids[:, :-1].contiguous(), ids[:, 1:].contiguous()
+    moments = []
+    for fails in (False, True):
+        torch.manual_seed(0)
+        with dev:
+            model = build_decoder(name, **changes)
+        trainer = DDPTrainer(model, dev, use_graph=False)
+        if fails:
+            def stop(*_):
+                raise ValueError("on purpose")
+            handle = model.blocks[0].register_full_backward_hook(stop)
+            with pytest.raises(ValueError):
+                trainer.step(tok, tgt)
+            handle.remove()
+        trainer.step(tok, tgt)
+        torch.cuda.synchronize()
+        moments.append(trainer.m.clone())
+    assert ((moments[0] - moments[1]).norm() / moments[0].norm()).item() < 1e-2

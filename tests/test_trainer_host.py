@@ -14,3 +14,69 @@ def test_optimizer_launch_takes_its_cap(monkeypatch, ctas):
     monkeypatch.setattr(ops, "adamw_step", lambda *a, **k: seen.append(k.get("ctas_per_sm")))
     trainer._adamw(0, 64, ctas)
     assert seen == [ctas]
+
+
+class _Kept(torch.autograd.Function):
+    """Hands a product to a queue in backward, or fails."""
+
+    @staticmethod
+    def forward(ctx, x, queue, sink, fail):
+        ctx.queue, ctx.sink, ctx.fail = queue, sink, fail
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, dy):
+        if ctx.fail:
+            raise ValueError("on purpose")
+        ctx.queue(ctx.sink)
+        return dy, None, None, None
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    """The queues of weight gradients on the host: what they would launch."""
+    import contextlib
+    from mccl_b200.ops import native
+    seen = []
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: None)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(native._C, "gemm_group", lambda items, accumulate: seen.append([it[2] for it in items]))
+    monkeypatch.setattr(native._C, "decoder_layer_wgrads", lambda items, B, S, H: seen.append([it[0] for it in items]))
+    return seen
+
+
+def _single(sink):
+    from mccl_b200.ops import native
+    native._products.add(torch.zeros(8, 16), torch.zeros(8, 16), sink, torch.nn.Parameter(torch.zeros(16, 16)))
+
+
+def _layer(sink):
+    from mccl_b200.ops import native
+    params = tuple(torch.nn.Parameter(torch.zeros(4)) for _ in range(12))
+    native._deferred.add((sink, None, None, [torch.zeros(4)] * 12), (1, 8, 1), params, torch.device("cpu"))
+
+
+@pytest.mark.parametrize("queue", [_single, _layer])
+def test_a_failed_backward_leaves_nothing_for_the_next(launches, queue):
+    from mccl_b200.ops import native
+    x = torch.ones(3, requires_grad=True)
+    with pytest.raises(ValueError):
+        _Kept.apply(_Kept.apply(x, queue, "lost", True), queue, "stale", False).sum().backward()
+    _Kept.apply(_Kept.apply(x, queue, "a", False), queue, "b", False).sum().backward()
+    assert launches == [["b", "a"]]
+    native.join_wgrad()
+    assert launches == [["b", "a"]]
+    # a pass inside another one (activation checkpointing) keeps its own
+    class Inner(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x.clone()
+
+        @staticmethod
+        def backward(ctx, dy):
+            with torch.enable_grad():
+                _Kept.apply(torch.ones(3, requires_grad=True), queue, "inner", False).sum().backward()
+            return dy
+    launches.clear()
+    _Kept.apply(Inner.apply(_Kept.apply(x, queue, "first", False)), queue, "last", False).sum().backward()
+    assert launches == [["inner"], ["last", "first"]]
