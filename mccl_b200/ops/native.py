@@ -332,7 +332,9 @@ class _Entry:
 
 class _Shared:
     """Weight gradients that go straight into a trainer's buffers, kept back until several can share a launch.  Flushed at the end
-    of backward at the latest (by an engine callback), and before anybody looks at the gradients of a bucket.
+    of backward at the latest (by an engine callback), and before anybody looks at the gradients of a bucket.  Where peers wait
+    for them (`_grad_awaited`) none is kept back: a bucket's collective starts with its last gradient, and the gain was measured
+    on one GPU only.
 
     The callback owns the entry and this table only knows it: the engine drops its callbacks when a pass fails, and what
     was kept back goes with them instead of joining the next pass's products."""
@@ -357,6 +359,8 @@ class _Shared:
             entry.items.append(item)
             entry.params.append(params)
             entry.size += size
+        if any(getattr(p, "_grad_awaited", False) for p in params):
+            self._flush(entry)
         return entry
 
     def _flush(self, entry) -> None:

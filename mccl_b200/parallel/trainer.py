@@ -221,6 +221,7 @@ class DDPTrainer:
             if self._per_bucket:
                 # ... and say so; gradients that come back through autograd fire its hook instead
                 p._grad_ready = report(p)
+                p._grad_awaited = self.world > 1
                 if self.world > 1:
                     p.register_post_accumulate_grad_hook(self._on_autograd_grad)
         # bf16 working copies of the parameters, refreshed by the optimizer kernel (the GEMMs

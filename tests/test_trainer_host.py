@@ -45,14 +45,20 @@ def launches(monkeypatch):
     return seen
 
 
-def _single(sink):
-    from mccl_b200.ops import native
-    native._products.add(torch.zeros(8, 16), torch.zeros(8, 16), sink, torch.nn.Parameter(torch.zeros(16, 16)))
+def _param(awaited, *shape):
+    p = torch.nn.Parameter(torch.zeros(*shape))
+    p._grad_awaited = awaited
+    return p
 
 
-def _layer(sink):
+def _single(sink, awaited=False):
     from mccl_b200.ops import native
-    params = tuple(torch.nn.Parameter(torch.zeros(4)) for _ in range(12))
+    native._products.add(torch.zeros(8, 16), torch.zeros(8, 16), sink, _param(awaited, 16, 16))
+
+
+def _layer(sink, awaited=False):
+    from mccl_b200.ops import native
+    params = tuple(_param(awaited, 4) for _ in range(12))
     native._deferred.add((sink, None, None, [torch.zeros(4)] * 12), (1, 8, 1), params, torch.device("cpu"))
 
 
@@ -80,3 +86,27 @@ def test_a_failed_backward_leaves_nothing_for_the_next(launches, queue):
     launches.clear()
     _Kept.apply(Inner.apply(_Kept.apply(x, queue, "first", False)), queue, "last", False).sum().backward()
     assert launches == [["inner"], ["last", "first"]]
+
+
+@pytest.mark.parametrize("queue", [_single, _layer])
+def test_gradients_that_peers_wait_for_are_not_kept_back(launches, queue):
+    x = torch.ones(3, requires_grad=True)
+    for name in "abc":
+        x = _Kept.apply(x, lambda sink: queue(sink, True), name, False)
+    x.sum().backward()
+    assert launches == [["c"], ["b"], ["a"]]
+
+
+@pytest.mark.parametrize("world", [1, 2])
+def test_trainer_says_whether_peers_wait(monkeypatch, world):
+    import mccl_b200
+    from mccl_b200.models import build_decoder
+    from mccl_b200.parallel import DDPTrainer, trainer
+    backend = type("Backend", (), {"device_comm": lambda self, index: object()})()
+    monkeypatch.setattr(trainer.dist, "is_initialized", lambda: world > 1)
+    monkeypatch.setattr(trainer.dist, "get_world_size", lambda group=None: world)
+    monkeypatch.setattr(trainer.dist, "get_rank", lambda group=None: 0)
+    monkeypatch.setattr(mccl_b200, "get_backend", lambda group=None: backend)
+    monkeypatch.setattr(DDPTrainer, "_sync_initial_params", lambda self, group: None)
+    t = DDPTrainer(build_decoder("tiny"), torch.device("cpu"), use_graph=False)
+    assert all(getattr(p, "_grad_awaited", False) == (world > 1) for p in t.model.parameters())
