@@ -406,22 +406,28 @@ class _Products(_Shared):
     tokens and shares a launch with them (1024 x 1024 and 3072 x 1024 over 4096 tokens: two launches of 28 and 33 us beside the
     optimizer, one of 35)."""
 
-    SMALL = 37    # 256 x 256 tiles: half of what the GPU works on at a time
-    MOST = 64     # beyond that a product is better alone
+    @staticmethod
+    def limits():
+        """(tiles of 256 x 256 up to which a product waits: half of what the SMs that products may use work on at a time; tiles
+        beyond which one joins none that waits: seven eighths, 64 on 148 SMs)."""
+        sms, cap = _C.gemm_sm_count(), _C.gemm_cta_limit()
+        pairs = (min(sms, cap) if cap > 0 else sms) // 2
+        return pairs // 2, pairs * 7 // 8
 
     def add(self, dz, x2, sink, weight) -> None:
         device, tokens = dz.device, dz.shape[0]
         tiles = -(-dz.shape[1] // 256) * -(-x2.shape[1] // 256)
+        small, most = self.limits()
         entry = self._pending.get((device, torch._C._current_graph_task_id()))
         waiting = entry is not None and entry.items and entry.kind == tokens and entry.stream == torch.cuda.current_stream(device)
-        if tiles > (self.MOST if waiting else self.SMALL) or (not waiting and not dz.is_contiguous()):
+        if tiles > (most if waiting else small) or (not waiting and not dz.is_contiguous()):
             if entry is not None:
                 self._flush(entry)
             _wgrad_gemm(dz, x2, sink)
             _notify(weight)
             return
         entry = self._enter(device, tokens, (dz.contiguous(), x2, sink), (weight,), tiles)
-        if entry.size > self.SMALL or len(entry.items) >= 4:
+        if entry.size > small or len(entry.items) >= 4:
             self._flush(entry)
 
     def _launch(self, kind, items) -> None:

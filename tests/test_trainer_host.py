@@ -110,3 +110,23 @@ def test_trainer_says_whether_peers_wait(monkeypatch, world):
     monkeypatch.setattr(DDPTrainer, "_sync_initial_params", lambda self, group: None)
     t = DDPTrainer(build_decoder("tiny"), torch.device("cpu"), use_graph=False)
     assert all(getattr(p, "_grad_awaited", False) == (world > 1) for p in t.model.parameters())
+
+
+def test_products_wait_by_the_sms_they_may_use(launches, monkeypatch):
+    """Half of the tiles that the GPU works on at a time: on 148 SMs, on fewer, and with a cap on the CTAs of products."""
+    from mccl_b200.ops import native
+    alone = []
+    monkeypatch.setattr(native, "_wgrad_gemm", lambda dz, x2, sink: alone.append(sink))
+
+    def queue(sink):   # 4 x 5 tiles
+        native._products.add(torch.zeros(8, 1024), torch.zeros(8, 1280), sink, _param(False, 1024, 1280))
+    for sms, cap, waits in ((148, 0, True), (148, 88, True), (148, 78, False), (80, 0, True), (78, 0, False)):
+        monkeypatch.setattr(native._C, "gemm_sm_count", lambda: sms)
+        monkeypatch.setattr(native._C, "gemm_cta_limit", lambda: cap)
+        launches.clear()
+        alone.clear()
+        _Kept.apply(torch.ones(3, requires_grad=True), queue, "a", False).sum().backward()
+        assert (launches, alone) == (([["a"]], []) if waits else ([], ["a"])), (sms, cap)
+    monkeypatch.setattr(native._C, "gemm_sm_count", lambda: 148)
+    monkeypatch.setattr(native._C, "gemm_cta_limit", lambda: 0)
+    assert native._products.limits() == (37, 64)
