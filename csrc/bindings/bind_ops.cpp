@@ -361,7 +361,7 @@ void bind_ops(py::module_& m) {
         return std::make_pair(o, lse);
       },
       py::arg("qkv"), py::arg("scale"), "Causal attention; returns (o [B, S, H*hd] bf16, lse [B, H, S] fp32, log2 domain).  S <= 256 and head_dim <= 64 (a "
-      "multiple of 8), or head_dim 64 with S a multiple of 128.");
+      "multiple of 8).");
   m.def("attention_supported", [](int64_t seq, int64_t head_dim) {
     return seq < (1 << 30) && head_dim < (1 << 30) && ops::attention_supported(static_cast<int>(seq), static_cast<int>(head_dim));
   });

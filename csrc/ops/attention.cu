@@ -21,7 +21,7 @@
 //   under elect.sync, no online rescale, and one wait where the products allow it.
 //   A tile row past the sequence or a column past the head dimension is zero fill of the TMA load, so ragged sizes take
 //   the same path.
-// Longer sequences (forward, head dimension 64): one warpgroup per 128 queries, looping over key blocks with the online softmax.
+// Longer sequences and wider heads are the caller's business.
 //
 // The reference has no attention kernel (its models call PyTorch's); this one exists because attention and the
 // copies around it are a tenth of the headline training step.  Every wait is bounded: on a timeout the kernel sets
@@ -40,14 +40,6 @@ constexpr int kBlk = 128;       // queries per CTA block, keys per inner block
 constexpr int kHd = 64;         // head dimension
 constexpr int kTile = kBlk * kHd * 2;   // bytes of a [128 x 64] bf16 tile: 16 KiB
 
-struct AttnDev {
-  __nv_bfloat16* o;        // [B, S, H, 64]
-  float* lse;              // [B, H, S]  log2-domain log-sum-exp: m + log2(l)
-  int S, H;
-  float scale_log2;        // softmax scale * log2(e)
-  int* err;
-};
-
 // Byte offset of 16-byte chunk `c` (0..7) of row `r` inside a [rows x 64] bf16 tile stored the way a TMA load with
 // the 128-byte swizzle stores it: rows of 128 bytes, 8-row groups of 1024 bytes, chunk index XORed with the row.
 __device__ __forceinline__ uint32_t sw128_offset(int r, int c) {
@@ -63,205 +55,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
-
-// -------------------------------------------------- forward, long sequences --
-__global__ void __launch_bounds__(128) attn_fwd_long_kernel(const __grid_constant__ CUtensorMap tm_qkv, AttnDev a) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* sQ = smem;                       // 16 KiB
-  uint8_t* sK = sQ + kTile;                 // 16 KiB: K_j is dead once S_j is in tensor memory, so one buffer will do
-  uint8_t* sV = sK + kTile;                 // 2 x 16 KiB
-  uint8_t* sP = sV + 2 * kTile;             // 32 KiB: two [128 x 64] sub-tiles
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(sP + 2 * kTile);
-  uint64_t* k_full = q_full + 1;
-  uint64_t* v_full = k_full + 1;            // [2]
-  uint64_t* mma_bar = v_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_bar + 1);
-  volatile int* bad = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int nblk = a.S / kBlk;
-  const int qi = nblk - 1 - static_cast<int>(blockIdx.x);   // long rows first
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int HD = a.H * kHd;
-  if (tid == 0) {
-    tc::mbar_init(q_full, 1);
-    tc::mbar_init(k_full, 1);
-    tc::mbar_init(&v_full[0], 1);
-    tc::mbar_init(&v_full[1], 1);
-    tc::mbar_init(mma_bar, 1);
-    *bad = 0;
-    tc::mbar_init_fence();
-    tc::tma_prefetch_desc(&tm_qkv);
-  }
-  if (warp == 0) tc::tmem_alloc(tmem_slot, 256);
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-  const uint32_t tmem_s = *tmem_slot, tmem_o = tmem_s + 128;
-  const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-  pdl_wait();
-  pdl_trigger();
-
-  const int row0 = b * a.S;
-  auto load_k = [&](int j) {
-    tc::mbar_expect_tx(k_full, kTile);
-    tc::tma_load_2d(sK, &tm_qkv, k_full, HD + h * kHd, row0 + j * kBlk);
-  };
-  auto load_v = [&](int j) {
-    const int st = j & 1;
-    tc::mbar_expect_tx(&v_full[st], kTile);
-    tc::tma_load_2d(sV + st * kTile, &tm_qkv, &v_full[st], 2 * HD + h * kHd, row0 + j * kBlk);
-  };
-  if (tid == 0) {
-    tc::mbar_expect_tx(q_full, kTile);
-    tc::tma_load_2d(sQ, &tm_qkv, q_full, h * kHd, row0 + qi * kBlk);
-    load_k(0);
-    load_v(0);
-    if (qi >= 1) load_v(1);
-  }
-
-  float m_run = -INFINITY, l_run = 0.f;
-  float o_acc[kHd];
-#pragma unroll
-  for (int d = 0; d < kHd; ++d) o_acc[d] = 0.f;
-  uint32_t mma_phase = 0;
-  const int q_row = qi * kBlk + tid;   // this thread's query index inside the sequence
-  bool ok = true;
-
-  for (int j = 0; j <= qi && ok; ++j) {
-    const int st = j & 1;
-    if (tid == 0) {
-      bool w = true;
-      if (j == 0) w = tc::mbar_wait(q_full, 0);
-      w = w && tc::mbar_wait(k_full, j & 1);
-      if (!w) *bad = 1;
-      tc::fence_after_sync();
-      if (w) {
-        constexpr uint32_t idesc = tc::idesc_bf16(kBlk, kBlk, false, false);
-        const uint64_t da = tc::smem_desc_k_sw128(sQ), db = tc::smem_desc_k_sw128(sK);
-#pragma unroll
-        for (int k4 = 0; k4 < kHd / UMMA_K; ++k4) tc::mma_bf16(tmem_s, da + 2 * k4, db + 2 * k4, idesc, k4 != 0);
-      }
-      tc::mma_commit(mma_bar);   // also on the failure path: releases the waiters below
-    }
-    ok = tc::mbar_wait(mma_bar, mma_phase) && *bad == 0;
-    mma_phase ^= 1u;
-    tc::fence_after_sync();
-    if (!__syncthreads_and(ok ? 1 : 0)) {
-      ok = false;
-      break;
-    }
-    if (tid == 0 && j + 1 <= qi) load_k(j + 1);   // S_j is in tensor memory: the K buffer is free again
-    // pass 1: row maximum of the (masked) scores
-    const bool diag = j == qi;
-    float mx = -INFINITY;
-#pragma unroll 1
-    for (int c0 = 0; c0 < kBlk; c0 += 32) {
-      float s[32];
-      tmem_ld32(tmem_s + lane_base + static_cast<uint32_t>(c0), s);
-#pragma unroll
-      for (int e = 0; e < 32; ++e) {
-        const bool masked = diag && (j * kBlk + c0 + e > q_row);
-        mx = masked ? mx : fmaxf(mx, s[e]);
-      }
-    }
-    const float m_new = fmaxf(m_run, mx * a.scale_log2);
-    const float alpha = exp2f(m_run - m_new);   // 0 on the first block (m_run = -inf)
-    // pass 2: probabilities, their sum, and P as the A operand of the next product
-    float rs = 0.f;
-#pragma unroll 1
-    for (int c0 = 0; c0 < kBlk; c0 += 32) {
-      float s[32];
-      tmem_ld32(tmem_s + lane_base + static_cast<uint32_t>(c0), s);
-      uint8_t* sub = sP + (c0 >> 6) * kTile;
-#pragma unroll
-      for (int c8 = 0; c8 < 4; ++c8) {
-        uint4 pk;
-        __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-        for (int e2 = 0; e2 < 4; ++e2) {
-          float p[2];
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int e = c8 * 8 + e2 * 2 + q;
-            const bool masked = diag && (j * kBlk + c0 + e > q_row);
-            p[q] = masked ? 0.f : exp2f(s[e] * a.scale_log2 - m_new);
-          }
-          hp[e2] = __floats2bfloat162_rn(p[0], p[1]);
-          // the sum uses the rounded values: they are what multiplies V
-          const float2 back = __bfloat1622float2(hp[e2]);
-          rs += back.x + back.y;
-        }
-        *reinterpret_cast<uint4*>(sub + sw128_offset(tid, ((c0 & 63) >> 3) + c8)) = pk;
-      }
-    }
-    l_run = l_run * alpha + rs;
-    m_run = m_new;
-    fence_async_smem();          // the MMA reads P through the async proxy
-    tc::fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      const bool w = tc::mbar_wait(&v_full[st], (j >> 1) & 1);
-      if (!w) *bad = 1;
-      tc::fence_after_sync();
-      if (w) {
-        constexpr uint32_t idesc = tc::idesc_bf16(kBlk, kHd, false, true);
-        const uint64_t dv = tc::smem_desc_mn_sw128(sV + st * kTile, kTile);
-#pragma unroll
-        for (int kk = 0; kk < kBlk / UMMA_K; ++kk) {
-          const uint64_t dp = tc::smem_desc_k_sw128(sP + (kk >> 2) * kTile) + 2 * (kk & 3);
-          tc::mma_bf16(tmem_o, dp, dv + 128 * kk, idesc, kk != 0);
-        }
-      }
-      tc::mma_commit(mma_bar);
-    }
-    ok = tc::mbar_wait(mma_bar, mma_phase) && *bad == 0;
-    mma_phase ^= 1u;
-    tc::fence_after_sync();
-    if (!__syncthreads_and(ok ? 1 : 0)) {
-      ok = false;
-      break;
-    }
-    // this key block's contribution, folded into the running output
-#pragma unroll
-    for (int c0 = 0; c0 < kHd; c0 += 32) {
-      float t[32];
-      tmem_ld32(tmem_o + lane_base + static_cast<uint32_t>(c0), t);
-#pragma unroll
-      for (int e = 0; e < 32; ++e) o_acc[c0 + e] = o_acc[c0 + e] * alpha + t[e];
-    }
-    tc::fence_before_sync();
-    __syncthreads();   // everybody has read S and O: the stage and both accumulators may be reused
-    if (tid == 0 && j + 2 <= qi) load_v(j + 2);
-  }
-
-  if (ok) {
-    const float inv = 1.f / l_run;
-    __nv_bfloat16* orow = a.o + (static_cast<size_t>(row0 + q_row) * a.H + h) * kHd;
-#pragma unroll
-    for (int c8 = 0; c8 < kHd / 8; ++c8) {
-      uint4 pk;
-      __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-      for (int e2 = 0; e2 < 4; ++e2) hp[e2] = __floats2bfloat162_rn(o_acc[c8 * 8 + 2 * e2] * inv, o_acc[c8 * 8 + 2 * e2 + 1] * inv);
-      reinterpret_cast<uint4*>(orow)[c8] = pk;
-    }
-    a.lse[(static_cast<size_t>(b) * a.H + h) * a.S + q_row] = m_run + log2f(l_run);
-  } else if (tid == 0) {
-    atomicExch(a.err, 11);
-    // loads that were issued must land before the CTA retires
-    tc::mbar_wait(q_full, 0, 1u << 20);
-  }
-  tc::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) {
-    tc::fence_after_sync();
-    tc::tmem_dealloc(tmem_s, 256);
-  }
-}
-
-constexpr int kLongSmem = 6 * kTile + 64 + 1024;   // 97 KiB: two CTAs per SM
 
 // ------------------------------------------------- forward, up to 256 keys --
 struct AttnArgs {
@@ -820,43 +613,24 @@ cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, cons
 
 cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse, int B, int S, int H, int hd, float softmax_scale,
                           cudaStream_t stream) {
-  if (B <= 0 || H <= 0) return cudaErrorNotSupported;
+  if (!attention_supported(S, hd) || B <= 0 || H <= 0) return cudaErrorNotSupported;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(o)) & 15u) return cudaErrorNotSupported;
-  const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  int* err = gemm_error_device_ptr();
-  if (!err) return cudaErrorNotSupported;
-  CUtensorMap tm;
+  static std::atomic<bool> configured{false};
+  cudaError_t rc = allow_smem(attn_fwd_kernel, kFwdSmem, configured);
+  if (rc != cudaSuccess) return rc;
+  CUtensorMap tq, to;
+  if (!encode_slots(&tq, qkv, B, S, 3 * H, hd) || !encode_slots(&to, o, B, S, H, hd, 32)) return cudaErrorNotSupported;
   (void)cudaGetLastError();
-  if (attention_supported(S, hd)) {
-    static std::atomic<bool> configured{false};
-    cudaError_t rc = allow_smem(attn_fwd_kernel, kFwdSmem, configured);
-    if (rc != cudaSuccess) return rc;
-    CUtensorMap to;
-    if (!encode_slots(&tm, qkv, B, S, 3 * H, hd) || !encode_slots(&to, o, B, S, H, hd, 32)) return cudaErrorNotSupported;
-    AttnArgs a = {};
-    a.lse = lse;
-    a.S = S;
-    a.H = H;
-    a.hd = hd;
-    a.scale = softmax_scale;
-    a.scale_log2 = scale_log2;
-    a.err = err;
-    MCCL_LAUNCH_PDL(attn_fwd_kernel, dim3((S + kBlk - 1) / kBlk, H, B), 256, kFwdSmem, stream, tm, to, a);
-  } else {
-    if (hd != kHd || S <= 0 || S % kBlk != 0) return cudaErrorNotSupported;
-    static std::atomic<bool> configured{false};
-    cudaError_t rc = allow_smem(attn_fwd_long_kernel, kLongSmem, configured);
-    if (rc != cudaSuccess) return rc;
-    if (!encode_map(&tm, qkv, B * S, 3 * H * kHd, 3 * H * kHd, kBlk)) return cudaErrorNotSupported;
-    AttnDev a;
-    a.o = o;
-    a.lse = lse;
-    a.S = S;
-    a.H = H;
-    a.scale_log2 = scale_log2;
-    a.err = err;
-    MCCL_LAUNCH_PDL(attn_fwd_long_kernel, dim3(S / kBlk, H, B), 128, kLongSmem, stream, tm, a);
-  }
+  AttnArgs a = {};
+  a.lse = lse;
+  a.S = S;
+  a.H = H;
+  a.hd = hd;
+  a.scale = softmax_scale;
+  a.scale_log2 = softmax_scale * 1.4426950408889634f;
+  a.err = gemm_error_device_ptr();
+  if (!a.err) return cudaErrorNotSupported;
+  MCCL_LAUNCH_PDL(attn_fwd_kernel, dim3((S + kBlk - 1) / kBlk, H, B), 256, kFwdSmem, stream, tq, to, a);
   count_launch();
   return launch_status();
 }

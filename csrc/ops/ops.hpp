@@ -81,7 +81,7 @@ cudaError_t embed_bwd(const long long* ids, const __nv_bfloat16* dy, float* dtok
 
 // ---- causal self-attention straight from the fused QKV projection.
 // qkv: [B, S, 3, H, hd] bf16; o: [B, S, H, hd]; lse: [B, H, S] fp32 (log2 domain, saved for backward).
-// Both ways: S <= 256 and hd <= 64 (a multiple of 8); forward also head dimension 64 with S a multiple of 128.
+// Both ways: S <= 256 and hd <= 64 (a multiple of 8).
 // cudaErrorNotSupported otherwise: the caller falls back.
 bool attention_supported(int S, int hd);
 cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse, int B, int S, int H, int hd, float softmax_scale,

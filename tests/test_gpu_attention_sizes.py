@@ -37,3 +37,15 @@ def test_forward_backward_and_column_sums(B, S, H, D):
     assert ((sums - 1 - d.float().sum((0, 1)).view(-1)).abs().max() / d.float().abs().sum((0, 1)).max()).item() < 1e-2
     torch.cuda.synchronize()
     assert _C.gemm_error_flag() == 0
+
+
+@pytest.mark.parametrize("S,D", [(257, 64), (384, 64), (128, 72), (64, 4)])
+def test_other_sizes_are_refused(S, D):
+    """On the host, with an error; the operator takes PyTorch's attention for them."""
+    from mccl_b200 import _C
+    q5 = torch.zeros(1, S, 3, 1, D, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(Exception):
+        _C.attn_fwd(q5, 1.0)
+    with pytest.raises(Exception):
+        _C.attn_bwd(q5, torch.zeros(1, S, D, device="cuda", dtype=torch.bfloat16), torch.zeros(1, S, D, device="cuda", dtype=torch.bfloat16),
+                    torch.zeros(1, 1, S, device="cuda"), 1.0)
