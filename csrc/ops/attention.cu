@@ -30,6 +30,7 @@
 #include "gemm_common.cuh"
 
 #include <atomic>
+#include <climits>
 
 namespace mccl {
 namespace ops {
@@ -101,8 +102,10 @@ __global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant_
   volatile int* bad = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qi = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);   // long rows first
-  const int h = blockIdx.y, b = blockIdx.z, nblk = qi + 1, nk = nblk * kBlk;
+  // one grid dimension: the others end at 65535, which a batch of short sequences passes
+  const int last = a.S > kBlk ? 1 : 0, unit = static_cast<int>(blockIdx.x) >> last;
+  const int qi = last - (static_cast<int>(blockIdx.x) & last);   // long rows first
+  const int b = unit / a.H, h = unit - b * a.H, nblk = qi + 1, nk = nblk * kBlk;
   if (warp == 0 && tc::elect_one()) {
     tc::mbar_init(qk_full, 1);
     tc::mbar_init(v_full, 1);
@@ -309,7 +312,7 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nblk = (a.S + kBlk - 1) / kBlk;   // 1 or 2
-  const int h = blockIdx.x, b = blockIdx.y;
+  const int b = static_cast<int>(blockIdx.x) / a.H, h = static_cast<int>(blockIdx.x) - b * a.H;
   if (warp == 0 && tc::elect_one()) {
     tc::mbar_init(&in_full[0], 1);
     tc::mbar_init(&in_full[1], 1);
@@ -580,11 +583,12 @@ cudaError_t allow_smem(K kernel, int bytes, std::atomic<bool>& done) {
 
 }  // namespace
 
+static_assert(2 * kBlk == 256, "one or two blocks of queries");
 bool attention_supported(int S, int hd) { return S >= 1 && S <= 2 * kBlk && hd >= 8 && hd <= kHd && hd % 8 == 0; }
 
 cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, const __nv_bfloat16* d_o, const float* lse,
                           __nv_bfloat16* dqkv, float* colsum, int B, int S, int H, int hd, float softmax_scale, cudaStream_t stream) {
-  if (!attention_supported(S, hd) || B <= 0 || H <= 0) return cudaErrorNotSupported;
+  if (!attention_supported(S, hd) || B <= 0 || H <= 0 || static_cast<long long>(B) * H > INT_MAX) return cudaErrorNotSupported;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o) |
        reinterpret_cast<uintptr_t>(dqkv)) & 15u)
     return cudaErrorNotSupported;
@@ -606,14 +610,15 @@ cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, cons
   a.scale_log2 = softmax_scale * 1.4426950408889634f;
   a.err = gemm_error_device_ptr();
   if (!a.err) return cudaErrorNotSupported;
-  MCCL_LAUNCH_PDL(attn_bwd_kernel, dim3(H, B), 256, kBwdSmem, stream, tq, tdo, to, tdqkv, a);
+  MCCL_LAUNCH_PDL(attn_bwd_kernel, H * B, 256, kBwdSmem, stream, tq, tdo, to, tdqkv, a);
   count_launch();
   return launch_status();
 }
 
 cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse, int B, int S, int H, int hd, float softmax_scale,
                           cudaStream_t stream) {
-  if (!attention_supported(S, hd) || B <= 0 || H <= 0) return cudaErrorNotSupported;
+  const int blocks = (S + kBlk - 1) / kBlk;
+  if (!attention_supported(S, hd) || B <= 0 || H <= 0 || static_cast<long long>(B) * H * blocks > INT_MAX) return cudaErrorNotSupported;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(o)) & 15u) return cudaErrorNotSupported;
   static std::atomic<bool> configured{false};
   cudaError_t rc = allow_smem(attn_fwd_kernel, kFwdSmem, configured);
@@ -630,7 +635,7 @@ cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse
   a.scale_log2 = softmax_scale * 1.4426950408889634f;
   a.err = gemm_error_device_ptr();
   if (!a.err) return cudaErrorNotSupported;
-  MCCL_LAUNCH_PDL(attn_fwd_kernel, dim3((S + kBlk - 1) / kBlk, H, B), 256, kFwdSmem, stream, tq, to, a);
+  MCCL_LAUNCH_PDL(attn_fwd_kernel, blocks * H * B, 256, kFwdSmem, stream, tq, to, a);
   count_launch();
   return launch_status();
 }

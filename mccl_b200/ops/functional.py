@@ -65,7 +65,7 @@ def causal_attention(qkv: torch.Tensor, n_heads: int) -> torch.Tensor:
     B, S = qkv.shape[0], qkv.shape[1]
     hd = qkv.numel() // (B * S * 3 * n_heads)
     q5 = qkv.view(B, S, 3, n_heads, hd)
-    if qkv.is_cuda and qkv.dtype == torch.bfloat16 and native_attention_supported(S, hd):
+    if qkv.is_cuda and qkv.dtype == torch.bfloat16 and native_attention_supported(S, hd) and B * n_heads * 2 < 2 ** 31:
         from .native import CausalAttentionFn
         return CausalAttentionFn.apply(q5, 1.0 / (hd ** 0.5))
     q, k, v = (t.transpose(1, 2) for t in q5.unbind(2))

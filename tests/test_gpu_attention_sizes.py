@@ -10,7 +10,8 @@ def _rel(a, b):
 
 
 @pytest.mark.parametrize("B,S,H,D", [(1, 1, 1, 64), (2, 24, 4, 32), (3, 127, 2, 64), (2, 128, 3, 8), (2, 129, 2, 40), (8, 200, 8, 64),
-                                     (2, 255, 1, 56), (2, 256, 12, 64)])
+                                     (2, 255, 1, 56), (2, 256, 12, 64),
+                                     (65536, 2, 1, 8), (1, 3, 65537, 8), (65600, 129, 1, 8)])
 def test_forward_backward_and_column_sums(B, S, H, D):
     from mccl_b200 import _C, ops
     torch.manual_seed(S * 7 + D)
