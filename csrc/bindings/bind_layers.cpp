@@ -191,15 +191,16 @@ void bind_layers(py::module_& m) {
         check(ops::embed_fwd(reinterpret_cast<const long long*>(ids.data_ptr<int64_t>()), tok.data_ptr<float>(), pos.has_value() ? pos->data_ptr<float>() : nullptr,
                              bf(x), T, d.S, D, static_cast<int>(tok.size(0)), st),
               "embedding");
-        // few tokens: the down projections as sums, all layers' zeroed at once, which the norm behind each finishes
+        // few tokens: the down projections in parts, which the norm behind each adds
         const bool as_sums = L > 0 && down_as_sums(d);
-        const int64_t TD = static_cast<int64_t>(T) * D;
-        at::Tensor sums;
+        at::Tensor room;
+        Parts parts;
         if (as_sums) {
-          sums = at::empty({L, TD}, opt16.dtype(at::kFloat));
-          check(cudaMemsetAsync(sums.data_ptr(), 0, static_cast<size_t>(L * TD) * 4, st), "sums");
+          parts.slabs = ops::gemm_slabs(product_in_parts(bf(x), w16[3], nullptr, T, D, F));
+          room = at::empty({parts.slabs.count * parts.slabs.stride}, opt16.dtype(at::kFloat));
+          parts.at = room.data_ptr<float>();
         }
-        Unfinished before = {nullptr, nullptr, nullptr};
+        Unfinished before = {parts, nullptr, nullptr};
         at::Tensor kept;   // what `before` points into
         auto f32 = [&](int l, int p, int64_t n) {
           const at::Tensor& t = layers[l * per + p];
@@ -214,9 +215,8 @@ void bind_layers(py::module_& m) {
           for (int l = 0; l < L; ++l) {
             const Weights w = {f32(l, LN1_W, D), f32(l, LN1_B, D), f32(l, QKV_B, 3 * D), f32(l, PROJ_B, D), f32(l, LN2_W, D), f32(l, LN2_B, D),
                                f32(l, UP_B, F), f32(l, DOWN_B, D), w16[l * 4], w16[l * 4 + 1], w16[l * 4 + 2], w16[l * 4 + 3]};
-            float* to = as_sums ? sums.data_ptr<float>() + l * TD : nullptr;
-            layer_forward(bf(x), bf(x2), w, s, d, eps, false, st, to, as_sums && l > 0 ? &before : nullptr);
-            before = {to, w.down_b, s.y};
+            layer_forward(bf(x), bf(x2), w, s, d, eps, false, st, as_sums ? &parts : nullptr, as_sums && l > 0 ? &before : nullptr);
+            before = {parts, w.down_b, s.y};
             if (!as_sums) std::swap(x, x2);
           }
         } else {
@@ -228,7 +228,7 @@ void bind_layers(py::module_& m) {
           kept = y;
           const at::Tensor q = qk.select(2, 0).transpose(1, 2), k = qk.select(2, 1).transpose(1, 2), v = qkv.select(2, 2).transpose(1, 2);
           for (int l = 0; l < L; ++l) {
-            if (as_sums && l > 0) check(ops::norm_sum_fwd(before.sums, nullptr, before.residual, bf(x), f32(l, 0, D), nullptr, bf(h), T, D, eps, st), "first norm");
+            if (as_sums && l > 0) finish(before, bf(x), f32(l, 0, D), nullptr, bf(h), T, D, eps, st, "first norm");
             else check(ops::norm_fwd(bf(x), f32(l, 0, D), nullptr, bf(h), nullptr, nullptr, T, D, eps, st), "first norm");
             product(bf(h), w16[l * 4], nullptr, bf(qkv), T, 3 * D, D, nullptr, false, nullptr, st, "qkv projection");
             check(ops::rope_qk_fwd(bf(qkv), cos_t->data_ptr<float>(), sin_t->data_ptr<float>(), bf(qk), T, d.S, d.H, hd, st), "rotary embedding");
@@ -243,8 +243,8 @@ void bind_layers(py::module_& m) {
               check(ops::swiglu_fwd(bf(gu), bf(act), T, F, st), "activation");
             }
             if (as_sums) {
-              before = {sums.data_ptr<float>() + l * TD, nullptr, bf(y)};
-              product_sums(bf(act), w16[l * 4 + 3], sums.data_ptr<float>() + l * TD, T, D, F, st, "down projection");
+              before = {parts, nullptr, bf(y)};
+              check(ops::gemm_to_slabs(product_in_parts(bf(act), w16[l * 4 + 3], parts.at, T, D, F), parts.slabs, st), "down projection");
             } else {
               product(bf(act), w16[l * 4 + 3], nullptr, bf(x2), T, D, F, bf(y), false, nullptr, st, "down projection");
               std::swap(x, x2);
@@ -252,7 +252,7 @@ void bind_layers(py::module_& m) {
           }
         }
         const float* final_b = lnf_b.has_value() ? lnf_b->data_ptr<float>() : nullptr;
-        if (as_sums) check(ops::norm_sum_fwd(before.sums, before.bias, before.residual, bf(x), lnf_w.data_ptr<float>(), final_b, bf(x2), T, D, eps, st), "final norm");
+        if (as_sums) finish(before, bf(x), lnf_w.data_ptr<float>(), final_b, bf(x2), T, D, eps, st, "final norm");
         else check(ops::norm_fwd(bf(x), lnf_w.data_ptr<float>(), final_b, bf(x2), nullptr, nullptr, T, D, eps, st), "final norm");
         at::Tensor logits = at::empty({d.B, d.S, V}, opt16);
         product(bf(x2), w16[L * 4], nullptr, bf(logits), T, V, D, nullptr, false, nullptr, st, "head");

@@ -168,17 +168,20 @@ void bind_ops(py::module_& m) {
           g.alpha = alpha->data_ptr<float>();
         }
         // A contraction far longer than the output is wide (the input gradient of an LM head: 32000 against 512) has too few
-        // tiles for the SMs; its fp32 partial sums go through a workspace (4096 x 512 x 32000: 123 -> 108 us).
+        // tiles for the SMs; parts of it go through a workspace (4096 x 512 x 32000: 123 -> 108 us).
         at::Tensor partial;
-        if (!out_fp32 && !out.has_value() && g.epilogue == ops::EPI_NONE && !g.residual && !g.mul && !g.colsum && ops::gemm_wants_partial_sums(g)) {
-          partial = at::zeros({M, N}, a.options().dtype(at::kFloat));
+        ops::Slabs slabs{};
+        if (!out_fp32 && !out.has_value() && g.epilogue == ops::EPI_NONE && !g.residual && !g.mul && !g.colsum && !g.a_mn_major && ops::gemm_wants_slabs(g)) {
+          slabs = ops::gemm_slabs(g);
+          partial = at::empty({slabs.count * slabs.stride}, a.options().dtype(at::kFloat));
           g.d = partial.data_ptr();
-          g.d_fp32 = g.accumulate = true;
+          g.d_fp32 = true;
           g.ldd = static_cast<int>(N);
-          g.alpha = nullptr;   // the cast multiplies
+          g.alpha = nullptr;   // the sum multiplies
         }
-        cudaError_t rc = ops::gemm_bf16_tn(g, stream_of(a));
-        if (rc == cudaSuccess && partial.defined()) rc = ops::cast_f32_bf16(partial.data_ptr<float>(), bf(d), M * N, stream_of(a), alpha.has_value() ? alpha->data_ptr<float>() : nullptr);
+        cudaError_t rc = partial.defined() ? ops::gemm_to_slabs(g, slabs, stream_of(a)) : ops::gemm_bf16_tn(g, stream_of(a));
+        if (rc == cudaSuccess && partial.defined())
+          rc = ops::sum_slabs_bf16(partial.data_ptr<float>(), slabs.count, slabs.stride, bf(d), M * N, alpha.has_value() ? alpha->data_ptr<float>() : nullptr, stream_of(a));
         MCCL_CHECK_T(rc == cudaSuccess, CudaError,
                      "gemm_bf16 [" << M << "x" << N << "x" << K << ", lda " << g.lda << ", ldb " << g.ldb << ", ldd " << g.ldd
                                    << "] failed: " << cudaGetErrorString(rc) << " " << ops::gemm_last_reason());

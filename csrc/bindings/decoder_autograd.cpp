@@ -153,12 +153,13 @@ struct CrossEntropyNode : torch::autograd::Function<CrossEntropyNode> {
     g.m = T;
     g.n = g.ldb = g.ldd = D;
     g.k = g.lda = V;
-    if (ops::gemm_wants_partial_sums(g)) {
-      at::Tensor partial = zeros_f32(static_cast<int64_t>(T) * D, head);
-      g.d_fp32 = g.accumulate = true;
-      g.d = partial.data_ptr();
-      check(ops::gemm_bf16_tn(g, st), "head backward");
-      check(ops::cast_f32_bf16(partial.data_ptr<float>(), bf(dh), static_cast<long long>(T) * D, st, upstream.data_ptr<float>()), "head backward");
+    if (ops::gemm_wants_slabs(g)) {
+      g.d_fp32 = true;
+      const ops::Slabs slabs = ops::gemm_slabs(g);
+      at::Tensor parts = at::empty({slabs.count * slabs.stride}, head.options());
+      g.d = parts.data_ptr();
+      check(ops::gemm_to_slabs(g, slabs, st), "head backward");
+      check(ops::sum_slabs_bf16(parts.data_ptr<float>(), slabs.count, slabs.stride, bf(dh), static_cast<long long>(T) * D, upstream.data_ptr<float>(), st), "head backward");
     } else {
       g.alpha = upstream.data_ptr<float>();
       check(ops::gemm_bf16_tn(g, st), "head backward");

@@ -172,40 +172,49 @@ inline void weight_gradients(const std::vector<Pending>& layers, const Dims& d, 
   check(ops::gemm_group(args.data(), static_cast<int>(args.size()), stream), "weight gradients");
 }
 
-// Whether the down projection of these sizes is better left as fp32 sums for the norm behind it: a single row of tiles that fills a
+// Whether the down projection of these sizes is better left in parts, which the norm behind it adds: a single row of tiles that fills a
 // quarter of the GPU at most, with a contraction long enough to share out.
 inline bool down_as_sums(const Dims& d) { return d.tokens() <= 128 && d.D <= 2048 && d.D % 8 == 0 && d.D / 64 * 4 <= ops::gemm_sm_count() && d.F >= 1024 && d.F >= d.D; }
-// sums[M, N] += x[M, K] · w[N, K]^T
-inline void product_sums(const bf16* x, const bf16* w, float* sums, int M, int N, int K, cudaStream_t stream, const char* what) {
+// x[M, K] · w[N, K]^T, to be left in parts
+inline ops::GemmArgs product_in_parts(const bf16* x, const bf16* w, float* parts, int M, int N, int K) {
   ops::GemmArgs g;
   g.a = x;
   g.b = w;
-  g.d = sums;
-  g.d_fp32 = g.accumulate = true;
+  g.d = parts;
+  g.d_fp32 = true;
   g.m = M;
   g.n = g.ldd = N;
   g.k = g.lda = g.ldb = K;
-  check(ops::gemm_bf16_tn(g, stream), what);
+  return g;
 }
+// Room for the parts of a layer's down projection: one, every layer's next norm has read it before it is written again.
+struct Parts {
+  float* at = nullptr;
+  ops::Slabs slabs{};
+};
 // What the layer before left for this one's first norm to finish, in place of x.
 struct Unfinished {
-  const float *sums, *bias;
+  Parts parts;
+  const float* bias;
   const bf16* residual;
 };
+inline void finish(const Unfinished& u, bf16* x, const float* w, const float* b, bf16* y, int rows, int dim, float eps, cudaStream_t st, const char* what) {
+  check(ops::norm_sum_fwd(u.parts.at, u.parts.slabs.count, u.parts.slabs.stride, u.bias, u.residual, x, w, b, y, rows, dim, eps, st), what);
+}
 
-// With `sums` the down projection is left there (zeros before) instead of in `out`; with `before` x is written here.
-inline void layer_forward(bf16* x, bf16* out, const Weights& w, const Slab& s, const Dims& d, float eps, bool keep, cudaStream_t st, float* sums = nullptr,
+// With `parts` the down projection is left there instead of in `out`; with `before` x is written here.
+inline void layer_forward(bf16* x, bf16* out, const Weights& w, const Slab& s, const Dims& d, float eps, bool keep, cudaStream_t st, const Parts* parts = nullptr,
                           const Unfinished* before = nullptr) {
   const int T = d.tokens(), D = d.D, F = d.F;
   const float scale = 1.f / std::sqrt(static_cast<float>(d.head_dim()));
-  if (before) check(ops::norm_sum_fwd(before->sums, before->bias, before->residual, x, w.ln1_w, w.ln1_b, s.h1, T, D, eps, st), "first norm");
+  if (before) finish(*before, x, w.ln1_w, w.ln1_b, s.h1, T, D, eps, st, "first norm");
   else check(ops::norm_fwd(x, w.ln1_w, w.ln1_b, s.h1, keep ? s.mean1 : nullptr, keep ? s.rstd1 : nullptr, T, D, eps, st), "first norm");
   product(s.h1, w.qkv, w.qkv_b, s.qkv, T, 3 * D, D, nullptr, false, nullptr, st, "qkv projection");
   check(ops::attention_fwd(s.qkv, s.o, s.lse, d.B, d.S, d.H, d.head_dim(), scale, st), "attention");
   product(s.o, w.proj, w.proj_b, s.y, T, D, D, x, false, nullptr, st, "output projection");
   check(ops::norm_fwd(s.y, w.ln2_w, w.ln2_b, s.h2, keep ? s.mean2 : nullptr, keep ? s.rstd2 : nullptr, T, D, eps, st), "second norm");
   product(s.h2, w.up, w.up_b, s.act, T, F, D, nullptr, true, keep ? s.gelu_grad : nullptr, st, "up projection");
-  if (sums) product_sums(s.act, w.down, sums, T, D, F, st, "down projection");
+  if (parts) check(ops::gemm_to_slabs(product_in_parts(s.act, w.down, parts->at, T, D, F), parts->slabs, st), "down projection");
   else product(s.act, w.down, w.down_b, out, T, D, F, s.y, false, nullptr, st, "down projection");
 }
 

@@ -114,56 +114,85 @@ __global__ void __launch_bounds__(256) norm_fwd_rows_kernel(const __nv_bfloat16*
   }
 }
 
-// x = bf16(sum + bias + residual), y = norm(x): the norm behind a product that was left as fp32 sums, one warp per row.  For a few
-// tokens, where a launch is nothing but latency: a 37 x 512 x 2048 product is eight tiles with 32 k-blocks each, 9.9 us; as
-// 64 pieces that add up in memory it takes 5, and this kernel no longer than the norm that would be here anyway (2.5).
-template <bool kLayerNorm, int kVecs>
-__global__ void __launch_bounds__(128) norm_sum_kernel(const float* __restrict__ sum, const float* __restrict__ bias, const __nv_bfloat16* __restrict__ residual,
-                                                       __nv_bfloat16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b,
-                                                       __nv_bfloat16* __restrict__ y, int rows, int dim, float eps) {
+// x = bf16(sum + bias + residual), y = norm(x): the norm behind a product that was left in parts.  For a few tokens, where a launch is
+// nothing but latency: a 37 x 512 x 2048 product is eight tiles with 32 k-blocks each, 9.9 us; as 64 pieces it takes 5, and this
+// kernel little longer than the norm that would be here anyway.  A CTA per row and eight columns per thread, so that the parts are
+// spread over as many SMs as there are rows and all of a thread's loads are in flight at once; added in order.  (A warp per
+// row, four rows per CTA: 1.8 us more a launch at 37 rows of 512, the forward of 16 layers 569.5 us against 539.0; parts that
+// add up in memory instead, which needs a memset and repeats only to rounding: 559.0.)
+template <bool kLayerNorm>
+__global__ void __launch_bounds__(256) norm_sum_kernel(const float* __restrict__ sum, int parts, long long stride, const float* __restrict__ bias,
+                                                       const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ x,
+                                                       const float* __restrict__ w, const float* __restrict__ b, __nv_bfloat16* __restrict__ y,
+                                                       int dim, float eps) {
   ::mccl::pdl_wait();
   ::mccl::pdl_trigger();
-  const int lane = threadIdx.x & 31, vecs = dim >> 3, row = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const size_t first = static_cast<size_t>(row) * vecs + lane;
-  float f[kVecs][8], total = 0.f, sq = 0.f;
+  __shared__ float s_red[2][8];
+  const int vec = threadIdx.x, vecs = dim >> 3, warps = static_cast<int>(blockDim.x) >> 5;
+  const bool mine = vec < vecs;
+  const size_t at = static_cast<size_t>(blockIdx.x) * vecs + vec;
+  float v[8], ww[8], bb[8], cc[8];
+  uint4 res = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-  for (int k = 0; k < kVecs; ++k)
-    if (lane + 32 * k < vecs) {
-      const float4* s = reinterpret_cast<const float4*>(sum) + 2 * (first + 32 * k);
-      const float4 s0 = __ldg(s), s1 = __ldg(s + 1);
-      float r[8], v[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-      unpack8(__ldg(reinterpret_cast<const uint4*>(residual) + first + 32 * k), r);
-      if (bias != nullptr) {
-        const float4* c = reinterpret_cast<const float4*>(bias) + 2 * (lane + 32 * k);
-        const float4 c0 = __ldg(c), c1 = __ldg(c + 1);
-        v[0] += c0.x, v[1] += c0.y, v[2] += c0.z, v[3] += c0.w, v[4] += c1.x, v[5] += c1.y, v[6] += c1.z, v[7] += c1.w;
-      }
+  for (int i = 0; i < 8; ++i) v[i] = ww[i] = bb[i] = cc[i] = 0.f;
+  auto load8 = [&](const float* from, float (&to)[8]) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(from) + 2 * vec), c = __ldg(reinterpret_cast<const float4*>(from) + 2 * vec + 1);
+    to[0] = a.x; to[1] = a.y; to[2] = a.z; to[3] = a.w; to[4] = c.x; to[5] = c.y; to[6] = c.z; to[7] = c.w;
+  };
+  if (mine) {
+    res = __ldg(reinterpret_cast<const uint4*>(residual) + at);
+    if (bias != nullptr) load8(bias, cc);
+    load8(w, ww);
+    if (kLayerNorm) load8(b, bb);
+    constexpr int kAhead = 8;
+    for (int p = 0; p < parts; p += kAhead) {
+      float4 t[kAhead][2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] += r[i];
-      const uint4 packed = pack8(v);
-      reinterpret_cast<uint4*>(x)[first + 32 * k] = packed;
-      unpack8(packed, f[k]);
+      for (int a = 0; a < kAhead; ++a)
+        if (p + a < parts) {
+          const float4* s = reinterpret_cast<const float4*>(sum + (p + a) * stride) + 2 * at;
+          t[a][0] = __ldg(s);
+          t[a][1] = __ldg(s + 1);
+        }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) total += f[k][i];
+      for (int a = 0; a < kAhead; ++a)
+        if (p + a < parts) {
+          v[0] += t[a][0].x; v[1] += t[a][0].y; v[2] += t[a][0].z; v[3] += t[a][0].w;
+          v[4] += t[a][1].x; v[5] += t[a][1].y; v[6] += t[a][1].z; v[7] += t[a][1].w;
+        }
     }
-  const float mean = kLayerNorm ? warp_sum(total) / dim : 0.f;
+    float r[8];
+    unpack8(res, r);
 #pragma unroll
-  for (int k = 0; k < kVecs; ++k)
-    if (lane + 32 * k < vecs) {
+    for (int i = 0; i < 8; ++i) v[i] = v[i] + cc[i] + r[i];
+    const uint4 packed = pack8(v);
+    reinterpret_cast<uint4*>(x)[at] = packed;
+    unpack8(packed, v);
+  }
+  auto block_sum = [&](float part, int set) {
+    part = warp_sum(part);
+    if ((threadIdx.x & 31) == 0) s_red[set][threadIdx.x >> 5] = part;
+    __syncthreads();
+    float all = 0.f;
+    for (int i = 0; i < warps; ++i) all += s_red[set][i];
+    return all;
+  };
+  float mean = 0.f, sq = 0.f;
+  if (kLayerNorm) {
+    float total = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) sq += (f[k][i] - mean) * (f[k][i] - mean);
-    }
-  const float rstd = rsqrtf(warp_sum(sq) / dim + eps);
+    for (int i = 0; i < 8; ++i) total += v[i];
+    mean = block_sum(mine ? total : 0.f, 0) / dim;
+  }
 #pragma unroll
-  for (int k = 0; k < kVecs; ++k)
-    if (lane + 32 * k < vecs) {
-      const int c = 8 * (lane + 32 * k);
-      float o[8];
+  for (int i = 0; i < 8; ++i) sq += (v[i] - mean) * (v[i] - mean);
+  const float rstd = rsqrtf(block_sum(mine ? sq : 0.f, 1) / dim + eps);
+  if (mine) {
+    float o[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = (f[k][i] - mean) * rstd * __ldg(w + c + i) + (kLayerNorm ? __ldg(b + c + i) : 0.f);
-      reinterpret_cast<uint4*>(y)[first + 32 * k] = pack8(o);
-    }
+    for (int i = 0; i < 8; ++i) o[i] = (v[i] - mean) * rstd * ww[i] + bb[i];
+    reinterpret_cast<uint4*>(y)[at] = pack8(o);
+  }
 }
 
 // Rows of any length: three passes over the row, the second and third from cache.
@@ -517,16 +546,12 @@ cudaError_t norm_fwd(const __nv_bfloat16* x, const float* w, const float* b, __n
   return ::mccl::launch_status();
 }
 
-cudaError_t norm_sum_fwd(const float* sum, const float* bias, const __nv_bfloat16* residual, __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y,
+cudaError_t norm_sum_fwd(const float* sum, int parts, long long stride, const float* bias, const __nv_bfloat16* residual, __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y,
                          int rows, int dim, float eps, cudaStream_t stream) {
-  if (dim % 8 != 0 || dim > 2048) return cudaErrorNotSupported;
-  const int vecs = (dim + 255) / 256, blocks = (rows + 3) / 4;
-#define MCCL_NORM_SUM(LN, V) MCCL_LAUNCH_PDL((norm_sum_kernel<LN, V>), blocks, 128, 0, stream, sum, bias, residual, x, w, b, y, rows, dim, eps)
-#define MCCL_NORM_SUM_V(LN) (vecs == 1 ? MCCL_NORM_SUM(LN, 1) : vecs == 2 ? MCCL_NORM_SUM(LN, 2) : vecs <= 4 ? MCCL_NORM_SUM(LN, 4) : MCCL_NORM_SUM(LN, 8))
-  if (b) MCCL_NORM_SUM_V(true);
-  else MCCL_NORM_SUM_V(false);
-#undef MCCL_NORM_SUM_V
-#undef MCCL_NORM_SUM
+  if (dim % 8 != 0 || dim > 2048 || parts < 1 || stride % 4 != 0) return cudaErrorNotSupported;
+  const int threads = (dim + 255) / 256 * 32;
+  if (b) MCCL_LAUNCH_PDL(norm_sum_kernel<true>, rows, threads, 0, stream, sum, parts, stride, bias, residual, x, w, b, y, dim, eps);
+  else MCCL_LAUNCH_PDL(norm_sum_kernel<false>, rows, threads, 0, stream, sum, parts, stride, bias, residual, x, w, b, y, dim, eps);
   count_launch();
   return ::mccl::launch_status();
 }
@@ -859,33 +884,64 @@ cudaError_t transpose_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, int rows
 }
 
 // ------------------------------------------------------------------ casts --
-__global__ void __launch_bounds__(256) cast_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n,
-                                                   const float* __restrict__ alpha) {
+__global__ void __launch_bounds__(256) cast_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n) {
   // dependent launch: the CTA may be resident before the previous kernel of the stream has finished
   ::mccl::pdl_wait();
   ::mccl::pdl_trigger();
-  const float s = alpha != nullptr ? __ldg(alpha) : 1.f;
   const long long n4 = n / 4;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const float4 f = reinterpret_cast<const float4*>(in)[i];
-    __nv_bfloat162 lo = __floats2bfloat162_rn(f.x * s, f.y * s), hi = __floats2bfloat162_rn(f.z * s, f.w * s);
+    __nv_bfloat162 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
     uint2 packed;
     packed.x = *reinterpret_cast<uint32_t*>(&lo);
     packed.y = *reinterpret_cast<uint32_t*>(&hi);
     reinterpret_cast<uint2*>(out)[i] = packed;
   }
   if (blockIdx.x == 0)
-    for (long long i = n4 * 4 + threadIdx.x; i < n; i += blockDim.x) out[i] = __float2bfloat16_rn(in[i] * s);
+    for (long long i = n4 * 4 + threadIdx.x; i < n; i += blockDim.x) out[i] = __float2bfloat16_rn(in[i]);
 }
 
-cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t stream, const float* alpha) {
+cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
   if ((reinterpret_cast<uintptr_t>(in) & 15u) || (reinterpret_cast<uintptr_t>(out) & 7u)) return cudaErrorNotSupported;
   long long blocks = (n / 4 + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
   if (blocks < 1) blocks = 1;
-  MCCL_LAUNCH_PDL(cast_kernel, static_cast<int>(blocks), 256, 0, stream, in, out, n, alpha);
+  MCCL_LAUNCH_PDL(cast_kernel, static_cast<int>(blocks), 256, 0, stream, in, out, n);
+  count_launch();
+  return ::mccl::launch_status();
+}
+
+// A product that was left in parts: 16 bytes of every part in flight per thread, added in order.
+__global__ void __launch_bounds__(256) sum_slabs_kernel(const float* __restrict__ in, int parts, long long stride, __nv_bfloat16* __restrict__ out,
+                                                        long long n, const float* __restrict__ alpha) {
+  ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
+  const float s = alpha != nullptr ? __ldg(alpha) : 1.f;
+  const long long n4 = n / 4;
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4; i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const float* p = in + 4 * i;
+    float4 f = __ldg(reinterpret_cast<const float4*>(p));
+#pragma unroll 4
+    for (int k = 1; k < parts; ++k) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(p + k * stride));
+      f.x += t.x; f.y += t.y; f.z += t.z; f.w += t.w;
+    }
+    __nv_bfloat162 lo = __floats2bfloat162_rn(f.x * s, f.y * s), hi = __floats2bfloat162_rn(f.z * s, f.w * s);
+    uint2 packed;
+    packed.x = *reinterpret_cast<uint32_t*>(&lo);
+    packed.y = *reinterpret_cast<uint32_t*>(&hi);
+    reinterpret_cast<uint2*>(out)[i] = packed;
+  }
+}
+
+cudaError_t sum_slabs_bf16(const float* in, int parts, long long stride, __nv_bfloat16* out, long long n, const float* alpha, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  if (parts < 1 || n % 4 != 0 || stride % 4 != 0 || (reinterpret_cast<uintptr_t>(in) & 15u) || (reinterpret_cast<uintptr_t>(out) & 7u)) return cudaErrorNotSupported;
+  long long blocks = (n / 4 + 255) / 256;
+  if (blocks > 148 * 8) blocks = 148 * 8;
+  MCCL_LAUNCH_PDL(sum_slabs_kernel, static_cast<int>(blocks), 256, 0, stream, in, parts, stride, out, n, alpha);
   count_launch();
   return ::mccl::launch_status();
 }

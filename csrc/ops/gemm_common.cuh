@@ -29,6 +29,7 @@ struct GemmDev {
   int d_fp32;
   int accumulate;
   int epilogue;
+  int slab_rows = 0;   // rows between the slabs of a product that is left in parts
   int atomic_add;  // fp32 output accumulated with red.global.add (split-K partial sums)
   int* err;  // device word set non-zero when a pipeline wait runs out
   TimelineBuf* tl;  // device timeline, or nullptr (off)

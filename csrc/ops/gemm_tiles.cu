@@ -20,6 +20,8 @@ MCCL_TILES_EXTERN_PAIR(false, false, OUT_F32, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16_SUM, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16_SCALED, 1)
+MCCL_TILES_EXTERN_PAIR(false, false, OUT_F32_SLABS, 1)
+MCCL_TILES_EXTERN_PAIR(false, true, OUT_F32_SLABS, 1)
 MCCL_TILES_EXTERN_PAIR(true, true, OUT_F32_SCALED, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_F32, 1)
 MCCL_TILES_EXTERN_PAIR(true, false, OUT_BF16, 1)
@@ -62,7 +64,7 @@ double cost(int bn, int tiles, int k, int workers, int splits, bool gelu, bool a
   return 3500 + (kind == 3 ? 2000 : 0) + (rounds - 1) * round + main_loop + epilogue;
 }
 
-Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, bool gelu, bool splittable) {
+Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, bool gelu, bool splittable, bool slabs = false) {
   Plan best;
   double best_cost = 0;
   const int k = args[0].k;
@@ -75,7 +77,7 @@ Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, boo
     int tiles = 0;
     for (int p = 0; p < count; ++p) tiles += ceil_div(args[p].m, bn == 256 ? 256 : 128) * ceil_div(args[p].n, bn);
     const int num_kb = ceil_div(k, 64);
-    if (splittable && operand_bytes < kRunsBytes && static_cast<long long>(tiles) * num_kb >= 8ll * workers) {
+    if (splittable && !slabs && operand_bytes < kRunsBytes && static_cast<long long>(tiles) * num_kb >= 8ll * workers) {
       // Equal runs of k-blocks for every worker: no last round that leaves SMs idle, at the price of up to two more partial
       // tiles per worker.  Workers are then at different places of K, so operands that do not stay in L2 are read several
       // times (the 262 MB of an LM head's gradient: 4096 x 512 x 32000 131 us against 123).
@@ -103,6 +105,9 @@ Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, boo
 }
 
 template <bool kAMn, bool kBMn, int kOut, int kMax = 1>
+cudaError_t run_plan(const GemmArgs* a, int count, const Plan& plan, cudaStream_t stream);
+
+template <bool kAMn, bool kBMn, int kOut, int kMax = 1>
 cudaError_t run(const GemmArgs* a, int count, int forced, cudaStream_t stream) {
   int sms = gemm_sm_count(), pairs = 0;
   if constexpr (kOut != OUT_GELU) pairs = max_pairs<256, kAMn, kBMn, kOut, kMax>();
@@ -113,7 +118,11 @@ cudaError_t run(const GemmArgs* a, int count, int forced, cudaStream_t stream) {
   }
   bool splittable = fp32_out(kOut);
   for (int p = 0; p < count; ++p) splittable = splittable && (a[p].accumulate || a[p].ldd == a[p].n);
-  const Plan plan = choose(a, count, forced, sms, pairs, kOut == OUT_GELU, splittable);
+  return run_plan<kAMn, kBMn, kOut, kMax>(a, count, choose(a, count, forced, sms, pairs, kOut == OUT_GELU, splittable), stream);
+}
+
+template <bool kAMn, bool kBMn, int kOut, int kMax>
+cudaError_t run_plan(const GemmArgs* a, int count, const Plan& plan, cudaStream_t stream) {
   if (plan.bn == 64) return launch_tiles<64, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
   if constexpr (kOut != OUT_GELU)
     if (plan.bn == 192) return launch_tiles<192, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
@@ -154,9 +163,40 @@ cudaError_t launch_gemm_tiles(const GemmArgs& a, int forced_bn, cudaStream_t str
 }
 
 // Measured on an LM head's input gradient (K 32000): 32 pair tiles (4096 x 512) 108 against 123 us, 48 (4096 x 768) 145 against
-// 152; with 64 tiles (4096 x 1024, K 8192) the zeroing, adding and casting cost more than the idle SMs, 67 against 43.
-bool gemm_wants_partial_sums(const GemmArgs& a) {
+// 152; with 64 tiles (4096 x 1024, K 8192) writing, adding and casting the parts cost more than the idle SMs, 67 against 43.
+bool gemm_wants_slabs(const GemmArgs& a) {
   return a.k >= 4096 && tiles::ceil_div(a.m, 256) * tiles::ceil_div(a.n, 256) * 10 <= gemm_sm_count() / 2 * 7;
+}
+
+namespace {
+tiles::Plan slab_plan(const GemmArgs& a) {
+  int sms = gemm_sm_count();
+  int pairs = a.b_mn_major ? tiles::max_pairs<256, false, true, tiles::OUT_F32_SLABS, 1>() : tiles::max_pairs<256, false, false, tiles::OUT_F32_SLABS, 1>();
+  const int limit = gemm_cta_limit();
+  if (limit > 0) {
+    sms = limit < sms ? limit : sms;
+    pairs = limit / 2 < pairs ? limit / 2 : pairs;
+  }
+  return tiles::choose(&a, 1, 0, sms, pairs, false, true, true);
+}
+}  // namespace
+
+Slabs gemm_slabs(const GemmArgs& a) {
+  const int rows = (a.m + 31) / 32 * 32;
+  return {slab_plan(a).splits, static_cast<long long>(rows) * a.n};
+}
+
+cudaError_t gemm_to_slabs(const GemmArgs& a, const Slabs& s, cudaStream_t stream) {
+  if (a.m <= 0 || a.n <= 0 || a.k <= 0 || a.a_mn_major || a.bias || a.residual || a.mul || a.colsum || a.alpha || a.accumulate || !a.d_fp32 ||
+      a.epilogue != EPI_NONE || a.ldd != a.n || s.count < 1 || s.count > tiles::ceil_div(a.k, BK))
+    return cudaErrorInvalidValue;
+  if (a.n % 8 != 0 || a.lda % 8 != 0 || a.ldb % 8 != 0 ||
+      ((reinterpret_cast<uintptr_t>(a.a) | reinterpret_cast<uintptr_t>(a.b) | reinterpret_cast<uintptr_t>(a.d)) & 15u))
+    return cudaErrorNotSupported;
+  const tiles::Plan plan = slab_plan(a);
+  if (plan.splits != s.count) return cudaErrorInvalidValue;   // the cap on the CTAs was moved in between
+  (void)cudaGetLastError();
+  return a.b_mn_major ? tiles::run_plan<false, true, tiles::OUT_F32_SLABS>(&a, 1, plan, stream) : tiles::run_plan<false, false, tiles::OUT_F32_SLABS>(&a, 1, plan, stream);
 }
 
 namespace {

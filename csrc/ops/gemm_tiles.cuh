@@ -40,6 +40,9 @@ namespace tiles {
 // OUT_BF16_SCALED, OUT_F32_SCALED: times the scalar at GemmDev::alpha (the upstream gradient of a loss).  Instantiations of their own: the
 // multiplications in the other epilogues, even where they were skipped, cost 2 us of a 134 us training step (instruction
 // fetch, and fewer loads in flight).
+// OUT_F32_SLABS: every part of K into a slab of its own (GemmDev::slab_rows rows further down in D), for a reader that adds the slabs in
+// order.  Partial sums that are added in memory arrive in any order, and a forward pass or an input gradient that went that way
+// no longer repeated bit for bit.
 // OUT_BF16_SUM: the bf16 output and, added into GemmDev::colsum, its column sums (a bias gradient).
 // OUT_SWIGLU (pair tile only): B is [gate | up], 2 n rows; the even CTA brings 128 rows of gate and the odd one the same 128 of up,
 // so that a tile's accumulator holds both factors of 128 outputs and silu(gate) * up is the epilogue.  The [m, 2 n] product
@@ -48,8 +51,8 @@ namespace tiles {
 // OUT_SWIGLU_GRAD (pair tile only): the input gradient of the product behind the activation, turned into the gradient of
 // [gate | up] (D, [m, 2 n]) with the saved [gate | up] (`aux`) on its way out; the [m, n] tensor between the two is neither
 // written nor read.
-enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3, OUT_SWIGLU = 4, OUT_SWIGLU_GRAD = 5, OUT_BF16_SCALED = 6, OUT_F32_SCALED = 7 };
-constexpr bool fp32_out(int out) { return out == OUT_F32 || out == OUT_F32_SCALED; }
+enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3, OUT_SWIGLU = 4, OUT_SWIGLU_GRAD = 5, OUT_BF16_SCALED = 6, OUT_F32_SCALED = 7, OUT_F32_SLABS = 8 };
+constexpr bool fp32_out(int out) { return out == OUT_F32 || out == OUT_F32_SCALED || out == OUT_F32_SLABS; }
 constexpr bool half_boxes(int out) { return out == OUT_GELU || out == OUT_SWIGLU || out == OUT_SWIGLU_GRAD; }   // 32-column output boxes
 
 // One product, or several with the same K whose tiles one launch works through (the weight gradients of one or more layers:
@@ -223,7 +226,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
   // splits >= 1: work items are (tile, part of K), taken in turn.  splits == 0: every worker gets an equal run of k-blocks,
   // across tile borders, and adds what it has of each tile into D.
   const int tiles = P.first[P.count];
-  const bool runs = kF32 && splits == 0;
+  const bool runs = kF32 && kOut != OUT_F32_SLABS && splits == 0;
   const int work_begin = runs ? static_cast<int>(static_cast<long long>(tiles) * all_kb * worker / workers) : worker;
   const int work_end = runs ? static_cast<int>(static_cast<long long>(tiles) * all_kb * (worker + 1) / workers) : tiles * splits;
 
@@ -265,7 +268,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
 
   // product, tile row, tile column and range of k-blocks of the work item at w, and where the next one is
   struct Item {
-    int p, m_blk, n_blk, kb0, kb1, next;
+    int p, m_blk, n_blk, kb0, kb1, next, piece;
   };
   auto item = [&](int w) {
     Item it;
@@ -275,12 +278,14 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
       it.kb0 = w - t * all_kb;
       it.kb1 = work_end - w < all_kb - it.kb0 ? it.kb0 + work_end - w : all_kb;
       it.next = w + it.kb1 - it.kb0;
+      it.piece = 0;
     } else {
       t = splits > 1 ? w / splits : w;
       const int s = w - t * splits;
       it.kb0 = splits > 1 ? all_kb * s / splits : 0;
       it.kb1 = splits > 1 ? all_kb * (s + 1) / splits : all_kb;
       it.next = w + workers;
+      it.piece = s;
     }
     it.p = 0;
     if constexpr (kMax > 1) {
@@ -468,7 +473,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
         }
       };
       if constexpr (kF32) {
-        const bool add = g.atomic_add || g.accumulate;
+        [[maybe_unused]] const bool add = g.atomic_add || g.accumulate;
 #pragma unroll 1
         for (int c = 0; c < S::kCols; c += 32) {
           uint32_t r[32];
@@ -487,7 +492,8 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           fence_async_smem();
           __syncwarp();
           if (tc::elect_one()) {
-            if (add) reduce_add_2d(map_d, stage, col0 + c, row0);
+            if constexpr (kOut == OUT_F32_SLABS) store_2d(map_d, stage, col0 + c, it.piece * g.slab_rows + row0);
+            else if (add) reduce_add_2d(map_d, stage, col0 + c, row0);
             else store_2d(map_d, stage, col0 + c, row0);
             bulk_commit();
           }
@@ -750,7 +756,7 @@ inline bool encode_groups(CUtensorMap* map, const void* base, int k, int cols, i
 }
 
 // Launches `workers` CTAs (pairs) over the tiles of `count` products with the same K, which is cut into `splits` (0: equal
-// runs of k-blocks; with anything but 1, fp32 sums are added into D).
+// runs of k-blocks; with anything but 1, fp32 sums are added into D, or go to slabs).
 template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut, int kMax>
 cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int splits, cudaStream_t stream) {
   using S = Shape<BN, kPair, kOut == OUT_GELU>;
@@ -772,14 +778,15 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
                      : kAMn ? encode_map(&P.a[p], a.a, a.k, a.m, a.lda, BK) : encode_map(&P.a[p], a.a, a.m, a.k, a.lda, BM);
     const bool okb = P.atoms[p] & 2 ? encode_groups(&P.b[p], a.b, a.k, a.n, a.ldb, S::kRowsB / 64)
                      : kBMn ? encode_map(&P.b[p], a.b, a.k, a.n, a.ldb, BK) : encode_map(&P.b[p], a.b, kOut == OUT_SWIGLU ? 2 * a.n : a.n, a.k, a.ldb, S::kRowsB);
-    if (!oka || !okb || !encode_out_map(&P.d[p], a.d, a.m, kOut == OUT_SWIGLU_GRAD ? 2 * a.n : a.n, a.ldd, fp32_out(kOut), half_boxes(kOut))) return cudaErrorNotSupported;
+    const int slab_rows = (a.m + 31) / 32 * 32;
+    if (!oka || !okb || !encode_out_map(&P.d[p], a.d, kOut == OUT_F32_SLABS ? slab_rows * splits : a.m, kOut == OUT_SWIGLU_GRAD ? 2 * a.n : a.n, a.ldd, fp32_out(kOut), half_boxes(kOut))) return cudaErrorNotSupported;
     P.m[p] = a.m;
     P.n[p] = a.n;
     constexpr int kTileN = kOut == OUT_SWIGLU ? BN / 2 : BN;
     P.n_tiles[p] = (a.n + kTileN - 1) / kTileN;
     P.first[p + 1] = P.first[p] + P.n_tiles[p] * ((a.m + (kPair ? 2 * BM : BM) - 1) / (kPair ? 2 * BM : BM));
     // partial sums are added into the output: start from zero unless the caller accumulates anyway
-    if (splits != 1 && !a.accumulate) {
+    if (splits != 1 && !a.accumulate && kOut != OUT_F32_SLABS) {
       cudaError_t rc = cudaMemsetAsync(a.d, 0, static_cast<size_t>(a.m) * a.n * sizeof(float), stream);
       if (rc != cudaSuccess) return rc;
     }
@@ -805,6 +812,7 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
   g.accumulate = a.accumulate ? 1 : 0;
   g.epilogue = a.epilogue;
   g.atomic_add = splits != 1 ? 1 : 0;
+  g.slab_rows = (a.m + 31) / 32 * 32;
   g.err = gemm_error_device_ptr();
   if (!g.err) return cudaErrorNotSupported;
   g.tl = timeline_device_ptr();

@@ -25,6 +25,11 @@ template cudaError_t launch_tiles<128, false, false, true, OUT_BF16_SCALED, 1>(c
 template cudaError_t launch_tiles<192, false, false, true, OUT_BF16_SCALED, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template cudaError_t launch_tiles<256, true, false, true, OUT_BF16_SCALED, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template int max_pairs<256, false, true, OUT_BF16_SCALED, 1>();
+template cudaError_t launch_tiles<64, false, false, true, OUT_F32_SLABS, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+template cudaError_t launch_tiles<128, false, false, true, OUT_F32_SLABS, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+template cudaError_t launch_tiles<192, false, false, true, OUT_F32_SLABS, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+template cudaError_t launch_tiles<256, true, false, true, OUT_F32_SLABS, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+template int max_pairs<256, false, true, OUT_F32_SLABS, 1>();
 template cudaError_t launch_tiles<64, false, true, false, OUT_BF16, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template cudaError_t launch_tiles<128, false, true, false, OUT_BF16, 1>(const GemmArgs*, int, int, int, cudaStream_t);
 template cudaError_t launch_tiles<192, false, true, false, OUT_BF16, 1>(const GemmArgs*, int, int, int, cudaStream_t);

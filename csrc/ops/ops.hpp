@@ -25,8 +25,9 @@ void count_launch(int n = 1);
 // x, y: [rows, dim] bf16; w, b: fp32; mean / rstd: fp32 [rows] saved for backward (both may be null).
 cudaError_t norm_fwd(const __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y, float* mean, float* rstd,
                      int rows, int dim, float eps, cudaStream_t stream);
-// x = bf16(sum + bias + residual) and y = norm(x), for a product left as fp32 sums [rows, dim]; bias may be null; dim up to 2048.
-cudaError_t norm_sum_fwd(const float* sum, const float* bias, const __nv_bfloat16* residual, __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y,
+// x = bf16(sum + bias + residual) and y = norm(x), for a product left in `parts` parts of fp32 [rows, dim], `stride` elements apart and added
+// in order; bias may be null; dim up to 2048.
+cudaError_t norm_sum_fwd(const float* sum, int parts, long long stride, const float* bias, const __nv_bfloat16* residual, __nv_bfloat16* x, const float* w, const float* b, __nv_bfloat16* y,
                          int rows, int dim, float eps, cudaStream_t stream);
 // dx: [rows, dim] bf16; dw, db: fp32 [dim].  With scratch (fp32, 2 * colsum_slabs(rows) * dim
 // elements) dw / db are overwritten by a two-stage, order-fixed reduction; with scratch == nullptr
@@ -63,8 +64,10 @@ cudaError_t mean_f32(const float* in, float* out, long long n, cudaStream_t stre
 
 // ---- out[c, r] = in[r, c] for a bf16 matrix [rows, cols].
 cudaError_t transpose_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, int rows, int cols, cudaStream_t stream);
-// fp32 → bf16 cast of n elements, times the device scalar alpha (null: one).
-cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t stream, const float* alpha = nullptr);
+// fp32 → bf16 cast of n elements.
+cudaError_t cast_f32_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t stream);
+// out = bf16(alpha * (part 0 + part 1 + ...)) over n elements; the parts are `stride` elements apart; alpha: device scalar (null: one).
+cudaError_t sum_slabs_bf16(const float* in, int parts, long long stride, __nv_bfloat16* out, long long n, const float* alpha, cudaStream_t stream);
 // The same for `count` tensors, tensor i into out[dst_offset[i], ...); 16-byte aligned sources and places.
 cudaError_t cast_many(const float* const* src, const long long* numel, const long long* dst_offset, int count, __nv_bfloat16* out,
                       cudaStream_t stream);
@@ -146,9 +149,16 @@ cudaError_t gemm_swiglu_grad(const GemmArgs& args, cudaStream_t stream);
 // (sixteen products per launch).  A product is a GemmArgs with both operands MN-major, fp32 output, no epilogue; all of them
 // accumulate, or none.
 cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream);
-// Whether a bf16 product without epilogue is better computed as fp32 partial sums, added into a zeroed fp32 [M, N], and cast:
-// a long contraction whose tiles leave much of the GPU idle.
-bool gemm_wants_partial_sums(const GemmArgs& args);
+// A product shared out over K: part i is left as fp32 sums [M, N] at i * `stride` elements of d, for a reader that adds the parts in order
+// (norm_sum_fwd, sum_slabs_bf16).  Plain product only, d_fp32, ldd = N, A not MN-major.  d has room for count * stride elements.
+struct Slabs {
+  int count;          // parts, chosen by sizes and by how many SMs products may use
+  long long stride;   // elements from one to the next (rows are rounded up to 32, and what is beyond M is written too)
+};
+Slabs gemm_slabs(const GemmArgs& args);
+cudaError_t gemm_to_slabs(const GemmArgs& args, const Slabs& slabs, cudaStream_t stream);
+// Whether a bf16 product without epilogue is better computed this way: a long contraction whose tiles leave much of the GPU idle.
+bool gemm_wants_slabs(const GemmArgs& args);
 // Caps the number of CTAs (= SMs) plain GEMM launches occupy from now on; 0 restores one CTA per SM.  A
 // data-parallel trainer lowers it during backward so that a few SMs stay free for the gradient collectives
 // that run beside the GEMMs.  The value is read at launch time, so it is baked into a captured CUDA graph.
