@@ -42,7 +42,8 @@ void bind_layers(py::module_& m) {
     c10::cuda::CUDAGuard guard(x.device());
     const Weights w = weights_of(params, d);
     need(dout, at::kBFloat16, x.numel(), "output gradient");
-    if (grads.empty()) {
+    const bool in_order = grads.empty();   // a trainer's buffers are added into as the sums arrive
+    if (in_order) {
       int64_t total = 0, at[kParams];
       for (int i = 0; i < kParams; ++i) {
         at[i] = total;
@@ -60,7 +61,7 @@ void bind_layers(py::module_& m) {
     Slab s;
     MCCL_CHECK_TENSOR(slab.is_cuda() && slab.numel() == Slab::place(&s, nullptr, d), "decoder layer: not the slab of this forward");
     Slab::place(&s, slab.data_ptr<uint8_t>(), d);
-    const auto [dx, tmp] = layer_backward(dout, x, w, s, g, d, defer);
+    const auto [dx, tmp] = layer_backward(dout, x, w, s, g, d, defer, in_order);
     return std::make_tuple(dx, grads, defer ? tmp : at::Tensor());
   });
   // The weight gradients of layers whose backward was called with defer: (output gradient, slab, the third result of
@@ -76,7 +77,8 @@ void bind_layers(py::module_& m) {
     for (const auto& [dout, slab, tmp, grads] : layers) {
       Pending p;
       need(dout, at::kBFloat16, TD, "output gradient");
-      need(tmp, at::kBFloat16, TD * 6 + static_cast<int64_t>(d.tokens()) * d.F, "gradients between the kernels");
+      need(tmp, at::kBFloat16, tmp.numel(), "gradients between the kernels");
+      MCCL_CHECK_TENSOR(tmp.numel() >= TD * 6 + static_cast<int64_t>(d.tokens()) * d.F, "decoder layer: not the gradients of this backward");
       MCCL_CHECK_TENSOR(slab.is_cuda() && slab.numel() == Slab::place(&p.s, nullptr, d) && grads.size() == kParams, "decoder layer: layers of one size expected");
       Slab::place(&p.s, slab.data_ptr<uint8_t>(), d);
       for (int i = 0; i < kParams; ++i) need(grads[i], at::kFloat, param_numel(d, i), "gradient buffer");

@@ -93,7 +93,7 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     }
     Slab s;
     Slab::place(&s, slab.data_ptr<uint8_t>(), d);
-    out[0] = layer_backward(dout, x, weights(params, flat, off.data()), s, g, d, false).first;
+    out[0] = layer_backward(dout, x, weights(params, flat, off.data()), s, g, d, false, true).first;
     return out;
   }
 };
@@ -114,10 +114,13 @@ struct NormNode : torch::autograd::Function<NormNode> {
     const int D = static_cast<int>(x.size(-1)), T = static_cast<int>(x.numel() / D);
     const float* mean = stats.data_ptr<float>();
     const int64_t at_b = (D + 7) / 8 * 8;
-    at::Tensor dx = at::empty_like(x), g = zeros_f32(at_b + D, w);
-    check(ops::norm_bwd_fused(bf(dy), bf(x), w.data_ptr<float>(), mean, mean + T, bf(dx), nullptr, g.data_ptr<float>(), g.data_ptr<float>() + at_b, nullptr, nullptr, T,
-                              D, true, stream_on(x)),
+    const int rows = ops::norm_bwd_parts(T, D);
+    at::Tensor dx = at::empty_like(x), g = at::empty({at_b + D}, stats.options()), parts = at::empty({2, rows, D}, stats.options());
+    float *dw = g.data_ptr<float>(), *pw = parts.data_ptr<float>(), *pb = pw + static_cast<int64_t>(rows) * D;
+    check(ops::norm_bwd_fused(bf(dy), bf(x), w.data_ptr<float>(), mean, mean + T, bf(dx), nullptr, pw, pb, nullptr, nullptr, T, D, true, stream_on(x), true),
           "final norm backward");
+    const ops::PartSum sums[2] = {{pw, dw, rows, D}, {pb, dw + at_b, rows, D}};
+    check(ops::sum_parts(sums, 2, stream_on(x)), "final norm backward");
     return {dx, g.as_strided({D}, {1}, 0), g.as_strided({D}, {1}, at_b), at::Tensor()};
   }
 };

@@ -5,6 +5,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "../core/errors.hpp"
@@ -123,9 +124,9 @@ inline cudaError_t gated(const bf16* x, const bf16* w, bf16* h, bf16* gu, int M,
   g.k = g.lda = g.ldb = K;
   return ops::gemm_swiglu(g, stream);
 }
-// dx[M, K] = dy[M, N] · w[N, K] (times mul, with its column sums added to colsum)
+// dx[M, K] = dy[M, N] · w[N, K] (times mul, with its column sums added to colsum, or in_order: left there in parts)
 inline void input_gradient(const bf16* dy, const bf16* w, bf16* dx, int M, int N, int K, const bf16* mul, float* colsum, cudaStream_t stream,
-                    const char* what) {
+                    const char* what, bool in_order = false) {
   ops::GemmArgs g;
   g.a = dy;
   g.b = w;
@@ -133,6 +134,7 @@ inline void input_gradient(const bf16* dy, const bf16* w, bf16* dx, int M, int N
   g.d = dx;
   g.mul = mul;
   g.colsum = colsum;
+  g.colsum_in_order = in_order;
   g.m = M;
   g.n = K;
   g.k = N;
@@ -160,7 +162,7 @@ struct Pending {
   Slab s;
   float *down, *up, *qkv, *proj;
 };
-inline void weight_gradients(const std::vector<Pending>& layers, const Dims& d, cudaStream_t stream) {
+inline void weight_gradients(const std::vector<Pending>& layers, const Dims& d, cudaStream_t stream, const ops::PartSum* sums = nullptr, int sum_count = 0) {
   const int T = d.tokens(), D = d.D, F = d.F;
   std::vector<ops::GemmArgs> args;
   for (const Pending& p : layers) {
@@ -169,7 +171,7 @@ inline void weight_gradients(const std::vector<Pending>& layers, const Dims& d, 
     args.push_back(weight_gradient(p.dqkv, p.s.h1, p.qkv, T, 3 * D, D));
     args.push_back(weight_gradient(p.dy, p.s.o, p.proj, T, D, D));
   }
-  check(ops::gemm_group(args.data(), static_cast<int>(args.size()), stream), "weight gradients");
+  check(ops::gemm_group(args.data(), static_cast<int>(args.size()), stream, sums, sum_count), "weight gradients");
 }
 
 // Whether the down projection of these sizes is better left in parts, which the norm behind it adds: a single row of tiles that fills a
@@ -225,30 +227,63 @@ inline Dims dims_of(const at::Tensor& x, int64_t B, int64_t S, int64_t H, int64_
   return {static_cast<int>(B), static_cast<int>(S), static_cast<int>(H), static_cast<int>(D), static_cast<int>(F)};
 }
 
-// Backward of a layer.  g: gradient buffers of the 12 parameters, added into.  Returns (dx, gradients between the kernels); with
-// defer the matrices' gradients are left for weight_gradients(), which needs the second.
+// The vectors' gradients of a layer as the kernels that hold the tensors leave them with in_order: one row per contributor.
+struct VectorParts {
+  float* part[kParams] = {};
+  int rows[kParams] = {};
+  static int64_t place(VectorParts* v, float* base, const Dims& d) {
+    const int T = d.tokens(), norm = ops::norm_bwd_parts(T, d.D), attention = ops::attention_bwd_parts(d.B, d.S);
+    int64_t at = 0;
+    for (int i : {LN1_W, LN1_B, QKV_B, PROJ_B, LN2_W, LN2_B, UP_B, DOWN_B}) {
+      v->rows[i] = i == QKV_B ? attention : (i == UP_B ? (T + 31) / 32 : norm);
+      v->part[i] = base + at;
+      at += static_cast<int64_t>(v->rows[i]) * param_numel(d, i);
+    }
+    return at;
+  }
+};
+
+// Backward of a layer.  g: gradient buffers of the 12 parameters, added into (in_order: the vectors' are written, as sums in an order that
+// does not depend on scheduling).  Returns (dx, gradients between the kernels); with defer the matrices' gradients are left
+// for weight_gradients(), which needs the second.
 inline std::pair<at::Tensor, at::Tensor> layer_backward(const at::Tensor& dout, const at::Tensor& x, const Weights& w, const Slab& s, float* const (&g)[kParams],
-                                                        const Dims& d, bool defer) {
+                                                        const Dims& d, bool defer, bool in_order) {
   const int T = d.tokens(), D = d.D, F = d.F;
   const float scale = 1.f / std::sqrt(static_cast<float>(d.head_dim()));
   cudaStream_t st = at::cuda::getCurrentCUDAStream(x.get_device()).stream();
   // dz [T, F], dqkv [T, 3 D], and three of [T, D]
   const int64_t TD = static_cast<int64_t>(T) * D;
-  at::Tensor tmp = at::empty({TD * 6 + static_cast<int64_t>(T) * F}, x.options());
+  const int64_t elems = TD * 6 + static_cast<int64_t>(T) * F;
+  VectorParts parts;
+  const int64_t room = in_order ? VectorParts::place(&parts, nullptr, d) : 0;   // fp32, behind the others
+  at::Tensor tmp = at::empty({elems + 2 * room}, x.options());
   bf16 *dh = bf(tmp), *dy = dh + TD, *d_o = dy + TD, *dqkv = d_o + TD, *dz = dqkv + 3 * TD;
   at::Tensor dx = at::empty_like(x);
-  input_gradient(bf(dout), w.down, dz, T, D, F, s.gelu_grad, g[UP_B], st, "down projection backward");
+  float* v[kParams];   // where the kernels leave the vectors' gradients
+  std::copy(std::begin(g), std::end(g), v);
+  if (in_order) {
+    VectorParts::place(&parts, reinterpret_cast<float*>(bf(tmp) + elems), d);
+    for (int i = 0; i < kParams; ++i)
+      if (parts.part[i]) v[i] = parts.part[i];
+  }
+  input_gradient(bf(dout), w.down, dz, T, D, F, s.gelu_grad, v[UP_B], st, "down projection backward", in_order);
   input_gradient(dz, w.up, dh, T, F, D, nullptr, nullptr, st, "up projection backward");
-  check(ops::norm_bwd_fused(dh, s.y, w.ln2_w, s.mean2, s.rstd2, dy, bf(dout), g[LN2_W], g[LN2_B], g[DOWN_B], g[PROJ_B], T, D, true, st),
+  check(ops::norm_bwd_fused(dh, s.y, w.ln2_w, s.mean2, s.rstd2, dy, bf(dout), v[LN2_W], v[LN2_B], v[DOWN_B], v[PROJ_B], T, D, true, st, in_order),
         "second norm backward");
   input_gradient(dy, w.proj, d_o, T, D, D, nullptr, nullptr, st, "output projection backward");
-  check(ops::attention_bwd(s.qkv, s.o, d_o, s.lse, dqkv, g[QKV_B], d.B, d.S, d.H, d.head_dim(), scale, st), "attention backward");
+  check(ops::attention_bwd(s.qkv, s.o, d_o, s.lse, dqkv, v[QKV_B], d.B, d.S, d.H, d.head_dim(), scale, st, in_order), "attention backward");
   input_gradient(dqkv, w.qkv, dh, T, 3 * D, D, nullptr, nullptr, st, "qkv projection backward");
-  check(ops::norm_bwd_fused(dh, bf(x), w.ln1_w, s.mean1, s.rstd1, bf(dx), dy, g[LN1_W], g[LN1_B], nullptr, nullptr, T, D, true, st),
+  check(ops::norm_bwd_fused(dh, bf(x), w.ln1_w, s.mean1, s.rstd1, bf(dx), dy, v[LN1_W], v[LN1_B], nullptr, nullptr, T, D, true, st, in_order),
         "first norm backward");
+  ops::PartSum sums[kParams];
+  int n = 0;
+  for (int i = 0; i < kParams; ++i)
+    if (parts.part[i]) sums[n++] = {parts.part[i], g[i], parts.rows[i], static_cast<int>(param_numel(d, i))};
   if (!defer) {
     const Pending p = {bf(dout), dz, dqkv, dy, s, g[DOWN_W], g[UP_W], g[QKV_W], g[PROJ_W]};
-    weight_gradients({p}, d, st);
+    weight_gradients({p}, d, st, sums, n);
+  } else if (in_order) {
+    check(ops::sum_parts(sums, n, st), "sums of the vectors' gradients");
   }
   return {dx, tmp};
 }

@@ -61,6 +61,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 struct AttnArgs {
   float* lse;                 // [B, H, S], log2 domain: m + log2(l)
   float* colsum;              // optional: column sums of dqkv are added here, fp32 [3 * H * hd]
+  int colsum_ld;              // when set: the sums of every 32 rows go to a row of their own of colsum, this many elements apart
   int S, H, hd;
   float scale, scale_log2;
   int* err;
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
   };
   // one row of 32 gradient columns [c0, c0 + 32) of part t (0: dQ, 1: dK, 2: dV) out of tensor memory into a tile that is
   // no longer needed; then the warp's 32 rows leave for block blk
-  auto stage_out = [&](uint8_t* tile, uint32_t taddr, int t, int c0) {
+  auto stage_out = [&](uint8_t* tile, uint32_t taddr, int t, int c0, int blk) {
     float v[32];
     tmem_ld32(taddr + lane_base + static_cast<uint32_t>(c0), v);
 #pragma unroll
@@ -376,7 +377,11 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
     }
     if (a.colsum != nullptr && c0 < a.hd) {   // rows past the sequence are zero
       const float sum = column_sum32(v, lane);
-      if (c0 + lane < a.hd) atomicAdd(a.colsum + (t * a.H + h) * a.hd + c0 + lane, sum);
+      if (c0 + lane < a.hd) {
+        float* to = a.colsum + static_cast<size_t>((b * nblk + blk) * 4 + (warp & 3)) * a.colsum_ld + (t * a.H + h) * a.hd + c0 + lane;
+        if (a.colsum_ld != 0) *to = sum;
+        else atomicAdd(to, sum);
+      }
     }
   };
   auto send_out = [&](const uint8_t* tile, int t, int blk) {
@@ -388,8 +393,8 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
   };
   auto key_block_out = [&](int j) {   // one warpgroup takes dK_j, the other dV_j; K_j and V_j have been read for the last time
     uint8_t* tile = (wg == 0 ? sK : sV) + j * kTile;
-    stage_out(tile, wg == 0 ? tm_dk : tm_dv, 1 + wg, 0);
-    stage_out(tile, wg == 0 ? tm_dk : tm_dv, 1 + wg, 32);
+    stage_out(tile, wg == 0 ? tm_dk : tm_dv, 1 + wg, 0, j);
+    stage_out(tile, wg == 0 ? tm_dk : tm_dv, 1 + wg, 32, j);
     tc::fence_before_sync();
     send_out(tile, 1 + wg, j);
   };
@@ -531,11 +536,11 @@ __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant_
   ok = __syncthreads_and((ok && *bad == 0) ? 1 : 0) != 0;
   if (ok) {
     if (nblk == 2) {   // one query block per warpgroup
-      stage_out(sQ + wg * kTile, tm_dq + static_cast<uint32_t>(wg * kHd), 0, 0);
-      stage_out(sQ + wg * kTile, tm_dq + static_cast<uint32_t>(wg * kHd), 0, 32);
+      stage_out(sQ + wg * kTile, tm_dq + static_cast<uint32_t>(wg * kHd), 0, 0, wg);
+      stage_out(sQ + wg * kTile, tm_dq + static_cast<uint32_t>(wg * kHd), 0, 32, wg);
       send_out(sQ + wg * kTile, 0, wg);
     } else {           // half of the columns per warpgroup
-      stage_out(sQ, tm_dq, 0, wg * 32);
+      stage_out(sQ, tm_dq, 0, wg * 32, 0);
       fence_async_smem();
       __syncthreads();
       if (wg == 0) send_out(sQ, 0, 0);
@@ -586,8 +591,10 @@ cudaError_t allow_smem(K kernel, int bytes, std::atomic<bool>& done) {
 static_assert(2 * kBlk == 256, "one or two blocks of queries");
 bool attention_supported(int S, int hd) { return S >= 1 && S <= 2 * kBlk && hd >= 8 && hd <= kHd && hd % 8 == 0; }
 
+int attention_bwd_parts(int B, int S) { return B * ((S + kBlk - 1) / kBlk) * 4; }
+
 cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, const __nv_bfloat16* d_o, const float* lse,
-                          __nv_bfloat16* dqkv, float* colsum, int B, int S, int H, int hd, float softmax_scale, cudaStream_t stream) {
+                          __nv_bfloat16* dqkv, float* colsum, int B, int S, int H, int hd, float softmax_scale, cudaStream_t stream, bool in_order) {
   if (!attention_supported(S, hd) || B <= 0 || H <= 0 || static_cast<long long>(B) * H > INT_MAX) return cudaErrorNotSupported;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o) |
        reinterpret_cast<uintptr_t>(dqkv)) & 15u)
@@ -603,6 +610,7 @@ cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, cons
   AttnArgs a = {};
   a.lse = const_cast<float*>(lse);
   a.colsum = colsum;
+  a.colsum_ld = in_order ? 3 * H * hd : 0;
   a.S = S;
   a.H = H;
   a.hd = hd;

@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(256) norm_bwd_fused_kernel(const __nv_bfloat16
                                                              const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx,
                                                              const __nv_bfloat16* __restrict__ dx_add, float* __restrict__ dw,
                                                              float* __restrict__ db, float* __restrict__ sum_add,
-                                                             float* __restrict__ sum_dx, int rows, int dim) {
+                                                             float* __restrict__ sum_dx, int rows, int dim, int in_order) {
   extern __shared__ float red[];   // [8 warps][kVecs * 256]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, vecs = dim >> 3;
   float aw[kVecs][8], ab[kVecs][8], sa[kSums ? kVecs : 1][8], sd[kSums ? kVecs : 1][8];
@@ -419,9 +419,60 @@ __global__ void __launch_bounds__(256) norm_bwd_fused_kernel(const __nv_bfloat16
       float t = 0.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) t += red[(set * 8 + i) * kVecs * 256 + c];
-      if (c < dim) atomicAdd(out + c, t);
+      if (c < dim) {
+        if (in_order) out[static_cast<size_t>(blockIdx.x) * dim + c] = t;
+        else atomicAdd(out + c, t);
+      }
     }
   }
+}
+
+// Sums of the rows that contributors left: 32 columns x 32 row lanes per block, lane l adds rows l, l + 32, ... with eight in flight,
+// then the lanes are added in order.  Nothing but latency: one round of loads for 256 rows.
+__global__ void __launch_bounds__(1024) sum_parts_kernel(const __grid_constant__ PartSums p) {
+  ::mccl::pdl_wait();
+  ::mccl::pdl_trigger();
+  __shared__ float lanes[32][33];
+  int i = 0;
+  while (i + 1 < p.count && static_cast<int>(blockIdx.x) >= p.first[i + 1]) ++i;
+  const PartSum s = p.s[i];
+  const int cx = threadIdx.x & 31, ly = threadIdx.x >> 5, c = (static_cast<int>(blockIdx.x) - p.first[i]) * 32 + cx;
+  float t = 0.f;
+  if (c < s.cols) {
+    for (int r0 = ly; r0 < s.rows; r0 += 256) {
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = r0 + 32 * k < s.rows ? __ldcg(s.in + static_cast<size_t>(r0 + 32 * k) * s.cols + c) : 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) t += v[k];
+    }
+  }
+  lanes[ly][cx] = t;
+  __syncthreads();
+  // warp w takes column w: its lanes are the row lanes
+  t = warp_sum(lanes[cx][ly]);
+  const int col = c - cx + ly;
+  if (cx == 0 && col < s.cols) s.out[col] = t;
+}
+
+cudaError_t PartSums::set(const PartSum* sums, int n) {
+  count = 0;
+  first[0] = 0;
+  if (n < 0 || n > kPartSums) return cudaErrorInvalidValue;
+  for (; count < n; ++count) {
+    s[count] = sums[count];
+    first[count + 1] = first[count] + (sums[count].cols + 31) / 32;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t sum_parts(const PartSum* sums, int count, cudaStream_t stream) {
+  PartSums p;
+  cudaError_t rc = p.set(sums, count);
+  if (rc != cudaSuccess || p.first[p.count] == 0) return rc;
+  MCCL_LAUNCH_PDL(sum_parts_kernel, p.first[count], 1024, 0, stream, p);
+  count_launch();
+  return ::mccl::launch_status();
 }
 
 // Column reductions over the rows: dw[c] = sum_r dy[r,c] * xhat[r,c] and
@@ -587,16 +638,19 @@ cudaError_t norm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const floa
   return ::mccl::launch_status();
 }
 
+int norm_bwd_parts(int rows, int dim) {
+  const int blocks = (rows + 7) / 8, most = dim <= 256 ? 2 * 148 : 148;
+  return blocks > most ? most : blocks;
+}
+
 cudaError_t norm_bwd_fused(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* w, const float* mean, const float* rstd,
                            __nv_bfloat16* dx, const __nv_bfloat16* dx_add, float* dw, float* db, float* sum_add, float* sum_dx, int rows,
-                           int dim, bool layernorm, cudaStream_t stream) {
+                           int dim, bool layernorm, cudaStream_t stream, bool in_order) {
   const int vecs = (dim + 255) / 256;
   const bool sums = sum_add != nullptr || sum_dx != nullptr;
   // the sums of a lane's columns live in registers: four sets of up to 32 or one of up to 64
   if (dim % 8 != 0 || vecs > (layernorm || sums ? 4 : 8) || (sum_add != nullptr && dx_add == nullptr)) return cudaErrorNotSupported;
-  int blocks = (rows + 7) / 8;
-  const int most = vecs == 1 ? 2 * 148 : 148;
-  if (blocks > most) blocks = most;
+  const int blocks = norm_bwd_parts(rows, dim);
   if (blocks < 1) return cudaSuccess;
   auto go = [&](auto kernel, int v, int sets, std::atomic<bool>& configured) -> cudaError_t {
     const int smem = sets * 8 * v * 256 * static_cast<int>(sizeof(float));
@@ -605,7 +659,7 @@ cudaError_t norm_bwd_fused(const __nv_bfloat16* dy, const __nv_bfloat16* x, cons
       if (rc != cudaSuccess) return rc;
       configured.store(true, std::memory_order_release);
     }
-    MCCL_LAUNCH_PDL(kernel, blocks, 256, smem, stream, dy, x, w, mean, rstd, dx, dx_add, dw, db, sum_add, sum_dx, rows, dim);
+    MCCL_LAUNCH_PDL(kernel, blocks, 256, smem, stream, dy, x, w, mean, rstd, dx, dx_add, dw, db, sum_add, sum_dx, rows, dim, in_order ? 1 : 0);
     count_launch();
     return ::mccl::launch_status();
   };

@@ -7,18 +7,19 @@ namespace ops {
 
 namespace tiles {
 #define MCCL_TILES_EXTERN(A, B, OUT, MAX)                                                                                     \
-  extern template cudaError_t launch_tiles<64, false, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t);          \
-  extern template cudaError_t launch_tiles<128, false, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t);
+  extern template cudaError_t launch_tiles<64, false, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t, const PartSums*);   \
+  extern template cudaError_t launch_tiles<128, false, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t, const PartSums*);
 #define MCCL_TILES_EXTERN_PAIR(A, B, OUT, MAX)                                                                                \
   MCCL_TILES_EXTERN(A, B, OUT, MAX)                                                                                           \
-  extern template cudaError_t launch_tiles<192, false, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t);         \
-  extern template cudaError_t launch_tiles<256, true, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t);          \
+  extern template cudaError_t launch_tiles<192, false, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t, const PartSums*);   \
+  extern template cudaError_t launch_tiles<256, true, A, B, OUT, MAX>(const GemmArgs*, int, int, int, cudaStream_t, const PartSums*);   \
   extern template int max_pairs<256, A, B, OUT, MAX>();
 MCCL_TILES_EXTERN(false, false, OUT_GELU, 1)
 MCCL_TILES_EXTERN_PAIR(false, false, OUT_BF16, 1)
 MCCL_TILES_EXTERN_PAIR(false, false, OUT_F32, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16_SUM, 1)
+MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16_PARTS, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_BF16_SCALED, 1)
 MCCL_TILES_EXTERN_PAIR(false, false, OUT_F32_SLABS, 1)
 MCCL_TILES_EXTERN_PAIR(false, true, OUT_F32_SLABS, 1)
@@ -29,9 +30,9 @@ MCCL_TILES_EXTERN_PAIR(true, false, OUT_F32, 1)
 MCCL_TILES_EXTERN_PAIR(true, true, OUT_BF16, 1)
 MCCL_TILES_EXTERN_PAIR(true, true, OUT_F32, 1)
 MCCL_TILES_EXTERN_PAIR(true, true, OUT_F32, kMaxGroup)
-extern template cudaError_t launch_tiles<256, true, false, false, OUT_SWIGLU, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+extern template cudaError_t launch_tiles<256, true, false, false, OUT_SWIGLU, 1>(const GemmArgs*, int, int, int, cudaStream_t, const PartSums*);
 extern template int max_pairs<256, false, false, OUT_SWIGLU, 1>();
-extern template cudaError_t launch_tiles<256, true, false, true, OUT_SWIGLU_GRAD, 1>(const GemmArgs*, int, int, int, cudaStream_t);
+extern template cudaError_t launch_tiles<256, true, false, true, OUT_SWIGLU_GRAD, 1>(const GemmArgs*, int, int, int, cudaStream_t, const PartSums*);
 extern template int max_pairs<256, false, true, OUT_SWIGLU_GRAD, 1>();
 #undef MCCL_TILES_EXTERN
 #undef MCCL_TILES_EXTERN_PAIR
@@ -105,10 +106,10 @@ Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, boo
 }
 
 template <bool kAMn, bool kBMn, int kOut, int kMax = 1>
-cudaError_t run_plan(const GemmArgs* a, int count, const Plan& plan, cudaStream_t stream);
+cudaError_t run_plan(const GemmArgs* a, int count, const Plan& plan, cudaStream_t stream, const PartSums* sums = nullptr);
 
 template <bool kAMn, bool kBMn, int kOut, int kMax = 1>
-cudaError_t run(const GemmArgs* a, int count, int forced, cudaStream_t stream) {
+cudaError_t run(const GemmArgs* a, int count, int forced, cudaStream_t stream, const PartSums* sums = nullptr) {
   int sms = gemm_sm_count(), pairs = 0;
   if constexpr (kOut != OUT_GELU) pairs = max_pairs<256, kAMn, kBMn, kOut, kMax>();
   const int limit = gemm_cta_limit();
@@ -118,17 +119,17 @@ cudaError_t run(const GemmArgs* a, int count, int forced, cudaStream_t stream) {
   }
   bool splittable = fp32_out(kOut);
   for (int p = 0; p < count; ++p) splittable = splittable && (a[p].accumulate || a[p].ldd == a[p].n);
-  return run_plan<kAMn, kBMn, kOut, kMax>(a, count, choose(a, count, forced, sms, pairs, kOut == OUT_GELU, splittable), stream);
+  return run_plan<kAMn, kBMn, kOut, kMax>(a, count, choose(a, count, forced, sms, pairs, kOut == OUT_GELU, splittable), stream, sums);
 }
 
 template <bool kAMn, bool kBMn, int kOut, int kMax>
-cudaError_t run_plan(const GemmArgs* a, int count, const Plan& plan, cudaStream_t stream) {
-  if (plan.bn == 64) return launch_tiles<64, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
+cudaError_t run_plan(const GemmArgs* a, int count, const Plan& plan, cudaStream_t stream, const PartSums* sums) {
+  if (plan.bn == 64) return launch_tiles<64, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream, sums);
   if constexpr (kOut != OUT_GELU)
-    if (plan.bn == 192) return launch_tiles<192, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
+    if (plan.bn == 192) return launch_tiles<192, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream, sums);
   if constexpr (kOut != OUT_GELU)
-    if (plan.bn == 256) return launch_tiles<256, true, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
-  return launch_tiles<128, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream);
+    if (plan.bn == 256) return launch_tiles<256, true, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream, sums);
+  return launch_tiles<128, false, kAMn, kBMn, kOut, kMax>(a, count, plan.workers, plan.splits, stream, sums);
 }
 
 template <int kOut>
@@ -150,7 +151,8 @@ cudaError_t launch_gemm_tiles(const GemmArgs& a, int forced_bn, cudaStream_t str
   (void)cudaGetLastError();   // a stale error of an earlier, unrelated call must not be blamed on this launch
   if (a.colsum) {
     if (gelu || a.d_fp32 || a.bias || a.residual || a.a_mn_major || !a.b_mn_major) return cudaErrorInvalidValue;
-    return tiles::run<false, true, tiles::OUT_BF16_SUM>(&a, 1, forced_bn, stream);
+    return a.colsum_in_order ? tiles::run<false, true, tiles::OUT_BF16_PARTS>(&a, 1, forced_bn, stream)
+                             : tiles::run<false, true, tiles::OUT_BF16_SUM>(&a, 1, forced_bn, stream);
   }
   if (a.alpha) {
     if (a.d_fp32 && a.a_mn_major && a.b_mn_major) return tiles::run<true, true, tiles::OUT_F32_SCALED>(&a, 1, forced_bn, stream);
@@ -222,7 +224,7 @@ cudaError_t run_swiglu(const GemmArgs& a, cudaStream_t stream) {
   if (tiles::choose(&alone, 1, 0, sms, pairs, false, false).bn != 256) return cudaErrorNotSupported;
   const int tiles = tiles::ceil_div(a.m, 256) * tiles::ceil_div(a.n, kTileN);
   (void)cudaGetLastError();
-  return tiles::launch_tiles<256, true, false, kBMn, kOut, 1>(&a, 1, tiles < pairs ? tiles : pairs, 1, stream);
+  return tiles::launch_tiles<256, true, false, kBMn, kOut, 1>(&a, 1, tiles < pairs ? tiles : pairs, 1, stream, nullptr);
 }
 }  // namespace
 
@@ -231,7 +233,9 @@ cudaError_t gemm_swiglu_grad(const GemmArgs& a, cudaStream_t stream) {
   return a.aux ? run_swiglu<true, tiles::OUT_SWIGLU_GRAD>(a, stream) : cudaErrorInvalidValue;
 }
 
-cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream) {
+cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream, const PartSum* sums, int sum_count) {
+  PartSums table;
+  if (cudaError_t rc = table.set(sums, sum_count); rc != cudaSuccess) return rc;
   for (int p = 0; p < count; ++p) {
     const GemmArgs& a = args[p];
     if (!a.a_mn_major || !a.b_mn_major || !a.d_fp32 || a.epilogue != EPI_NONE || a.residual || a.mul || a.colsum || a.k != args[0].k ||
@@ -244,7 +248,7 @@ cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream) {
   (void)cudaGetLastError();
   for (int p = 0; p < count; p += tiles::kMaxGroup) {
     const int c = count - p < tiles::kMaxGroup ? count - p : tiles::kMaxGroup;
-    cudaError_t rc = tiles::run<true, true, tiles::OUT_F32, tiles::kMaxGroup>(args + p, c, 0, stream);
+    cudaError_t rc = tiles::run<true, true, tiles::OUT_F32, tiles::kMaxGroup>(args + p, c, 0, stream, p == 0 && sum_count > 0 ? &table : nullptr);
     if (rc != cudaSuccess) return rc;
   }
   return cudaSuccess;

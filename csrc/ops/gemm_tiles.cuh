@@ -32,6 +32,7 @@
 #include "../core/launch.hpp"
 
 #include <atomic>
+#include <type_traits>
 
 namespace mccl {
 namespace ops {
@@ -44,6 +45,7 @@ namespace tiles {
 // order.  Partial sums that are added in memory arrive in any order, and a forward pass or an input gradient that went that way
 // no longer repeated bit for bit.
 // OUT_BF16_SUM: the bf16 output and, added into GemmDev::colsum, its column sums (a bias gradient).
+// OUT_BF16_PARTS: the sums of every 32 rows are written to a row of their own instead, for finish_sums or sum_parts.
 // OUT_SWIGLU (pair tile only): B is [gate | up], 2 n rows; the even CTA brings 128 rows of gate and the odd one the same 128 of up,
 // so that a tile's accumulator holds both factors of 128 outputs and silu(gate) * up is the epilogue.  The [m, 2 n] product
 // itself, which backward reads, is written too where `aux` is given.  As a kernel of its own the activation read it back:
@@ -51,15 +53,19 @@ namespace tiles {
 // OUT_SWIGLU_GRAD (pair tile only): the input gradient of the product behind the activation, turned into the gradient of
 // [gate | up] (D, [m, 2 n]) with the saved [gate | up] (`aux`) on its way out; the [m, n] tensor between the two is neither
 // written nor read.
-enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3, OUT_SWIGLU = 4, OUT_SWIGLU_GRAD = 5, OUT_BF16_SCALED = 6, OUT_F32_SCALED = 7, OUT_F32_SLABS = 8 };
+enum Out : int { OUT_BF16 = 0, OUT_GELU = 1, OUT_F32 = 2, OUT_BF16_SUM = 3, OUT_SWIGLU = 4, OUT_SWIGLU_GRAD = 5, OUT_BF16_SCALED = 6, OUT_F32_SCALED = 7, OUT_F32_SLABS = 8, OUT_BF16_PARTS = 9 };
 constexpr bool fp32_out(int out) { return out == OUT_F32 || out == OUT_F32_SCALED || out == OUT_F32_SLABS; }
 constexpr bool half_boxes(int out) { return out == OUT_GELU || out == OUT_SWIGLU || out == OUT_SWIGLU_GRAD; }   // 32-column output boxes
 
 // One product, or several with the same K whose tiles one launch works through (the weight gradients of one or more layers:
 // alone, a 512 x 2048 gradient is 64 tiles and leaves half the SMs without one).
 constexpr int kMaxGroup = 16;
+struct NoSums {};
+struct WithSums {
+  PartSums sums;   // finished by the epilogue warps while the first tile's main loop runs
+};
 template <int kMax>
-struct Problems {
+struct Problems : std::conditional_t<(kMax > 1), WithSums, NoSums> {
   CUtensorMap a[kMax], b[kMax], d[kMax];
   CUtensorMap x;              // the second output of the GELU instantiation, or the extra input of the bf16 ones
   int m[kMax], n[kMax];
@@ -198,10 +204,40 @@ __device__ __forceinline__ void unpack8(const uint4& pk, float (&v)[8]) {
   }
 }
 
+// Sums that kernels before this one left in parts (bias and norm gradients), by the W epilogue warps of each CTA: 32 columns at a time,
+// rows dealt out to the warps with eight in flight, the warps' shares added in order.  A launch of its own for them is 4 us per layer
+// (70M training loop 3870 -> 3941 us); here nobody waits for it (3868).
+template <int W>
+__device__ __forceinline__ void finish_sums(const PartSums& p, float* red, int warp, int lane) {
+  const int groups = p.first[p.count];
+  for (int q = blockIdx.x; q < groups; q += gridDim.x) {
+    int i = 0;
+    while (i + 1 < p.count && q >= p.first[i + 1]) ++i;
+    const float* in = p.s[i].in;
+    const int rows = p.s[i].rows, cols = p.s[i].cols, c = (q - p.first[i]) * 32 + lane;
+    float t = 0.f;
+    if (c < cols)
+      for (int r0 = warp; r0 < rows; r0 += 8 * W) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = r0 + W * k < rows ? __ldcg(in + static_cast<size_t>(r0 + W * k) * cols + c) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t += v[k];
+      }
+    red[warp * 32 + lane] = t;
+    asm volatile("bar.sync 1, %0;" ::"n"(W * 32) : "memory");
+    if (warp == 0 && c < cols) {
+      for (int w = 1; w < W; ++w) t += red[w * 32 + lane];
+      p.s[i].out[c] = t;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(W * 32) : "memory");
+  }
+}
+
 template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut, int kMax>
 __global__ void __launch_bounds__(Shape<BN, kPair, kOut == OUT_GELU>::kThreads, 1)
 gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits) {
-  constexpr bool kBf16 = kOut == OUT_BF16 || kOut == OUT_BF16_SUM, kF32 = fp32_out(kOut), kScaled = kOut == OUT_BF16_SCALED || kOut == OUT_F32_SCALED;
+  constexpr bool kSum = kOut == OUT_BF16_SUM || kOut == OUT_BF16_PARTS, kBf16 = kOut == OUT_BF16 || kSum, kF32 = fp32_out(kOut), kScaled = kOut == OUT_BF16_SCALED || kOut == OUT_F32_SCALED;
   using S = Shape<BN, kPair, kOut == OUT_GELU>;
   constexpr int kStages = S::kStages, kTileM = kPair ? 2 * BM : BM;
   constexpr bool kGated = kOut == OUT_SWIGLU;
@@ -427,6 +463,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
     bool ok = true;
     int i = 0;
     uint32_t xparity = 0;
+    if constexpr (kMax > 1) finish_sums<S::kEpiWarps>(P.sums, reinterpret_cast<float*>(smem + S::kStagingOff), e, lane);
     float alpha = 1.f;
     if constexpr (kScaled) alpha = __ldg(g.alpha);
     for (int w = work_begin; w < work_end; ++i) {
@@ -678,12 +715,12 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
               }
             }
             *stage_unit(stage, lane, j) = pack8(v);
-            if constexpr (kOut == OUT_BF16_SUM) {
+            if constexpr (kSum) {
 #pragma unroll
               for (int q = 0; q < 8; ++q) r[jj * 8 + q] = __float_as_uint(v[q]);
             }
           }
-          if constexpr (kOut == OUT_BF16_SUM) {
+          if constexpr (kSum) {
             // sums of 32 columns over the warp's 32 rows by halving: 31 shuffles, lane l ends up with column l
 #pragma unroll
             for (int o = 16; o >= 1; o >>= 1) {
@@ -694,7 +731,10 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
                 r[q] = __float_as_uint(((lane & o) ? hi : lo) + other);
               }
             }
-            if (col0 + 32 * h + lane < n) atomicAdd(g.colsum + col0 + 32 * h + lane, __uint_as_float(r[0]));
+            if (col0 + 32 * h + lane < n) {
+              if constexpr (kOut == OUT_BF16_PARTS) g.colsum[static_cast<size_t>(row0 >> 5) * n + col0 + 32 * h + lane] = __uint_as_float(r[0]);
+              else atomicAdd(g.colsum + col0 + 32 * h + lane, __uint_as_float(r[0]));
+            }
           }
         }
         if (inside) {
@@ -758,7 +798,7 @@ inline bool encode_groups(CUtensorMap* map, const void* base, int k, int cols, i
 // Launches `workers` CTAs (pairs) over the tiles of `count` products with the same K, which is cut into `splits` (0: equal
 // runs of k-blocks; with anything but 1, fp32 sums are added into D, or go to slabs).
 template <int BN, bool kPair, bool kAMn, bool kBMn, int kOut, int kMax>
-cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int splits, cudaStream_t stream) {
+cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int splits, cudaStream_t stream, const PartSums* sums = nullptr) {
   using S = Shape<BN, kPair, kOut == OUT_GELU>;
   auto kernel = gemm_tile_kernel<BN, kPair, kAMn, kBMn, kOut, kMax>;
   static std::atomic<bool> configured{false};
@@ -768,6 +808,10 @@ cudaError_t launch_tiles(const GemmArgs* args, int count, int workers, int split
     configured.store(true, std::memory_order_release);
   }
   Problems<kMax> P;
+  if constexpr (kMax > 1) {
+    P.sums.count = P.sums.first[0] = 0;
+    if (sums) P.sums = *sums;
+  }
   P.count = count;
   P.first[0] = 0;
   for (int p = 0; p < count; ++p) {

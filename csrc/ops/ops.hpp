@@ -38,9 +38,25 @@ cudaError_t norm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const floa
                      cudaStream_t stream, const __nv_bfloat16* dx_add = nullptr, int parts = 3);
 // The same backward in one pass: dw, db (LayerNorm) and, where given, the column sums of dx_add and of dx are ADDED into fp32
 // [dim] buffers.  dim <= 1024, or 2048 for RMSNorm without column sums; cudaErrorNotSupported otherwise.
+// With in_order each of the four (those given) is a block [norm_bwd_parts(rows, dim), dim] instead, written and not added into, for sum_parts.
 cudaError_t norm_bwd_fused(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* w, const float* mean, const float* rstd,
                            __nv_bfloat16* dx, const __nv_bfloat16* dx_add, float* dw, float* db, float* sum_add, float* sum_dx, int rows,
-                           int dim, bool layernorm, cudaStream_t stream);
+                           int dim, bool layernorm, cudaStream_t stream, bool in_order = false);
+int norm_bwd_parts(int rows, int dim);
+// Sums whose parts a kernel left in rows: out[c] = in[0, c] + in[1, c] + ... in an order that depends on sizes alone.
+struct PartSum {
+  const float* in;   // [rows, cols]
+  float* out;        // [cols]
+  int rows, cols;
+};
+constexpr int kPartSums = 8;
+struct PartSums {
+  PartSum s[kPartSums];
+  int first[kPartSums + 1];   // first group of 32 columns of each
+  int count;
+  cudaError_t set(const PartSum* sums, int n);
+};
+cudaError_t sum_parts(const PartSum* sums, int count, cudaStream_t stream);
 // out[c] = sum over rows of in[r, c] (bias gradients).  scratch: colsum_slabs(rows) * dim floats,
 // or nullptr to add into out atomically in one pass.
 cudaError_t colsum_bf16(const __nv_bfloat16* in, float* out, float* scratch, int rows, int dim, cudaStream_t stream);
@@ -89,9 +105,12 @@ cudaError_t embed_bwd(const long long* ids, const __nv_bfloat16* dy, float* dtok
 bool attention_supported(int S, int hd);
 cudaError_t attention_fwd(const __nv_bfloat16* qkv, __nv_bfloat16* o, float* lse, int B, int S, int H, int hd, float softmax_scale,
                           cudaStream_t stream);
-// dqkv: [B, S, 3, H, hd] bf16, every element written.  colsum (optional, fp32 [3 * H * hd]): its column sums are added here.
+// dqkv: [B, S, 3, H, hd] bf16, every element written.  colsum (optional, fp32 [3 * H * hd]): its column sums are added here, or with in_order
+// written to a block [attention_bwd_parts(B, S), 3 * H * hd] for sum_parts.
 cudaError_t attention_bwd(const __nv_bfloat16* qkv, const __nv_bfloat16* o, const __nv_bfloat16* d_o, const float* lse,
-                          __nv_bfloat16* dqkv, float* colsum, int B, int S, int H, int hd, float softmax_scale, cudaStream_t stream);
+                          __nv_bfloat16* dqkv, float* colsum, int B, int S, int H, int hd, float softmax_scale, cudaStream_t stream,
+                          bool in_order = false);
+int attention_bwd_parts(int B, int S);
 
 // ---- rotary embedding of the fused QKV projection's output (pairs of even and odd elements; cos / sin: fp32
 // [>= seq, head_dim / 2]; token t has position t % seq).  qkv [tokens, 3, H, hd] -> qk [tokens, 2, H, hd].
@@ -129,6 +148,7 @@ struct GemmArgs {
   const __nv_bfloat16* residual = nullptr;  // [M, N] added after bias / activation, row stride ldd
   const __nv_bfloat16* mul = nullptr;       // [M, N]: D = acc * mul (e.g. the saved gelu'(z): the input gradient through a GELU), row stride ldd
   float* colsum = nullptr;                  // [N] fp32: column sums of D are added here (bf16 output without bias or residual, B MN-major)
+  bool colsum_in_order = false;             // colsum is [ceil(M / 32), N] instead: the sums of 32 rows each, written, for sum_parts
   int m = 0, n = 0, k = 0;
   int lda = 0, ldb = 0, ldd = 0;
   bool d_fp32 = false;
@@ -148,7 +168,8 @@ cudaError_t gemm_swiglu_grad(const GemmArgs& args, cudaStream_t stream);
 // Up to any number of weight gradients dW[N, K] = dY[tokens, N]^T · X[tokens, K] over the same tokens, worked through together
 // (sixteen products per launch).  A product is a GemmArgs with both operands MN-major, fp32 output, no epilogue; all of them
 // accumulate, or none.
-cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream);
+// `sums` (up to kPartSums, of kernels before this one) are finished by the first launch beside its products, see sum_parts.
+cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream, const PartSum* sums = nullptr, int sum_count = 0);
 // A product shared out over K: part i is left as fp32 sums [M, N] at i * `stride` elements of d, for a reader that adds the parts in order
 // (norm_sum_fwd, sum_slabs_bf16).  Plain product only, d_fp32, ldd = N, A not MN-major.  d has room for count * stride elements.
 struct Slabs {

@@ -34,3 +34,29 @@ def test_product_in_parts(m, n, k, mn_major):
     for _ in range(20):
         assert torch.equal(_C.gemm_bf16(a, bb, b_t=mn_major)[0], d)
     assert _C.gemm_error_flag() == 0
+
+
+@pytest.mark.parametrize("name,changes,B,S", [("tiny", {}, 8, 24), ("tiny", {"vocab": 8192}, 1, 1), ("tiny", {"n_heads": 2, "max_seq": 256}, 2, 129),
+                                              ("70m", {"n_layers": 2}, 16, 256), ("110m", {"n_layers": 1, "vocab": 512}, 3, 200)])
+@pytest.mark.parametrize("one_call", [True, False])
+def test_vector_gradients_of_a_training_loop(monkeypatch, name, changes, B, S, one_call):
+    """Biases and norms, in the loss's own call and through the layers' nodes."""
+    from mccl_b200.models import build_decoder
+    torch.manual_seed(0)
+    model = build_decoder(name, **changes).cuda()
+    if not one_call:
+        monkeypatch.setattr(type(model), "_loss_in_one_call", lambda self, *a: None)
+    tok = torch.randint(0, model.cfg.vocab, (B, S + 1), device="cuda")
+
+    def grads():
+        model.zero_grad(set_to_none=True)
+        loss = model(tok[:, :-1], tok[:, 1:])
+        loss.backward()
+        return loss.detach(), {n: p.grad for n, p in model.named_parameters() if p.dim() == 1}
+    l0, g0 = grads()
+    assert len(g0) == 8 * model.cfg.n_layers + 2
+    for _ in range(10):
+        l1, g1 = grads()
+        assert torch.equal(l0, l1)
+        for n in g0:
+            assert torch.equal(g0[n], g1[n]), n
