@@ -276,20 +276,6 @@ __global__ void __launch_bounds__(256, 2) attn_fwd_kernel(const __grid_constant_
 constexpr int kFwdSmem = 6 * kTile + 2048 + 64 + 1024;   // 99 KiB: two CTAs per SM
 
 // ------------------------------------------------ backward, up to 256 keys --
-// Sum of each of 32 per-lane values over the warp's lanes, by halving: lane l returns column l.
-__device__ __forceinline__ float column_sum32(float (&v)[32], int lane) {
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-#pragma unroll
-    for (int q = 0; q < o; ++q) {
-      const float lo = v[q], hi = v[q + o];
-      const float other = __shfl_xor_sync(0xffffffffu, (lane & o) ? lo : hi, o);
-      v[q] = ((lane & o) ? hi : lo) + other;
-    }
-  }
-  return v[0];
-}
-
 // Tensor memory, 512 columns: [0,128) S  [128,256) dP  [256,384) dQ_0, dQ_1  [384,448) dK_j  [448,512) dV_j
 __global__ void __launch_bounds__(256, 1) attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv,
                                                           const __grid_constant__ CUtensorMap tm_do,

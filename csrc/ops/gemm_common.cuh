@@ -3,6 +3,7 @@
 // descriptor encoder.
 #pragma once
 
+#include "bf16x8.cuh"
 #include "ops.hpp"
 #include "tcgen05.cuh"
 

@@ -187,23 +187,6 @@ __device__ __forceinline__ void bulk_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
-  uint4 pk;
-  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-  return pk;
-}
-__device__ __forceinline__ void unpack8(const uint4& pk, float (&v)[8]) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&pk);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 t = __bfloat1622float2(h[i]);
-    v[2 * i] = t.x;
-    v[2 * i + 1] = t.y;
-  }
-}
-
 // Sums that kernels before this one left in parts (bias and norm gradients), by the W epilogue warps of each CTA: 32 columns at a time,
 // rows dealt out to the warps with eight in flight, the warps' shares added in order.  A launch of its own for them is 4 us per layer
 // (70M training loop 3870 -> 3941 us); here nobody waits for it (3868).
@@ -686,6 +669,7 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
           tc::tmem_ld_wait();
           if (h == 1) last_read();
           if (!inside) continue;
+          [[maybe_unused]] float sums[32];
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj) {
             const int j = 4 * h + jj;
@@ -717,23 +701,14 @@ gemm_tile_kernel(const __grid_constant__ Problems<kMax> P, GemmDev g, int splits
             *stage_unit(stage, lane, j) = pack8(v);
             if constexpr (kSum) {
 #pragma unroll
-              for (int q = 0; q < 8; ++q) r[jj * 8 + q] = __float_as_uint(v[q]);
+              for (int q = 0; q < 8; ++q) sums[jj * 8 + q] = v[q];
             }
           }
           if constexpr (kSum) {
-            // sums of 32 columns over the warp's 32 rows by halving: 31 shuffles, lane l ends up with column l
-#pragma unroll
-            for (int o = 16; o >= 1; o >>= 1) {
-#pragma unroll
-              for (int q = 0; q < o; ++q) {
-                const float lo = __uint_as_float(r[q]), hi = __uint_as_float(r[q + o]);
-                const float other = __shfl_xor_sync(0xffffffffu, (lane & o) ? lo : hi, o);
-                r[q] = __float_as_uint(((lane & o) ? hi : lo) + other);
-              }
-            }
+            const float sum = column_sum32(sums, lane);   // over the warp's 32 rows
             if (col0 + 32 * h + lane < n) {
-              if constexpr (kOut == OUT_BF16_PARTS) g.colsum[static_cast<size_t>(row0 >> 5) * n + col0 + 32 * h + lane] = __uint_as_float(r[0]);
-              else atomicAdd(g.colsum + col0 + 32 * h + lane, __uint_as_float(r[0]));
+              if constexpr (kOut == OUT_BF16_PARTS) g.colsum[static_cast<size_t>(row0 >> 5) * n + col0 + 32 * h + lane] = sum;
+              else atomicAdd(g.colsum + col0 + 32 * h + lane, sum);
             }
           }
         }

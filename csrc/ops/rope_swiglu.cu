@@ -5,6 +5,7 @@
 // and access, consecutive threads on consecutive addresses.  They replace chains of strided element-wise operators that
 // went over fp32 intermediates (even / odd slices, stack, cast, chunk, concatenation).
 #include "../core/launch.hpp"
+#include "bf16x8.cuh"
 #include "ops.hpp"
 
 namespace mccl {
@@ -14,22 +15,6 @@ namespace {
 
 constexpr int kThreads = 256;
 
-__device__ __forceinline__ void unpack8(const uint4& raw, float (&f)[8]) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 t = __bfloat1622float2(h[i]);
-    f[2 * i] = t.x;
-    f[2 * i + 1] = t.y;
-  }
-}
-__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
-  uint4 raw;
-  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-  return raw;
-}
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 int blocks_for(long long units) {
