@@ -115,8 +115,8 @@ struct NormNode : torch::autograd::Function<NormNode> {
     const float* mean = stats.data_ptr<float>();
     const int64_t at_b = (D + 7) / 8 * 8;
     const int rows = ops::norm_bwd_parts(T, D);
-    at::Tensor dx = at::empty_like(x), g = at::empty({at_b + D}, stats.options()), parts = at::empty({2, rows, D}, stats.options());
-    float *dw = g.data_ptr<float>(), *pw = parts.data_ptr<float>(), *pb = pw + static_cast<int64_t>(rows) * D;
+    at::Tensor dx = at::empty_like(x), g = at::empty({2 * at_b + 2 * static_cast<int64_t>(rows) * D}, stats.options());   // the sums, and the parts they are made of
+    float *dw = g.data_ptr<float>(), *pw = dw + 2 * at_b, *pb = pw + static_cast<int64_t>(rows) * D;
     check(ops::norm_bwd_fused(bf(dy), bf(x), w.data_ptr<float>(), mean, mean + T, bf(dx), nullptr, pw, pb, nullptr, nullptr, T, D, true, stream_on(x), true),
           "final norm backward");
     const ops::PartSum sums[2] = {{pw, dw, rows, D}, {pb, dw + at_b, rows, D}};

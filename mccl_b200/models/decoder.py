@@ -114,8 +114,10 @@ def _stock(m: nn.Module) -> bool:
 
 
 def _untouched(m: nn.Module) -> bool:
-    """The same, and nobody wants to see the module's own calls."""
-    return (_stock(m) and "forward" not in m.__dict__ and not any(_GLOBAL_HOOKS)
+    """Whether a native call may stand in for this projection, and nobody wants to see the module's own calls.  (Host time counts
+    here: twice per layer in loops that run operator by operator.)"""
+    t = type(m)
+    return (t.forward is _LINEAR_FORWARD and t.__call__ is _MODULE_CALL and "forward" not in m.__dict__ and not any(_GLOBAL_HOOKS)
             and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks))
 
 
@@ -152,7 +154,7 @@ class _Structure:
                 and list(map(type, self.modules)) == self.types
                 and not any(map(dict.__contains__, self.own, itertools.repeat("forward")))
                 and list(map(operator.itemgetter("eps"), self.norms)) == self.eps
-                and all(getattr(cls, name) is f for cls, methods in _STOCK.items() for name, f in methods.items()))
+                and all([getattr(cls, name) is f for cls, name, f in _STOCK_METHODS]))
 
 
 def _structure(module: nn.Module, device, children):
@@ -190,7 +192,7 @@ class Norm(nn.Module):
         """(norm(x), x as it should be fed to the residual connection).  The native path hands x through the
         norm operator so that backward adds the residual gradient in the norm-backward kernel
         (MCCL_FUSE_RESIDUAL_GRAD=0: x is returned untouched)."""
-        if native and _FUSE_RESIDUAL_GRAD and _stock(self) and "forward" not in self.__dict__:
+        if native and _FUSE_RESIDUAL_GRAD and type(self).forward is _NORM_FORWARD and "forward" not in self.__dict__:
             from .. import ops
             return ops.norm_residual(x, self.weight, self.bias, self.eps)
         return self.forward(x, native), x
@@ -296,8 +298,9 @@ class Block(nn.Module):
         if cfg.act == "swiglu":
             if native:
                 from .. import ops
-                if all(_untouched(m) and m.bias is None for m in (self.gate_up, self.down)):
-                    return ops.mlp_swiglu(h, self.gate_up.weight, self.down.weight, residual=x)
+                first, second = self.gate_up, self.down
+                if _untouched(first) and _untouched(second) and first.bias is None and second.bias is None:
+                    return ops.mlp_swiglu(h, first.weight, second.weight, residual=x)
                 h = ops.swiglu(self.gate_up(h, native))   # not what the fused call computes, or somebody wants to see the calls
             else:
                 g, u = self.gate_up(h, native).chunk(2, dim=-1)
@@ -313,6 +316,8 @@ class Block(nn.Module):
 #: Modules that the native calls can stand for, and the methods whose work they do.
 _STOCK = {cls: {name: getattr(cls, name) for name in ("forward", "with_residual") if hasattr(cls, name)}
           for cls in (Block, Norm, Linear, nn.Embedding, nn.ModuleList)}
+_STOCK_METHODS = [(cls, name, f) for cls, methods in _STOCK.items() for name, f in methods.items()]
+_LINEAR_FORWARD, _NORM_FORWARD, _MODULE_CALL = Linear.forward, Norm.forward, nn.Module.__call__
 
 
 class Decoder(nn.Module):
@@ -354,8 +359,9 @@ class Decoder(nn.Module):
         return self.ln_f(x, native)
 
     def _layers(self, device):
-        """(structure, the layers' parameters in the order the native calls take them), or None where those calls do not stand for
-        this model: a module or a method was replaced, parameters are missing or of other sizes, somebody watches the calls."""
+        """The structure with the layers' parameters in the order the native calls take them (`layers`) and those around them (`outer`), or
+        None where those calls do not stand for this model: a module or a method was replaced, parameters are missing or of
+        other sizes, somebody watches the calls."""
         cls = type(self)
         if cls.hidden is not Decoder.hidden or cls.head_weight is not Decoder.head_weight or "hidden" in self.__dict__ or "head_weight" in self.__dict__:
             return None
@@ -377,7 +383,10 @@ class Decoder(nn.Module):
                     and lnf.get("weight") is not None and lnf["weight"].numel() == cfg.d_model and (lnf.get("bias") is None) == (cfg.norm != "layernorm")
                     and getattr(self.head, "bias", None) is None and (self.pos is None) == (cfg.pos == "rope") and s.eps[0] == cfg.eps)
             s.layers = layers if fits else False
-        return None if s.layers is False else (s, s.layers)
+            if fits:
+                tok, pos, head = self.tok.weight, None if self.pos is None else self.pos.weight, self.head_weight()
+                s.outer = (tok, pos, self.ln_f.weight, self.ln_f.bias, head)
+        return None if s.layers is False else s
 
     def _fused_gelu(self, tokens: torch.Tensor) -> bool:
         cfg = self.cfg
@@ -391,37 +400,38 @@ class Decoder(nn.Module):
     def _loss_in_one_call(self, tokens: torch.Tensor, targets: torch.Tensor):
         """The training loss through C++ autograd nodes, or None where that does not apply (a trainer's gradient buffers, frozen
         or replaced parameters, hooks)."""
-        found = self._layers(tokens.device)
-        if found is None or not self._fused_gelu(tokens) or targets.dtype != torch.int64 or targets.numel() != tokens.numel():
+        if not self._fused_gelu(tokens) or targets.dtype != torch.int64 or targets.numel() != tokens.numel():
             return None
-        s, layers = found
-        if hasattr(self.tok.weight, "_grad_sink") or not all(p.requires_grad for p in s.params):
+        s = self._layers(tokens.device)
+        if s is None:
+            return None
+        tok, pos, lnf_w, lnf_b, head = s.outer
+        if hasattr(tok, "_grad_sink") or not all(p.requires_grad for p in s.params):
             return None
         from .. import _C
-        return _C.decoder_loss(tokens, targets, self.tok.weight, self.pos.weight, layers, self.ln_f.weight, self.ln_f.bias,
-                               self.head_weight(), self.cfg.n_heads, self.cfg.eps)
+        return _C.decoder_loss(tokens, targets, tok, pos, s.layers, lnf_w, lnf_b, head, self.cfg.n_heads, self.cfg.eps)
 
     def _forward_without_gradients(self, tokens: torch.Tensor):
         """Logits from one native call over the whole decoder, or None where it does not apply."""
         cfg = self.cfg
         from .. import _C
         rope = cfg.pos == "rope"
-        found = self._layers(tokens.device)
-        if found is None:
+        s = self._layers(tokens.device)
+        if s is None:
             return None
+        tok, pos, lnf_w, lnf_b, head = s.outer
         if rope:
-            if (tokens.dim() != 2 or tokens.dtype != torch.int64 or cfg.d_model % 64 or cfg.d_ff % 64 or self.head_weight().shape[0] % 8
+            if (tokens.dim() != 2 or tokens.dtype != torch.int64 or cfg.d_model % 64 or cfg.d_ff % 64 or head.shape[0] % 8
                     or cfg.norm != "rmsnorm" or cfg.act != "swiglu" or cfg.head_dim % 8 or torch.is_autocast_enabled()):
                 return None
         elif not self._fused_gelu(tokens):
             return None
-        layers, head = found[1], self.head_weight()
+        layers = s.layers
         if hasattr(head, "_bf16"):   # a trainer keeps bf16 copies of the matrices up to date
             layers = [getattr(p, "_bf16", p) if p.dim() == 2 else p for p in layers]
             head = head._bf16
         tables = _rope_tables(tokens.shape[1], cfg.head_dim, tokens.device) if rope else (None, None)
-        return _C.decoder_fwd(tokens, self.tok.weight, None if self.pos is None else self.pos.weight, layers, self.ln_f.weight, self.ln_f.bias, head,
-                              cfg.n_heads, cfg.eps, *tables)
+        return _C.decoder_fwd(tokens, tok, pos, layers, lnf_w, lnf_b, head, cfg.n_heads, cfg.eps, *tables)
 
     def head_weight(self) -> torch.Tensor:
         return self.tok.weight if self.head is None else self.head.weight

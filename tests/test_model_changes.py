@@ -103,7 +103,7 @@ def _projections(name):
 def test_structure_is_watched(name):
     dev = torch.device("cpu")
     plain = _model(name)
-    assert plain._layers(dev) is not None and plain._layers(dev)[1] is plain._layers(dev)[1]
+    assert plain._layers(dev) is not None and plain._layers(dev).layers is plain._layers(dev).layers
     for which in _projections(name):
         for label, change in ASIDE.items():
             m = copy.deepcopy(plain)
@@ -116,7 +116,7 @@ def test_structure_is_watched(name):
         change(m, "qkv")
         found = m._layers(dev)
         want = [p for b in m.blocks for p in b._ordered()]
-        assert found is not None and len(found[1]) == len(want) and all(a is b for a, b in zip(found[1], want)), label
+        assert found is not None and len(found.layers) == len(want) and all(a is b for a, b in zip(found.layers, want)), label
 
 
 def test_hooks_on_every_module_are_seen():
