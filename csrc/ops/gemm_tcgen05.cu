@@ -43,6 +43,15 @@ void set_gemm_kernel(const std::string& name) {
   g_gemm_kernel_override.store(name.empty() ? -2 : kernel_index(name), std::memory_order_relaxed);
 }
 
+int gemm_kernel_choice() {
+  static const int env_choice = [] {
+    const char* v = std::getenv("MCCL_GEMM_KERNEL");
+    return kernel_index(v ? v : "");
+  }();
+  const int forced = g_gemm_kernel_override.load(std::memory_order_relaxed);
+  return forced != -2 ? forced : env_choice;
+}
+
 const char* gemm_last_reason() { return t_reason; }
 
 cudaError_t gemm_bf16_tn(const GemmArgs& a, cudaStream_t stream) {
@@ -63,12 +72,7 @@ cudaError_t gemm_bf16_tn(const GemmArgs& a, cudaStream_t stream) {
   if (a.residual && (reinterpret_cast<uintptr_t>(a.residual) & 15u)) return unsupported("residual pointer must be 16-byte aligned");
   if (a.mul && ((reinterpret_cast<uintptr_t>(a.mul) & 15u) || a.d_fp32)) return unsupported("mul must be 16-byte aligned and the output bf16");
   if (a.a_mn_major && a.m % 8 != 0) return unsupported("an MN-major A needs M to be a multiple of 8");
-  static const int env_choice = [] {
-    const char* v = std::getenv("MCCL_GEMM_KERNEL");
-    return kernel_index(v ? v : "");
-  }();
-  const int forced = g_gemm_kernel_override.load(std::memory_order_relaxed);
-  const int choice = forced != -2 ? forced : env_choice;
+  const int choice = gemm_kernel_choice();
   const bool gelu = a.epilogue == EPI_BIAS_GELU || a.epilogue == EPI_GELU || a.epilogue == EPI_BIAS_GELU_D || a.epilogue == EPI_GELU_D;
   if (a.alpha && (gelu || a.bias || a.residual || a.mul || a.colsum)) return cudaErrorInvalidValue;
   const bool tile_only = a.k % BK != 0 || a.colsum || a.alpha || (gelu && !a.aux);   // what only the tile kernel does

@@ -167,11 +167,13 @@ cudaError_t launch_gemm_tiles(const GemmArgs& a, int forced_bn, cudaStream_t str
 // Measured on an LM head's input gradient (K 32000): 32 pair tiles (4096 x 512) 108 against 123 us, 48 (4096 x 768) 145 against
 // 152; with 64 tiles (4096 x 1024, K 8192) writing, adding and casting the parts cost more than the idle SMs, 67 against 43.
 bool gemm_wants_slabs(const GemmArgs& a) {
-  return a.k >= 4096 && tiles::ceil_div(a.m, 256) * tiles::ceil_div(a.n, 256) * 10 <= gemm_sm_count() / 2 * 7;
+  if (a.m <= 0 || a.n <= 0 || a.a_mn_major || a.n % 8 != 0 || a.lda % 8 != 0 || a.ldb % 8 != 0 ||
+      ((reinterpret_cast<uintptr_t>(a.a) | reinterpret_cast<uintptr_t>(a.b)) & 15u))
+    return false;   // gemm_bf16_tn says why
+  return a.k >= 4096 && gemm_kernel_choice() >= 0 && tiles::ceil_div(a.m, 256) * tiles::ceil_div(a.n, 256) * 10 <= gemm_sm_count() / 2 * 7;
 }
 
-namespace {
-tiles::Plan slab_plan(const GemmArgs& a) {
+Slabs gemm_slabs(const GemmArgs& a) {
   int sms = gemm_sm_count();
   int pairs = a.b_mn_major ? tiles::max_pairs<256, false, true, tiles::OUT_F32_SLABS, 1>() : tiles::max_pairs<256, false, false, tiles::OUT_F32_SLABS, 1>();
   const int limit = gemm_cta_limit();
@@ -179,13 +181,9 @@ tiles::Plan slab_plan(const GemmArgs& a) {
     sms = limit < sms ? limit : sms;
     pairs = limit / 2 < pairs ? limit / 2 : pairs;
   }
-  return tiles::choose(&a, 1, 0, sms, pairs, false, true, true);
-}
-}  // namespace
-
-Slabs gemm_slabs(const GemmArgs& a) {
-  const int rows = (a.m + 31) / 32 * 32;
-  return {slab_plan(a).splits, static_cast<long long>(rows) * a.n};
+  const int choice = gemm_kernel_choice();
+  const tiles::Plan plan = tiles::choose(&a, 1, choice > 0 ? choice : 0, sms, pairs, false, true, true);
+  return {plan.splits, static_cast<long long>((a.m + 31) / 32 * 32) * a.n, plan.bn, plan.workers};
 }
 
 cudaError_t gemm_to_slabs(const GemmArgs& a, const Slabs& s, cudaStream_t stream) {
@@ -195,8 +193,11 @@ cudaError_t gemm_to_slabs(const GemmArgs& a, const Slabs& s, cudaStream_t stream
   if (a.n % 8 != 0 || a.lda % 8 != 0 || a.ldb % 8 != 0 ||
       ((reinterpret_cast<uintptr_t>(a.a) | reinterpret_cast<uintptr_t>(a.b) | reinterpret_cast<uintptr_t>(a.d)) & 15u))
     return cudaErrorNotSupported;
-  const tiles::Plan plan = slab_plan(a);
-  if (plan.splits != s.count) return cudaErrorInvalidValue;   // the cap on the CTAs was moved in between
+  if (s.workers < 1) return cudaErrorInvalidValue;
+  tiles::Plan plan;
+  plan.bn = s.tile;
+  plan.workers = s.workers;
+  plan.splits = s.count;
   (void)cudaGetLastError();
   return a.b_mn_major ? tiles::run_plan<false, true, tiles::OUT_F32_SLABS>(&a, 1, plan, stream) : tiles::run_plan<false, false, tiles::OUT_F32_SLABS>(&a, 1, plan, stream);
 }

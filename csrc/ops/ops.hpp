@@ -175,6 +175,7 @@ cudaError_t gemm_group(const GemmArgs* args, int count, cudaStream_t stream, con
 struct Slabs {
   int count;          // parts, chosen by sizes and by how many SMs products may use
   long long stride;   // elements from one to the next (rows are rounded up to 32, and what is beyond M is written too)
+  int tile, workers;  // the rest of the choice: a cap on the CTAs that moves between the two calls changes nothing
 };
 Slabs gemm_slabs(const GemmArgs& args);
 cudaError_t gemm_to_slabs(const GemmArgs& args, const Slabs& slabs, cudaStream_t stream);
@@ -188,6 +189,8 @@ void set_gemm_cta_limit(int ctas);
 // "pair256" (that tile), "persistent" (one CTA per SM); "" = default.
 void set_gemm_kernel(const std::string& name);
 int gemm_cta_limit();
+// What set_gemm_kernel or MCCL_GEMM_KERNEL asks for: a tile (64 ... 256), 0 for one of the kernel's choosing, -1 for the persistent kernel.
+int gemm_kernel_choice();
 int gemm_sm_count();
 // Why the last gemm_bf16_tn call on this thread returned cudaErrorNotSupported ("" otherwise).
 const char* gemm_last_reason();

@@ -60,3 +60,23 @@ def test_vector_gradients_of_a_training_loop(monkeypatch, name, changes, B, S, o
         assert torch.equal(l0, l1)
         for n in g0:
             assert torch.equal(g0[n], g1[n]), n
+
+
+@pytest.mark.parametrize("kernel", ["tile64", "tile128", "tile192", "pair256", "persistent"])
+@pytest.mark.parametrize("m,n,k", [(37, 512, 4096), (257, 264, 4480)])
+def test_product_in_parts_on_a_chosen_kernel(kernel, m, n, k):
+    """The hand-chosen tile holds for products in parts, and a cap on the CTAs for how many parts there are."""
+    from mccl_b200 import _C
+    torch.manual_seed(m)
+    a, b = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(k, n, device="cuda").bfloat16()
+    want = a.double() @ b.double()
+    try:
+        for cap in (0, 20):
+            _C.set_gemm_kernel(kernel)
+            _C.set_gemm_cta_limit(cap)
+            d, _ = _C.gemm_bf16(a, b, b_t=True)
+            assert ((d.double() - want).norm() / want.norm()).item() < 2.5e-3
+    finally:
+        _C.set_gemm_kernel("")
+        _C.set_gemm_cta_limit(0)
+    assert _C.gemm_error_flag() == 0
