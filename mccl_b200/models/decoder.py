@@ -393,7 +393,7 @@ class Decoder(nn.Module):
         from .. import _C
         from ..ops.functional import native_attention_supported
         return (cfg.pos == "learned" and cfg.norm == "layernorm" and cfg.act == "gelu" and tokens.dim() == 2 and tokens.dtype == torch.int64
-                and self.head_weight().shape[0] % 8 == 0 and tokens.shape[1] <= cfg.max_seq and not torch.is_autocast_enabled()
+                and tokens.shape[1] <= cfg.max_seq and not torch.is_autocast_enabled()
                 and native_attention_supported(tokens.shape[1], cfg.head_dim)
                 and _C.decoder_layer_supported(tokens.shape[1], cfg.n_heads, cfg.d_model, cfg.d_ff))
 
@@ -406,7 +406,7 @@ class Decoder(nn.Module):
         if s is None:
             return None
         tok, pos, lnf_w, lnf_b, head = s.outer
-        if hasattr(tok, "_grad_sink") or not all(p.requires_grad for p in s.params):
+        if head.shape[0] % 8 or hasattr(tok, "_grad_sink") or not all(p.requires_grad for p in s.params):
             return None
         from .. import _C
         return _C.decoder_loss(tokens, targets, tok, pos, s.layers, lnf_w, lnf_b, head, self.cfg.n_heads, self.cfg.eps)
@@ -420,8 +420,10 @@ class Decoder(nn.Module):
         if s is None:
             return None
         tok, pos, lnf_w, lnf_b, head = s.outer
+        if head.shape[0] % 8:
+            return None
         if rope:
-            if (tokens.dim() != 2 or tokens.dtype != torch.int64 or cfg.d_model % 64 or cfg.d_ff % 64 or head.shape[0] % 8
+            if (tokens.dim() != 2 or tokens.dtype != torch.int64 or cfg.d_model % 64 or cfg.d_ff % 64
                     or cfg.norm != "rmsnorm" or cfg.act != "swiglu" or cfg.head_dim % 8 or torch.is_autocast_enabled()):
                 return None
         elif not self._fused_gelu(tokens):
