@@ -218,10 +218,10 @@ class DDPTrainer:
             self._param_bucket[p] = bi
             # native operators write gradients straight into the flat buffer ...
             p._grad_sink = p.grad
+            p._grad_awaited = self.world > 1   # peers wait for the bucket this gradient completes
             if self._per_bucket:
                 # ... and say so; gradients that come back through autograd fire its hook instead
                 p._grad_ready = report(p)
-                p._grad_awaited = self.world > 1
                 if self.world > 1:
                     p.register_post_accumulate_grad_hook(self._on_autograd_grad)
         # bf16 working copies of the parameters, refreshed by the optimizer kernel (the GEMMs
@@ -344,6 +344,9 @@ class DDPTrainer:
         except BaseException:
             # what this backward has added already is not part of the next step's gradients
             if self._fused_zero and not torch.cuda.is_current_stream_capturing():
+                for s in (self.opt_stream, self.comm_stream, self.wgrad_stream):   # what still writes or reads the gradients
+                    if s is not None:
+                        torch.cuda.current_stream(self.device).wait_stream(s)
                 self.flat_g.zero_()
             raise
         finally:
