@@ -76,7 +76,8 @@ cudaError_t gemm_bf16_tn(const GemmArgs& a, cudaStream_t stream) {
   const bool gelu = a.epilogue == EPI_BIAS_GELU || a.epilogue == EPI_GELU || a.epilogue == EPI_BIAS_GELU_D || a.epilogue == EPI_GELU_D;
   if (a.alpha && (gelu || a.bias || a.residual || a.mul || a.colsum)) return cudaErrorInvalidValue;
   const bool tile_only = a.k % BK != 0 || a.colsum || a.alpha || (gelu && !a.aux);   // what only the tile kernel does
-  cudaError_t rc = choice == kPersistent && !tile_only ? launch_gemm_persistent(a, FusedDev{}, 0, stream) : launch_gemm_tiles(a, choice, stream);
+  cudaError_t rc = choice == kPersistent && !tile_only ? launch_gemm_persistent(a, FusedDev{}, 0, stream)
+                                                         : launch_gemm_tiles(a, choice > 0 ? choice : 0, stream);
   if (rc == cudaErrorNotSupported) return unsupported("cuTensorMapEncodeTiled rejected an operand");
   return rc;
 }

@@ -102,6 +102,8 @@ Plan choose(const GemmArgs* args, int count, int forced, int sms, int pairs, boo
       }
     }
   }
+  // a tile that was asked for and cannot run (a pair under a cap of one CTA, a wide tile with GELU): one that can
+  if (best.bn == 0 && forced) return choose(args, count, 0, sms, pairs, gelu, splittable, slabs);
   return best;
 }
 

@@ -112,6 +112,32 @@ def test_norm_backward_in_one_pass(rows, dim, layernorm):
         assert _rel(gb - 1, db) < 1e-4
 
 
+@pytest.mark.parametrize("kernel", ["persistent", "tile64", "tile192", "pair256"])
+def test_layer_on_a_chosen_kernel(kernel):
+    """What the chosen kernel does not do (ragged contractions, column sums, GELU without its second output, products times a scalar)
+    goes to one that does."""
+    from mccl_b200 import _C
+    a, b = _pair("tiny")
+    tok = torch.randint(0, a.cfg.vocab, (3, 34), device="cuda")
+    try:
+        for cap in (0, 1):
+            _C.set_gemm_kernel(kernel)
+            _C.set_gemm_cta_limit(cap)
+            with torch.no_grad():
+                assert _rel(a(tok), b(tok)) < 2e-2
+            a.zero_grad(set_to_none=True)
+            b.zero_grad(set_to_none=True)
+            a(tok[:, :-1], tok[:, 1:]).backward()
+            b(tok[:, :-1], tok[:, 1:]).backward()
+            for (n, p), (_, q) in zip(a.named_parameters(), b.named_parameters()):
+                if "qkv.bias" not in n:
+                    assert _rel(p.grad, q.grad) < 4e-2, n
+    finally:
+        _C.set_gemm_kernel("")
+        _C.set_gemm_cta_limit(0)
+    assert _C.gemm_error_flag() == 0
+
+
 def test_cast_many():
     from mccl_b200 import _C
     ts = [torch.randn(n, device="cuda") for n in (1, 7, 8192, 8193, 100_001)] + [torch.randn(130, 70, device="cuda") for _ in range(150)]
